@@ -154,16 +154,17 @@ int small_b200_conv2d_f32(const small_b200_layer *L, const float *in, const floa
 int small_b200_conv2d_maxpool_f32_supported(const small_b200_layer *conv, const small_b200_layer *pool);
 int small_b200_conv2d_maxpool_f32(const small_b200_layer *conv, const small_b200_layer *pool, const float *in,
                                   const float *filt, const float *bias, float *out, void *stream);
-/* The same layer on the tensor cores (tcgen05 kind::tf32 with the 3xTF32 operand split, fp32
+/* The same layer on the tensor cores (tcgen05 kind::f16 on pairs of half-precision words, fp32
  * accumulation in tensor memory), stride 1 only.  Each fp32 operand x enters the tensor core as
- * hi = x (its 13 low mantissa bits are ignored) and lo = x - hi; the lo copy of the activations
- * is made inside the kernel, in shared memory.  The caller provides the filter re-laid for the
- * tensor core:
+ * hi = half(x * 2^e) and lo = half(x * 2^e - hi), 22 bits like the two words of a 3xTF32 split (which
+ * the functions are named after); the power of two belongs to the filter as a whole and to each patch
+ * of 16 input channels of a tile, brings its largest magnitude to at least 2^6 and at most 65504, and is
+ * undone in fp32.  The activations are split inside the kernel, in shared memory.  The caller
+ * provides the filter re-laid for the tensor core:
  *   filt_prepared  small_b200_filter_prepare_tf32x3(filt), once per set of weights,
- *                  2 * K*C*Fh*Fw floats: per CTA tile and tap the filter as [c/4][k][4 c]
- *                  (what the tensor core reads directly) followed by its lo copy; for K = 16 or 32
- *                  the lo rows of every 4-channel chunk follow its hi rows directly
- *                  ([c/4][hi k | lo k][4 c]).  The layout depends on K alone; treat it as opaque.
+ *                  2 * K*C*Fh*Fw floats: per CTA tile and tap the hi and lo halves as
+ *                  [c/8][hi k | lo k][8 c] (what the tensor core reads directly), then the inverse
+ *                  of the filter's scale.  The layout depends on K alone; treat it as opaque.
  * ..._supported() says whether a shape is covered (1) or not (0).  The reference has no
  * counterpart of the preparation call (its filters are used as packed). */
 int small_b200_conv2d_f32_tf32x3_supported(const small_b200_layer *L);

@@ -1,53 +1,53 @@
-// conv_tf32x3.cu -- fp32 dense convolution (stride 1) on the 5th-generation tensor cores with
-// the 3xTF32 split: every fp32 operand x is fed as hi = x (the tensor core ignores the low 13
-// mantissa bits) and lo = x - trunc_tf32(x) (exact in fp32), and each product is accumulated as
-// a_lo*b_hi + a_hi*b_lo + a_hi*b_hi in fp32 tensor memory.  The dropped a_lo*b_lo term is
-// 2^-22 relative, so the result stays within the 1e-5 gate against the reference's fp32 loop
-// nest (include/small/abstract_layer.hpp:1368-1823, FLOAT_CONV_TILE_C).
+// conv_f16x3.cu -- fp32 dense convolution (stride 1) on the 5th-generation tensor cores, every fp32 operand as a
+// pair of half-precision words with a block scale.
+//
+// Arithmetic.  v * 2^e = hi + lo with hi = half(v * 2^e), lo = half(v * 2^e - hi), both truncated: 11 + 11 bits, the
+// very words of a 3xTF32 split (where the tensor core itself drops the low bits of a tf32 operand).  A product is a_lo*b_hi + a_hi*b_lo + a_hi*b_hi in fp32 tensor memory; the
+// dropped a_lo*b_lo is 2^-22 relative.  The power of two 2^e belongs to a block -- the whole filter, and a tile's patch
+// of 16 input channels -- and brings its largest magnitude to 2^13 or more, so the pair keeps its 22 bits down to 2^-16
+// of that magnitude and an absolute error below 2^-38 of it under that; it is undone in the FMA with which the
+// accumulation warps add a partial sum to their fp32 registers.  kind::f16 covers 16 channels per instruction where
+// kind::tf32 covers 8 at the same cost (N/2 cycles of the pipe, 128 + N operand rows of 32 bytes), so a layer needs half
+// the instructions, half the operand traffic in shared memory and half the filter bytes of the 3xTF32 form this
+// replaced: 1024 -> 1024 channels 3x3 on 64 images of 13x13 0.800 -> 0.464 ms, 16 -> 32 at 208x208 with the max
+// pool 0.198 -> 0.162, 128 -> 256 at 26x26 0.122 -> 0.075.  Against fp64 the 9216-term sums of the first are off by
+// 5.2e-7 of the largest (3xTF32: 7.3e-7; the fp32 loop nest of include/small/abstract_layer.hpp:1368-1823, whose
+// FLOAT_CONV_TILE_C this replaces: 5.7e-6).
 //
 // GEMM orientation: D[k][pixel] = sum_c W[k][c] * X[pixel][c].  The output channels are the
 // tensor core's M (one tile of 128, or 64 for layers with fewer channels), the pixels its N
-// (64..256 per CTA).  One tcgen05.mma of kind::tf32 covers only 8 input channels and occupies
-// the tensor pipe for N/2 cycles whatever M is, with a floor of about 80 cycles (measured with
-// two issuing threads: 83 cycles at N = 128, 96 at N = 192, 128 at N = 256), so wide-N instructions
-// are what keeps the pipe busy.  Every MMA reads its operands from shared memory (10 KB at N = 192):
-// at full rate that alone is 107 of the 128 bytes per cycle shared memory delivers, which makes
-// shared-memory bandwidth, not the tensor pipe, the ceiling of the wide layers.
+// (64..256 per CTA); wide-N instructions are what keeps the pipe busy.  An instruction reads 10 KB of operands at
+// N = 192 in its 96 cycles, and filter stages and patches arrive in the same memory: together about 150 bytes per cycle
+// at full rate against 128, so shared-memory bandwidth, and on long runs the power cap, bound the wide layers.
 //
-// Layers with 32 or 64 output channels turn the GEMM around (PIXM): 128 pixels are the M of one MMA
-// and all output channels its N, D[pixel][k].  Both dimensions of the instruction are then used in
-// full (a 64-row M costs the same pipe time as 128 rows), an MMA takes N/2 = 16 or 32 cycles, and a
-// thread of the accumulation warps owns one pixel with all its channels: its sums go to the packed
-// output as 64-byte runs without any transposition.  Three threads issue the MMAs there.
+// Layers with 16, 32 or 64 output channels turn the GEMM around (PIXM): 128 pixels are the M of one MMA
+// and all output channels its N, D[pixel][k].  A thread of the accumulation warps owns one pixel with all
+// its channels: its sums go to the packed output as 64-byte runs without any transposition.  Three threads issue
+// the MMAs there.
 // Variants of the pixel-major kernel (template arguments MERGED, POOL): for 16 / 32 output channels
-// [W_hi | W_lo] is one operand of 2K columns (four MMAs per tap instead of six, TcArgs::merged); layers of
-// one 16-channel block then sum the whole window in tensor memory (TcArgs::row_skip); for 32 / 64 output
+// [W_hi | W_lo] is one operand of 2K columns (two MMAs per tap instead of three, TcArgs::merged); for 32 / 64 output
 // channels on wide images a following 2x2 stride-2 max pool can run in the epilogue (TcArgs::pool).
 //
 // Implicit GEMM without im2col ("linear shift"):
 //   For one image and one block of 16 input channels, TMA copies a patch of the packed
 //   activations [rows][PW columns][16 ch] (64 bytes per pixel) into shared memory.
 //   PW = W + max(pad_l, pad_r): the zero column(s) that TMA's out-of-bounds fill produces at the
-//   left edge of every row also serve as the right padding of the row above.  The copy writes
-//   the patch in the 64-byte swizzle, and that IS a K-major operand of the tensor core: rows of
-//   64 bytes (one pixel's 16 channels), 8-pixel groups 512 bytes apart; the hardware applies the
-//   swizzle to absolute shared-memory addresses, so a descriptor may start at any pixel.  The raw
-//   fp32 patch serves as the hi operand as it is; four splitter warps write the lo copy to the
-//   same offsets of a second buffer.  Output pixel (r, c) is GEMM column m = r*PW + c, and filter
-//   tap (kh, kw) of that pixel sits at patch entry m + kh*PW + kw: consecutive pixels are
-//   consecutive rows for EVERY tap, so a tap only moves the descriptor's start address by 64 bytes
+//   left edge of every row also serve as the right padding of the row above.  Four splitter warps turn every
+//   64-byte row into its 32 bytes of hi and 32 bytes of lo halves, in place and in the 64-byte swizzle, and that IS a
+//   K-major operand of the tensor core: rows of 64 bytes, 8-pixel groups 512 bytes apart; the hardware applies the
+//   swizzle to absolute shared-memory addresses, so a descriptor may start at any pixel.  Output pixel (r, c) is GEMM
+//   column m = r*PW + c, and filter tap (kh, kw) of that pixel sits at patch entry m + kh*PW + kw: consecutive pixels
+//   are consecutive rows for EVERY tap, so a tap only moves the descriptor's start address by 64 bytes
 //   per pixel.  Columns with c >= Wo are junk and are not stored.
-//   (A no-swizzle K-major patch needs 16-byte box rows from TMA, which it moves at about one row
-//   per 9 cycles, or a re-layout pass through shared memory: both were slower.)
-//   The filter [K/16][C/16][tap][16 c][16 k] has the output channel contiguous (MN-major).
-//   kind::tf32 did not accept an MN-major no-swizzle operand on this hardware (a one-MMA
-//   experiment returned zeros, while the K-major form was exact), so the filter is re-laid once
-//   per set of weights into [K/MT][C/16][tap][c/4][MT k][4 c] (prepare_filter_kernel), MT =
-//   output channels per CTA.  One tap of one CTA is then a single contiguous run of MT*64 bytes
-//   that IS the K-major canonical layout and arrives by one bulk copy; its lo copy is made by the
-//   same preparation step and loaded next to it (making it in shared memory like the patch's
-//   cost more shared-memory bandwidth than the tensor core could spare).
+//   The filter [K/16][C/16][tap][16 c][16 k] is re-laid once per set of weights into
+//   [K/MT][C/16][tap][c/8][hi k | lo k][8 c] (prepare_filter_kernel), MT = output channels per CTA: the K-major
+//   canonical layout, hi and lo rows of a chunk one behind the other.  The taps of a group are then one contiguous run
+//   that arrives by one bulk copy.
 #include "tc_common.cuh"
+
+#include <cuda_fp16.h>
+
+#include <cstring>
 
 namespace
 {
@@ -55,6 +55,8 @@ using namespace sb;
 
 constexpr int W_STAGES_MAX = 6; // filter stages, each one group of taps (a kernel row)
 constexpr int X_SLOTS_MAX = 3;
+constexpr int BOX_PX = 32; // widest box of a TMA load: 256 elements of 8 bytes
+constexpr int SCALE_RING = 16; // patches whose block scale is remembered: slots + unflushed accumulator buffers, rounded up
 
 // Division of a non-negative int below 2^31 by a divisor fixed per launch: one multiply-high, an add and a
 // shift instead of the two dozen instructions of a 32-bit division.  Every role decodes a tile per tile and
@@ -84,6 +86,7 @@ struct TcArgs
     int tiled;         // 0: tiles are ranges of full-width rows; 1: TH x TW pixel tiles
     int TW, TH, tiles_x; // tiled mode: valid columns / rows of a tile, tiles per row of tiles
     int MT;            // output channels per CTA (tensor-core M): 128 or 64
+    int WR;            // channel rows a filter stage has room for: MT, or K in pixel-major tiles (N = K rows are read)
     int k_tiles;       // ceil(K / MT)
     int x_slots, w_stages;
     int pixm;          // 1: pixels on the tensor core's M, output channels on its N (K = 32 or 64)
@@ -103,6 +106,11 @@ struct TcArgs
     // columns).  Only the strides differ: input rows are a whole image apart, and so are output rows.
     int rows_view;
     long long o_kb_stride, o_row_stride;
+    // How a patch is fetched.  0: one TMA box of PW pixels x PR rows (x cg planes), zeros outside the image.  1: runs of
+    // consecutive pixels by untiled bulk copies (1x1 layers have no halo): one run per plane of a tile (tiled), or one per
+    // image row (rows_view with rows wider than a box).  x_row / x_plane: floats from a row / plane to the next.
+    int runs;
+    long long x_row, x_plane;
     int accumulate, act;
     float slope;
     unsigned smem_bytes;
@@ -112,13 +120,12 @@ struct TcArgs
     int ksplit;          // 2: a cluster of two CTAs shares a tile, each reduces half of the channel blocks
     int tile_base;       // first tile of this launch (a layer may run as two launches, see the launch code)
     int w_resident;      // 1: every group of a tile has a filter stage of its own, loaded once per CTA (see fit_rings)
-    // Filters with 16 or 32 output channels are prepared with the lo rows of every 4-channel chunk right
-    // behind its hi rows ([slab][c/4][hi k | lo k][4 c], interleaved_filter()): a pixel-major MMA then
-    // takes [W_hi | W_lo] as ONE operand of 2K columns (the MERGED kernel, see its issuer).
+    // 16 or 32 output channels: a pixel-major MMA takes [W_hi | W_lo] (the rows lie one behind the other in every
+    // 8-channel chunk) as ONE operand of 2K columns (the MERGED kernel, see its issuer).
     int merged;
-    // Layers of one 16-channel block with the merged operand sum a WHOLE window in tensor memory (group = taps,
-    // at most 18 full-size accumulations): one flush and one round of hand-overs per tile instead of one per
-    // kernel row, and the issuing threads take whole tiles in turn.  row_skip: descriptor units from the last
+    // Windows of at most nine taps are summed WHOLE in tensor memory where the stages fit (group = taps: at most nine
+    // full-size accumulations, as many as one kernel row of two-word tf32 operands used to need): one flush and
+    // one round of hand-overs per patch instead of one per kernel row.  row_skip: descriptor units from the last
     // tap of a kernel row to the first tap of the next one, beyond the one-pixel step.
     int row_skip;
     // 1: a 2x2 stride-2 max pool follows in the epilogue (pixel-major tiled plans only); the output strides
@@ -130,55 +137,74 @@ struct TcArgs
 // Output channels per CTA, a function of K alone so that filter preparation and the
 // convolution agree.
 __host__ __device__ inline int pick_mt(int K) { return K >= 128 ? 128 : 64; }
-// Layout of the prepared filter, a function of K alone for the same reason.
-__host__ __device__ inline bool interleaved_filter(int K) { return K == 16 || K == 32; }
 
-// packed filter [K/16][slab][16 c][16 k] -> hi and lo copies in [K/MT][slab][c/4][kv k][4 c];
-// kv = MT except in a last, partial tile (K % MT channels).  inter: one array [slab][c/4][hi K | lo K][4 c].
+// Largest magnitude of the filter (finite values; the sign bit cleared, floats compare like integers).
+__global__ void __launch_bounds__(256) filter_max_kernel(long long n, const float *__restrict__ w, uint32_t *__restrict__ top)
+{
+    uint32_t m = 0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    {
+        const uint32_t b = __float_as_uint(__ldg(w + i)) & 0x7fffffffu;
+        m = max(m, b < 0x7f800000u ? b : 0u);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && m)
+        atomicMax(top, m);
+}
+
+// Block scale of a set of operands whose largest magnitude has the bits `top`: the power of two that brings it
+// into [2^13, 2^14), and its inverse.  Exponents are held to where both are normal numbers.
+__device__ __forceinline__ float scale_up(uint32_t top)
+{
+    const uint32_t e = max(top >> 23, 15u);
+    return __uint_as_float((267u - e) << 23);
+}
+__device__ __forceinline__ float scale_down(uint32_t top)
+{
+    const uint32_t e = max(top >> 23, 15u);
+    return __uint_as_float((e - 13u) << 23);
+}
+
+// packed filter [K/16][slab][16 c][16 k] -> half-precision pairs [K/MT][slab][c/8][hi kv | lo kv][8 c]; kv = MT
+// except in a last, partial tile (K % MT channels).  head[0] = the inverse of the filter's block scale.
 __global__ void __launch_bounds__(256)
-prepare_filter_kernel(long long n, int slabs, int MT, int K, int inter, const float *__restrict__ w,
-                      float *__restrict__ hi, float *__restrict__ lo)
+prepare_filter_kernel(long long n, int slabs, int MT, int K, const float *__restrict__ w, const uint32_t *__restrict__ top,
+                      __half *__restrict__ pairs, float *__restrict__ head)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
+    const uint32_t t0 = *top;
+    if (i == 0)
+        head[0] = scale_down(t0);
     const int k16 = (int)(i & 15), c = (int)((i >> 4) & 15);
     const long long t = i >> 8;            // kb16 * slabs + slab
     const int slab = (int)(t % slabs);
     const int k = (int)(t / slabs) * 16 + k16;
     const int tile = k / MT;
     const int kv = (K - tile * MT) < MT ? (K - tile * MT) : MT;
-    const long long o = (long long)tile * MT * slabs * 16 + ((long long)slab * 4 + (c >> 2)) * kv * 4 +
-                        (long long)(k - tile * MT) * 4 + (c & 3);
-    const float v = w[i];
-    const float vl = v - __uint_as_float(__float_as_uint(v) & 0xffffe000u);
-    if (inter)
-    {
-        const long long oi = (((long long)slab * 4 + (c >> 2)) * 2 * K + k) * 4 + (c & 3);
-        hi[oi] = v;
-        hi[oi + (long long)K * 4] = vl;
-        return;
-    }
-    hi[o] = v;
-    lo[o] = vl;
+    const long long o = ((long long)tile * MT * slabs * 16 + (long long)slab * kv * 16) * 2 +
+                        (long long)(c >> 3) * kv * 16 + (long long)(k - tile * MT) * 8 + (c & 7);
+    const float v = w[i] * scale_up(t0);
+    const __half h = __float2half_rz(v);
+    pairs[o] = h;
+    pairs[o + (long long)kv * 8] = __float2half_rz(v - __half2float(h));
 }
 
 // Tensor-core accumulation truncates: every MMA adds into the fp32 accumulator with
 // round-toward-zero, a one-sided error that grows with the number of accumulations (measured
 // here: 3e-5 of the output range after 1700 MMAs).  So tensor memory only ever holds the sum
-// of one kernel row of one channel block (6 MMAs per tap); eight accumulation warps pull
-// these partial sums out with tcgen05.ld and add them into fp32 registers with
-// round-to-nearest, while the tensor core already works on the next groups of taps in the other
+// of one group of taps (a window of up to nine, or a kernel row) of one channel block, its small cross terms first;
+// eight accumulation warps pull these partial sums out with tcgen05.ld and add them into fp32 registers with
+// round-to-nearest, while the tensor core already works on the next groups in the other
 // accumulator buffers of tensor memory (two of 192 or 256 columns, four when a buffer needs at
 // most 128).
 //
-// warp 0: TMA producer, warps 1..2: MMA issuers (warp 3 idle), warps 4..11: accumulation +
+// warp 0: TMA producer, warps 1..2 (pixel-major 1..3): MMA issuers, warps 4..11: accumulation +
 // epilogue (lane quarter = warp % 4, pixel half = (warp - 4) / 4), warps 12..15: operand
-// splitters (lo copy of every patch).  The first and last warpgroups give registers
-// back (setmaxnreg) so that the accumulation warps can hold 128 running sums per thread
-// without spilling.
+// splitters.
 //
-// The unit of the filter pipeline is a GROUP of taps (one kernel row): one bulk copy and one
+// The unit of the filter pipeline is a GROUP of taps: one bulk copy and one
 // tcgen05.commit, which frees the filter stage for the producer and hands the partial sums to
 // the accumulation warps.
 constexpr int ACC_WARPS = 8;
@@ -188,14 +214,75 @@ constexpr int SPLIT_THREADS = 128;
 constexpr int NUM_THREADS = 512;
 constexpr int COLS_PER_THREAD = 128;
 
-__device__ __forceinline__ float4 lo_of(const float4 v)
+// Two fp32 values, already multiplied by their block scale, as a pair of half-precision words: hi = v,
+// lo = v - hi, both cut to 11 bits as a tf32 operand is.  (Rounded to nearest the 9216-term sums come out at 3.0e-7 of the
+// largest instead of 5.2e-7, but then results drift from the 3xTF32 form's by more than either is off: 2.5e-5 of a
+// YOLO head, whose box sizes are exponentials, against 2e-6 with the same words.)
+__device__ __forceinline__ void split2(float a, float b, uint32_t &hi, uint32_t &lo)
 {
-    float4 r;
-    r.x = v.x - __uint_as_float(__float_as_uint(v.x) & 0xffffe000u);
-    r.y = v.y - __uint_as_float(__float_as_uint(v.y) & 0xffffe000u);
-    r.z = v.z - __uint_as_float(__float_as_uint(v.z) & 0xffffe000u);
-    r.w = v.w - __uint_as_float(__float_as_uint(v.w) & 0xffffe000u);
-    return r;
+    asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
+    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
+    asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b - f.y), "f"(a - f.x));
+}
+__device__ __forceinline__ uint32_t finite_abs(float v)
+{
+    const uint32_t b = __float_as_uint(v) & 0x7fffffffu;
+    return b < 0x7f800000u ? b : 0u;
+}
+__device__ __forceinline__ uint32_t finite_max(const float4 v)
+{
+    return max(max(finite_abs(v.x), finite_abs(v.y)), max(finite_abs(v.z), finite_abs(v.w)));
+}
+__device__ __forceinline__ float max_abs(const float4 v)
+{
+    return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+}
+// Largest of the splitter threads' values; `words` is used again only after another call.
+__device__ __forceinline__ uint32_t split_reduce(uint32_t m, uint32_t *words, int w, int lane)
+{
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0)
+        words[w] = m;
+    asm volatile("bar.sync 2, 128;" ::: "memory");
+    const uint4 t = *reinterpret_cast<const uint4 *>(words);
+    return max(max(t.x, t.y), max(t.z, t.w));
+}
+// U pieces of 8 channels (piece u = half u & 1 of patch row u / 2; u, u + 128, ...) into hi and lo halves, in place.
+// Returns the largest magnitude of those that belong to the patch (`valid` rows of the first plane, `valid2` of the
+// second, `entries` further on).  Neither the reads nor the writes are predicated -- rows behind the patch hold whatever
+// the slot held before and are never stored from -- because the predicates cost more than the work: 1090 cycles for
+// 256 rows by four warps one predicated piece at a time, 950 four at a time, 440 without the predicates (shared memory
+// delivers about 74 bytes per cycle to loads and stores, which makes 430 the floor).
+template <int U>
+__device__ __forceinline__ float split_pieces(float4 *piece, int u0, float up, uint32_t entries, int valid, int valid2)
+{
+    float4 v[U][2];
+    float fm = 0.f;
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+    {
+        const int u = u0 + q * SPLIT_THREADS, late = (u >> 2) & 1;
+        v[q][0] = piece[2 * u + late];
+        v[q][1] = piece[2 * u + 1 - late];
+    }
+    __syncwarp(); // a row belongs to two lanes: both have read it
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+    {
+        const int u = u0 + q * SPLIT_THREADS, sw = (u >> 2) & 3, late = sw & 1, h = u & 1, r = u >> 1;
+        uint4 hi, lo; // of the chunks in the order they were read
+        split2(v[q][0].x * up, v[q][0].y * up, hi.x, lo.x);
+        split2(v[q][0].z * up, v[q][0].w * up, hi.y, lo.y);
+        split2(v[q][1].x * up, v[q][1].y * up, hi.z, lo.z);
+        split2(v[q][1].z * up, v[q][1].w * up, hi.w, lo.w);
+        const float top = fmaxf(max_abs(v[q][0]), max_abs(v[q][1]));
+        fm = fmaxf(fm, (r < valid || (uint32_t)(r - (int)entries) < (uint32_t)valid2) ? top : 0.f);
+        uint4 *row = reinterpret_cast<uint4 *>(piece + (2 * u & ~3));
+        // late rows: chunks read in the other order, lo half written first
+        row[(h + 2 * late) ^ sw] = late ? make_uint4(lo.z, lo.w, lo.x, lo.y) : hi;
+        row[(h + 2 - 2 * late) ^ sw] = late ? make_uint4(hi.z, hi.w, hi.x, hi.y) : lo;
+    }
+    return fm;
 }
 
 // One tile of work: an image, a range of pixels and a block of MT output channels.
@@ -207,10 +294,6 @@ struct Tile
     int tw_valid, th_valid;    // real outputs per patch row / patch rows that hold outputs
 };
 
-// FAST = false keeps the plain divisions: the whole-window instantiations (MERGED == 2) are at the edge of their
-// register budget, and with the multiply-high form the compiler's spill landed in their MMA issue loop
-// (16 -> 32 channels at 208x208: 0.203 -> 0.225 ms), so they divide the slow way.
-template <bool FAST = true>
 __device__ __forceinline__ Tile decode_tile(const TcArgs &a, int t)
 {
     // Pixel tile fastest, then the image, channel tile slowest.  The CTAs that run at the same time then
@@ -221,18 +304,18 @@ __device__ __forceinline__ Tile decode_tile(const TcArgs &a, int t)
     // all 75 MB of filter again: 541 MB of DRAM reads per launch for 126 MB of algorithmic bytes (176 MB
     // now, and the layer 3 % faster).
     Tile T;
-    const int t1 = FAST ? a.by_px_tiles.div(t) : t / a.px_tiles, pt = t - t1 * a.px_tiles;
-    T.kt = FAST ? a.by_N.div(t1) : t1 / a.N;
+    const int t1 = a.by_px_tiles.div(t), pt = t - t1 * a.px_tiles;
+    T.kt = a.by_N.div(t1);
     T.n = t1 - T.kt * a.N;
     if (!a.tiled)
     {
         const int m0 = pt * a.NPX;
-        T.row_base = FAST ? a.by_PW.div(m0) : m0 / a.PW; T.col_base = 0; T.m_local0 = m0 - T.row_base * a.PW;
+        T.row_base = a.by_PW.div(m0); T.col_base = 0; T.m_local0 = m0 - T.row_base * a.PW;
         T.tw_valid = a.Wo; T.th_valid = a.Ho;
     }
     else
     {
-        const int ty = FAST ? a.by_tiles_x.div(pt) : pt / a.tiles_x, tx = pt - ty * a.tiles_x;
+        const int ty = a.by_tiles_x.div(pt), tx = pt - ty * a.tiles_x;
         T.row_base = ty * a.TH; T.col_base = tx * a.TW; T.m_local0 = 0;
         T.tw_valid = (a.Wo - T.col_base) < a.TW ? (a.Wo - T.col_base) : a.TW; T.th_valid = a.TH;
     }
@@ -253,8 +336,8 @@ __device__ __forceinline__ Tile decode_tile(const TcArgs &a, int t)
 
 template <bool PERSIST, bool SPLIT, bool PIXM = false, int MERGED = 0, bool POOL = false> // MERGED: 1 merged operand, 2 with whole-window groups
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restrict__ filt,
-                   const float *__restrict__ filt_lo, const TcArgs a, const float *__restrict__ bias, float *__restrict__ out, int *status)
+conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restrict__ in, const __half *__restrict__ filt,
+                  const float *__restrict__ filt_scale, const TcArgs a, const float *__restrict__ bias, float *__restrict__ out, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t x_full[X_SLOTS_MAX], x_ready[X_SLOTS_MAX], x_empty[X_SLOTS_MAX];
@@ -262,15 +345,17 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
     __shared__ __align__(8) uint64_t t_full[4], t_empty[4];
     __shared__ __align__(8) uint64_t peer_staged, peer_done; // split reduction: hand-over between the two CTAs
     __shared__ uint32_t tmem_base_s;
+    __shared__ __align__(8) uint64_t x_redo;   // a patch fetched again because its block scale did not fit
+    __shared__ float patch_down[SCALE_RING];   // inverse of the block scale of each patch in flight
+    __shared__ __align__(16) uint32_t split_top[3][4];      // the splitter warps' maxima of the patch at hand
     __shared__ int acc_failed; // an accumulation warp gave up on a wait: all eight leave at the same tile
 
     const uint32_t entries = (uint32_t)a.PR * a.PW;
     const uint32_t x_bytes = entries * 64 * (uint32_t)a.cg;     // one patch [plane][entry][16 floats]
-    const uint32_t x_part = (x_bytes + 1023u) & ~1023u;         // hi (or lo) copy; keeps the swizzle pattern anchored
-    const uint32_t w_part = (uint32_t)a.MT * 64;               // one hi (or lo) tap tile
-    uint8_t *sX = smem;                                              // [slot][hi|lo][entry][64 B, 64-byte swizzle]
-    uint8_t *sW = sX + (size_t)a.x_slots * 2 * x_part;              // [stage][hi|lo][tap in group][c/4][MT k][16 B]
-    const uint32_t w_half_stage = (uint32_t)a.group * w_part;       // hi (or lo) tiles of one stage
+    const uint32_t x_part = (x_bytes + 4095u) & ~4095u;         // a patch slot: whole passes of the splitters (64 rows each)
+    uint8_t *sX = smem;                                              // [slot][entry][64 B, 64-byte swizzle]
+    uint8_t *sW = sX + (size_t)a.x_slots * x_part;                  // [stage][tap in group][c/8][hi kv | lo kv][16 B]
+    const uint32_t w_stage = (uint32_t)a.group * a.WR * 64;         // bytes of one filter stage
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint32_t tmem_cols = 32;
@@ -289,27 +374,47 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
     const int first_tile = a.tile_base + (split ? blockIdx.x / 2 : blockIdx.x), tile_step = gridDim.x;
 
     // patch number pc / group number gc count over every tile of this CTA
-    auto issue_patch = [&](const Tile &T, int cb, int pc) {
-        const int slot = pc % a.x_slots;
-        mbar_expect_tx(&x_full[slot], x_bytes);
-        tma_load_4d(sX + (size_t)slot * 2 * x_part, &map_x, 0, T.col_base - a.pad_l, T.row_base - a.pad_t,
-                    (T.n * a.cbs + cb_begin + cb) * a.cg, &x_full[slot]);
+    // pixels of a tile's patch that a copy delivers, per plane: every entry of a box (zeros outside the image), or
+    // what lies inside the image where the patch is fetched as runs
+    auto patch_rows = [&](const Tile &T) -> int {
+        if (!a.runs)
+            return (int)entries;
+        if (a.tiled)
+            return min(a.PW, a.W - T.col_base);
+        return min(a.PR, a.H - T.row_base) * a.PW;
     };
-    auto issue_filter = [&](const Tile &T, int g, int gc) {
-        const int st = gc % a.w_stages;
-        uint8_t *wd = sW + (size_t)st * 2 * w_half_stage;
-        const size_t off = (size_t)T.kt * a.MT * steps * 16 + (size_t)(g + cb_begin * groups_per_cb) * a.group * T.kv * 16;
-        mbar_expect_tx(&w_full[st], 2u * a.group * T.kv * 64);
-        if (MERGED)
+    auto fetch_patch = [&](const Tile &T, int cb, int slot, uint64_t *bar) {
+        uint8_t *dst = sX + (size_t)slot * x_part;
+        const int plane = (T.n * a.cbs + cb_begin + cb) * a.cg;
+        if (!a.runs)
         {
-            // hi and lo rows of a chunk lie side by side in one array: one run of twice the length
-            tma_load_1d(wd, filt + 2 * off, 2u * a.group * T.kv * 64, &w_full[st]);
+            mbar_expect_tx(bar, x_bytes);
+            tma_load_3d(dst, &map_x, (T.col_base - a.pad_l) * 8, T.row_base - a.pad_t, plane, bar);
             return;
         }
-        // the group's taps are contiguous, [tap][c/4][kv k][4 c]: a partial last tile (kv < MT) simply
-        // is a shorter run, and the MMA descriptors take kv * 16 bytes as the chunk stride
-        tma_load_1d(wd, filt + off, (uint32_t)a.group * T.kv * 64, &w_full[st]);
-        tma_load_1d(wd + w_half_stage, filt_lo + off, (uint32_t)a.group * T.kv * 64, &w_full[st]);
+        const uint32_t bytes = (uint32_t)patch_rows(T) * 64;
+        mbar_expect_tx(bar, bytes * (uint32_t)a.cg);
+        for (int p = 0; p < a.cg; ++p)
+        {
+            const float *src = in + (long long)(plane + p) * a.x_plane + (long long)T.row_base * a.x_row + (long long)T.col_base * CB;
+            uint8_t *d = dst + (size_t)p * entries * 64;
+            if (a.tiled)
+                tma_load_1d(d, src, bytes, bar);
+            else
+                for (uint32_t done = 0; done < bytes; done += (uint32_t)a.PW * 64, src += a.x_row)
+                    tma_load_1d(d + done, src, (uint32_t)a.PW * 64, bar);
+        }
+    };
+    auto issue_patch = [&](const Tile &T, int cb, int slot) { fetch_patch(T, cb, slot, &x_full[slot]); };
+    auto reload_patch = [&](const Tile &, int t, int cb, int slot) {
+        fetch_patch(decode_tile(a, t), cb, slot, &x_redo);
+    };
+    auto issue_filter = [&](const Tile &T, int g, int st) {
+        // the group's taps are contiguous, [tap][c/8][hi kv | lo kv][8 c]: one run; a partial last tile (kv < MT)
+        // simply is a shorter one, and the MMA descriptors take 2 * kv * 16 bytes as the chunk stride
+        const size_t off = (size_t)T.kt * a.MT * steps * 32 + (size_t)(g + cb_begin * groups_per_cb) * a.group * T.kv * 32;
+        mbar_expect_tx(&w_full[st], (uint32_t)a.group * T.kv * 64);
+        tma_load_1d(sW + (size_t)st * w_stage, filt + off, (uint32_t)a.group * T.kv * 64, &w_full[st]);
     };
 
     if (warp == 0)
@@ -319,18 +424,18 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
             acc_failed = 0;
             for (int i = 0; i < X_SLOTS_MAX; ++i)
             {
-                mbar_init(&x_full[i], 1); mbar_init(&x_ready[i], SPLIT_THREADS); mbar_init(&x_empty[i], PIXM ? 3 : 2);
+                mbar_init(&x_full[i], 1); mbar_init(&x_ready[i], 1); mbar_init(&x_empty[i], PIXM ? 3 : 2);
             }
             for (int i = 0; i < W_STAGES_MAX; ++i)
             {
                 mbar_init(&w_full[i], 1); mbar_init(&g_done[i], 1);
             }
             for (int i = 0; i < 4; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], ACC_WARPS); }
-            mbar_init(&peer_staged, ACC_WARPS); mbar_init(&peer_done, ACC_WARPS);
+            mbar_init(&x_redo, 1); mbar_init(&peer_staged, ACC_WARPS); mbar_init(&peer_done, ACC_WARPS);
             fence_barrier_init();
             // The first patch and the first filter stage only need their barriers: their round
             // trip to memory overlaps the tensor-memory allocation and the CTA-wide barrier.
-            const Tile T = decode_tile<MERGED != 2>(a, first_tile);
+            const Tile T = decode_tile(a, first_tile);
             issue_patch(T, 0, 0);
             issue_filter(T, 0, 0);
         }
@@ -348,7 +453,22 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
 
     if (warp < FIRST_ACC_WARP || warp >= FIRST_SPLIT_WARP)
     {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+        // The launch has 512 x 128 registers; the roles' shares add up to that at most (setmaxnreg draws on nothing else):
+        // 128 x 88 + 256 x 168 + 128 x 88, pixel-major tiles 128 x 88 + 256 x 144 + 128 x 112.
+        if (warp < FIRST_ACC_WARP)
+        {
+            if (PIXM)
+                asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+            else
+                asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+        }
+        else
+        {
+            if (PIXM)
+                asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");
+            else
+                asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+        }
         if (warp == 0 && lane == 0)
         {
             // ---------------- producer ----------------
@@ -358,56 +478,66 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
             // the MMAs of a tile with one or two channel blocks.  The look-ahead never waits (a wait
             // here would hold back the filter stages); only the patch of the group at hand does.
             // The patch cursor (p_t, p_cb) walks the same (tile, channel block) sequence as everybody else.
-            int pc = 1, gc = 0, q = 0; // pc: patches issued (patch 0 already is), q: patches the groups have entered
+            // Ring positions are counters that wrap (here and in the other roles): a division by a ring's depth is some
+            // forty instructions of straight-line code in every step of every role.
+            int pc = 1, q = 0;             // patches issued (patch 0 already is), patches the groups have entered
+            int slot = a.x_slots > 1 ? 1 : 0; // where patch pc goes, and the parity of the slot's last release
+            uint32_t freed = a.x_slots > 1 ? 1 : 0;
             int p_t = first_tile, p_cb = 1;
-            Tile PT = decode_tile<MERGED != 2>(a, p_t); // decoded once per tile (the decode divides)
+            Tile PT = decode_tile(a, p_t); // decoded once per tile
             auto step_cursor = [&]() {
                 if (p_cb == cbs_l)
                 {
                     p_cb = 0;
                     p_t += tile_step;
                     if (PERSIST && p_t < a.total_tiles)
-                        PT = decode_tile<MERGED != 2>(a, p_t);
+                        PT = decode_tile(a, p_t);
                 }
             };
             step_cursor();
             auto next_patch = [&]() {
-                issue_patch(PT, p_cb, pc);
+                issue_patch(PT, p_cb, slot);
                 ++pc;
                 ++p_cb;
+                if (++slot == a.x_slots) { slot = 0; freed ^= 1; }
                 step_cursor();
             };
+            int st = 0;
+            uint32_t w_freed = 1; // parity of the filter stage's last release; the first round finds all stages free
+            bool w_first = true, first = true;
             SB_TILE_LOOP(ok)
             {
-                const Tile T = decode_tile<MERGED != 2>(a, t);
-                for (int g = 0; g < groups && ok; ++g, ++gc)
+                const Tile T = decode_tile(a, t);
+                int in_cb = 0;
+                for (int g = 0; g < groups && ok; ++g)
                 {
-                    if (g % groups_per_cb == 0)
+                    if (in_cb == 0)
                     {
                         if (pc <= q) // the look-ahead has not reached this group's patch: now it must go
                         {
-                            const int slot = pc % a.x_slots, xuse = pc / a.x_slots;
-                            if (xuse > 0) // all issuers' MMAs on the slot's previous patch are done
-                                ok = mbar_wait(&x_empty[slot], (xuse - 1) & 1, status, 11);
+                            if (pc >= a.x_slots) // all issuers' MMAs on the slot's previous patch are done
+                                ok = mbar_wait(&x_empty[slot], freed, status, 11);
                             if (!ok)
                                 break;
                             next_patch();
                         }
                         ++q;
                     }
+                    if (++in_cb == groups_per_cb)
+                        in_cb = 0;
                     while (pc < q - 1 + a.x_slots && (PERSIST ? p_t < a.total_tiles : p_t == first_tile) &&
-                           (pc < a.x_slots || mbar_test(&x_empty[pc % a.x_slots], ((pc / a.x_slots) - 1) & 1)))
+                           (pc < a.x_slots || mbar_test(&x_empty[slot], freed)))
                         next_patch();
-                    if (gc == 0)
-                        continue; // so is filter stage 0
-                    if (a.w_resident && gc >= a.w_stages)
+                    if (a.w_resident && !w_first)
                         continue; // the whole filter is in shared memory since the CTA's first tile
-                    const int st = gc % a.w_stages, wuse = gc / a.w_stages;
-                    if (wuse > 0)
-                        ok = mbar_wait(&g_done[st], (wuse - 1) & 1, status, 12);
+                    if (!w_first)
+                        ok = mbar_wait(&g_done[st], w_freed, status, 12);
                     if (!ok)
                         break;
-                    issue_filter(T, g, gc);
+                    if (!first) // filter stage 0 already is on its way
+                        issue_filter(T, g, st);
+                    first = false;
+                    if (++st == a.w_stages) { st = 0; w_first = false; w_freed ^= 1; }
                 }
             }
         }
@@ -436,15 +566,13 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
             // patch: rows of 64 bytes (one pixel's 16 channels) in the 64-byte swizzle the bulk copy
             // wrote; 8-pixel groups are 512 bytes apart; a pixel further is 4 descriptor units
             const uint64_t x_desc_base = make_smem_desc(smem_u32(sX), 16, 512, 4);
-            const uint32_t idesc = make_idesc(1 /*f32*/, 2 /*tf32*/, 2 /*tf32*/, 0 /*A K-major*/, 0 /*B K-major*/,
+            const uint32_t idesc = make_idesc(1 /*f32*/, 0 /*f16*/, 0 /*f16*/, 0 /*A K-major*/, 0 /*B K-major*/,
                                               PIXM ? 128u : (uint32_t)a.MT, PIXM ? (uint32_t)a.K : (uint32_t)a.NPX);
-            const uint32_t idesc_wide = make_idesc(1, 2, 2, 0, 0, 128u, 2u * (uint32_t)a.K); // MERGED: N = [hi | lo]
-            const uint64_t x_lo_off = x_part >> 4, w_lo_off = w_half_stage >> 4;
-            constexpr uint32_t w_rows = MERGED ? 2u : 1u; // rows of a 4-channel chunk: kv, or kv hi + kv lo
-            const uint64_t x_half = 2; // channels 8..15 of the block
+            const uint32_t idesc_wide = make_idesc(1, 0, 0, 0, 0, 128u, 2u * (uint32_t)a.K); // MERGED: N = [hi | lo]
+            const uint64_t x_lo_off = 2; // a pixel's row: 32 bytes of hi halves, 32 bytes of lo halves
             const uint64_t tap_step = (uint64_t)a.tap_step;
-            const uint64_t w_stage_step = (uint64_t)2 * w_half_stage >> 4;
-            const uint64_t x_slot_step = (uint64_t)2 * x_part >> 4;
+            const uint64_t w_stage_step = (uint64_t)w_stage >> 4;
+            const uint64_t x_slot_step = (uint64_t)x_part >> 4;
             int slot = 0, xphase = 0, st = 0, wphase = 0, g = 0; // g counts groups over all tiles
             uint64_t x_slot_off = 0, w_stage_off = 0;
             SB_TILE_LOOP(ok)
@@ -459,11 +587,11 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
                     T.m_local0 = 0; T.kv = a.K;
                 }
                 else
-                    T = decode_tile<MERGED != 2>(a, t);
+                    T = decode_tile(a, t);
                 const uint64_t x_desc0 = x_desc_base + (uint64_t)T.m_local0 * 4;
-                // filter stage: [tap][c/4][kv rows][16 B], kv = channels of this tile
-                const uint64_t w_desc0 = make_smem_desc(smem_u32(sW), (uint32_t)T.kv * 16 * w_rows, 128, 0);
-                const uint64_t w_tap = (uint64_t)T.kv * 4 * w_rows, w_half = (uint64_t)T.kv * 2 * w_rows;
+                // filter stage: [tap][c/8][kv hi rows | kv lo rows][16 B], kv = channels of this tile
+                const uint64_t w_desc0 = make_smem_desc(smem_u32(sW), (uint32_t)T.kv * 32, 128, 0);
+                const uint64_t w_tap = (uint64_t)T.kv * 4, w_lo_off = (uint64_t)T.kv;
                 for (int cb = 0; cb < cbs_l && ok; ++cb)
                 {
                     ok = mbar_wait(&x_ready[slot], xphase, status, 13);
@@ -489,8 +617,8 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
                             {
                                 // [W_hi | W_lo] is one operand of 2K columns: x_hi times it gives the hi*hi sums in
                                 // columns [0, K) and one cross term in [K, 2K), x_lo * W_hi adds the other cross
-                                // term there.  Four instructions per tap and 128 pixels instead of six, the 128-pixel
-                                // operand read from shared memory four times instead of six, and the small terms
+                                // term there.  Two instructions per tap and 128 pixels instead of three, the 128-pixel
+                                // operand read from shared memory twice instead of three times, and the small terms
                                 // never meet a full-size accumulator; the accumulation warps add the two halves.
                                 const uint32_t d0 = tmem + (uint32_t)((g & tb_mask) * mtiles * 2 * a.K);
                                 int kw = 0;
@@ -498,14 +626,12 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
                                 {
                                     for (int mt = 0; mt < mtiles; ++mt)
                                     {
-                                        const uint64_t xa = xh + (uint64_t)mt * 512, xl = xa + x_lo_off;
+                                        const uint64_t xa = xh + (uint64_t)mt * 512;
                                         const uint32_t d = d0 + (uint32_t)(mt * 2 * a.K);
-                                        tc_mma_tf32(d, xa, wh, idesc_wide, tp == 0 ? 0u : 1u);
-                                        tc_mma_tf32(d + (uint32_t)a.K, xl, wh, idesc, 1u);
-                                        tc_mma_tf32(d, xa + x_half, wh + w_half, idesc_wide, 1u);
-                                        tc_mma_tf32(d + (uint32_t)a.K, xl + x_half, wh + w_half, idesc, 1u);
+                                        tc_mma_f16(d, xa, wh, idesc_wide, tp == 0 ? 0u : 1u);
+                                        tc_mma_f16(d + (uint32_t)a.K, xa + x_lo_off, wh, idesc, 1u);
                                     }
-                                    if (MERGED == 2 && ++kw == a.Fw) // the group spans kernel rows: on to the next patch row
+                                    if (++kw == a.Fw) // on to the next patch row (0 where a group is one row)
                                     {
                                         kw = 0;
                                         xh += (uint64_t)a.row_skip;
@@ -518,44 +644,44 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
                                 // The small cross terms of the whole group first, the hi*hi terms last: the
                                 // tensor core adds into its accumulator with truncation, an error of one ulp OF
                                 // THE ACCUMULATOR per MMA, so only the MMAs issued while it holds full-size sums
-                                // (two per tap instead of six) contribute a full-size error.
+                                // (one per tap instead of three) contribute a full-size error.
                                 uint64_t wh2 = wh, xh2 = xh;
+                                int kw = 0, kw2 = 0;
                                 for (int tp = 0; tp < a.group; ++tp, wh += w_tap, xh += tap_step)
                                 {
                                     const uint64_t wl = wh + w_lo_off;
                                     for (int mt = 0; mt < mtiles; ++mt)
                                     {
-                                        const uint64_t xa = xh + (uint64_t)mt * 512, xl = xa + x_lo_off; // 128 pixels on
+                                        const uint64_t xa = xh + (uint64_t)mt * 512; // 128 pixels on
                                         const uint32_t d = d0 + (uint32_t)(mt * a.K);
-                                        tc_mma_tf32(d, xa, wl, idesc, tp == 0 ? 0u : 1u);
-                                        tc_mma_tf32(d, xl, wh, idesc, 1u);
-                                        tc_mma_tf32(d, xa + x_half, wl + w_half, idesc, 1u);
-                                        tc_mma_tf32(d, xl + x_half, wh + w_half, idesc, 1u);
+                                        tc_mma_f16(d, xa, wl, idesc, tp == 0 ? 0u : 1u);
+                                        tc_mma_f16(d, xa + x_lo_off, wh, idesc, 1u);
                                     }
+                                    if (++kw == a.Fw) { kw = 0; xh += (uint64_t)a.row_skip; }
                                 }
                                 for (int tp = 0; tp < a.group; ++tp, wh2 += w_tap, xh2 += tap_step)
+                                {
                                     for (int mt = 0; mt < mtiles; ++mt)
-                                    {
-                                        const uint64_t xa = xh2 + (uint64_t)mt * 512;
-                                        const uint32_t d = d0 + (uint32_t)(mt * a.K);
-                                        tc_mma_tf32(d, xa, wh2, idesc, 1u);
-                                        tc_mma_tf32(d, xa + x_half, wh2 + w_half, idesc, 1u);
-                                    }
+                                        tc_mma_f16(d0 + (uint32_t)(mt * a.K), xh2 + (uint64_t)mt * 512, wh2, idesc, 1u);
+                                    if (++kw2 == a.Fw) { kw2 = 0; xh2 += (uint64_t)a.row_skip; }
+                                }
                             }
-                            const uint32_t d = tmem + (uint32_t)((g & tb_mask) * a.NPX);
-                            uint64_t wh2 = wh, xh2 = xh; // cross terms first, hi*hi last (see the pixel-major loop)
-                            for (int tp = 0; !PIXM && tp < a.group; ++tp, wh += w_tap, xh += tap_step)
+                            else
                             {
-                                const uint64_t xl = xh + x_lo_off, wl = wh + w_lo_off;
-                                tc_mma_tf32(d, wl, xh, idesc, tp == 0 ? 0u : 1u);
-                                tc_mma_tf32(d, wh, xl, idesc, 1u);
-                                tc_mma_tf32(d, wl + w_half, xh + x_half, idesc, 1u);
-                                tc_mma_tf32(d, wh + w_half, xl + x_half, idesc, 1u);
-                            }
-                            for (int tp = 0; !PIXM && tp < a.group; ++tp, wh2 += w_tap, xh2 += tap_step)
-                            {
-                                tc_mma_tf32(d, wh2, xh2, idesc, 1u);
-                                tc_mma_tf32(d, wh2 + w_half, xh2 + x_half, idesc, 1u);
+                                const uint32_t d = tmem + (uint32_t)((g & tb_mask) * a.NPX);
+                                uint64_t wh2 = wh, xh2 = xh; // cross terms first, hi*hi last (see the pixel-major loop)
+                                int kw = 0, kw2 = 0;
+                                for (int tp = 0; tp < a.group; ++tp, wh += w_tap, xh += tap_step)
+                                {
+                                    tc_mma_f16(d, wh + w_lo_off, xh, idesc, tp == 0 ? 0u : 1u);
+                                    tc_mma_f16(d, wh, xh + x_lo_off, idesc, 1u);
+                                    if (++kw == a.Fw) { kw = 0; xh += (uint64_t)a.row_skip; }
+                                }
+                                for (int tp = 0; tp < a.group; ++tp, wh2 += w_tap, xh2 += tap_step)
+                                {
+                                    tc_mma_f16(d, wh2, xh2, idesc, 1u);
+                                    if (++kw2 == a.Fw) { kw2 = 0; xh2 += (uint64_t)a.row_skip; }
+                                }
                             }
                             // the stage is free for the producer and the group's partial sums are
                             // complete for the accumulation warps: one commit serves both while the
@@ -580,34 +706,87 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
         else if (warp >= FIRST_SPLIT_WARP)
         {
             // ---------------- operand splitters ----------------
+            // The copy left rows of 64 bytes (16 channels of a pixel).  Each is replaced in place by its hi and lo
+            // halves, 32 bytes each, in the 64-byte swizzle the MMAs read (16-byte chunk j of row i at chunk
+            // j ^ ((i >> 1) & 3)).  A thread takes 8 channels at a time, neighbouring lanes a row; rows 2, 3 of every
+            // four touch their two chunks in the other order, so that neither the reads nor the writes of a warp
+            // meet in a bank.
+            // The block scale: a CTA starts from its first patch's largest magnitude (brought to 2^13..2^14) and keeps the
+            // power of two as long as every patch's largest scaled magnitude stays in [2^6, 65504); the pass that converts
+            // also finds that magnitude.  (Finding it first took as long as the conversion: a second pass over shared
+            // memory and a barrier in front of every patch.)  A patch outside the range is fetched and converted again.
             const int sid = tid - FIRST_SPLIT_WARP * 32;
-            bool ok = true;
-            int pc = 0;
+            bool ok = true, known = false;
+            int slot = 0, scale_at = 0;
+            uint32_t phase = 0, turn = 0;
+            uint32_t redone = 0;
+            float up = 1.f, down = 1.f;
             SB_TILE_LOOP(ok)
-                for (int cb = 0; cb < cbs_l && ok; ++cb, ++pc)
+            {
+                Tile T = {};
+                if (a.runs)
+                    T = decode_tile(a, t);
+                const int valid = patch_rows(T), valid2 = a.cg > 1 ? valid : 0; // pixels of the first / second plane
+                const int total = (int)(x_part >> 5); // pieces, whole passes of the warps: the slot has room for them
+                for (int cb = 0; cb < cbs_l && ok; ++cb)
                 {
-                    const int slot = pc % a.x_slots;
-                    ok = mbar_wait(&x_full[slot], (pc / a.x_slots) & 1, status, 17);
+                    ok = mbar_wait(&x_full[slot], phase, status, 17);
                     if (!ok)
                         break;
+                    float4 *piece = reinterpret_cast<float4 *>(sX + (size_t)slot * x_part);
+                    uint32_t m = 0;
+                    for (int round = 0; round < 2; ++round)
                     {
-                        // The patch as the bulk copy wrote it is the hi operand (the tensor core
-                        // ignores the 13 low mantissa bits of an fp32 word read as tf32); the lo copy
-                        // takes the same place in its own buffer, so the swizzle needs no thought.
-                        const float4 *xh = reinterpret_cast<const float4 *>(sX + (size_t)slot * 2 * x_part);
-                        float4 *xl = reinterpret_cast<float4 *>(sX + (size_t)slot * 2 * x_part + x_part);
-                        const uint32_t total = x_bytes >> 4;
-                        for (uint32_t i = (uint32_t)sid; i < total; i += SPLIT_THREADS)
-                            xl[i] = lo_of(xh[i]);
+                        if (!known)
+                        {
+                            for (int u = sid; u < total; u += SPLIT_THREADS)
+                                if ((u >> 1) < valid || (uint32_t)((u >> 1) - (int)entries) < (uint32_t)valid2)
+                                    m = max(m, max(finite_max(piece[2 * u]), finite_max(piece[2 * u + 1])));
+                            m = split_reduce(m, split_top[2], warp - FIRST_SPLIT_WARP, lane);
+                            up = scale_up(m);
+                            down = scale_down(m);
+                        }
+                        float fm = 0.f;
+                        int base = sid;
+                        for (; base + 3 * SPLIT_THREADS < total; base += 4 * SPLIT_THREADS)
+                            fm = fmaxf(fm, split_pieces<4>(piece, base, up, entries, valid, valid2));
+                        for (; base < total; base += SPLIT_THREADS)
+                            fm = fmaxf(fm, split_pieces<1>(piece, base, up, entries, valid, valid2));
+                        fence_proxy_async();
+                        m = split_reduce(__float_as_uint(fm * up), split_top[turn], warp - FIRST_SPLIT_WARP, lane);
+                        // 0: all zero; not below 65504: would have overflowed (or an infinity in the input, which no
+                        // scale helps: it stays one)
+                        if (!known || m == 0 || (m >= 0x42800000u && m < 0x477fe000u))
+                            break;
+                        if (sid == 0)
+                            reload_patch(T, t, cb, slot);
+                        ok = mbar_wait(&x_redo, redone & 1, status, 18);
+                        ++redone;
+                        if (!ok)
+                            break;
+                        known = false;
+                        m = 0;
                     }
-                    fence_proxy_async();
-                    mbar_arrive(&x_ready[slot]);
+                    known = m != 0; // an all-zero patch says nothing about the next one
+                    if (sid == 0)
+                    {
+                        patch_down[scale_at] = down;
+                        mbar_arrive(&x_ready[slot]);
+                    }
+                    turn ^= 1;
+                    scale_at = (scale_at + 1) % SCALE_RING;
+                    if (++slot == a.x_slots) { slot = 0; phase ^= 1; }
                 }
+            }
         }
     }
     else
     {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");
+        if (!PIXM)
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+        else
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+        const float w_down = __ldg(filt_scale);             // inverse of the filter's block scale
         const float act_ns = act_neg_scale(a.act, a.slope); // activation: v > 0 ? v : v * act_ns
         if (PIXM)
         {
@@ -621,10 +800,10 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
             const bool active = mt < mtiles;
             const size_t plane = (size_t)a.o_kb_stride;
             bool ok = true;
-            int gc = 0;
-            SB_TILE_LOOP(ok)
+            int gc = 0, pc = 0; // groups flushed, patches they came from
+            for (int t = first_tile, once_ = 0; (PERSIST ? (t < a.total_tiles) : (once_ == 0)) && ok; t += tile_step, ++once_, ++pc)
             {
-                const Tile T = decode_tile<MERGED != 2>(a, t);
+                const Tile T = decode_tile(a, t);
                 // the bias seeds the sums (these loads overlap the wait for the first group)
                 constexpr int ACC = MERGED ? 32 : 64; // output channels a thread can hold
                 float acc[ACC];
@@ -635,13 +814,18 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
                                                             : make_float4(0.f, 0.f, 0.f, 0.f);
                     acc[4 * c4] = b.x; acc[4 * c4 + 1] = b.y; acc[4 * c4 + 2] = b.z; acc[4 * c4 + 3] = b.w;
                 }
+                int in_cb = 0;
                 for (int g = 0; g < groups && ok; ++g, ++gc)
                 {
+                    if (in_cb == groups_per_cb) { in_cb = 0; ++pc; }
+                    ++in_cb;
                     const int tb = gc & 3;
                     ok = mbar_wait(&t_full[tb], (gc >> 2) & 1, status, 15, 1u << 24);
                     if (!ok)
                         break;
                     tc_fence_after_sync();
+                    // the group's sums are those of operands scaled by powers of two: undone here, in the same FMA
+                    const float down = *reinterpret_cast<volatile float *>(&patch_down[pc % SCALE_RING]) * w_down;
                     if (active)
                     {
                         const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) +
@@ -656,18 +840,18 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
                             {
 #pragma unroll
                                 for (int e = 0; e < 16; ++e)
-                                    acc[e] += __uint_as_float(v[e]) + __uint_as_float(v[16 + e]);
+                                    acc[e] = fmaf(__uint_as_float(v[e]) + __uint_as_float(v[16 + e]), down, acc[e]);
                             }
                             else
                             {
 #pragma unroll
                                 for (int e = 0; e < 32; ++e)
-                                    acc[e] += __uint_as_float(v[e]);
+                                    acc[e] = fmaf(__uint_as_float(v[e]), down, acc[e]);
                                 tmem_ld32(tbase + 32u, v);
                                 tmem_ld_wait();
 #pragma unroll
                                 for (int e = 0; e < 32; ++e)
-                                    acc[e] += __uint_as_float(v[e]);
+                                    acc[e] = fmaf(__uint_as_float(v[e]), down, acc[e]);
                             }
                         }
                         else // K = 64
@@ -681,7 +865,7 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
                                 tmem_ld_wait();
 #pragma unroll
                                 for (int e = 0; e < 32; ++e)
-                                    acc[piece * 32 + e] += __uint_as_float(v[e]);
+                                    acc[piece * 32 + e] = fmaf(__uint_as_float(v[e]), down, acc[piece * 32 + e]);
                             }
                         }
                     }
@@ -707,7 +891,7 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
                     // before it and all leave together (see the channel-major epilogue).
                     constexpr int HALF = ACC / 2;
                     const int ml = mt * 128 + quarter * 32 + lane; // tiled plans: m_local0 = 0
-                    const int rl = (MERGED == 2 ? ml / a.PW : a.by_PW.div(ml)), cl = ml - rl * a.PW;
+                    const int rl = a.by_PW.div(ml), cl = ml - rl * a.PW;
                     const int upper = lane & 1;
                     float *xrow = reinterpret_cast<float *>(smem + a.stage_off) +
                                   ((size_t)(rl >> 1) * (a.PW >> 1) + (cl >> 1)) * (ACC + 4) + upper * HALF;
@@ -756,7 +940,7 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
                 else if (ok && active)
                 {
                     const int ml = T.m_local0 + mt * 128 + quarter * 32 + lane;
-                    const int rl = (MERGED == 2 ? ml / a.PW : a.by_PW.div(ml)), cl = ml - rl * a.PW;
+                    const int rl = a.by_PW.div(ml), cl = ml - rl * a.PW;
                     const int r = T.row_base + rl, c = T.col_base + cl;
                     if (cl < T.tw_valid && rl < T.th_valid && r < a.Ho)
                     {
@@ -803,8 +987,10 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
         const int psub = lane >> 2, q4 = lane & 3; // 8 pixels x 4 float4 per warp and step
         const size_t plane = (size_t)a.o_kb_stride;
         bool ok = true;
-        int gc = 0;
-        SB_TILE_LOOP(ok)
+        int gc = 0, pc = 0; // groups flushed, patches they came from
+        int st = 0;
+        uint32_t st_phase = 0;
+        for (int t = first_tile, once_ = 0; (PERSIST ? (t < a.total_tiles) : (once_ == 0)) && ok; t += tile_step, ++once_, ++pc)
         {
             const Tile T = decode_tile(a, t);
             // the bias of this thread's channel seeds its sums (rank 0 only when two CTAs share a tile)
@@ -813,16 +999,23 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
 #pragma unroll
             for (int c = 0; c < COLS_PER_THREAD; ++c)
                 acc[c] = seed;
+            int in_cb = 0;
             for (int g = 0; g < groups && ok; ++g, ++gc)
             {
+                if (in_cb == groups_per_cb) { in_cb = 0; ++pc; }
+                ++in_cb;
                 const int tb = gc & (a.tbufs - 1);
                 if (a.tbufs > a.w_stages)
                     ok = mbar_wait(&t_full[tb], (gc >> (a.tbufs == 4 ? 2 : 1)) & 1, status, 15, 1u << 24);
                 else
-                    ok = mbar_wait(&g_done[gc % a.w_stages], (gc / a.w_stages) & 1, status, 15, 1u << 24);
+                    {
+                    ok = mbar_wait(&g_done[st], st_phase, status, 15, 1u << 24);
+                    if (++st == a.w_stages) { st = 0; st_phase ^= 1; }
+                }
                 if (!ok)
                     break;
                 tc_fence_after_sync();
+                const float down = *reinterpret_cast<volatile float *>(&patch_down[pc % SCALE_RING]) * w_down;
                 const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(tb * a.NPX + col0);
 #pragma unroll
                 for (int piece = 0; piece < COLS_PER_THREAD / 32; ++piece)
@@ -834,7 +1027,7 @@ conv_tf32x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__res
                         tmem_ld_wait();
 #pragma unroll
                         for (int e = 0; e < 32; ++e)
-                            acc[piece * 32 + e] += __uint_as_float(v[e]);
+                            acc[piece * 32 + e] = fmaf(__uint_as_float(v[e]), down, acc[piece * 32 + e]);
                     }
                 }
                 tc_fence_before_sync();
@@ -1012,11 +1205,12 @@ bool fit_rings(TcArgs &a, bool need_two)
     a.row_skip = (a.cg == 1 && a.group != a.Fw) ? (a.PW - a.Fw) * 4 : 0;
     const size_t limit = 226 * 1024;
     const int entries = a.PR * a.PW;
-    const size_t x_part = ((size_t)entries * 64 * a.cg + 1023) & ~(size_t)1023;
-    const size_t w_part = (size_t)a.MT * 64 * a.group;
+    const size_t x_part = ((size_t)entries * 64 * a.cg + 4095) & ~(size_t)4095;
+    a.WR = a.pixm ? a.K : a.MT;
+    const size_t w_part = (size_t)a.WR * 64 * a.group; // one filter stage
     const size_t staging = (size_t)64 * (a.MT + 16) * 4; // 32 pixels of each half of the tile
     // {patch slots, filter stages (>= 2: a commit serves both rings)}
-    static const int pref[][2] = {{3, 3}, {2, 3}, {2, 2}, {1, 3}, {1, 2}};
+    static const int pref[][2] = {{3, 6}, {3, 4}, {3, 3}, {2, 3}, {3, 2}, {2, 2}, {1, 3}, {1, 2}};
     // persistent where it pays and fits: narrow layers (64-channel tiles: small filter stages and
     // staging rows, little work per tile); wide ones need the shared memory for deeper rings
     // Pixel-major persistent tiles whose whole filter fits: one stage per group of a tile, loaded once
@@ -1033,7 +1227,7 @@ bool fit_rings(TcArgs &a, bool need_two)
         if (stages <= W_STAGES_MAX)
             for (int xs = 3; xs >= 2; --xs)
             {
-                const size_t ops = (size_t)xs * 2 * x_part + (size_t)stages * 2 * w_part;
+                const size_t ops = (size_t)xs * x_part + (size_t)stages * w_part;
                 const size_t smem = ops + pool_rows;
                 if (smem <= limit)
                 {
@@ -1049,7 +1243,7 @@ bool fit_rings(TcArgs &a, bool need_two)
             const int xs = p[0] < a.cbs || persistent ? p[0] : a.cbs;
             if (need_two && xs < 2 && a.cbs >= 2)
                 continue;
-            const size_t ops = (size_t)xs * 2 * x_part + (size_t)p[1] * 2 * w_part;
+            const size_t ops = (size_t)xs * x_part + (size_t)p[1] * w_part;
             const size_t full = (size_t)a.NPX * (a.MT + 16) * 4; // one tile per CTA stages the whole tile
             const size_t smem = persistent ? ops + (a.pixm ? pool_rows : staging) : (ops > full ? ops : full);
             if (smem <= limit)
@@ -1072,7 +1266,7 @@ bool plan_tiled(const small_b200_layer *L, TcArgs &a)
     double best = 0.0;
     int best_tw = 0, best_th = 0;
     const int cap = 256, gran = a.pixm ? 128 : 64;
-    for (int tw = 8; tw <= a.Wo && tw + a.Fw - 1 <= cap; tw += (a.pool ? 2 : 1))
+    for (int tw = 8; tw <= a.Wo && tw + a.Fw - 1 <= BOX_PX; tw += (a.pool ? 2 : 1))
     {
         const int pw = tw + a.Fw - 1;
         int th = (cap - tw) / pw + 1;
@@ -1105,7 +1299,7 @@ bool plan_tiled(const small_b200_layer *L, TcArgs &a)
 }
 
 // Tiling and shared-memory plan of one layer; false when the shape is not covered.
-bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool whole)
+bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool whole, bool rows_view)
 {
     if (!L || L->stride != 1 || row_stride(L) != 1 || L->C % CB != 0 || L->K % CB != 0 || L->C <= 0 || L->K <= 0)
         return false;
@@ -1114,6 +1308,7 @@ bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool 
     a = TcArgs{};
     a.N = L->N; a.C = L->C; a.K = L->K; a.H = L->H; a.W = L->W; a.Fh = L->Fh; a.Fw = L->Fw;
     a.pad_t = L->pad_t; a.pad_l = L->pad_l;
+    a.x_row = (long long)a.W * CB; a.x_plane = (long long)a.H * a.W * CB;
     a.Ho = out_dim(L->H, L->pad_t, L->pad_b, L->Fh, 1);
     a.Wo = out_dim(L->W, L->pad_l, L->pad_r, L->Fw, 1);
     a.cbs = L->C / CB; a.taps = L->Fh * L->Fw;
@@ -1125,12 +1320,12 @@ bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool 
     a.cg = 1; a.tap_step = 4;
     // few output channels: pixels on the tensor core's M (see the kernel's PIXM paths)
     a.pixm = pixm ? 1 : 0;
-    a.merged = (pixm && interleaved_filter(a.K)) ? 1 : 0;
+    a.merged = (pixm && a.K <= 32) ? 1 : 0;
     a.row_skip = 0;
     if (whole)
     {
-        // the whole window in one group (TcArgs::row_skip): one channel block, at most 3x3
-        if (!a.merged || a.cbs != 1 || a.Fh < 2 || a.taps > 9)
+        // the whole window in one group (TcArgs::row_skip): at most 3x3
+        if (a.Fh < 2 || a.taps > 9)
             return false;
         a.group = a.taps;
     }
@@ -1145,12 +1340,41 @@ bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool 
     }
     if (a.Ho == 0 || a.Wo == 0)
         return true;
-    if (L->W + (L->pad_l > L->pad_r ? L->pad_l : L->pad_r) > 64)
-        return plan_tiled(L, a);
     // 1x1 layer: two channel blocks per patch and per group (see TcArgs::cg)
+    const bool pointwise = a.taps == 1 && !L->pad_t && !L->pad_b && !L->pad_l && !L->pad_r;
     if (a.taps == 1 && a.cbs % 2 == 0)
     {
         a.cg = 2; a.cbs /= 2; a.taps = 2; a.group = 2;
+    }
+    if (pointwise && !rows_view)
+    {
+        // no neighbourhoods: an image is one row of pixels, a tile a run of NPX of them
+        a.W *= a.H; a.H = 1; a.Wo = a.W; a.Ho = 1;
+        a.tiled = 1; a.TH = 1; a.PR = 1; a.runs = 1;
+        const int gran = a.pixm ? 128 : 64, tiles256 = (a.W + 255) / 256;
+        for (int npx = ((a.W + tiles256 - 1) / tiles256 + gran - 1) / gran * gran; npx >= gran; npx -= gran)
+        {
+            a.NPX = a.TW = a.PW = npx;
+            a.tiles_x = a.px_tiles = (a.W + npx - 1) / npx;
+            if (a.cg > 1)
+                a.tap_step = npx * 4;
+            if (fit_rings(a, npx > 128))
+                return true;
+        }
+        return false;
+    }
+    if (rows_view)
+    {
+        a.x_row = (long long)a.C * a.W; a.x_plane = (long long)a.W * CB;
+        a.runs = a.PW > BOX_PX ? 1 : 0;
+    }
+    else if (a.PW > BOX_PX)
+    {
+        if (a.cg > 1) // a padded 1x1 layer: one channel block at a time
+        {
+            a.cbs *= 2; a.cg = 1; a.taps = 1; a.group = 1;
+        }
+        return plan_tiled(L, a);
     }
     // GEMM columns of one image: the last valid one is (Ho-1)*PW + Wo-1
     const int m_img = (a.Ho - 1) * a.PW + a.Wo;
@@ -1182,22 +1406,20 @@ bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool 
         }
     return false;
 }
-bool plan_as(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool = false)
+bool plan_as(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool rows_view)
 {
-    // whole-window groups only where the filter stays resident in shared memory
-    if (pixm && plan_as_g(L, a, pixm, pool, true) && (a.w_resident || a.Ho == 0 || a.Wo == 0))
+    // pixel-major: whole-window groups only where the filter stays resident in shared memory; channel-major: where
+    // two stages of a whole window and two patches fit
+    if (plan_as_g(L, a, pixm, pool, true, rows_view) && (a.Ho == 0 || a.Wo == 0 || (pixm ? a.w_resident : a.x_slots >= 2)))
         return true;
-    return plan_as_g(L, a, pixm, pool, false);
+    return plan_as_g(L, a, pixm, pool, false, rows_view);
 }
-bool plan_shape(const small_b200_layer *L, TcArgs &a)
+bool plan_shape(const small_b200_layer *L, TcArgs &a, bool rows_view = false)
 {
     const bool want_pixm = L && (L->K == 16 || L->K == 32 || L->K == 64);
-    if (want_pixm && plan_as(L, a, true))
+    if (want_pixm && plan_as(L, a, true, false, rows_view))
         return true;
-    // the interleaved filter layout is only read by the pixel-major kernel
-    if (L && interleaved_filter(L->K))
-        return false;
-    return plan_as(L, a, false);
+    return plan_as(L, a, false, false, rows_view);
 }
 bool plan(const small_b200_layer *L, TcArgs &a)
 {
@@ -1206,7 +1428,7 @@ bool plan(const small_b200_layer *L, TcArgs &a)
     {
         small_b200_layer V = *L; // the batch as the rows of one image (TcArgs::rows_view)
         V.N = 1; V.H = L->N; V.W = L->H * L->W;
-        if (plan_shape(&V, a))
+        if (plan_shape(&V, a, true))
         {
             a.rows_view = 1;
             a.o_kb_stride = (long long)V.W * CB;
@@ -1231,7 +1453,7 @@ bool plan_pooled(const small_b200_layer *L, const small_b200_layer *pool, TcArgs
     if (pool->Fh != 2 || pool->Fw != 2 || pool->stride != 2 || row_stride(pool) != 2 || pool->pad_t || pool->pad_b ||
         pool->pad_l || pool->pad_r)
         return false;
-    if (!plan_as(L, a, true, true))
+    if (!plan_as(L, a, true, true, false))
         return false;
     if (pool->H != a.Ho || pool->W != a.Wo || pool->C != L->K || pool->N != L->N)
         return false;
@@ -1269,8 +1491,15 @@ int small_b200_filter_prepare_tf32x3(const small_b200_layer *L, const float *fil
     if (!L || L->C % CB != 0 || L->K % CB != 0 || L->C <= 0 || L->K <= 0 || L->Fh <= 0 || L->Fw <= 0)
         return fail(SMALL_B200_INVALID_ARGUMENT, "Conv2D<float> (3xTF32) ERROR: shape not covered by the tensor-core path.");
     const long long n = (long long)L->K * L->C * L->Fh * L->Fw;
-    prepare_filter_kernel<<<(unsigned)((n + 255) / 256), 256, 0, as_stream(stream)>>>(
-        n, (L->C / CB) * L->Fh * L->Fw, pick_mt(L->K), L->K, interleaved_filter(L->K) ? 1 : 0, filt, prepared, prepared + n);
+    // [0, n) floats: the half-precision pairs; behind them the inverse of the block scale and the largest magnitude
+    uint32_t *top = reinterpret_cast<uint32_t *>(prepared + n + 1);
+    SB_CUDA(cudaMemsetAsync(top, 0, sizeof(uint32_t), as_stream(stream)));
+    const long long blocks = (n + 255) / 256;
+    filter_max_kernel<<<(unsigned)(blocks < 1024 ? blocks : 1024), 256, 0, as_stream(stream)>>>(n, filt, top);
+    if (int rc = launched("filter_max_kernel"))
+        return rc;
+    prepare_filter_kernel<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(
+        n, (L->C / CB) * L->Fh * L->Fw, pick_mt(L->K), L->K, filt, top, reinterpret_cast<__half *>(prepared), prepared + n);
     return launched("prepare_filter_kernel");
 }
 
@@ -1311,31 +1540,29 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
 
     CUtensorMap mx;
     {
-        // activations [N*cbs][H][W][16 floats]
-        const uint64_t dims[4] = {16, (uint64_t)a.W, (uint64_t)a.H, (uint64_t)a.N * a.cbs * a.cg};
-        uint64_t strides[3] = {64, (uint64_t)a.W * 64, (uint64_t)a.H * a.W * 64};
-        if (a.rows_view) // rows are images (C*P floats apart), planes the channel blocks of one image
-        {
-            strides[1] = (uint64_t)a.C * a.W * 4;
-            strides[2] = (uint64_t)a.W * 64;
-        }
-        const uint32_t box[4] = {16, (uint32_t)a.PW, (uint32_t)a.PR, (uint32_t)a.cg};
-        if (int rc = make_tensor_map(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, in, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B))
+        // activations [N*cbs][H][W][8 x 8 bytes]: whole rows of the image are the innermost dimension.  (A map with a
+        // pixel's 64 bytes innermost moves one 64-byte row per 9 to 12 cycles, whatever memory delivers.)
+        const uint64_t dims[3] = {(uint64_t)a.W * 8, (uint64_t)a.H, (uint64_t)a.N * a.cbs * a.cg};
+        const uint64_t strides[2] = {(uint64_t)a.x_row * 4, (uint64_t)a.x_plane * 4};
+        const uint32_t box[3] = {(uint32_t)a.PW * 8, (uint32_t)a.PR, (uint32_t)a.cg};
+        if (a.runs)
+            memset(&mx, 0, sizeof(mx));
+        else if (int rc = make_tensor_map(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, in, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE))
             return rc;
     }
     static PerDeviceOnce configured;
     int dev;
     if (configured.needed(&dev))
     {
-        SB_CUDA(cudaFuncSetAttribute(conv_tf32x3_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_tf32x3_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_tf32x3_kernel<true, false, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_tf32x3_kernel<true, false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_tf32x3_kernel<true, false, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_tf32x3_kernel<true, false, true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_tf32x3_kernel<true, false, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_tf32x3_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_tf32x3_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         configured.mark(dev);
     }
     int *status = device_status_ptr();
@@ -1365,7 +1592,8 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
             blocks = 2 * tiles;
         }
     }
-    const float *flo_ = filt_prepared + (size_t)a.K * a.C * a.Fh * a.Fw;
+    const __half *filt = reinterpret_cast<const __half *>(filt_prepared);
+    const float *filt_scale = filt_prepared + (size_t)a.K * a.C * a.Fh * a.Fw;
     auto launch_split = [&](const TcArgs &ta, long long nblocks) -> int {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)nblocks); cfg.blockDim = dim3(NUM_THREADS);
@@ -1374,7 +1602,7 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
-        SB_CUDA(cudaLaunchKernelEx(&cfg, conv_tf32x3_kernel<false, true>, mx, filt_prepared, flo_, ta, bias, out, status));
+        SB_CUDA(cudaLaunchKernelEx(&cfg, conv_f16x3_kernel<false, true>, mx, in, filt, filt_scale, ta, bias, out, status));
         return SMALL_B200_OK;
     };
     // One tile per CTA and a last wave that fills less than half of the SMs (512 tiles on 148 SMs: three
@@ -1390,21 +1618,21 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         {
             TcArgs a1 = a;
             a1.tile_base = 0;
-            conv_tf32x3_kernel<false, false><<<(unsigned)full, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
-                mx, filt_prepared, flo_, a1, bias, out, status);
-            if (int rc = launched("conv_tf32x3_kernel"))
+            conv_f16x3_kernel<false, false><<<(unsigned)full, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
+                mx, in, filt, filt_scale, a1, bias, out, status);
+            if (int rc = launched("conv_f16x3_kernel"))
                 return rc;
             TcArgs a2 = a;
             a2.tile_base = (int)full; a2.ksplit = 2;
             if (int rc = launch_split(a2, 2 * rem))
                 return rc;
-            return launched("conv_tf32x3_kernel");
+            return launched("conv_f16x3_kernel");
         }
     }
     const bool whole = a.merged && a.cg == 1 && a.group != a.Fw; // whole-window groups (TcArgs::row_skip)
 #define SB_LAUNCH_PIXM(M, P) \
-    conv_tf32x3_kernel<true, false, true, M, P><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>( \
-        mx, filt_prepared, flo_, a, bias, out, status)
+    conv_f16x3_kernel<true, false, true, M, P><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>( \
+        mx, in, filt, filt_scale, a, bias, out, status)
     if (a.pool && whole)
         SB_LAUNCH_PIXM(2, true);
     else if (a.pool && a.merged)
@@ -1417,20 +1645,20 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         SB_LAUNCH_PIXM(1, false);
 #undef SB_LAUNCH_PIXM
     else if (a.pixm)
-        conv_tf32x3_kernel<true, false, true><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
-            mx, filt_prepared, filt_prepared + (size_t)a.K * a.C * a.Fh * a.Fw, a, bias, out, status);
+        conv_f16x3_kernel<true, false, true><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
+            mx, in, filt, filt_scale, a, bias, out, status);
     else if (a.persistent)
-        conv_tf32x3_kernel<true, false><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
-            mx, filt_prepared, filt_prepared + (size_t)a.K * a.C * a.Fh * a.Fw, a, bias, out, status);
+        conv_f16x3_kernel<true, false><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
+            mx, in, filt, filt_scale, a, bias, out, status);
     else if (a.ksplit == 2)
     {
         if (int rc = launch_split(a, blocks))
             return rc;
     }
     else
-        conv_tf32x3_kernel<false, false><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
-            mx, filt_prepared, filt_prepared + (size_t)a.K * a.C * a.Fh * a.Fw, a, bias, out, status);
-    return launched("conv_tf32x3_kernel");
+        conv_f16x3_kernel<false, false><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
+            mx, in, filt, filt_scale, a, bias, out, status);
+    return launched("conv_f16x3_kernel");
 }
 } // namespace
 
