@@ -117,7 +117,7 @@ struct TcArgs
     unsigned stage_off;  // byte offset of the output staging rows (0: they alias the operand buffers)
     int total_tiles;     // N * px_tiles * k_tiles
     int persistent;      // 1: one CTA per SM walks over the tiles; 0: one tile per CTA
-    int ksplit;          // 2: a cluster of two CTAs shares a tile, each reduces half of the channel blocks
+    int ksplit;          // > 1: a cluster of that many CTAs shares a tile, each reduces a part of the channel blocks
     int tile_base;       // first tile of this launch (a layer may run as two launches, see the launch code)
     int w_resident;      // 1: every group of a tile has a filter stage of its own, loaded once per CTA (see fit_rings)
     // 16 or 32 output channels: a pixel-major MMA takes [W_hi | W_lo] (the rows lie one behind the other in every
@@ -362,16 +362,15 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     while ((int)tmem_cols < (PIXM ? a.tbufs * (a.NPX >> 7) * a.K * (MERGED ? 2 : 1) : a.tbufs * a.NPX))
         tmem_cols <<= 1;
 
-    // Split reduction (one tile per CTA only): the two CTAs of a cluster take one half of the channel
-    // blocks each; rank 1 hands its sums to rank 0 through shared memory at the end.  It turns the
-    // 3.46 waves of the 13x13 layers at batch 64 into 7 half-waves.
+    // Split reduction (one tile per CTA only): the CTAs of a cluster take a part of the channel blocks each, leave their
+    // sums in shared memory at the end, and each adds up and stores its share of the tile.
     constexpr bool split = SPLIT && !PERSIST;
-    const uint32_t crank = split ? cluster_ctarank() : 0u;
-    const int cbs_l = split ? a.cbs / 2 : a.cbs;     // channel blocks this CTA reduces
-    const int cb_begin = (int)crank * cbs_l;
+    const int crank = split ? (int)cluster_ctarank() : 0, S = split ? a.ksplit : 1;
+    const int cb_begin = split ? crank * a.cbs / S : 0;
+    const int cbs_l = split ? (crank + 1) * a.cbs / S - cb_begin : a.cbs; // channel blocks this CTA reduces
     const int steps = a.cbs * a.taps;
     const int groups_per_cb = a.taps / a.group, groups = cbs_l * groups_per_cb;
-    const int first_tile = a.tile_base + (split ? blockIdx.x / 2 : blockIdx.x), tile_step = gridDim.x;
+    const int first_tile = a.tile_base + (split ? blockIdx.x / (unsigned)S : blockIdx.x), tile_step = gridDim.x;
 
     // patch number pc / group number gc count over every tile of this CTA
     // pixels of a tile's patch that a copy delivers, per plane: every entry of a box (zeros outside the image), or
@@ -431,7 +430,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                 mbar_init(&w_full[i], 1); mbar_init(&g_done[i], 1);
             }
             for (int i = 0; i < 4; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], ACC_WARPS); }
-            mbar_init(&x_redo, 1); mbar_init(&peer_staged, ACC_WARPS); mbar_init(&peer_done, ACC_WARPS);
+            mbar_init(&x_redo, 1); mbar_init(&peer_staged, ACC_WARPS * S); mbar_init(&peer_done, ACC_WARPS * S);
             fence_barrier_init();
             // The first patch and the first filter stage only need their barriers: their round
             // trip to memory overlaps the tensor-memory allocation and the CTA-wide barrier.
@@ -993,7 +992,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
         for (int t = first_tile, once_ = 0; (PERSIST ? (t < a.total_tiles) : (once_ == 0)) && ok; t += tile_step, ++once_, ++pc)
         {
             const Tile T = decode_tile(a, t);
-            // the bias of this thread's channel seeds its sums (rank 0 only when two CTAs share a tile)
+            // the bias of this thread's channel seeds its sums (rank 0 only when several CTAs share a tile)
             const float seed = (bias && crank == 0 && lane_has_row && k_local < T.kv) ? __ldg(bias + T.kt * a.MT + k_local) : 0.f;
             float acc[COLS_PER_THREAD];
 #pragma unroll
@@ -1061,26 +1060,58 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                     }
                 }
                 asm volatile("bar.sync 1, 256;" ::: "memory"); // the eight accumulation warps
-                uint32_t peer_stage = 0;
                 if (split)
                 {
-                    if (crank == 1)
+                    // Every warp tells every CTA of the cluster that its sums are staged; when all have, the units of the
+                    // tile (8 pixels x 16 channels) go round over the warps of the cluster, each of which adds up the
+                    // S staged parts in rank order and stores.  Nobody leaves before all have read.
+                    if (lane < S)
                     {
-                        // hand the staged half-sums to rank 0, then stay until it has read them
-                        if (lane == 0)
+                        asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                        mbar_arrive_remote(map_to_cta(&peer_staged, (uint32_t)lane));
+                    }
+                    __syncwarp();
+                    ok = mbar_wait_cluster(&peer_staged, 0, status, 20) && ok;
+                    const int pgs = a.NPX / 8, units = pgs * kbs;
+                    for (int u = crank * ACC_WARPS + warp - FIRST_ACC_WARP; ok && u < units; u += S * ACC_WARPS)
+                    {
+                        const int kb = u / pgs, px = (u - kb * pgs) * 8 + psub;
+                        const int ml = T.m_local0 + px;
+                        const int rl = a.by_PW.div(ml), cl = ml - rl * a.PW;
+                        const int r = T.row_base + rl, c = T.col_base + cl;
+                        if (cl < T.tw_valid && rl < T.th_valid && r < a.Ho)
                         {
-                            asm volatile("fence.acq_rel.cluster;" ::: "memory");
-                            mbar_arrive_remote(map_to_cta(&peer_staged, 0));
+                            const float *sp = stage + (size_t)px * pitch + kb * CB + q4 * 4;
+                            float4 part[8]; // all loads out together: a round trip to another SM takes about 1000 cycles
+#pragma unroll
+                            for (int q = 0; q < 8; ++q)
+                                if (q < S)
+                                    part[q] = ld_cluster_f4(map_to_cta(sp, (uint32_t)q));
+                            float4 x = part[0];
+#pragma unroll
+                            for (int q = 1; q < 8; ++q)
+                                if (q < S)
+                                {
+                                    x.x += part[q].x; x.y += part[q].y; x.z += part[q].z; x.w += part[q].w;
+                                }
+                            float *o = obase + (size_t)r * a.o_row_stride + (size_t)c * CB + (size_t)kb * plane;
+                            if (a.accumulate)
+                            {
+                                const float4 s4 = *reinterpret_cast<const float4 *>(o);
+                                x.x += s4.x; x.y += s4.y; x.z += s4.z; x.w += s4.w;
+                            }
+                            x.x = apply_act_ns(x.x, act_ns); x.y = apply_act_ns(x.y, act_ns);
+                            x.z = apply_act_ns(x.z, act_ns); x.w = apply_act_ns(x.w, act_ns);
+                            *reinterpret_cast<float4 *>(o) = x;
                         }
-                        ok = mbar_wait_cluster(&peer_done, 0, status, 21) && false; // rank 1 stores nothing
                     }
-                    else
-                    {
-                        ok = ok && mbar_wait_cluster(&peer_staged, 0, status, 20);
-                        peer_stage = map_to_cta(stage, 1);
-                    }
+                    __syncwarp();
+                    if (lane < S)
+                        mbar_arrive_remote(map_to_cta(&peer_done, (uint32_t)lane));
+                    __syncwarp();
+                    mbar_wait_cluster(&peer_done, 0, status, 21);
                 }
-                if (ok)
+                else if (ok)
                 {
                     for (int pg = warp - FIRST_ACC_WARP; pg < a.NPX / 8; pg += ACC_WARPS)
                     {
@@ -1091,18 +1122,12 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                         if (cl < T.tw_valid && rl < T.th_valid && r < a.Ho)
                         {
                             const float *sp = stage + (size_t)px * pitch + q4 * 4;
-                            const uint32_t rp = peer_stage + (uint32_t)(((size_t)px * pitch + q4 * 4) * 4);
                             float *o = obase + (size_t)r * a.o_row_stride + (size_t)c * CB;
 #pragma unroll
                             for (int kb = 0; kb < 8; ++kb)
                               if (kb < kbs)
                             {
                                 float4 x = *reinterpret_cast<const float4 *>(sp + kb * CB);
-                                if (split)
-                                {
-                                    const float4 y = ld_cluster_f4(rp + (uint32_t)(kb * CB * 4)); // rank 1's half
-                                    x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
-                                }
                                 float *ok_ = o + (size_t)kb * plane;
                                 if (a.accumulate)
                                 {
@@ -1115,13 +1140,6 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                             }
                         }
                     }
-                }
-                if (split && crank == 0)
-                {
-                    // rank 1 may leave: its staging rows have been read
-                    __syncwarp();
-                    if (lane == 0)
-                        mbar_arrive_remote(map_to_cta(&peer_done, 1));
                 }
             }
             else
@@ -1261,11 +1279,11 @@ bool fit_rings(TcArgs &a, bool need_two)
 // halo stays small (a range of full-width rows of a 208-wide image drags two whole rows of halo
 // along for every 256 outputs).  GEMM column j of a tile is patch-linear: row j / PW, column j % PW,
 // columns >= TW of each patch row are junk.
-bool plan_tiled(const small_b200_layer *L, TcArgs &a)
+bool plan_tiled(const small_b200_layer *L, TcArgs &a, int cap)
 {
     double best = 0.0;
     int best_tw = 0, best_th = 0;
-    const int cap = 256, gran = a.pixm ? 128 : 64;
+    const int gran = a.pixm ? 128 : 64;
     for (int tw = 8; tw <= a.Wo && tw + a.Fw - 1 <= BOX_PX; tw += (a.pool ? 2 : 1))
     {
         const int pw = tw + a.Fw - 1;
@@ -1299,7 +1317,7 @@ bool plan_tiled(const small_b200_layer *L, TcArgs &a)
 }
 
 // Tiling and shared-memory plan of one layer; false when the shape is not covered.
-bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool whole, bool rows_view)
+bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool whole, bool rows_view, int npx_cap)
 {
     if (!L || L->stride != 1 || row_stride(L) != 1 || L->C % CB != 0 || L->K % CB != 0 || L->C <= 0 || L->K <= 0)
         return false;
@@ -1336,7 +1354,7 @@ bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool 
         if (!pixm || a.accumulate || a.Ho % 2 || a.Wo % 2 || a.Fw % 2 == 0 || a.Ho == 0 || a.Wo == 0 ||
             L->W + (L->pad_l > L->pad_r ? L->pad_l : L->pad_r) <= 64)
             return false;
-        return plan_tiled(L, a);
+        return plan_tiled(L, a, npx_cap);
     }
     if (a.Ho == 0 || a.Wo == 0)
         return true;
@@ -1351,8 +1369,8 @@ bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool 
         // no neighbourhoods: an image is one row of pixels, a tile a run of NPX of them
         a.W *= a.H; a.H = 1; a.Wo = a.W; a.Ho = 1;
         a.tiled = 1; a.TH = 1; a.PR = 1; a.runs = 1;
-        const int gran = a.pixm ? 128 : 64, tiles256 = (a.W + 255) / 256;
-        for (int npx = ((a.W + tiles256 - 1) / tiles256 + gran - 1) / gran * gran; npx >= gran; npx -= gran)
+        const int gran = a.pixm ? 128 : 64, tiles_cap = (a.W + npx_cap - 1) / npx_cap;
+        for (int npx = ((a.W + tiles_cap - 1) / tiles_cap + gran - 1) / gran * gran; npx >= gran; npx -= gran)
         {
             a.NPX = a.TW = a.PW = npx;
             a.tiles_x = a.px_tiles = (a.W + npx - 1) / npx;
@@ -1374,13 +1392,13 @@ bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool 
         {
             a.cbs *= 2; a.cg = 1; a.taps = 1; a.group = 1;
         }
-        return plan_tiled(L, a);
+        return plan_tiled(L, a, npx_cap);
     }
     // GEMM columns of one image: the last valid one is (Ho-1)*PW + Wo-1
     const int m_img = (a.Ho - 1) * a.PW + a.Wo;
-    const int tiles256 = (m_img + 255) / 256;
+    const int tiles_cap = (m_img + npx_cap - 1) / npx_cap;
     const int gran = a.pixm ? 128 : 64;
-    int npx_first = ((m_img + tiles256 - 1) / tiles256 + gran - 1) / gran * gran;
+    int npx_first = ((m_img + tiles_cap - 1) / tiles_cap + gran - 1) / gran * gran;
     // First pass: only plans that keep two patches in flight (a layer with few channel blocks
     // per CTA otherwise waits for every patch's load and lo copy), even at a narrower tile;
     // second pass: anything that fits.
@@ -1406,29 +1424,29 @@ bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool 
         }
     return false;
 }
-bool plan_as(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool rows_view)
+bool plan_as(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool rows_view, int npx_cap)
 {
     // pixel-major: whole-window groups only where the filter stays resident in shared memory; channel-major: where
     // two stages of a whole window and two patches fit
-    if (plan_as_g(L, a, pixm, pool, true, rows_view) && (a.Ho == 0 || a.Wo == 0 || (pixm ? a.w_resident : a.x_slots >= 2)))
+    if (plan_as_g(L, a, pixm, pool, true, rows_view, npx_cap) && (a.Ho == 0 || a.Wo == 0 || (pixm ? a.w_resident : a.x_slots >= 2)))
         return true;
-    return plan_as_g(L, a, pixm, pool, false, rows_view);
+    return plan_as_g(L, a, pixm, pool, false, rows_view, npx_cap);
 }
-bool plan_shape(const small_b200_layer *L, TcArgs &a, bool rows_view = false)
+bool plan_shape(const small_b200_layer *L, TcArgs &a, bool rows_view, int npx_cap)
 {
     const bool want_pixm = L && (L->K == 16 || L->K == 32 || L->K == 64);
-    if (want_pixm && plan_as(L, a, true, false, rows_view))
+    if (want_pixm && plan_as(L, a, true, false, rows_view, 256))
         return true;
-    return plan_as(L, a, false, false, rows_view);
+    return plan_as(L, a, false, false, rows_view, npx_cap);
 }
-bool plan(const small_b200_layer *L, TcArgs &a)
+bool plan(const small_b200_layer *L, TcArgs &a, int npx_cap = 256)
 {
     if (L && L->Fh == 1 && L->Fw == 1 && L->stride == 1 && !L->pad_t && !L->pad_b && !L->pad_l && !L->pad_r &&
         L->N > 1 && L->H > 0 && L->W > 0 && (long long)L->H * L->W <= 64)
     {
         small_b200_layer V = *L; // the batch as the rows of one image (TcArgs::rows_view)
         V.N = 1; V.H = L->N; V.W = L->H * L->W;
-        if (plan_shape(&V, a, true))
+        if (plan_shape(&V, a, true, npx_cap))
         {
             a.rows_view = 1;
             a.o_kb_stride = (long long)V.W * CB;
@@ -1436,7 +1454,7 @@ bool plan(const small_b200_layer *L, TcArgs &a)
             return true;
         }
     }
-    if (!plan_shape(L, a))
+    if (!plan_shape(L, a, false, npx_cap))
         return false;
     a.o_kb_stride = (long long)a.Ho * a.Wo * CB;
     a.o_row_stride = (long long)a.Wo * CB;
@@ -1453,7 +1471,7 @@ bool plan_pooled(const small_b200_layer *L, const small_b200_layer *pool, TcArgs
     if (pool->Fh != 2 || pool->Fw != 2 || pool->stride != 2 || row_stride(pool) != 2 || pool->pad_t || pool->pad_b ||
         pool->pad_l || pool->pad_r)
         return false;
-    if (!plan_as(L, a, true, true, false))
+    if (!plan_as(L, a, true, true, false, 256))
         return false;
     if (pool->H != a.Ho || pool->W != a.Wo || pool->C != L->K || pool->N != L->N)
         return false;
@@ -1526,13 +1544,123 @@ int small_b200_conv2d_maxpool_f32_tf32x3(const small_b200_layer *conv, const sma
 
 namespace
 {
+// Cycles of one channel block (or bundle) of a channel-major tile: its MMAs (32 + N/4 cycles each for their operands, N/2
+// for the pipe), the filter stage's way into shared memory (about 40 bytes per cycle), or the splitters' passes.
+double block_cycles(const TcArgs &a)
+{
+    const double mma = 3.0 * a.taps * (a.NPX / 2 > 32 + a.NPX / 4 ? a.NPX / 2 : 32 + a.NPX / 4);
+    const double filter = a.taps * a.MT * 64 / 40.0;
+    const double split = 600 + 1100.0 * a.PR * a.PW * a.cg / 256;
+    return mma > filter ? (mma > split ? mma : split) : (filter > split ? filter : split);
+}
+// How a channel-major layer is cut: tile width (plans of at most 256, 192, 128, 64 pixels), how many CTAs of a cluster
+// share a tile's reduction, and the same for the tiles of a last, partial wave where that runs as a launch of its own
+// behind the full ones (rem_split, 0: one launch).  Small batches leave most SMs idle without it: 1024 -> 1024
+// channels on one 13x13 image are 8 tiles of 192 pixels.  The estimate counts whole waves of CTAs; the fixed costs are
+// those of starting a CTA (8000 cycles from its first instruction to its first finished sums, most of it cold code and
+// the first filter stage) and of the exchange between the CTAs of a cluster (2000 until all are there, 4000 to 7000 to
+// read the parts from the other SMs at some 13 bytes per cycle); a second launch costs another start.
+// One image: conv8 of Tiny-YOLOv2 (1024 -> 1024 at 13x13) 62 -> 25 us, conv7 56 -> 19, conv6 33 -> 13, conv5 24 -> 13.
+struct Cut
+{
+    int npx_cap, split, rem_split;
+};
+// Clusters of S such CTAs (one per SM) that the current device runs at a time: they may not cross the borders of its
+// groups of SMs (148 SMs: 74 pairs, 33 clusters of 4, 22 of 6, 15 of 8).
+int resident_clusters(int S)
+{
+    static std::atomic<int> known[64][9];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64)
+        dev = 0;
+    int n = known[dev][S].load(std::memory_order_relaxed);
+    if (n)
+        return n;
+    n = num_sms() / S;
+    if (S > 1)
+    {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)S); cfg.blockDim = dim3(NUM_THREADS);
+        cfg.dynamicSmemBytes = 226 * 1024;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        int q = 0;
+        if (cudaOccupancyMaxActiveClusters(&q, conv_f16x3_kernel<false, true>, &cfg) == cudaSuccess && q > 0)
+            n = q;
+        else
+            cudaGetLastError();
+    }
+    known[dev][S].store(n, std::memory_order_relaxed);
+    return n;
+}
+Cut choose_cut(const small_b200_layer *L)
+{
+    const double start = 8000, exchange = 6000;
+    const long long sms = num_sms();
+    static const int widths[] = {1, 2, 3, 4, 6, 8};
+    Cut best{256, 1, 0};
+    double best_cost = 0;
+    int last_npx = 0;
+    for (int cap = 256; cap >= 64; cap -= 64)
+    {
+        TcArgs a;
+        if (!plan(L, a, cap) || a.pixm || a.persistent || a.NPX == last_npx)
+            continue;
+        last_npx = a.NPX;
+        const long long tiles = (long long)a.N * a.px_tiles * a.k_tiles;
+        const double t = block_cycles(a);
+        for (int S : widths)
+        {
+            if (S > a.cbs)
+                break;
+            const long long room = resident_clusters(S);
+            const double each = t * ((a.cbs + S - 1) / S) + start + (S > 1 ? exchange : 0);
+            const double cost = ((tiles + room - 1) / room) * each;
+            // a finer cut has to promise something: the exchange is an estimate
+            if (best_cost == 0 || cost < 0.95 * best_cost)
+            {
+                best_cost = cost; best = Cut{cap, S, 0};
+            }
+            const long long full = tiles / sms, rem = tiles % sms;
+            if (S > 1 && full > 0 && rem > 0)
+            {
+                const double mixed = full * (t * a.cbs + start) + ((rem + room - 1) / room) * each + start;
+                if (mixed < 0.95 * best_cost)
+                {
+                    best_cost = mixed; best = Cut{cap, 1, S};
+                }
+            }
+        }
+    }
+    return best;
+}
+
 int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float *in, const float *filt_prepared,
            const float *bias, float *out, void *stream)
 {
     if (int rc = check_window_layer(L, "Conv2D<float>", true, 2))
         return rc;
+    static PerDeviceOnce configured;
+    int dev;
+    if (configured.needed(&dev))
+    {
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        configured.mark(dev);
+    }
     TcArgs a;
-    if (pool ? !plan_pooled(L, pool, a) : !plan(L, a))
+    const Cut cut = pool ? Cut{256, 1, 0} : choose_cut(L);
+    if (pool ? !plan_pooled(L, pool, a) : !plan(L, a, cut.npx_cap))
         return fail(SMALL_B200_INVALID_ARGUMENT, pool ? "Conv2D+MaxPool2D<float> (3xTF32) ERROR: shape not covered by the fused tensor-core path."
                                                       : "Conv2D<float> (3xTF32) ERROR: shape not covered by the tensor-core path.");
     if (a.N == 0 || a.Ho == 0 || a.Wo == 0)
@@ -1550,21 +1678,6 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         else if (int rc = make_tensor_map(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, in, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE))
             return rc;
     }
-    static PerDeviceOnce configured;
-    int dev;
-    if (configured.needed(&dev))
-    {
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        configured.mark(dev);
-    }
     int *status = device_status_ptr();
     if (!status)
         return fail(SMALL_B200_CUDA_ERROR, "device status word not available");
@@ -1576,22 +1689,8 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
     long long blocks = tiles;
     if (a.persistent && blocks > num_sms())
         blocks = num_sms();
-    a.ksplit = 1;
-    if (!a.persistent && a.cbs * a.cg >= 64 && a.cbs % 2 == 0)
-    {
-        // a cluster of two CTAs per tile, each reducing half of the channel blocks, when that
-        // shortens the tail: 512 tiles on 148 SMs are 4 rounds, 1024 half tiles are 7 half rounds
-        const long long sms = num_sms();
-        const long long rounds1 = (tiles + sms - 1) / sms, rounds2 = (2 * tiles + sms - 1) / sms;
-        // a 1x1 layer's half tile is too little work to pay for the hand-over between the two CTAs
-        // unless the tiles alone leave SMs idle (measured: 512 tiles of 1024->256 at 13x13 0.22 ms
-        // whole, 0.25 ms split; 64 tiles of 1024->128 0.050 ms whole, 0.035 ms split)
-        if (rounds2 * 100 <= rounds1 * 2 * 93 && (a.cg == 1 || 2 * tiles <= sms))
-        {
-            a.ksplit = 2;
-            blocks = 2 * tiles;
-        }
-    }
+    a.ksplit = (a.pixm || a.persistent) ? 1 : cut.split;
+    blocks *= a.ksplit;
     const __half *filt = reinterpret_cast<const __half *>(filt_prepared);
     const float *filt_scale = filt_prepared + (size_t)a.K * a.C * a.Fh * a.Fw;
     auto launch_split = [&](const TcArgs &ta, long long nblocks) -> int {
@@ -1600,38 +1699,28 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         cfg.dynamicSmemBytes = ta.smem_bytes; cfg.stream = as_stream(stream);
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        attr[0].val.clusterDim.x = (unsigned)ta.ksplit; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
         SB_CUDA(cudaLaunchKernelEx(&cfg, conv_f16x3_kernel<false, true>, mx, in, filt, filt_scale, ta, bias, out, status));
         return SMALL_B200_OK;
     };
-    // One tile per CTA and a last wave that fills less than half of the SMs (512 tiles on 148 SMs: three
-    // full waves and 68 tiles): that wave runs as clusters of two CTAs that split the reduction, in a
-    // launch of its own behind the full waves, and takes a little over half a round instead of a whole
-    // one.  (Splitting EVERY tile of such a layer was measured slower: 512 -> 1024 channels at 13x13
-    // 0.415 -> 0.425 ms; the exchange between the two CTAs costs about a sixth of a half tile.)
-    if (!a.pixm && !a.persistent && a.ksplit == 1 && a.cbs % 2 == 0 && a.cbs >= 8 && a.cg == 1)
+    if (!a.pixm && !a.persistent && cut.rem_split)
     {
-        const long long sms = num_sms();
-        const long long full = tiles / sms * sms, rem = tiles - full;
-        if (full > 0 && rem > 0 && 2 * rem <= sms)
-        {
-            TcArgs a1 = a;
-            a1.tile_base = 0;
-            conv_f16x3_kernel<false, false><<<(unsigned)full, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
-                mx, in, filt, filt_scale, a1, bias, out, status);
-            if (int rc = launched("conv_f16x3_kernel"))
-                return rc;
-            TcArgs a2 = a;
-            a2.tile_base = (int)full; a2.ksplit = 2;
-            if (int rc = launch_split(a2, 2 * rem))
-                return rc;
-            return launched("conv_f16x3_kernel");
-        }
+        const long long full = tiles / num_sms() * num_sms(), rem = tiles - full;
+        TcArgs a1 = a;
+        a1.tile_base = 0;
+        conv_f16x3_kernel<false, false><<<(unsigned)full, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_scale, a1, bias, out, status);
+        if (int rc = launched("conv_f16x3_kernel"))
+            return rc;
+        TcArgs a2 = a;
+        a2.tile_base = (int)full; a2.ksplit = cut.rem_split;
+        if (int rc = launch_split(a2, a2.ksplit * rem))
+            return rc;
+        return launched("conv_f16x3_kernel");
     }
     const bool whole = a.merged && a.cg == 1 && a.group != a.Fw; // whole-window groups (TcArgs::row_skip)
 #define SB_LAUNCH_PIXM(M, P) \
-    conv_f16x3_kernel<true, false, true, M, P><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>( \
+    conv_f16x3_kernel<true, false, true, M, P><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(\
         mx, in, filt, filt_scale, a, bias, out, status)
     if (a.pool && whole)
         SB_LAUNCH_PIXM(2, true);
@@ -1645,19 +1734,16 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         SB_LAUNCH_PIXM(1, false);
 #undef SB_LAUNCH_PIXM
     else if (a.pixm)
-        conv_f16x3_kernel<true, false, true><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
-            mx, in, filt, filt_scale, a, bias, out, status);
+        conv_f16x3_kernel<true, false, true><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_scale, a, bias, out, status);
     else if (a.persistent)
-        conv_f16x3_kernel<true, false><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
-            mx, in, filt, filt_scale, a, bias, out, status);
-    else if (a.ksplit == 2)
+        conv_f16x3_kernel<true, false><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_scale, a, bias, out, status);
+    else if (a.ksplit > 1)
     {
         if (int rc = launch_split(a, blocks))
             return rc;
     }
     else
-        conv_f16x3_kernel<false, false><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(
-            mx, in, filt, filt_scale, a, bias, out, status);
+        conv_f16x3_kernel<false, false><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_scale, a, bias, out, status);
     return launched("conv_f16x3_kernel");
 }
 } // namespace
