@@ -207,6 +207,16 @@ int small_b200_conv2d_f32_tf32x3_noalloc(const small_b200_layer *L, const float 
  * DepthwiseConv2D_Bias_ReLU (fused_interface_abstract.hpp:1419). */
 int small_b200_dwconv2d_f32(const small_b200_layer *L, const float *in, const float *filt,
                             const float *bias, float *out, void *stream);
+/* DepthwiseConv2D(+bias)(+activation) followed by a 1x1 Conv2D(+bias)(+activation), a depthwise-separable
+ * block of include/small/models/MobileNetTiny.hpp, as ONE kernel (the reference's fused pairs are the other
+ * way round, Conv2D_ReLU_DepthwiseConv2D_ReLU).  Covered: depthwise 3x3 with stride 1 or 2, up to 384 input
+ * channels; ..._supported() says so, other pairs run as two calls.
+ * The 1x1 filter is re-laid once per set of weights into 2*K*C floats
+ * (small_b200_filter_prepare_dwconv2d_conv2d_f32; opaque). */
+int small_b200_dwconv2d_conv2d_f32_supported(const small_b200_layer *dw, const small_b200_layer *pw);
+int small_b200_filter_prepare_dwconv2d_conv2d_f32(const small_b200_layer *pw, const float *filt, float *prepared, void *stream);
+int small_b200_dwconv2d_conv2d_f32(const small_b200_layer *dw, const small_b200_layer *pw, const float *in, const float *dw_filt,
+                                   const float *dw_bias, const float *pw_prepared, const float *pw_bias, float *out, void *stream);
 /* small::GroupConv2D / PartialGroupConv2D<FloatBuffer> (:1265, :1402): `groups` independent
  * convolutions, each from L->C input channels to L->K output channels (the reference's
  * interface passes its input_channels argument for both).  Layouts of the loop nest with

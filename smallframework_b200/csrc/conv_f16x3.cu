@@ -58,24 +58,6 @@ constexpr int X_SLOTS_MAX = 3;
 constexpr int BOX_PX = 32; // widest box of a TMA load: 256 elements of 8 bytes
 constexpr int SCALE_RING = 16; // patches whose block scale is remembered: slots + unflushed accumulator buffers, rounded up
 
-// Division of a non-negative int below 2^31 by a divisor fixed per launch: one multiply-high, an add and a
-// shift instead of the two dozen instructions of a 32-bit division.  Every role decodes a tile per tile and
-// the accumulation warps turn a GEMM column into a pixel with a division by the patch width; these run on the
-// schedulers the MMA-issuing threads need.
-struct FastDiv
-{
-    uint32_t mul, shift;
-    __host__ void set(int d)
-    {
-        uint32_t s = 0;
-        while ((1ull << s) < (unsigned long long)d)
-            ++s;
-        shift = s;
-        mul = (uint32_t)((((1ull << 32) * ((1ull << s) - (unsigned long long)d)) / (unsigned long long)d) + 1);
-    }
-    __device__ __forceinline__ int div(int x) const { return (int)((__umulhi((uint32_t)x, mul) + (uint32_t)x) >> shift); }
-};
-
 struct TcArgs
 {
     int N, C, K, H, W, Ho, Wo, Fh, Fw, pad_t, pad_l;

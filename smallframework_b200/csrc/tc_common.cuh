@@ -29,6 +29,23 @@ int make_tensor_map(CUtensorMap *map, CUtensorMapDataType dt, int rank, const vo
                     CUtensorMapSwizzle swizzle);
 
 #ifdef __CUDACC__
+// Division of a non-negative int below 2^31 by a divisor fixed per launch: one multiply-high, an add and a
+// shift instead of the two dozen instructions of a 32-bit division.  Tiles and
+// pixels are decoded on the schedulers the MMA-issuing threads need.
+struct FastDiv
+{
+    uint32_t mul, shift;
+    __host__ void set(int d)
+    {
+        uint32_t s = 0;
+        while ((1ull << s) < (unsigned long long)d)
+            ++s;
+        shift = s;
+        mul = (uint32_t)((((1ull << 32) * ((1ull << s) - (unsigned long long)d)) / (unsigned long long)d) + 1);
+    }
+    __device__ __forceinline__ int div(int x) const { return (int)((__umulhi((uint32_t)x, mul) + (uint32_t)x) >> shift); }
+};
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -180,6 +197,14 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, i
                  ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4),
                  "r"(smem_u32(bar))
                  : "memory");
+}
+
+// One lane of the (converged) warp; the compiler keeps what surrounds it uniform.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
 }
 
 // ---- tcgen05 ------------------------------------------------------------------------------

@@ -319,7 +319,7 @@ class Chain:
     tensors at the two ends."""
 
     def __init__(self, layers, batch, dtype="f32", device="cuda", tensor_core="auto", fuse_pool=True,
-                 fuse_u8=True):
+                 fuse_u8=True, fuse_dw=True):
         """tensor_core: "auto" = fp32 convolutions run on the tensor cores where the library
         prefers them there (small_b200_conv2d_f32_tf32x3_preferred); True = every covered
         layer; False = CUDA cores only.  fuse_pool: a CUDA-core convolution followed by a 2x2
@@ -328,7 +328,9 @@ class Chain:
         producer and enqueue_layer() does nothing for it.  fuse_u8: a uint8 convolution followed by a
         3x3 depthwise convolution (the reference's Conv2D_ReLU_DepthwiseConv2D_ReLU pairing), or by the
         global average pool and the dense layer that end the keyword-spotting network, runs as one kernel
-        where the library covers the shapes; the absorbed layers are entered in `fused_into` likewise."""
+        where the library covers the shapes; the absorbed layers are entered in `fused_into` likewise.
+        fuse_dw: an fp32 depthwise convolution followed by a 1x1 convolution (a depthwise-separable block) runs as
+        one kernel where the library covers the pair and tensor_core allows it."""
         self.layers, self.batch, self.dtype = layers, batch, dtype
         self.fuse_pool = fuse_pool
         self.tensor_core = tensor_core
@@ -361,11 +363,28 @@ class Chain:
             for key in ("src", "dst"):
                 if key in L and L[key] not in self.named:
                     self.named[L[key]] = torch.zeros(max_act, dtype=self.tdtype, device=self.dev)
-        # tensor-core fp32 path: filters re-laid once (hi + lo copies)
+        self.fused_into = {}  # index of an absorbed layer -> index of the layer whose kernel computes it
+        # depthwise-separable blocks: the 1x1 filter re-laid once
+        self.blocks = {}
+        if dtype == "f32" and tensor_core and fuse_dw:
+            for i in range(len(layers) - 1):
+                L, Pn = layers[i], layers[i + 1]
+                if L["op"] != "dwconv" or Pn["op"] != "conv" or "src" in L or "src" in Pn:
+                    continue
+                dd, dp = self._desc(L, padded(L["C"])), self._desc(Pn, padded(Pn["C"]))
+                if not lib().small_b200_dwconv2d_conv2d_f32_supported(C.byref(dd), C.byref(dp)):
+                    continue
+                wt = self.params[i + 1][0]
+                prep = torch.empty(2 * wt.numel(), dtype=torch.float32, device=self.dev)
+                check(lib().small_b200_filter_prepare_dwconv2d_conv2d_f32(C.byref(dp), wt.data_ptr(), prep.data_ptr(),
+                                                                          torch.cuda.current_stream().cuda_stream))
+                self.blocks[i] = prep
+                self.fused_into[i + 1] = i
+        # tensor-core fp32 path: filters re-laid once (hi + lo words)
         self.prepared = [None] * len(layers)
         if dtype == "f32" and tensor_core:
             for i, L in enumerate(layers):
-                if L["op"] != "conv" or (i == 0 and L["C"] % CB != 0):
+                if L["op"] != "conv" or (i == 0 and L["C"] % CB != 0) or i in self.fused_into:
                     continue
                 d = self._desc(L, padded(L["C"]))
                 # "auto": the library's own choice (the C++ platform headers ask the same function)
@@ -379,11 +398,10 @@ class Chain:
                                                              torch.cuda.current_stream().cuda_stream))
                 self.prepared[i] = prep
             torch.cuda.synchronize()
-        self.fused_into = {}  # index of a max pool -> index of the convolution that absorbs it
         if dtype == "f32" and fuse_pool:
             for i in range(len(layers) - 1):
                 L, Pn = layers[i], layers[i + 1]
-                if L["op"] != "conv" or Pn["op"] != "maxpool" or "src" in L:
+                if L["op"] != "conv" or Pn["op"] != "maxpool" or "src" in L or i in self.fused_into:
                     continue
                 dc = self._desc(L, L["C"] if i == 0 else padded(L["C"]))
                 dp = self._desc(Pn, padded(Pn["C"]))
@@ -465,6 +483,10 @@ class Chain:
                                                  p(bs), p(dst), stream))
         elif L["op"] == "conv":
             check(getattr(l, f"small_b200_conv2d_{sfx}")(C.byref(d), p(src), p(wt), p(bs), p(dst), stream))
+        elif L["op"] == "dwconv" and i in self.blocks:
+            dp = self._desc(self.layers[i + 1], padded(self.layers[i + 1]["C"]))
+            check(l.small_b200_dwconv2d_conv2d_f32(C.byref(d), C.byref(dp), p(src), p(wt), p(bs), p(self.blocks[i]),
+                                                   p(self.params[i + 1][1]), p(dst), stream))
         elif L["op"] == "dwconv":
             check(getattr(l, f"small_b200_dwconv2d_{sfx}")(C.byref(d), p(src), p(wt), p(bs), p(dst), stream))
         elif L["op"] == "maxpool":
