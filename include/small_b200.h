@@ -207,13 +207,26 @@ int small_b200_conv2d_f32_tf32x3_noalloc(const small_b200_layer *L, const float 
  * DepthwiseConv2D_Bias_ReLU (fused_interface_abstract.hpp:1419). */
 int small_b200_dwconv2d_f32(const small_b200_layer *L, const float *in, const float *filt,
                             const float *bias, float *out, void *stream);
+/* The same convolution for layers of at most twelve million multiply-adds, where latency is all there is:
+ * the reduction is shared by the threads of many CTAs (its own order of additions).  ..._preferred() says
+ * whether a layer is that small (the executors ask it before the tensor-core choice); other layers run
+ * small_b200_conv2d_f32. */
+int small_b200_conv2d_f32_small_preferred(const small_b200_layer *L);
+int small_b200_conv2d_f32_small(const small_b200_layer *L, const float *in, const float *filt, const float *bias, float *out, void *stream);
+/* AveragePool2D over the whole image, a dense layer (1x1 convolution, + bias, + activation) on the averages
+ * and, with softmax != 0, SoftMax over its K outputs: the tail of a classifier (Resnet8Tiny.hpp,
+ * MobileNetTiny.hpp) as ONE kernel.  Covered: up to 2048 channels and 256 outputs. */
+int small_b200_avgpool_dense_f32_supported(const small_b200_layer *pool, const small_b200_layer *dense);
+int small_b200_avgpool_dense_f32(const small_b200_layer *pool, const small_b200_layer *dense, int32_t softmax, const float *in,
+                                 const float *filt, const float *bias, float *out, void *stream);
 /* DepthwiseConv2D(+bias)(+activation) followed by a 1x1 Conv2D(+bias)(+activation), a depthwise-separable
  * block of include/small/models/MobileNetTiny.hpp, as ONE kernel (the reference's fused pairs are the other
  * way round, Conv2D_ReLU_DepthwiseConv2D_ReLU).  Covered: depthwise 3x3 with stride 1 or 2, up to 384 input
- * channels; ..._supported() says so, other pairs run as two calls.
- * The 1x1 filter is re-laid once per set of weights into 2*K*C floats
+ * channels; ..._supported() says so, other pairs run as two calls, and ..._preferred() where two calls are the
+ * shorter way.  The 1x1 filter is re-laid once per set of weights into 2*K*C floats
  * (small_b200_filter_prepare_dwconv2d_conv2d_f32; opaque). */
 int small_b200_dwconv2d_conv2d_f32_supported(const small_b200_layer *dw, const small_b200_layer *pw);
+int small_b200_dwconv2d_conv2d_f32_preferred(const small_b200_layer *dw, const small_b200_layer *pw);
 int small_b200_filter_prepare_dwconv2d_conv2d_f32(const small_b200_layer *pw, const float *filt, float *prepared, void *stream);
 int small_b200_dwconv2d_conv2d_f32(const small_b200_layer *dw, const small_b200_layer *pw, const float *in, const float *dw_filt,
                                    const float *dw_bias, const float *pw_prepared, const float *pw_bias, float *out, void *stream);

@@ -74,7 +74,12 @@ SIGNATURES = {
     "small_b200_conv2d_f32_tf32x3": [_LP, _VP, _VP, _VP, _VP, _VP],
     "small_b200_conv2d_f32_tf32x3_noalloc": [_LP, _VP, _VP, _VP, _VP, _VP],
     "small_b200_dwconv2d_f32": [_LP, _VP, _VP, _VP, _VP, _VP],
+    "small_b200_conv2d_f32_small_preferred": [_LP],
+    "small_b200_conv2d_f32_small": [_LP, _VP, _VP, _VP, _VP, _VP],
+    "small_b200_avgpool_dense_f32_supported": [_LP, _LP],
+    "small_b200_avgpool_dense_f32": [_LP, _LP, C.c_int32, _VP, _VP, _VP, _VP, _VP],
     "small_b200_dwconv2d_conv2d_f32_supported": [_LP, _LP],
+    "small_b200_dwconv2d_conv2d_f32_preferred": [_LP, _LP],
     "small_b200_filter_prepare_dwconv2d_conv2d_f32": [_LP, _VP, _VP, _VP],
     "small_b200_dwconv2d_conv2d_f32": [_LP, _LP, _VP, _VP, _VP, _VP, _VP, _VP, _VP],
     "small_b200_groupconv2d_f32": [_LP, C.c_int32, _VP, _VP, _VP, _VP, _VP],

@@ -15,6 +15,12 @@
 
 #include "common.cuh"
 
+namespace sb
+{
+bool conv_small_preferred(const small_b200_layer *L); // conv_small_f32.cu
+int conv_small_f32(const small_b200_layer *L, const float *in, const float *filt, const float *bias, float *out, cudaStream_t st);
+} // namespace sb
+
 namespace
 {
 using namespace sb;
@@ -640,6 +646,12 @@ int conv2d_f32_impl(const small_b200_layer *L, int pool, const float *in, const 
     if (a.N == 0 || a.Ho == 0 || a.Wo == 0)
         return SMALL_B200_OK;
     cudaStream_t st = as_stream(stream);
+
+    // Small layers, except where the pair with a following max pool is one staged kernel (it and the two calls give the same
+    // bits, which callers may rely on; executors ask small_b200_conv2d_f32_small_preferred() themselves).
+    const bool poolable = a.sh == 1 && L->stride == 1 && L->C >= CB && a.K % 32 == 0 && a.Ho % 2 == 0 && a.Wo % 2 == 0;
+    if (!pool && !poolable && conv_small_preferred(L))
+        return conv_small_f32(L, in, filt, bias, out, st);
 
     if (L->C < CB)
     {

@@ -25,6 +25,12 @@
 // 3072 cycles per tile against 2980 for the tile's bytes).
 #include "tc_common.cuh"
 
+namespace sb
+{
+bool conv_small_preferred(const small_b200_layer *L); // conv_small_f32.cu
+double conv_small_us(const small_b200_layer *L);
+} // namespace sb
+
 namespace
 {
 using namespace sb;
@@ -583,6 +589,15 @@ int small_b200_dwconv2d_conv2d_f32_supported(const small_b200_layer *dw, const s
     DpArgs a;
     int R;
     return plan_dwpw(dw, pw, a, R) ? 1 : 0;
+}
+
+// Layers of a small batch: where the depthwise layer (3 to 4 us) and the latency kernel for the 1x1 layer together stay below
+// this kernel's 6 (16 channels) to 13 us (256), two launches are the shorter way.
+int small_b200_dwconv2d_conv2d_f32_preferred(const small_b200_layer *dw, const small_b200_layer *pw)
+{
+    if (!small_b200_dwconv2d_conv2d_f32_supported(dw, pw))
+        return 0;
+    return conv_small_preferred(pw) && 3.5 + conv_small_us(pw) < 6.5 + 0.03 * dw->C ? 0 : 1;
 }
 
 int small_b200_filter_prepare_dwconv2d_conv2d_f32(const small_b200_layer *pw, const float *filt, float *prepared, void *stream)

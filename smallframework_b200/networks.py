@@ -329,7 +329,9 @@ class Chain:
         3x3 depthwise convolution (the reference's Conv2D_ReLU_DepthwiseConv2D_ReLU pairing), or by the
         global average pool and the dense layer that end the keyword-spotting network, runs as one kernel
         where the library covers the shapes; the absorbed layers are entered in `fused_into` likewise.
-        fuse_dw: an fp32 depthwise convolution followed by a 1x1 convolution (a depthwise-separable block) runs as
+        "auto" also runs layers of a few million multiply-adds in the latency kernel
+        (small_b200_conv2d_f32_small_preferred) and a global average pool with the dense layer and the softmax behind it as
+        one kernel.  fuse_dw: an fp32 depthwise convolution followed by a 1x1 convolution (a depthwise-separable block) runs as
         one kernel where the library covers the pair and tensor_core allows it."""
         self.layers, self.batch, self.dtype = layers, batch, dtype
         self.fuse_pool = fuse_pool
@@ -364,6 +366,14 @@ class Chain:
                 if key in L and L[key] not in self.named:
                     self.named[L[key]] = torch.zeros(max_act, dtype=self.tdtype, device=self.dev)
         self.fused_into = {}  # index of an absorbed layer -> index of the layer whose kernel computes it
+        # layers too small for the tensor cores' fixed costs, and the tail of a classifier as one kernel
+        self.small, self.tails = set(), set()
+        if dtype == "f32" and tensor_core == "auto":
+            for i, L in enumerate(layers):
+                cin = L["C"] if i == 0 else padded(L["C"])
+                if L["op"] == "conv" and lib().small_b200_conv2d_f32_small_preferred(C.byref(self._desc(L, cin))):
+                    self.small.add(i)
+            self._find_tails()
         # depthwise-separable blocks: the 1x1 filter re-laid once
         self.blocks = {}
         if dtype == "f32" and tensor_core and fuse_dw:
@@ -372,7 +382,9 @@ class Chain:
                 if L["op"] != "dwconv" or Pn["op"] != "conv" or "src" in L or "src" in Pn:
                     continue
                 dd, dp = self._desc(L, padded(L["C"])), self._desc(Pn, padded(Pn["C"]))
-                if not lib().small_b200_dwconv2d_conv2d_f32_supported(C.byref(dd), C.byref(dp)):
+                pick = lib().small_b200_dwconv2d_conv2d_f32_preferred if tensor_core == "auto" else \
+                    lib().small_b200_dwconv2d_conv2d_f32_supported
+                if not pick(C.byref(dd), C.byref(dp)):
                     continue
                 wt = self.params[i + 1][0]
                 prep = torch.empty(2 * wt.numel(), dtype=torch.float32, device=self.dev)
@@ -384,7 +396,7 @@ class Chain:
         self.prepared = [None] * len(layers)
         if dtype == "f32" and tensor_core:
             for i, L in enumerate(layers):
-                if L["op"] != "conv" or (i == 0 and L["C"] % CB != 0) or i in self.fused_into:
+                if L["op"] != "conv" or (i == 0 and L["C"] % CB != 0) or i in self.fused_into or i in self.small:
                     continue
                 d = self._desc(L, padded(L["C"]))
                 # "auto": the library's own choice (the C++ platform headers ask the same function)
@@ -401,7 +413,7 @@ class Chain:
         if dtype == "f32" and fuse_pool:
             for i in range(len(layers) - 1):
                 L, Pn = layers[i], layers[i + 1]
-                if L["op"] != "conv" or Pn["op"] != "maxpool" or "src" in L or i in self.fused_into:
+                if L["op"] != "conv" or Pn["op"] != "maxpool" or "src" in L or i in self.fused_into or i in self.small:
                     continue
                 dc = self._desc(L, L["C"] if i == 0 else padded(L["C"]))
                 dp = self._desc(Pn, padded(Pn["C"]))
@@ -439,6 +451,25 @@ class Chain:
         self.kernels_per_step = 0
         self._descs = []
 
+    def _find_tails(self):
+        """Average pool over the whole image -> dense layer [-> softmax], where nobody else reads what lies between."""
+        layers, uses = self.layers, {}
+        for L in layers:
+            if "src" in L:
+                uses[L["src"]] = uses.get(L["src"], 0) + 1
+        feeds = lambda a, b: ("src" in a) == ("src" in b) and ("src" not in a or (a["dst"] == b["src"] and uses[b["src"]] == 1))
+        for i in range(len(layers) - 1):
+            P, D = layers[i], layers[i + 1]
+            if P["op"] != "avgpool" or D["op"] != "conv" or not feeds(P, D):
+                continue
+            dp, dd = self._desc(P, padded(P["C"])), self._desc(D, padded(D["C"]))
+            if not lib().small_b200_avgpool_dense_f32_supported(C.byref(dp), C.byref(dd)):
+                continue
+            self.tails.add(i)
+            self.fused_into[i + 1] = i
+            if i + 2 < len(layers) and layers[i + 2]["op"] == "softmax" and feeds(D, layers[i + 2]):
+                self.fused_into[i + 2] = i
+
     def absorbed(self, i):
         """Indices of the layers that run inside layer i's kernel, in order."""
         return sorted(k for k, v in self.fused_into.items() if v == i)
@@ -462,7 +493,14 @@ class Chain:
         if i in self.fused_into:
             return  # computed by its producer
         follow = self.absorbed(i)
-        if L["op"] == "conv" and follow and self.dtype == "u8":
+        if i in self.tails:
+            D = self.layers[i + 1]
+            w2, b2 = self.params[i + 1]
+            check(l.small_b200_avgpool_dense_f32(C.byref(d), C.byref(self._desc(D, padded(D["C"]))), int(len(follow) > 1), p(src),
+                                                 p(w2), p(b2), p(dst), stream))
+        elif L["op"] == "conv" and i in self.small:
+            check(l.small_b200_conv2d_f32_small(C.byref(d), p(src), p(wt), p(bs), p(dst), stream))
+        elif L["op"] == "conv" and follow and self.dtype == "u8":
             ds = [self._desc(self.layers[k], padded(self.layers[k]["C"])) for k in follow]
             w2, b2 = self.params[follow[-1]]
             if len(follow) == 1:
@@ -512,8 +550,9 @@ class Chain:
             if "src" in L:
                 if L["op"] == "alias":
                     names[L["dst"]] = names[L["src"]]
-                plan.append((names[L["src"]], names[L["dst"]]))
-                src = names[L["dst"]]
+                last = self.layers[(self.absorbed(i) or [i])[-1]]
+                plan.append((names[L["src"]], names[last["dst"]]))
+                src = names[last["dst"]]
                 continue
             dst = self.bufs[1] if src is self.bufs[0] else self.bufs[0]
             plan.append((src, dst))
