@@ -182,13 +182,25 @@ class DarknetModel:
                                                                    None, 0.0, packed.data_ptr(), bias.data_ptr(), st))
             d = self._desc(r)
             prepared = None
-            use_tc = tensor_core and self.lib.small_b200_conv2d_f32_tf32x3_supported(C.byref(d)) and (
+            small = tensor_core == "auto" and self.lib.small_b200_conv2d_f32_small_preferred(C.byref(d))
+            use_tc = tensor_core and not small and self.lib.small_b200_conv2d_f32_tf32x3_supported(C.byref(d)) and (
                 tensor_core is True or self.lib.small_b200_conv2d_f32_tf32x3_preferred(C.byref(d)))
             if use_tc:
                 prepared = torch.empty(2 * packed.numel(), device=self.dev)
                 check(self.lib.small_b200_filter_prepare_tf32x3(C.byref(d), packed.data_ptr(), prepared.data_ptr(), st))
-            self.params.append((packed, bias, prepared))
+            self.params.append((packed, bias, prepared, small))
+        self._find_pools(tensor_core)
         self.stream.synchronize()
+        # The whole network as one CUDA graph, recorded now on a stream of its own (one launch per inference instead of
+        # some two dozen calls); a call made while somebody else records this stream enqueues the layers one by one.
+        self.graph = None
+        if all(r.get("scale", 2) == 2 for r in self.plan):  # other scales are inference()'s to refuse
+            side, self.graph = torch.cuda.Stream(device=self.dev), C.c_void_p()
+            check(self.lib.small_b200_graph_begin(side.cuda_stream))
+            try:
+                self._enqueue(side.cuda_stream)
+            finally:
+                check(self.lib.small_b200_graph_end(side.cuda_stream, C.byref(self.graph)))
 
     def _desc(self, r):
         return self.Layer(self.batch, r["Cp"], r["Kp"], r["H"], r["W"], r["size"], r["size"], r["stride"], *r["pads"],
@@ -199,20 +211,62 @@ class DarknetModel:
             return self.x
         return self.out[i] if self.out[i] is not None else self._src(self.plan[i]["parents"][0])
 
+    def _find_pools(self, tensor_core):
+        """Convolutions whose output only a following 2x2 max pool reads run with it as one kernel where the library covers
+        the pair: self.pooled[convolution] = pool."""
+        self.pooled, readers = {}, {}
+        for r in self.plan:
+            for p in r["parents"]:
+                readers[p] = readers.get(p, 0) + 1
+        for i, r in enumerate(self.plan[:-1]):
+            nxt = self.plan[i + 1]
+            if r["op"] != "conv" or nxt["op"] != "maxpool" or nxt["parents"] != [i] or readers[i] != 1:
+                continue
+            _, _, prepared, small = self.params[i]
+            dc, dp = self._desc(r), self._desc(nxt)
+            covered = self.lib.small_b200_conv2d_maxpool_f32_tf32x3_supported if prepared is not None else \
+                self.lib.small_b200_conv2d_maxpool_f32_supported
+            if tensor_core == "auto" and not small and covered(C.byref(dc), C.byref(dp)):
+                self.pooled[i] = i + 1
+
     def inference(self, x=None):
         """Enqueues the network; returns the device tensors of the yolo layers, each
         [batch][predictions][5 + classes]."""
-        l, check, st = self.lib, self.check, self.stream.cuda_stream
         if x is not None:
             self.x.copy_(self.torch.as_tensor(x, device=self.dev).reshape(-1))
-        heads = []
+        if self.graph is None or self.torch.cuda.is_current_stream_capturing():
+            self._enqueue(self.stream.cuda_stream)
+        else:
+            self.check(self.lib.small_b200_graph_launch(self.graph, self.stream.cuda_stream))
+        return [self.out[i].view(self.batch, r["preds"], r["classes"] + 5) for i, r in enumerate(self.plan) if r["op"] == "yolo"]
+
+    def __del__(self):
+        try:
+            if self.graph:
+                self.lib.small_b200_graph_destroy(self.graph)
+        except Exception:
+            pass
+
+    def _enqueue(self, st):
+        l, check = self.lib, self.check
+        done = set(self.pooled.values())
         for i, r in enumerate(self.plan):
             src = [self._src(p) for p in r["parents"]]
             dst = self.out[i]
+            if i in done:
+                continue  # its convolution wrote it
             if r["op"] == "conv":
-                packed, bias, prepared = self.params[i]
+                packed, bias, prepared, small = self.params[i]
                 d = self._desc(r)
-                if prepared is not None:
+                if i in self.pooled:
+                    dp, dst = self._desc(self.plan[self.pooled[i]]), self.out[self.pooled[i]]
+                    fn = l.small_b200_conv2d_maxpool_f32 if prepared is None else l.small_b200_conv2d_maxpool_f32_tf32x3
+                    check(fn(C.byref(d), C.byref(dp), src[0].data_ptr(), (packed if prepared is None else prepared).data_ptr(),
+                             bias.data_ptr(), dst.data_ptr(), st))
+                elif small:
+                    check(l.small_b200_conv2d_f32_small(C.byref(d), src[0].data_ptr(), packed.data_ptr(), bias.data_ptr(),
+                                                        dst.data_ptr(), st))
+                elif prepared is not None:
                     check(l.small_b200_conv2d_f32_tf32x3(C.byref(d), src[0].data_ptr(), prepared.data_ptr(), bias.data_ptr(),
                                                          dst.data_ptr(), st))
                 else:
@@ -238,8 +292,6 @@ class DarknetModel:
                 check(l.small_b200_yolo_decode_f32(self.batch, r["Cp"], r["H"], r["W"], len(r["anchors"]), r["classes"],
                                                    float(r["img"] // r["H"]), a.ctypes.data, src[0].data_ptr(),
                                                    dst.data_ptr(), st))
-                heads.append(dst.view(self.batch, r["preds"], r["classes"] + 5))
-        return heads
 
     def detect(self, x=None, confidence_threshold=0.25, iou_threshold=0.45, max_candidates=16384, max_detections=1024):
         """Darknet::process_outputs per image: numpy arrays [n, 7] of x, y, w, h, objectness, class score, class id."""
