@@ -549,7 +549,11 @@ class Chain:
                 continue
             if "src" in L:
                 if L["op"] == "alias":
-                    names[L["dst"]] = names[L["src"]]
+                    # The two names trade buffers where the source is written again before anyone reads it: a layer from
+                    # dst to src would otherwise work in place, with some CTAs writing what others still have to read.
+                    kept = next((M.get("src") == L["src"] or bool(M.get("accumulate")) for M in self.layers[i + 1:]
+                                 if L["src"] in (M.get("src"), M.get("dst"))), False)
+                    names[L["dst"]], names[L["src"]] = names[L["src"]], names[L["src"] if kept else L["dst"]]
                 last = self.layers[(self.absorbed(i) or [i])[-1]]
                 plan.append((names[L["src"]], names[last["dst"]]))
                 src = names[last["dst"]]

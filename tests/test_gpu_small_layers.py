@@ -9,7 +9,7 @@ from oracle.bindings import same_pads, shape
 from smallframework_b200 import interface as S
 from smallframework_b200 import packing as P
 from smallframework_b200._lib import Layer, check, lib
-from tests.gpu_util import CB, fbuf, oracle_conv_batch, rel_max_err
+from tests.gpu_util import CB, fbuf, oracle_conv_batch, oracle_layer, rel_max_err
 
 CASES = [
     # C, K, H, W, Fh, Fw, stride, pads, batch
@@ -79,3 +79,29 @@ def test_layers_that_are_not_small():
     pool = Layer(1, 64, 64, 8, 8, 4, 4, 1, 0, 0, 0, 0, 0, 0, 0.0, 0, 0, 0, 0, 0, 0)
     dense = Layer(1, 64, 16, 1, 1, 1, 1, 1, 0, 0, 0, 0, 0, 0, 0.0, 0, 0, 0, 0, 0, 0)
     assert not lib().small_b200_avgpool_dense_f32_supported(C.byref(pool), C.byref(dense))  # not the whole image
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch", [1, 21])
+def test_residual_chain_never_works_in_place(oracle, batch):
+    """A shortcut convolution behind an alias reads one buffer and writes another, and the chain gives what the oracle gives."""
+    import torch
+    from smallframework_b200 import networks
+    layers = networks.resnet8(seed=0)
+    chain = networks.Chain(layers, batch, "f32")
+    assert all(io is None or L["op"] == "alias" or io[0].data_ptr() != io[1].data_ptr() for L, io in zip(layers, chain.io_plan()))
+    x = np.random.default_rng(batch).uniform(0, 1, (batch, chain.x.numel() // batch)).astype(np.float32)
+    chain.x.copy_(torch.from_numpy(x.reshape(-1)))
+    torch.cuda.synchronize()
+    chain.enqueue()
+    torch.cuda.synchronize()
+    got = chain.y.cpu().numpy().reshape(batch, -1)
+    for n in (0, batch // 2, batch - 1):
+        named, cur = {"in": x[n]}, None
+        for i, L in enumerate(layers):
+            if L["op"] == "alias":
+                named[L["dst"]] = named[L["src"]]
+                continue
+            seed = named[L["dst"]].copy() if L.get("accumulate") else None
+            cur = named[L["dst"]] = oracle_layer(oracle, L, i == 0, named[L["src"]], seed=seed)
+        assert rel_max_err(got[n, :cur.size], cur) <= 2e-5
