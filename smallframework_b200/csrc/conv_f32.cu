@@ -19,6 +19,8 @@ namespace sb
 {
 bool conv_small_preferred(const small_b200_layer *L); // conv_small_f32.cu
 int conv_small_f32(const small_b200_layer *L, const float *in, const float *filt, const float *bias, float *out, cudaStream_t st);
+bool conv_gather_preferred(const small_b200_layer *L); // conv_gather_f32.cu
+int conv_gather_f32(const small_b200_layer *L, const float *in, const float *filt, const float *bias, float *out, cudaStream_t st);
 } // namespace sb
 
 namespace
@@ -652,6 +654,9 @@ int conv2d_f32_impl(const small_b200_layer *L, int pool, const float *in, const 
     const bool poolable = a.sh == 1 && L->stride == 1 && L->C >= CB && a.K % 32 == 0 && a.Ho % 2 == 0 && a.Wo % 2 == 0;
     if (!pool && !poolable && conv_small_preferred(L))
         return conv_small_f32(L, in, filt, bias, out, st);
+    // Strided windows (stride 1 has the tensor-core entry points of its own, for callers that ask for them).
+    if (!pool && (a.sh != 1 || L->stride != 1) && conv_gather_preferred(L))
+        return conv_gather_f32(L, in, filt, bias, out, st);
 
     if (L->C < CB)
     {
