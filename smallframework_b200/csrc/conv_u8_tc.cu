@@ -90,6 +90,9 @@ struct PwArgs
     int tiles;   // ceil(P / 128)
     int nblocks; // K / NT
     int bulk;    // 1: a channel block of a tile is one contiguous run of pixels (plain bulk copies)
+    int images;  // images per tile where one leaves half of it empty or more, else 0
+    int N;
+    FastDiv by_tiles, by_P;
     long long out_pix_stride, out_plane_stride, out_group_stride; // bytes
     int zero_in, zero_filt, lshift, rshift, mult, k_zero;
 };
@@ -157,8 +160,16 @@ pw_u8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const PwArgs a, const
                 ok = mbar_wait(&done_bar[s], ((i >> 1) - 1) & 1, status, 3);
             if (!ok)
                 break;
-            const int tile = item % a.tiles, g = item / a.tiles;
-            if (a.bulk)
+            const int g = a.by_tiles.div(item), tile = item - g * a.tiles;
+            if (a.images)
+            {
+                // small images: a row of the copy is a channel block of an image (P * 16 contiguous bytes), so a channel block of
+                // the tile is the images' pixels one after the other; rows past the batch read as zero
+                mbar_expect_tx(&full_bar[s], (uint32_t)(a.cbs * a.images * a.P * CB));
+                for (int cb = 0; cb < a.cbs; ++cb)
+                    tma_load_3d(sA + (size_t)s * a_bytes + (size_t)cb * TILE_M * CB, &map_a, 0, tile * a.images, cb, &full_bar[s]);
+            }
+            else if (a.bulk)
             {
                 // [cb][pixel][16 B] in memory as in shared memory: one run per channel block (a tiled
                 // copy with 16-byte rows moves a row every few cycles and set the pace of this kernel);
@@ -204,6 +215,7 @@ pw_u8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const PwArgs a, const
     else if (warp < PW_EPI_WARPS)
     {
         const int px_t = (warp & 3) * 32 + lane;      // this thread's pixel of the tile = its TMEM lane
+        const int image = a.images ? a.by_P.div(px_t) : 0;
         constexpr int CPW = NT >= 32 ? NT / 2 : NT;  // output channels per warp group
         const int c_begin = (warp >> 2) * CPW;
         // per-channel constants: k_zero + bias + C*zI*zF + zI * (column sum of the filter)
@@ -227,7 +239,7 @@ pw_u8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const PwArgs a, const
         for (int item = blockIdx.x; item < total && ok; item += gridDim.x, ++i)
         {
             const int s = i & 1;
-            const int tile = item % a.tiles, g = item / a.tiles;
+            const int g = a.by_tiles.div(item), tile = item - g * a.tiles;
             ok = mbar_wait(&full_bar[s], (i >> 1) & 1, status, 6);
             if (!ok)
                 break;
@@ -249,9 +261,10 @@ pw_u8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const PwArgs a, const
             if (!ok)
                 break;
             tc_fence_after_sync();
-            const int p = tile * TILE_M + px_t;
+            const int n = a.images ? tile * a.images + image : g, p = a.images ? px_t - image * a.P : tile * TILE_M + px_t;
+            const bool live = a.images ? image < a.images && n < a.N : p < a.P;
             const int base = a.zero_filt * asum;
-            uint8_t *orow = out + (size_t)g * a.out_group_stride + (size_t)p * a.out_pix_stride;
+            uint8_t *orow = out + (size_t)n * a.out_group_stride + (size_t)p * a.out_pix_stride;
 #pragma unroll
             for (int cc = 0; cc < CPW; cc += 16)
             {
@@ -272,10 +285,8 @@ pw_u8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const PwArgs a, const
                     q[4 * e4 + 3] = (int)r[4 * e4 + 3] + base + cr.w;
                 }
                 const uint4 o = requant_pack16(q, a.lshift, a.rshift, a.mult);
-                if (p < a.P)
-                {
+                if (live)
                     *reinterpret_cast<uint4 *>(orow + (size_t)((nb * NT + c0) / CB) * a.out_plane_stride) = o;
-                }
             }
             // stage s of shared memory and buffer s of tensor memory are free again
             tc_fence_before_sync();
@@ -569,9 +580,26 @@ int conv2d_u8_tensor_core(const small_b200_layer *L, const uint8_t *in, const ui
         a.out_group_stride = (long long)(L->K / CB) * HW * CB;
     }
     a.tiles = (a.P + TILE_M - 1) / TILE_M;
+    CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_UINT8;
+    // Two images and more fit a tile (P <= 64): as many as do, since a tile costs the same (barriers, MMAs, the requantisation
+    // of 128 rows) whatever it holds.  2048 images: 256 -> 256 channels at 3x3 49.8 -> 7.1 us, 128 -> 128 at 6x6 24.0 -> 10.5,
+    // 64 -> 128 at 6x6 23.0 -> 10.0; a single image is where it was.
+    a.images = a.bulk && a.P <= TILE_M / 2 && a.groups > 1 ? TILE_M / a.P : 0;
+    a.N = L->N;
+    if (a.images)
+    {
+        if (a.images > L->N)
+            a.images = L->N;
+        type = CU_TENSOR_MAP_DATA_TYPE_FLOAT64; // pairs of them are pixels; nothing is converted
+        dims[0] = 2 * (uint64_t)HW; dims[1] = (uint64_t)L->N; dims[2] = (uint64_t)cbs;
+        strides[0] = (uint64_t)cbs * HW * CB; strides[1] = (uint64_t)HW * CB;
+        box[0] = 2 * (uint32_t)HW; box[1] = (uint32_t)a.images; box[2] = 1;
+        a.tiles = (L->N + a.images - 1) / a.images;
+        a.groups = 1;
+    }
+    a.by_tiles.set(a.tiles); a.by_P.set(a.P);
     CUtensorMap map;
-    if (int rc = make_tensor_map(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, in, dims, strides, box,
-                                 CU_TENSOR_MAP_SWIZZLE_NONE))
+    if (int rc = make_tensor_map(&map, type, 3, in, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE))
         return rc;
     switch (nt)
     {

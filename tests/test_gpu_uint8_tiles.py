@@ -1,0 +1,80 @@
+"""uint8 kernels that work on tiles of several images or planes, at the edges of their tiles: bit-exact against the oracle."""
+import numpy as np
+import pytest
+
+from oracle.bindings import Quant, same_pads, shape
+from smallframework_b200 import _lib
+from smallframework_b200 import interface as S
+from smallframework_b200 import packing as P
+from tests.gpu_util import CB, qbuf
+from tests.test_gpu_uint8 import _out, _quant
+
+pytestmark = pytest.mark.gpu
+
+DW_CASES = [
+    # C, H, W, pads (None: same), batch
+    (32, 3, 3, None, 70),                # whole planes, an odd number of rows, a last CTA that is not full
+    (128, 6, 6, None, 40),
+    (16, 48, 48, None, 3),               # runs of rows
+    (48, 45, 37, None, 2),               # a short last run with an odd number of rows, a last strip that is not full
+    (16, 1, 1, None, 5),
+    (16, 2, 300, None, 1),
+    (16, 9, 7, (0, 0, 0, 0), 2),
+    (16, 5, 6, (2, 4, 3, 1), 2),         # rows and columns of nothing but padding
+]
+
+
+@pytest.mark.parametrize("case", DW_CASES, ids=lambda c: "C{}_{}x{}_p{}_n{}".format(*c))
+@pytest.mark.parametrize("zp", [(0, -128), (-128, -128), (-113, -121), (-255, -250), (3, -7)], ids=lambda z: "zi{}_zf{}".format(*z))
+def test_depthwise_3x3_tiles(oracle, case, zp):
+    import torch
+    C, H, W, pads, N = case
+    pads = pads or same_pads(H, W, 3, 3, 1)
+    rng = np.random.default_rng(C * H + W + zp[0] + 1000)
+    q = _quant(rng, 9, zp)
+    x = P.pack_activation(rng.integers(0, 256, (N, C, H, W)).astype(np.uint8))
+    w = P.pack_dw_filter(rng.integers(0, 256, (C, 3, 3)).astype(np.uint8))
+    bias = rng.integers(-4096, 4097, C).astype(np.int32)
+    sh = shape(C, C, H, W, 3, 3, 1, pads, CB)
+    ho, wo = sh.out_hw()
+    I, F, O = qbuf(x, zp[0]), qbuf(w, zp[1]), _out(N * C * ho * wo, q)
+    S.DepthwiseConv2D_Bias_Activation(3, 3, 1, *pads, C, H, W, I, F, torch.from_numpy(bias).cuda(), O, batch=N)
+    want = np.stack([oracle.conv2d_u8(sh, q, x[n], w, bias=bias, depthwise=True) for n in range(N)])
+    assert _lib.device_status() == 0
+    assert np.array_equal(O.numpy().reshape(N, -1), want)
+    assert want.min() < want.max()
+
+
+@pytest.mark.parametrize("case", [(32, 16, 8, 8, 5), (256, 256, 3, 3, 31), (64, 128, 6, 6, 8), (128, 32, 1, 2, 130), (96, 48, 5, 13, 4)],
+                         ids=lambda c: "C{}_K{}_{}x{}_n{}".format(*c))
+@pytest.mark.parametrize("zp", [(0, -128), (-113, -121)], ids=lambda z: "zi{}_zf{}".format(*z))
+def test_pointwise_tiles_of_several_images(oracle, case, zp):
+    C, K, H, W, N = case
+    rng = np.random.default_rng(C + K + N)
+    q = _quant(rng, C, zp)
+    x = P.pack_activation(rng.integers(0, 256, (N, C, H, W)).astype(np.uint8))
+    w = P.pack_conv_filter(rng.integers(0, 256, (K, C, 1, 1)).astype(np.uint8))
+    sh = shape(C, K, H, W, 1, 1, 1, (0, 0, 0, 0), CB)
+    I, F, O = qbuf(x, zp[0]), qbuf(w, zp[1]), _out(N * K * H * W, q)
+    S.Conv2D(1, 1, 1, 0, 0, 0, 0, K, C, H, W, I, F, O, batch=N, path="tensor_core")
+    want = np.stack([oracle.conv2d_u8(sh, q, x[n], w) for n in range(N)])
+    assert _lib.device_status() == 0
+    assert np.array_equal(O.numpy().reshape(N, -1), want)
+    assert want.min() < want.max()
+
+
+@pytest.mark.parametrize("hw", [(1, 1), (8, 8), (5, 13), (16, 16), (1, 257)], ids=lambda s: "{}x{}".format(*s))
+def test_global_average_pool_sizes(oracle, hw):
+    H, W = hw
+    C, N = 48, 7
+    rng = np.random.default_rng(H * W)
+    x = rng.integers(0, 256, (N, C, H, W)).astype(np.uint8)
+    x[0] = 255                           # the largest sum
+    x = P.pack_activation(x)
+    rshift = int(np.floor(np.log2(H * W)))
+    q = Quant(0, 0, 0, rshift, min(int(2.0 ** (31 + rshift) / (H * W) * 0.99), (1 << 31) - 1), 0)
+    sh = shape(C, C, H, W, H, W, 1, (0, 0, 0, 0), CB)
+    I, O = qbuf(x, 0), _out(N * C, q)
+    S.AveragePool2D(H, W, 1, 0, 0, 0, 0, C, H, W, I, O, batch=N)
+    want = np.stack([oracle.pool2d_u8(sh, q, x[n], average=True) for n in range(N)])
+    assert np.array_equal(O.numpy().reshape(N, -1), want)
