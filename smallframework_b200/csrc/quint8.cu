@@ -11,6 +11,9 @@
 // buffer between input-channel blocks (q_abstract_layer.hpp:1144), which is why its
 // callers over-allocate outputs four times; nothing of that is needed here.
 #include "common.cuh"
+#include "tc_common.cuh"
+
+#include <algorithm>
 
 namespace
 {
@@ -393,104 +396,221 @@ dwconv_u8_dp4a_kernel(const QArgs a, const uint8_t *__restrict__ in, const uint8
     *reinterpret_cast<uint4 *>(out + o * CB) = requant_pack16(acc, a.lshift, a.rshift, a.mult);
 }
 
-// Depthwise 3x3, stride 1, a row strip per thread: TW neighbouring outputs of one row x 8
-// channels.  The three taps of a kernel COLUMN of one input pixel are transposed once and serve
-// the (up to) three outputs that see this input column through kw = 0, 1, 2, so a strip of TW
-// outputs costs TW + 2 transposes instead of 3 * TW, and the index arithmetic is paid once per
-// strip.  Filter words in shared memory: [cb][half][kw][8 ch] = (w[0][kw], w[1][kw], w[2][kw], 0)
-// as signed bytes.
-template <bool SIGNED_IN, int TW>
-__global__ void __launch_bounds__(256, 3)
-dwconv3x3_u8_rows_kernel(const QArgs a, const uint8_t *__restrict__ in, const uint8_t *__restrict__ filt,
-                         const int32_t *__restrict__ bias, uint8_t *__restrict__ out, int strips, int pad_t, int pad_l)
+// Depthwise 3x3, stride 1, through shared memory.  A tile is whole planes (an image's channel block) where they are small,
+// else a run of rows of one plane; CTAs are persistent and fetch the next tile before they compute one.  Pixels are copied 16
+// bytes a thread (a bulk copy a row took some 50 cycles each, more than all else for rows of 3 or 6 pixels) into a pitch
+// that has room for the padding, which holds the byte -zero_in, whose contribution (a + zero_in) * w is nothing: every tap is
+// inside.  A thread computes 2 rows x TW pixels of 4 channels.  The four rows a kernel column covers for the two output
+// rows are byte-transposed once; against the filter column (w0, w1, w2, 0) they give the upper output, against
+// (0, w0, w1, w2) the lower one, so that a transpose of 8 permutes serves up to 24 sums of products.  Filter bytes are
+// signed, w' = w - 128, and the input stays unsigned:
+//   sum (a + zI)(w + zF) = sum a w' + (128 + zF) sum a + zI sum (w + zF)
+// with the last term in the seed of the requantisation and the second one (SUM_A: another three dp4a a column) only
+// where zF != -128.  The output goes back through shared memory as one bulk copy.
+// What bounds it: the integer pipes (three dp4a, two or three instructions of transposes and loads, four and a half of
+// requantisation per output byte).  Reading strips of a row straight from global memory, 96 bytes apart from lane to lane,
+// was bound by L1 wavefronts, with twice the transposes.  2048 images, us before -> now: 16 channels at 48x48 102 -> 70, 32 at
+// 24x24 52 -> 36, 64 at 12x12 29 -> 22, 128 at 6x6 16.5 -> 13.6, 256 at 3x3 9.2 -> 10.9 (half the rows of its last pairs
+// are nothing); a whole MobileNet's 13 layers 330 -> 285.
+// TW is odd: eight strips, TW * 16 bytes apart, times four quarters of a pixel then touch all 32 banks.
+constexpr int DW_THREADS = 256;
+struct DwTile
 {
-    extern __shared__ __align__(16) unsigned sw[]; // [cb][half][kw][8]
-    const int cbs = a.C / CB;
-    for (int i = threadIdx.x; i < cbs * 48; i += blockDim.x)
+    int N, cbs, H, W, Ho, Wo, pad_t, pad_l;
+    int planes;    // planes per tile (more than one only when a tile covers all rows)
+    int rows, row_tiles; // output rows per tile (even, or all of them), tiles down a plane
+    int strips, pairs, pitch, in_rows; // pitch and in_rows in pixels and rows of shared memory
+    int zero_in, sum_a;  // sum_a: 128 + zero_filt
+    int lshift, rshift, mult, k_zero;
+    int tiles;
+    unsigned in_bytes, out_bytes, out_at, w_at; // bytes of a stage; offsets
+    FastDiv by_row_tiles, by_cbs, by_strips, by_pairs, by_pitch, by_in_rows, by_copy_rows, by_W;
+};
+
+template <int TW, bool SUM_A>
+__global__ void __launch_bounds__(DW_THREADS, 3)
+dwconv3x3_u8_tile_kernel(const DwTile a, const uint8_t *__restrict__ in, const uint8_t *__restrict__ filt,
+                         const int32_t *__restrict__ bias, uint8_t *__restrict__ out)
+{
+    extern __shared__ __align__(128) uint8_t smem[]; // [stage][plane][in_rows][pitch][16], [stage][plane][rows][Wo][16], filter
+    const int tid = threadIdx.x, first = blockIdx.x, step = gridDim.x;
+    // padding: columns, and the rows that are padding in every tile, once for both stages
+    const unsigned pad = (unsigned)(-a.zero_in & 255) * 0x01010101u;
+    const bool whole = a.row_tiles == 1;
+    for (int st = 0; st < 2 && first + st * step < a.tiles; ++st)
+        for (int i = tid; i < a.planes * a.in_rows * a.pitch; i += DW_THREADS)
+        {
+            const int lr = a.by_pitch.div(i), x = i - lr * a.pitch - a.pad_l, r = lr - a.by_in_rows.div(lr) * a.in_rows - a.pad_t;
+            if (x < 0 || x >= a.W || (whole && (r < 0 || r >= a.H)))
+                *reinterpret_cast<uint4 *>(smem + st * a.in_bytes + (size_t)i * CB) = make_uint4(pad, pad, pad, pad);
+        }
+    // per channel block [kw][16] words (w0, w1, w2, 0), then [16] seeds
+    unsigned *words = reinterpret_cast<unsigned *>(smem + a.w_at);
+    for (int i = tid; i < a.cbs * CB; i += DW_THREADS)
     {
-        const int j = i % 8, kw = (i / 8) % 3, half = (i / 24) % 2, cb = i / 48;
-        const int ch = half * 8 + j;
-        unsigned wv = 0;
-        for (int kh = 0; kh < 3; ++kh)
-            wv |= (unsigned)(filt[(((size_t)cb * 3 + kh) * 3 + kw) * CB + ch] ^ 0x80u) << (8 * kh);
-        sw[i] = wv;
-    }
-    __syncthreads();
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long total = (long long)a.N * cbs * a.Ho * strips * 2;
-    if (i >= total)
-        return;
-    const int half = (int)(i & 1); i >>= 1;
-    const int strip = (int)(i % strips); i /= strips;
-    const int oh = (int)(i % a.Ho); i /= a.Ho; // i = n * cbs + cb
-    const int cb = (int)(i % cbs);
-    const uint8_t *plane = in + (size_t)i * a.H * a.W * CB + half * 8;
-    const int ow0 = strip * TW;
-    unsigned wreg[3][8];
-    {
-        const uint4 *wp = reinterpret_cast<const uint4 *>(sw + ((size_t)cb * 2 + half) * 24);
+        const int cb = i >> 4, ch = i & 15;
+        const uint8_t *w = filt + (size_t)cb * 9 * CB + ch;
+        int sum = 0;
 #pragma unroll
         for (int kw = 0; kw < 3; ++kw)
         {
-            const uint4 w0 = wp[kw * 2], w1 = wp[kw * 2 + 1];
-            wreg[kw][0] = w0.x; wreg[kw][1] = w0.y; wreg[kw][2] = w0.z; wreg[kw][3] = w0.w;
-            wreg[kw][4] = w1.x; wreg[kw][5] = w1.y; wreg[kw][6] = w1.z; wreg[kw][7] = w1.w;
-        }
-    }
-    int acc[TW][8];
+            unsigned v = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-    {
-        const int s0 = a.k_zero + (bias ? bias[cb * CB + half * 8 + j] : 0);
-#pragma unroll
-        for (int o = 0; o < TW; ++o)
-            acc[o][j] = s0;
-    }
-    const int ih0 = oh - pad_t;
-    const bool rok0 = ih0 >= 0 && ih0 < a.H, rok1 = ih0 + 1 >= 0 && ih0 + 1 < a.H, rok2 = ih0 + 2 >= 0 && ih0 + 2 < a.H;
-    const uint8_t *row0 = plane + (size_t)ih0 * a.W * CB, *row1 = row0 + (size_t)a.W * CB, *row2 = row1 + (size_t)a.W * CB;
-#pragma unroll
-    for (int x = 0; x < TW + 2; ++x)
-    {
-        const int xi = ow0 - pad_l + x;
-        if (xi < 0 || xi >= a.W)
-            continue; // a padded column adds nothing
-        uint2 r0 = make_uint2(0u, 0u), r1 = make_uint2(0u, 0u), r2 = make_uint2(0u, 0u);
-        if (rok0) r0 = *reinterpret_cast<const uint2 *>(row0 + (size_t)xi * CB);
-        if (rok1) r1 = *reinterpret_cast<const uint2 *>(row1 + (size_t)xi * CB);
-        if (rok2) r2 = *reinterpret_cast<const uint2 *>(row2 + (size_t)xi * CB);
-        if (SIGNED_IN)
-        {
-            if (rok0) { r0.x ^= 0x80808080u; r0.y ^= 0x80808080u; }
-            if (rok1) { r1.x ^= 0x80808080u; r1.y ^= 0x80808080u; }
-            if (rok2) { r2.x ^= 0x80808080u; r2.y ^= 0x80808080u; }
-        }
-        unsigned c[8];
-        transpose4x4(r0.x, r1.x, r2.x, 0u, c);
-        transpose4x4(r0.y, r1.y, r2.y, 0u, c + 4);
-#pragma unroll
-        for (int kw = 0; kw < 3; ++kw)
-        {
-            const int o = x - kw; // output o of the strip sees input column x through tap column kw
-            if (o >= 0 && o < TW)
+            for (int kh = 0; kh < 3; ++kh)
             {
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    acc[o][j] = dp4a_in<SIGNED_IN>(c[j], wreg[kw][j], acc[o][j]);
+                const int b = w[(kh * 3 + kw) * CB];
+                sum += b - 128 + a.sum_a;
+                v |= (unsigned)(b ^ 0x80) << (8 * kh);
             }
+            words[(cb * 4 + kw) * CB + ch] = v;
         }
+        words[(cb * 4 + 3) * CB + ch] = (unsigned)(a.k_zero + (bias ? bias[cb * CB + ch] : 0) + a.zero_in * sum);
     }
-    uint8_t *orow = out + (((size_t)i * a.Ho + oh) * a.Wo) * CB + half * 8;
-#pragma unroll
-    for (int o = 0; o < TW; ++o)
-    {
-        if (ow0 + o < a.Wo)
+    // A tile's rows: copies of those of the image; rows that are padding (in runs of rows only) are written.
+    auto fetch = [&](int tile, int st) {
+        const int unit = a.by_row_tiles.div(tile), oh0 = (tile - unit * a.row_tiles) * a.rows, plane0 = unit * a.planes;
+        const int planes = min(a.planes, a.N * a.cbs - plane0), top = oh0 - a.pad_t;
+        const int r_lo = max(top, 0), r_hi = min(top + a.in_rows, a.H), count = max(r_hi - r_lo, 0);
+        uint8_t *stage = smem + st * a.in_bytes;
+        const uint32_t to = smem_u32(stage) + (uint32_t)(((r_lo - top) * a.pitch + a.pad_l) * CB);
+        const uint8_t *from = in + ((size_t)plane0 * a.H + r_lo) * a.W * CB;
+        for (int i = tid; i < planes * count * a.W; i += DW_THREADS)
         {
-            uint2 v;
-            v.x = requant_pack4(acc[o][0], acc[o][1], acc[o][2], acc[o][3], a.lshift, a.rshift, a.mult);
-            v.y = requant_pack4(acc[o][4], acc[o][5], acc[o][6], acc[o][7], a.lshift, a.rshift, a.mult);
-            *reinterpret_cast<uint2 *>(orow + (size_t)(ow0 + o) * CB) = v;
+            const int row = a.by_W.div(i), pl = whole ? a.by_copy_rows.div(row) : 0, r = row - pl * count;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + (uint32_t)(((pl * a.in_rows + r) * a.pitch + i - row * a.W) * CB)),
+                         "l"(from + (size_t)(pl * (a.H - count) * a.W + i) * CB)
+                         : "memory");
         }
+        if (!whole && count < a.in_rows)
+            for (int i = tid; i < a.in_rows * a.pitch; i += DW_THREADS)
+            {
+                const int r = a.by_pitch.div(i) + top;
+                if (r < r_lo || r >= r_hi)
+                    *reinterpret_cast<uint4 *>(stage + (size_t)i * CB) = make_uint4(pad, pad, pad, pad);
+            }
+    };
+    auto store = [&](int tile, int st) { // by one thread, after all of them have fenced and met
+        const int unit = a.by_row_tiles.div(tile), oh0 = (tile - unit * a.row_tiles) * a.rows, plane0 = unit * a.planes;
+        const int planes = min(a.planes, a.N * a.cbs - plane0), rows = min(a.rows, a.Ho - oh0);
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out + ((size_t)plane0 * a.Ho + oh0) * a.Wo * CB),
+                     "r"(smem_u32(smem + a.out_at + st * a.out_bytes)), "r"((unsigned)(planes * rows * a.Wo * CB))
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    };
+    __syncthreads();
+    fetch(first, 0);
+    const bool fast = requant_is_fast(a.lshift, a.rshift, a.mult);
+    const int per_plane = a.pairs * a.strips;
+    int st = 0;
+    for (int tile = first; tile < a.tiles; tile += step)
+    {
+        // One meeting per tile: this tile's copies have landed, everyone is through with the tile before it (its output can
+        // go, its stage be filled again), and the output before that one has been read.
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        fence_proxy_async();
+        if (tid == 0)
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        __syncthreads();
+        if (tid == 0 && tile != first)
+            store(tile - step, st ^ 1);
+        if (tile + step < a.tiles)
+            fetch(tile + step, st ^ 1);
+        const int unit = a.by_row_tiles.div(tile), oh0 = (tile - unit * a.row_tiles) * a.rows, plane0 = unit * a.planes;
+        const int planes = min(a.planes, a.N * a.cbs - plane0), rows = min(a.rows, a.Ho - oh0);
+        const uint8_t *sI = smem + st * a.in_bytes;
+        uint8_t *sO = smem + a.out_at + st * a.out_bytes;
+        for (int i = tid; i < planes * per_plane * 4; i += DW_THREADS)
+        {
+            const int q = i & 3, row = a.by_strips.div(i >> 2), strip = (i >> 2) - row * a.strips, pl = a.by_pairs.div(row);
+            const int r = 2 * (row - pl * a.pairs), ow0 = strip * TW;
+            const unsigned *src = reinterpret_cast<const unsigned *>(sI + ((size_t)(pl * a.in_rows + r) * a.pitch + ow0) * CB) + q;
+            const int cb = plane0 + pl - a.by_cbs.div(plane0 + pl) * a.cbs;
+            const uint4 *wp = reinterpret_cast<const uint4 *>(words + cb * 4 * CB) + q;
+            unsigned w[3][4];
+#pragma unroll
+            for (int kw = 0; kw < 3; ++kw)
+            {
+                const uint4 v = wp[kw * 4];
+                w[kw][0] = v.x; w[kw][1] = v.y; w[kw][2] = v.z; w[kw][3] = v.w;
+            }
+            const uint4 sv = wp[12];
+            const int seed[4] = {(int)sv.x, (int)sv.y, (int)sv.z, (int)sv.w};
+            int acc[2][TW][4];
+            int asum[2][SUM_A ? TW : 1][4];
+#pragma unroll
+            for (int o = 0; o < TW; ++o)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                {
+                    acc[0][o][j] = acc[1][o][j] = 0;
+                    if (SUM_A)
+                        asum[0][o][j] = asum[1][o][j] = 0;
+                }
+#pragma unroll
+            for (int x = 0; x < TW + 2; ++x)
+            {
+                unsigned c[4];
+                transpose4x4(src[x * 4], src[(a.pitch + x) * 4], src[(2 * a.pitch + x) * 4], src[(3 * a.pitch + x) * 4], c);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                {
+#pragma unroll
+                    for (int kw = 0; kw < 3; ++kw)
+                        if (x - kw >= 0 && x - kw < TW)
+                        {
+                            acc[0][x - kw][j] = dp4a_us(c[j], w[kw][j], acc[0][x - kw][j]);
+                            acc[1][x - kw][j] = dp4a_us(c[j], w[kw][j] << 8, acc[1][x - kw][j]);
+                            if (SUM_A)
+                            {
+                                asum[0][x - kw][j] = dp4a_us(c[j], 0x00010101u, asum[0][x - kw][j]);
+                                asum[1][x - kw][j] = dp4a_us(c[j], 0x01010100u, asum[1][x - kw][j]);
+                            }
+                        }
+                }
+            }
+            if (SUM_A)
+#pragma unroll
+                for (int o = 0; o < TW; ++o)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                    {
+                        acc[0][o][j] += a.sum_a * asum[0][o][j];
+                        acc[1][o][j] += a.sum_a * asum[1][o][j];
+                    }
+            long long seeds[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                seeds[j] = requant_seed(seed[j], a.mult);
+            unsigned *dst = reinterpret_cast<unsigned *>(sO + ((size_t)(pl * a.rows + r) * a.Wo + ow0) * CB) + q;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int o = 0; o < TW; ++o)
+                    if (ow0 + o < a.Wo && r + h < rows)
+                    {
+                        unsigned v;
+                        if (fast)
+                        {
+                            const int bit = 1 << (a.rshift - 2), sh1 = a.rshift - 1;
+                            v = pack4_sat(requant_seeded_raw(acc[h][o][0], a.mult, seeds[0], bit, sh1),
+                                          requant_seeded_raw(acc[h][o][1], a.mult, seeds[1], bit, sh1),
+                                          requant_seeded_raw(acc[h][o][2], a.mult, seeds[2], bit, sh1),
+                                          requant_seeded_raw(acc[h][o][3], a.mult, seeds[3], bit, sh1));
+                        }
+                        else
+                            v = requant_pack4_general(acc[h][o][0] + seed[0], acc[h][o][1] + seed[1], acc[h][o][2] + seed[2],
+                                                      acc[h][o][3] + seed[3], a.lshift, a.rshift, a.mult);
+                        dst[(h * a.Wo + o) * 4] = v;
+                    }
+        }
+        st ^= 1;
+    }
+    fence_proxy_async();
+    __syncthreads();
+    if (tid == 0)
+    {
+        store(first + (a.tiles - 1 - first) / step * step, st ^ 1);
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
 }
 
@@ -708,8 +828,71 @@ conv2d_u8_c1_dp4a_kernel(const QArgs a, const uint8_t *__restrict__ in, const ui
     }
 }
 
-// Global average pool (window = whole image, no padding): one warp per image and 16-channel
-// block; lanes stride over the pixels, then a shuffle tree adds the 16 channel sums.
+// Global average pool (window = whole image, no padding) of at most 256 pixels: LANES lanes per image and 16-channel block
+// stride over the pixels.  A channel's sum fits 16 bits, so two channels share a register; the last two steps of the
+// reduction halve the channels a lane answers for, and four lanes requantise and store four channels each.  A warp for a
+// 3x3 plane with every lane adding and requantising all 16 channels took 21.4 us for 2048 images of 256 channels, all of
+// it shuffles and multiplications (the bytes are 1 us).  Four lanes up to 64 pixels: beyond, 16 loads a lane and more
+// in a row cost more than three steps of shuffles.
+template <int LANES>
+__global__ void __launch_bounds__(256)
+global_avgpool_small_u8_kernel(const QArgs a, const uint8_t *__restrict__ in, uint8_t *__restrict__ out)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, plane = t / LANES;
+    const int l = threadIdx.x & (LANES - 1), px = a.H * a.W;
+    const bool live = plane < (long long)a.N * (a.C / CB);
+    unsigned even[4] = {0u, 0u, 0u, 0u}, odd[4] = {0u, 0u, 0u, 0u};
+    if (live)
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(in) + plane * px;
+#pragma unroll 4
+        for (int p = l; p < px; p += LANES)
+        {
+            const uint4 v = __ldg(src + p);
+            const unsigned w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+            {
+                even[k] += w[k] & 0x00ff00ffu;
+                odd[k] += (w[k] >> 8) & 0x00ff00ffu;
+            }
+        }
+    }
+#pragma unroll
+    for (int off = LANES / 2; off > 2; off >>= 1)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+        {
+            even[k] += __shfl_xor_sync(0xffffffffu, even[k], off);
+            odd[k] += __shfl_xor_sync(0xffffffffu, odd[k], off);
+        }
+#pragma unroll
+    for (int off = 2; off > 0; off >>= 1) // lanes with the bit keep the upper half of what is left
+    {
+        const bool up = l & off;
+#pragma unroll
+        for (int k = 0; k < off; ++k)
+        {
+            const unsigned ge = up ? even[k] : even[k + off], go = up ? odd[k] : odd[k + off];
+            const unsigned ke = up ? even[k + off] : even[k], ko = up ? odd[k + off] : odd[k];
+            even[k] = ke + __shfl_xor_sync(0xffffffffu, ge, off);
+            odd[k] = ko + __shfl_xor_sync(0xffffffffu, go, off);
+        }
+    }
+    if (live && l < 4)
+    {
+        const int zero = px * a.zero_in + a.k_zero;
+        unsigned o = 0;
+        const unsigned sums[4] = {even[0] & 0xffffu, odd[0] & 0xffffu, even[0] >> 16, odd[0] >> 16};
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            o |= (unsigned)(requant_dev((int)sums[k] + zero, a.lshift, a.rshift, a.mult) & 255) << (8 * k);
+        reinterpret_cast<unsigned *>(out)[plane * 4 + l] = o;
+    }
+}
+
+// The same for larger images: one warp per image and 16-channel block; lanes stride over the pixels, then a shuffle tree adds
+// the 16 channel sums.
 __global__ void __launch_bounds__(256)
 global_avgpool_u8_kernel(const QArgs a, const uint8_t *__restrict__ in, uint8_t *__restrict__ out)
 {
@@ -802,6 +985,78 @@ int check_partial_u8(const small_b200_layer *L, const char *name, int channels, 
     return SMALL_B200_OK;
 }
 
+// -1: not a shape of the tiled depthwise kernel.
+int launch_dw_tile(const small_b200_layer *L, const QArgs &q, const uint8_t *in, const uint8_t *filt, const int32_t *bias, uint8_t *out,
+                   cudaStream_t st)
+{
+    if (q.Fh != 3 || q.Fw != 3 || q.stride != 1 || row_stride(L) != 1 || q.zero_in > 0 || q.zero_in < -255) // padding has to be a byte
+        return -1;
+    DwTile a{};
+    a.N = q.N; a.cbs = q.C / CB; a.H = q.H; a.W = q.W; a.Ho = q.Ho; a.Wo = q.Wo; a.pad_t = q.pad_t; a.pad_l = q.pad_l;
+    a.zero_in = q.zero_in; a.sum_a = 128 + q.zero_filt;
+    a.lshift = q.lshift; a.rshift = q.rshift; a.mult = q.mult; a.k_zero = q.k_zero;
+    const long long total_planes = (long long)q.N * a.cbs;
+    // Strips of 5 or of 3, by the instructions they take (two rows, four channels a thread); with sums of the input the
+    // accumulators of 5 would not fit the registers.
+    auto cost = [&](int tw) { return (q.Wo + tw - 1) / tw * (tw * 76 + (tw + 2) * 14); };
+    const int tw = !a.sum_a && cost(5) <= cost(3) ? 5 : 3;
+    a.strips = (q.Wo + tw - 1) / tw;
+    a.pitch = (a.strips * tw + 2) | 1; // odd: row pairs, two pitches apart, use different banks
+    if (q.W + q.pad_l > a.pitch || q.W > 4096 || q.H > 0x10000)
+        return -1;
+    auto bytes = [&](int planes, int rows) {
+        const int in_rows = (rows + 1) / 2 * 2 + 2;
+        a.in_bytes = (unsigned)((planes * in_rows * a.pitch * CB + 127) & ~127);
+        a.out_bytes = (unsigned)((planes * rows * q.Wo * CB + 127) & ~127);
+        a.out_at = 2 * a.in_bytes;
+        a.w_at = a.out_at + 2 * a.out_bytes;
+        return (long long)a.w_at + a.cbs * 4 * CB * 4;
+    };
+    // The tile: the one with the shortest estimated time, rounds of a CTA's threads plus about half a round for a tile's
+    // barrier and copies, at three CTAs an SM (what the registers leave; so many hide each other's waits).
+    const long long cap = 72 * 1024, room = 3LL * num_sms();
+    int best_planes = 0, best_rows = 0;
+    double best = 1e30;
+    auto consider = [&](int planes, int rows) {
+        const long long items = (long long)planes * ((rows + 1) / 2) * a.strips * 4;
+        const long long tiles = (total_planes + planes - 1) / planes * ((q.Ho + rows - 1) / rows);
+        const double time = (double)((tiles + room - 1) / room) * ((double)((items + DW_THREADS - 1) / DW_THREADS) + 0.5);
+        if (time < best) { best = time; best_planes = planes; best_rows = rows; }
+    };
+    for (int planes = 1; planes <= 256 && planes <= total_planes && bytes(planes, q.Ho) <= cap; ++planes)
+        consider(planes, q.Ho);
+    for (int rows = 2; rows < q.Ho && bytes(1, rows) <= cap; rows += 2)
+        consider(1, rows);
+    if (!best_planes)
+        return -1;
+    a.planes = best_planes; a.rows = best_rows;
+    a.row_tiles = (q.Ho + a.rows - 1) / a.rows;
+    a.pairs = (a.rows + 1) / 2; a.in_rows = 2 * a.pairs + 2;
+    const size_t smem = (size_t)bytes(a.planes, a.rows);
+    const long long tiles = (total_planes + a.planes - 1) / a.planes * a.row_tiles;
+    if (tiles > 0x3fffffffLL || total_planes > 0x3fffffffLL)
+        return -1;
+    a.tiles = (int)tiles;
+    const unsigned blocks = (unsigned)(tiles < room ? tiles : room);
+    const int copy_rows = std::min(a.H, a.in_rows - a.pad_t); // rows of the image in a tile of whole planes
+    if (copy_rows <= 0)
+        return -1;
+    a.by_row_tiles.set(a.row_tiles); a.by_cbs.set(a.cbs); a.by_strips.set(a.strips); a.by_pairs.set(a.pairs);
+    a.by_pitch.set(a.pitch); a.by_in_rows.set(a.in_rows); a.by_copy_rows.set(copy_rows); a.by_W.set(a.W);
+    static PerDeviceOnce configured;
+    int dev;
+    if (configured.needed(&dev))
+    {
+        SB_CUDA(cudaFuncSetAttribute(dwconv3x3_u8_tile_kernel<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+        SB_CUDA(cudaFuncSetAttribute(dwconv3x3_u8_tile_kernel<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+        SB_CUDA(cudaFuncSetAttribute(dwconv3x3_u8_tile_kernel<5, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+        configured.mark(dev);
+    }
+    auto kern = a.sum_a ? dwconv3x3_u8_tile_kernel<3, true> : tw == 5 ? dwconv3x3_u8_tile_kernel<5, false> : dwconv3x3_u8_tile_kernel<3, false>;
+    kern<<<blocks, DW_THREADS, smem, st>>>(a, in, filt, bias, out);
+    return launched("dwconv3x3_u8_tile_kernel");
+}
+
 template <int OP>
 int launch_window(const small_b200_layer *L, const char *name, int max_stride, const uint8_t *in,
                   const uint8_t *filt, const int32_t *bias, uint8_t *out, void *stream)
@@ -828,28 +1083,11 @@ int launch_window(const small_b200_layer *L, const char *name, int max_stride, c
     }
     if (items == 0)
         return SMALL_B200_OK;
-    if (OP == 0 && a.zero_filt == -128 && (a.zero_in == 0 || a.zero_in == -128) && a.Fh == 3 && a.Fw == 3 &&
-        a.stride == 1 && a.C <= 2048 && a.Wo >= 3)
+    if (OP == 0)
     {
-        // 3x3 stride 1: row strips of 4, 5 or 6 outputs per thread, whichever tiles the width best
-        const bool sgn = a.zero_in != 0;
-        cudaStream_t st = as_stream(stream);
-        int tw = 6, waste = 1 << 30;
-        for (int t = 6; t >= 4; --t)
-        {
-            const int w_ = (a.Wo + t - 1) / t * t - a.Wo;
-            if (w_ < waste) { waste = w_; tw = t; }
-        }
-        const int strips = (a.Wo + tw - 1) / tw;
-        const long long threads = (long long)a.N * (a.C / CB) * a.Ho * strips * 2;
-        const unsigned blocks = (unsigned)((threads + 255) / 256);
-        const size_t smem = (size_t)(a.C / CB) * 48 * 4;
-#define SB_DW_ROWS(S, T) dwconv3x3_u8_rows_kernel<S, T><<<blocks, 256, smem, st>>>(a, in, filt, bias, out, strips, L->pad_t, L->pad_l)
-        if (tw == 6) { if (sgn) SB_DW_ROWS(true, 6); else SB_DW_ROWS(false, 6); }
-        else if (tw == 5) { if (sgn) SB_DW_ROWS(true, 5); else SB_DW_ROWS(false, 5); }
-        else { if (sgn) SB_DW_ROWS(true, 4); else SB_DW_ROWS(false, 4); }
-#undef SB_DW_ROWS
-        return launched("dwconv3x3_u8_rows_kernel");
+        const int rc = launch_dw_tile(L, a, in, filt, bias, out, as_stream(stream));
+        if (rc >= 0)
+            return rc;
     }
     if (OP == 0 && a.zero_filt == -128 && (a.zero_in == 0 || a.zero_in == -128) && a.Fh * a.Fw <= 64 && a.C <= 2048)
     {
@@ -872,6 +1110,14 @@ int launch_window(const small_b200_layer *L, const char *name, int max_stride, c
     if (OP == 2 && a.Fh == a.H && a.Fw == a.W && !L->pad_t && !L->pad_b && !L->pad_l && !L->pad_r)
     {
         const long long warps = (long long)a.N * (a.C / CB);
+        const int px = a.H * a.W;
+        if (px <= 256)
+        {
+            const int lanes = px <= 64 ? 4 : 32;
+            (lanes == 4 ? global_avgpool_small_u8_kernel<4> : global_avgpool_small_u8_kernel<32>)
+                <<<(unsigned)((warps * lanes + 255) / 256), 256, 0, as_stream(stream)>>>(a, in, out);
+            return launched("global_avgpool_small_u8_kernel");
+        }
         global_avgpool_u8_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, as_stream(stream)>>>(a, in, out);
         return launched("global_avgpool_u8_kernel");
     }
