@@ -19,6 +19,8 @@
 // sums of the filter tile are taken from the shared-memory tiles by the epilogue threads.
 #include "tc_common.cuh"
 
+#include <algorithm>
+
 namespace sb
 {
 static __device__ int g_device_status = 0;
@@ -90,9 +92,10 @@ struct PwArgs
     int tiles;   // ceil(P / 128)
     int nblocks; // K / NT
     int bulk;    // 1: a channel block of a tile is one contiguous run of pixels (plain bulk copies)
-    int images;  // images per tile where one leaves half of it empty or more, else 0
+    int images;  // an image's last rem <= 64 pixels share a tile with those of the images after it, this many in all (0: no such tiles)
+    int rem, main; // main: tiles before the first shared one
     int N;
-    FastDiv by_tiles, by_P;
+    FastDiv by_tiles, by_rem;
     long long out_pix_stride, out_plane_stride, out_group_stride; // bytes
     int zero_in, zero_filt, lshift, rshift, mult, k_zero;
 };
@@ -127,7 +130,7 @@ pw_u8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const PwArgs a, const
     uint8_t *sB = smem + 2 * (size_t)a_bytes; // [NT/16][cbs][16][16]
 
     const int nb = blockIdx.y;
-    const int total = a.groups * a.tiles;
+    const int total = a.main + (a.images ? (a.N + a.images - 1) / a.images : 0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
     if (warp == PW_EPI_WARPS)
@@ -161,13 +164,14 @@ pw_u8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const PwArgs a, const
             if (!ok)
                 break;
             const int g = a.by_tiles.div(item), tile = item - g * a.tiles;
-            if (a.images)
+            if (item >= a.main)
             {
-                // small images: a row of the copy is a channel block of an image (P * 16 contiguous bytes), so a channel block of
-                // the tile is the images' pixels one after the other; rows past the batch read as zero
-                mbar_expect_tx(&full_bar[s], (uint32_t)(a.cbs * a.images * a.P * CB));
+                // a row of the copy is the last rem pixels of an image's channel block (contiguous bytes), so a channel block of the
+                // tile is the images' pixels one after the other; rows past the batch read as zero
+                mbar_expect_tx(&full_bar[s], (uint32_t)(a.cbs * a.images * a.rem * CB));
                 for (int cb = 0; cb < a.cbs; ++cb)
-                    tma_load_3d(sA + (size_t)s * a_bytes + (size_t)cb * TILE_M * CB, &map_a, 0, tile * a.images, cb, &full_bar[s]);
+                    tma_load_3d(sA + (size_t)s * a_bytes + (size_t)cb * TILE_M * CB, &map_a, 2 * (a.P - a.rem), (item - a.main) * a.images, cb,
+                                &full_bar[s]);
             }
             else if (a.bulk)
             {
@@ -215,7 +219,7 @@ pw_u8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const PwArgs a, const
     else if (warp < PW_EPI_WARPS)
     {
         const int px_t = (warp & 3) * 32 + lane;      // this thread's pixel of the tile = its TMEM lane
-        const int image = a.images ? a.by_P.div(px_t) : 0;
+        const int image = a.images ? a.by_rem.div(px_t) : 0;
         constexpr int CPW = NT >= 32 ? NT / 2 : NT;  // output channels per warp group
         const int c_begin = (warp >> 2) * CPW;
         // per-channel constants: k_zero + bias + C*zI*zF + zI * (column sum of the filter)
@@ -261,8 +265,10 @@ pw_u8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const PwArgs a, const
             if (!ok)
                 break;
             tc_fence_after_sync();
-            const int n = a.images ? tile * a.images + image : g, p = a.images ? px_t - image * a.P : tile * TILE_M + px_t;
-            const bool live = a.images ? image < a.images && n < a.N : p < a.P;
+            const bool shared = item >= a.main;
+            const int n = shared ? (item - a.main) * a.images + image : g;
+            const int p = shared ? a.P - a.rem + px_t - image * a.rem : tile * TILE_M + px_t;
+            const bool live = shared ? image < a.images && n < a.N : p < a.P;
             const int base = a.zero_filt * asum;
             uint8_t *orow = out + (size_t)n * a.out_group_stride + (size_t)p * a.out_pix_stride;
 #pragma unroll
@@ -325,7 +331,7 @@ int launch_pw(const CUtensorMap &map, const PwArgs &a, size_t smem, const uint8_
         per_sm = 8;
     if (per_sm < 1)
         per_sm = 1;
-    const long long total = (long long)a.groups * a.tiles;
+    const long long total = (long long)a.main + (a.images ? (a.N + a.images - 1) / a.images : 0);
     long long gx = (long long)num_sms() * per_sm / a.nblocks;
     if (gx < 1)
         gx = 1;
@@ -581,23 +587,24 @@ int conv2d_u8_tensor_core(const small_b200_layer *L, const uint8_t *in, const ui
     }
     a.tiles = (a.P + TILE_M - 1) / TILE_M;
     CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_UINT8;
-    // Two images and more fit a tile (P <= 64): as many as do, since a tile costs the same (barriers, MMAs, the requantisation
-    // of 128 rows) whatever it holds.  2048 images: 256 -> 256 channels at 3x3 49.8 -> 7.1 us, 128 -> 128 at 6x6 24.0 -> 10.5,
-    // 64 -> 128 at 6x6 23.0 -> 10.0; a single image is where it was.
-    a.images = a.bulk && a.P <= TILE_M / 2 && a.groups > 1 ? TILE_M / a.P : 0;
+    // An image's pixels past the last full tile share tiles where at least two images' fit one, since a tile costs the same
+    // (barriers, MMAs, the requantisation of 128 rows) whatever it holds.  2048 images, one tile or more an image before ->
+    // now: 256 -> 256 channels at 3x3 49.8 -> 7.1 us, 128 -> 128 at 6x6 24.0 -> 10.5, 64 -> 64 at 12x12 (16 pixels past a tile)
+    // 25 -> 16, 32 -> 32 at 24x24 (64 past four) 34 -> 32; a single image is where it was.
     a.N = L->N;
+    a.rem = a.P % TILE_M;
+    a.images = a.bulk && a.rem > 0 && a.rem <= TILE_M / 2 && a.groups > 1 ? std::min(TILE_M / a.rem, L->N) : 0;
+    a.by_rem.set(a.rem > 0 ? a.rem : 1);
     if (a.images)
     {
-        if (a.images > L->N)
-            a.images = L->N;
         type = CU_TENSOR_MAP_DATA_TYPE_FLOAT64; // pairs of them are pixels; nothing is converted
         dims[0] = 2 * (uint64_t)HW; dims[1] = (uint64_t)L->N; dims[2] = (uint64_t)cbs;
         strides[0] = (uint64_t)cbs * HW * CB; strides[1] = (uint64_t)HW * CB;
-        box[0] = 2 * (uint32_t)HW; box[1] = (uint32_t)a.images; box[2] = 1;
-        a.tiles = (L->N + a.images - 1) / a.images;
-        a.groups = 1;
+        box[0] = 2 * (uint32_t)a.rem; box[1] = (uint32_t)a.images; box[2] = 1;
+        a.tiles = a.P / TILE_M;
     }
-    a.by_tiles.set(a.tiles); a.by_P.set(a.P);
+    a.main = a.groups * a.tiles;
+    a.by_tiles.set(a.tiles > 0 ? a.tiles : 1);
     CUtensorMap map;
     if (int rc = make_tensor_map(&map, type, 3, in, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE))
         return rc;
