@@ -614,140 +614,229 @@ dwconv3x3_u8_tile_kernel(const DwTile a, const uint8_t *__restrict__ in, const u
     }
 }
 
-// Dense convolution whose whole reduction is at most 32 bytes: a 1x1 layer on 16 channels, or a first
-// layer (1..3 channels, [H][W][C] image) whose window holds at most 32 values, e.g. 3x3 on 3 channels.
-// These are streaming layers -- one 16-byte load (or a few byte loads) and one 16-byte store per pixel
-// and block of output channels -- with too little arithmetic for the tensor core to matter.  A thread
-// makes one output pixel: its reduction row sits in up to eight registers of four bytes, the filter in
-// shared memory as words of four reduction bytes, [word][output channel], so one 128-bit broadcast
-// fetch feeds four dp4a.  Filter zero point -128, input zero point 0 or -128 (operands enter shifted);
-// taps outside the image are zero bytes, i.e. skipped, as in the reference.
-// FIX333: the 3x3 window on 3 channels.  A kernel row of the window is 9 contiguous bytes of the
-// [H][W][3] image: three aligned 32-bit loads and two funnel shifts instead of nine byte loads; rows at
-// the left border, or whose aligned reads would pass the end of the buffer, take the byte path.
-template <bool SIGNED_IN, bool FIRST, bool FIX333 = false>
+// Dense convolution whose whole reduction is at most 32 bytes: a 1x1 layer on 16 or 32 channels, or a first layer (1..3
+// channels, [H][W][C] image) whose window holds at most 32 values, e.g. 3x3 on 3 channels.  These are streaming layers
+// with too little arithmetic for the tensor core to matter: what bounds them is the integer pipes (a dp4a for four products,
+// four and a half instructions of requantisation per output byte), and before that shared memory, if every
+// pixel fetches the filter for itself (64 four-byte broadcasts a pixel; 2.3 of the 3 cycles an output took).  So a thread makes
+// PX pixels, 32 apart, and a 16-byte fetch of four channels' filter words feeds 4 * PX dp4a; one pixel a thread where
+// there are not enough of them to fill the machine.  Two and not four: with 128 registers the gathers of eight warps a CTA had
+// too little to hide behind (first layer 138 us against 100).  2048 images, us before -> now: 3x3 on 3 channels, stride 2
+// at 96x96 113 -> 99 (225 -> 100 with padding on all sides); 16 -> 16 channels at 48x48 69 -> 57; 16 -> 32 at 24x24 49 -> 27
+// (as an implicit GEMM before).
+// Filter bytes are signed, w' = w - 128, the input stays unsigned, taps outside the image hold the byte -zero_in:
+//   sum (a + zI)(w + zF) = sum a w' + (128 + zF) sum a + zI sum (w + zF)
+// with the last term in the seed of the requantisation and the second one counted once per pixel.
+struct OneArgs
+{
+    int total, H, W, Ho, Wo, C, K, Fh, Fw, R, stride, pad_t, pad_l;
+    int zero_in, sum_a; // sum_a: 128 + zero_filt
+    int lshift, rshift, mult, k_zero;
+    long long in_bytes;
+    FastDiv by_hw, by_Wo;
+};
+enum { ONE_1X1, ONE_333, ONE_FIRST };
+
+// The reduction row of output pixel g: WORDS words of four bytes.
+template <int WORDS, int KIND>
+__device__ __forceinline__ void one_gather(const OneArgs &a, const uint8_t *__restrict__ in, int g, unsigned pad, unsigned (&x)[WORDS])
+{
+    const int n = a.by_hw.div(g), p = g - n * a.Ho * a.Wo, oh = a.by_Wo.div(p), ow = p - oh * a.Wo;
+    const int ih0 = oh * a.stride - a.pad_t, iw0 = ow * a.stride - a.pad_l;
+    if (KIND == ONE_1X1)
+    {
+        const bool inside = (unsigned)ih0 < (unsigned)a.H && (unsigned)iw0 < (unsigned)a.W;
+        const uint8_t *src = in + (((size_t)n * (WORDS / 4) * a.H + ih0) * a.W + iw0) * CB;
+#pragma unroll
+        for (int cb = 0; cb < WORDS / 4; ++cb)
+        {
+            const uint4 v = inside ? __ldg(reinterpret_cast<const uint4 *>(src + (size_t)cb * a.H * a.W * CB)) : make_uint4(pad, pad, pad, pad);
+            x[4 * cb] = v.x; x[4 * cb + 1] = v.y; x[4 * cb + 2] = v.z; x[4 * cb + 3] = v.w;
+        }
+        return;
+    }
+    if (KIND == ONE_333)
+    {
+        // A kernel row is 9 contiguous bytes: three aligned words and two funnel shifts; where the aligned words would pass an
+        // end of the buffer, bytes.
+        const uint8_t *row0 = in + ((long long)n * a.H + ih0) * a.W * 3 + iw0 * 3;
+        const int vb = min(9, (a.W - iw0) * 3), skip = max(0, -iw0) * 3; // bytes of a row's run inside the image: [skip, vb)
+        unsigned r0[3], r1[3], r2[3];
+#pragma unroll
+        for (int kh = 0; kh < 3; ++kh)
+        {
+            r0[kh] = r1[kh] = pad; r2[kh] = pad & 0xffu;
+            if ((unsigned)(ih0 + kh) >= (unsigned)a.H)
+                continue;
+            const uint8_t *run = row0 + (long long)kh * a.W * 3;
+            const uintptr_t base = reinterpret_cast<uintptr_t>(run) & ~(uintptr_t)3;
+            if (base >= reinterpret_cast<uintptr_t>(in) && base + 12 <= reinterpret_cast<uintptr_t>(in) + (uintptr_t)a.in_bytes)
+            {
+                const unsigned *wp = reinterpret_cast<const unsigned *>(base);
+                const unsigned sh = (unsigned)(reinterpret_cast<uintptr_t>(run) & 3) * 8;
+                const unsigned w0 = __ldg(wp), w1 = __ldg(wp + 1), w2 = __ldg(wp + 2);
+                r0[kh] = __funnelshift_r(w0, w1, sh);
+                r1[kh] = __funnelshift_r(w1, w2, sh);
+                r2[kh] = (w2 >> sh) & 0xffu;
+                if (vb < 9 || skip > 0)
+                {
+#pragma unroll
+                    for (int b = 0; b < 9; ++b)
+                        if (b < skip || b >= vb)
+                        {
+                            unsigned &r = b < 4 ? r0[kh] : b < 8 ? r1[kh] : r2[kh];
+                            const unsigned m = 0xffu << (8 * (b & 3));
+                            r = (r & ~m) | (pad & m);
+                        }
+                }
+            }
+            else
+            {
+#pragma unroll
+                for (int b = 0; b < 9; ++b)
+                    if (b >= skip && b < vb)
+                    {
+                        unsigned &r = b < 4 ? r0[kh] : b < 8 ? r1[kh] : r2[kh];
+                        const unsigned m = 0xffu << (8 * (b & 3));
+                        r = (r & ~m) | (unsigned)run[b] << (8 * (b & 3));
+                    }
+            }
+        }
+        x[0] = r0[0]; x[1] = r1[0];
+        x[2] = r2[0] | (r0[1] << 8);
+        x[3] = (r0[1] >> 24) | (r1[1] << 8);
+        x[4] = (r1[1] >> 24) | (r2[1] << 8) | (r0[2] << 16);
+        x[5] = (r0[2] >> 16) | (r1[2] << 16);
+        x[6] = (r1[2] >> 16) | (r2[2] << 16);
+        return;
+    }
+    const uint8_t *img = in + (size_t)n * a.C * a.H * a.W;
+    int kh = 0, kw = 0, c = 0;
+#pragma unroll
+    for (int j = 0; j < WORDS; ++j)
+        x[j] = 0u;
+#pragma unroll
+    for (int r = 0; r < 4 * WORDS; ++r) // unrolled: x[] stays in registers
+    {
+        const int ih = ih0 + kh, iw = iw0 + kw;
+        if (r < a.R)
+        {
+            const unsigned v = (unsigned)ih < (unsigned)a.H && (unsigned)iw < (unsigned)a.W ? img[((size_t)ih * a.W + iw) * a.C + c] : pad & 0xffu;
+            x[r >> 2] |= v << (8 * (r & 3));
+        }
+        if (++c == a.C)
+        {
+            c = 0;
+            if (++kw == a.Fw) { kw = 0; ++kh; }
+        }
+    }
+}
+
+template <int WORDS, int KIND, int PX>
 __global__ void __launch_bounds__(256)
-conv2d_u8_onestep_kernel(const QArgs a, int words, const uint8_t *__restrict__ in, const uint8_t *__restrict__ filt,
+conv2d_u8_onestep_kernel(const OneArgs a, const uint8_t *__restrict__ in, const uint8_t *__restrict__ filt,
                          const int32_t *__restrict__ bias, uint8_t *__restrict__ out)
 {
-    extern __shared__ __align__(16) unsigned smem_u[]; // [K/16][words][16 k]
-    const int R = a.Fh * a.Fw * a.C; // reduction length in bytes (<= 32)
-    const int kbs = a.K / CB;
-    for (int i = threadIdx.x; i < kbs * words * CB; i += blockDim.x)
+    extern __shared__ __align__(16) unsigned smem_u[]; // [K/4][WORDS + 1][4 k]: filter words, then the seeds
+    for (int i = threadIdx.x; i < a.K; i += blockDim.x)
     {
-        const int k = i % CB, j = (i / CB) % words, kb = i / (CB * words);
-        unsigned wv = 0;
-        for (int t = 0; t < 4; ++t)
+        const uint8_t *w = filt + (size_t)(i / CB) * a.R * CB + (i % CB); // filter [K/16][R rows][16 k] for both layouts
+        unsigned *row = smem_u + (size_t)(i / 4) * (WORDS + 1) * 4 + (i & 3);
+        int sum = 0;
+#pragma unroll
+        for (int j = 0; j < WORDS; ++j)
         {
-            const int r = 4 * j + t;
-            if (r < R) // filter [K/16][R rows][16 k] for both layouts
-                wv |= (unsigned)(filt[((size_t)kb * R + r) * CB + k] ^ 0x80u) << (8 * t);
+            unsigned wv = 0;
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (4 * j + t < a.R)
+                {
+                    const int b = w[(4 * j + t) * CB];
+                    sum += b - 128 + a.sum_a;
+                    wv |= (unsigned)(b ^ 0x80) << (8 * t);
+                }
+            row[j * 4] = wv;
         }
-        smem_u[i] = wv;
+        row[WORDS * 4] = (unsigned)(a.k_zero + (bias ? bias[i] : 0) + a.zero_in * sum);
     }
     __syncthreads();
-    const long long total = (long long)a.N * a.Ho * a.Wo;
-    const int hw = a.Ho * a.Wo;
+    const unsigned pad = (unsigned)(-a.zero_in & 255) * 0x01010101u;
+    const int hw = a.Ho * a.Wo, kbs = a.K / CB, bit = 1 << max(a.rshift - 2, 0), sh1 = a.rshift - 1;
+    const bool fast = requant_is_fast(a.lshift, a.rshift, a.mult);
     // a CTA keeps its copy of the filter for many pixels
-    for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += (long long)gridDim.x * blockDim.x)
+    for (long long base = (long long)blockIdx.x * 256 * PX + (threadIdx.x >> 5) * 32 * PX + (threadIdx.x & 31); base < a.total;
+         base += (long long)gridDim.x * 256 * PX)
     {
-    const int n = (int)(g / hw), p = (int)(g - (long long)n * hw);
-    const int oh = p / a.Wo, ow = p - oh * a.Wo;
-    const int ih0 = oh * a.stride - a.pad_t, iw0 = ow * a.stride - a.pad_l;
-    unsigned x[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-    bool gathered = false;
-    if (FIRST && FIX333)
-    {
-        const uint8_t *img = in + (size_t)n * 3 * a.H * a.W;
-        const uint8_t *in_end = in + (size_t)a.N * 3 * a.H * a.W;
-        const uint8_t *last = img + ((size_t)(ih0 + 2 < a.H ? ih0 + 2 : a.H - 1) * a.W + iw0) * 3;
-        if (iw0 >= 0 && ih0 + 2 >= 0 && (reinterpret_cast<uintptr_t>(last) & ~(uintptr_t)3) + 12 <= reinterpret_cast<uintptr_t>(in_end))
-        {
-            const int vb = (a.W - iw0) >= 3 ? 9 : (a.W - iw0) * 3; // bytes of a row's run inside the image
-            const unsigned f = SIGNED_IN ? 0x80808080u : 0u;
-            unsigned r0[3], r1[3], r2[3];
+        const int g0 = (int)base;
+        unsigned x[PX][WORDS];
+        int sa[PX];
 #pragma unroll
-            for (int kh = 0; kh < 3; ++kh)
-            {
-                const int ih = ih0 + kh;
-                r0[kh] = r1[kh] = r2[kh] = 0u;
-                if (ih >= 0 && ih < a.H)
-                {
-                    const uintptr_t addr = reinterpret_cast<uintptr_t>(img + ((size_t)ih * a.W + iw0) * 3);
-                    const unsigned *wp = reinterpret_cast<const unsigned *>(addr & ~(uintptr_t)3);
-                    const unsigned sh = (unsigned)(addr & 3) * 8;
-                    const unsigned w0 = wp[0], w1 = wp[1], w2 = wp[2];
-                    r0[kh] = __funnelshift_r(w0, w1, sh) ^ f;
-                    r1[kh] = __funnelshift_r(w1, w2, sh) ^ f;
-                    r2[kh] = ((w2 >> sh) ^ f) & 0xffu;
-                    if (vb <= 6) { r2[kh] = 0u; r1[kh] &= 0x0000ffffu; }
-                    if (vb <= 3) { r1[kh] = 0u; r0[kh] &= 0x00ffffffu; }
-                }
-            }
-            x[0] = r0[0]; x[1] = r1[0];
-            x[2] = r2[0] | (r0[1] << 8);
-            x[3] = (r0[1] >> 24) | (r1[1] << 8);
-            x[4] = (r1[1] >> 24) | (r2[1] << 8) | (r0[2] << 16);
-            x[5] = (r0[2] >> 16) | (r1[2] << 16);
-            x[6] = (r1[2] >> 16) | (r2[2] << 16);
-            gathered = true;
-        }
-    }
-    if (FIRST && !gathered)
-    {
-        const uint8_t *img = in + (size_t)n * a.C * a.H * a.W;
-        int kh = 0, kw = 0, c = 0;
+        for (int t = 0; t < PX; ++t)
+            one_gather<WORDS, KIND>(a, in, min(g0 + 32 * t, a.total - 1), pad, x[t]);
 #pragma unroll
-        for (int r = 0; r < 32; ++r) // unrolled: x[] stays in registers
+        for (int t = 0; t < PX; ++t)
         {
-            const int ih = ih0 + kh, iw = iw0 + kw;
-            if (r < R && ih >= 0 && ih < a.H && iw >= 0 && iw < a.W)
+            sa[t] = 0;
+            if (a.sum_a)
             {
-                const unsigned v = (unsigned)img[((size_t)ih * a.W + iw) * a.C + c] ^ (SIGNED_IN ? 0x80u : 0u);
-                x[r >> 2] |= v << (8 * (r & 3));
-            }
-            if (++c == a.C)
-            {
-                c = 0;
-                if (++kw == a.Fw)
-                {
-                    kw = 0;
-                    ++kh;
-                }
+                unsigned s = 0;
+#pragma unroll
+                for (int j = 0; j < WORDS; ++j)
+                    s = __dp4a(x[t][j], 0x01010101u, s);
+                sa[t] = a.sum_a * (int)s;
             }
         }
-    }
-    if (!FIRST && ih0 >= 0 && ih0 < a.H && iw0 >= 0 && iw0 < a.W) // 1x1 window on one block of 16 channels
-    {
-        const uint4 v = *reinterpret_cast<const uint4 *>(in + (((size_t)n * a.H + ih0) * a.W + iw0) * CB);
-        const unsigned f = SIGNED_IN ? 0x80808080u : 0u;
-        x[0] = v.x ^ f; x[1] = v.y ^ f; x[2] = v.z ^ f; x[3] = v.w ^ f;
-    }
-    uint8_t *o = out + ((size_t)n * kbs * hw + p) * CB;
-    for (int kb = 0; kb < kbs; ++kb)
-    {
-        int acc[CB];
-#pragma unroll
-        for (int k = 0; k < CB; ++k)
-            acc[k] = a.k_zero + (bias ? bias[kb * CB + k] : 0);
-        const uint4 *w4 = reinterpret_cast<const uint4 *>(smem_u + (size_t)kb * words * CB);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
+        for (int kb = 0; kb < kbs; ++kb)
         {
-            if (j >= words)
-                break;
+            unsigned o[PX][4];
 #pragma unroll
             for (int k4 = 0; k4 < 4; ++k4)
             {
-                const uint4 wv = w4[j * 4 + k4];
-                acc[4 * k4 + 0] = dp4a_in<SIGNED_IN>(x[j], wv.x, acc[4 * k4 + 0]);
-                acc[4 * k4 + 1] = dp4a_in<SIGNED_IN>(x[j], wv.y, acc[4 * k4 + 1]);
-                acc[4 * k4 + 2] = dp4a_in<SIGNED_IN>(x[j], wv.z, acc[4 * k4 + 2]);
-                acc[4 * k4 + 3] = dp4a_in<SIGNED_IN>(x[j], wv.w, acc[4 * k4 + 3]);
+                const uint4 *w4 = reinterpret_cast<const uint4 *>(smem_u) + (size_t)(kb * 4 + k4) * (WORDS + 1);
+                int acc[PX][4];
+#pragma unroll
+                for (int t = 0; t < PX; ++t)
+                    acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = sa[t];
+#pragma unroll
+                for (int j = 0; j < WORDS; ++j)
+                {
+                    const uint4 wv = w4[j];
+#pragma unroll
+                    for (int t = 0; t < PX; ++t)
+                    {
+                        acc[t][0] = dp4a_us(x[t][j], wv.x, acc[t][0]);
+                        acc[t][1] = dp4a_us(x[t][j], wv.y, acc[t][1]);
+                        acc[t][2] = dp4a_us(x[t][j], wv.z, acc[t][2]);
+                        acc[t][3] = dp4a_us(x[t][j], wv.w, acc[t][3]);
+                    }
+                }
+                const uint4 c = w4[WORDS];
+                if (fast)
+                {
+                    const long long s0 = requant_seed((int)c.x, a.mult), s1 = requant_seed((int)c.y, a.mult),
+                                    s2 = requant_seed((int)c.z, a.mult), s3 = requant_seed((int)c.w, a.mult);
+#pragma unroll
+                    for (int t = 0; t < PX; ++t)
+                        o[t][k4] = pack4_sat(requant_seeded_raw(acc[t][0], a.mult, s0, bit, sh1), requant_seeded_raw(acc[t][1], a.mult, s1, bit, sh1),
+                                             requant_seeded_raw(acc[t][2], a.mult, s2, bit, sh1), requant_seeded_raw(acc[t][3], a.mult, s3, bit, sh1));
+                }
+                else
+#pragma unroll
+                    for (int t = 0; t < PX; ++t)
+                        o[t][k4] = requant_pack4_general(acc[t][0] + (int)c.x, acc[t][1] + (int)c.y, acc[t][2] + (int)c.z, acc[t][3] + (int)c.w,
+                                                         a.lshift, a.rshift, a.mult);
+            }
+#pragma unroll
+            for (int t = 0; t < PX; ++t)
+            {
+                const int g = g0 + 32 * t;
+                if (g < a.total)
+                {
+                    const int n = a.by_hw.div(g);
+                    *reinterpret_cast<uint4 *>(out + (((size_t)n * kbs + kb) * hw + (g - n * hw)) * CB) = make_uint4(o[t][0], o[t][1], o[t][2], o[t][3]);
+                }
             }
         }
-        *reinterpret_cast<uint4 *>(o + (size_t)kb * hw * CB) = requant_pack16(acc, a.lshift, a.rshift, a.mult);
-    }
     }
 }
 
@@ -1142,6 +1231,69 @@ int conv2d_u8_ring(const small_b200_layer *L, const uint8_t *in, const uint8_t *
 
 namespace
 {
+// Layers whose whole reduction is at most 32 bytes and whose padding is a byte.
+bool one_step_covers(const small_b200_layer *L)
+{
+    return (long long)L->C * L->Fh * L->Fw <= 32 && (L->C < CB || (L->Fh == 1 && L->Fw == 1)) && L->zero_in <= 0 && L->zero_in >= -255 &&
+           L->K <= 1024;
+}
+// ... and which the kernel does faster than the tensor cores.  2048 images, us, this kernel and those: 16 -> 32 channels at
+// 24x24 27 and 49, 16 -> 64 48 and 68, 16 -> 128 at 12x12 25 and 29; but 32 -> 32 at 24x24 37 and 34, and a few images of 32
+// channels 5 and 4.
+bool one_step_preferred(const small_b200_layer *L)
+{
+    return one_step_covers(L) && (L->C < CB || (L->C == CB && L->K <= 128));
+}
+
+template <int WORDS, int KIND>
+int launch_onestep(const OneArgs &a, const uint8_t *in, const uint8_t *filt, const int32_t *bias, uint8_t *out, cudaStream_t st)
+{
+    const size_t smem = (size_t)a.K * (WORDS + 1) * 4; // at most 36 KB
+    constexpr int PX = 2;
+    const long long sms = num_sms(), many = (long long)PX * 256;
+    if (a.total >= sms * many) // four pixels a thread once that leaves a CTA for every SM
+    {
+        const long long nb = std::min((a.total + many - 1) / many, sms * 8);
+        conv2d_u8_onestep_kernel<WORDS, KIND, PX><<<(unsigned)nb, 256, smem, st>>>(a, in, filt, bias, out);
+    }
+    else
+        conv2d_u8_onestep_kernel<WORDS, KIND, 1><<<(unsigned)((a.total + 255) / 256), 256, smem, st>>>(a, in, filt, bias, out);
+    return launched("conv2d_u8_onestep_kernel");
+}
+
+// -1: not covered.
+int conv2d_u8_onestep(const small_b200_layer *L, const QArgs &q, const uint8_t *in, const uint8_t *filt, const int32_t *bias, uint8_t *out,
+                      cudaStream_t st)
+{
+    const long long px = (long long)q.Ho * q.Wo;
+    if (!one_step_covers(L) || row_stride(L) != q.stride || px > 0x3fffffffLL || reinterpret_cast<uintptr_t>(in) % 16 ||
+        reinterpret_cast<uintptr_t>(out) % 16)
+        return -1;
+    OneArgs a{};
+    a.H = q.H; a.W = q.W; a.Ho = q.Ho; a.Wo = q.Wo; a.C = q.C; a.K = q.K; a.Fh = q.Fh; a.Fw = q.Fw; a.R = q.C * q.Fh * q.Fw;
+    a.stride = q.stride; a.pad_t = q.pad_t; a.pad_l = q.pad_l;
+    a.zero_in = q.zero_in; a.sum_a = 128 + q.zero_filt;
+    a.lshift = q.lshift; a.rshift = q.rshift; a.mult = q.mult; a.k_zero = q.k_zero;
+    a.by_hw.set((int)px); a.by_Wo.set(q.Wo);
+    // images in portions of less than 2^30 pixels
+    const long long per = 0x3fffffffLL / px, in_image = (long long)q.C * q.H * q.W, out_image = px * q.K;
+    for (long long n = 0; n < q.N; n += per)
+    {
+        const long long images = std::min(per, (long long)q.N - n);
+        a.total = (int)(images * px);
+        a.in_bytes = images * in_image;
+        const uint8_t *x = in + n * in_image;
+        uint8_t *y = out + n * out_image;
+        const int rc = q.C >= 2 * CB                                ? launch_onestep<8, ONE_1X1>(a, x, filt, bias, y, st)
+                       : q.C == CB                                  ? launch_onestep<4, ONE_1X1>(a, x, filt, bias, y, st)
+                       : q.C == 3 && q.Fh == 3 && q.Fw == 3 ? launch_onestep<7, ONE_333>(a, x, filt, bias, y, st)
+                                                                    : launch_onestep<8, ONE_FIRST>(a, x, filt, bias, y, st);
+        if (rc)
+            return rc;
+    }
+    return SMALL_B200_OK;
+}
+
 // path: 0 = the faster kernel for the shape, 1 = CUDA cores only, 2 = tensor cores or an error
 int conv2d_u8_dispatch(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
                        uint8_t *out, void *stream, int path)
@@ -1167,50 +1319,31 @@ int conv2d_u8_dispatch(const small_b200_layer *L, const uint8_t *in, const uint8
         requant_in_place_kernel<<<1, 1024, 0, as_stream(stream)>>>(a.Ho * a.Wo, a, out);
         return launched("requant_in_place_kernel");
     }
-    const int tc = tensor_core ? conv2d_u8_tensor_core(L, in, filt, bias, out, as_stream(stream)) : -1;
-    if (tc >= 0)
-        return tc;
     QArgs a; fill(L, a, true);
     if (a.N == 0 || a.Ho == 0 || a.Wo == 0)
         return SMALL_B200_OK;
+    if (path == 0 && L->C >= CB && one_step_preferred(L))
+    {
+        const int one = conv2d_u8_onestep(L, a, in, filt, bias, out, as_stream(stream));
+        if (one >= 0)
+            return one;
+    }
+    const int tc = tensor_core ? conv2d_u8_tensor_core(L, in, filt, bias, out, as_stream(stream)) : -1;
+    if (tc >= 0)
+        return tc;
     if (tensor_core)
     {
         const int tc1 = conv2d_u8_one_channel_tc(L, in, filt, bias, out, as_stream(stream));
         if (tc1 >= 0)
             return tc1;
     }
-    // A reduction of one 32-byte step (a 1x1 layer on 16 channels, a 3x3 first layer on 3) is a streaming
-    // layer with nothing for the tensor core to do: measured on MobileNet-v1 0.25 uint8 at batch 2048, the
-    // implicit GEMM takes 0.43 ms for the 3x3x3 first layer and 0.188 ms for 16 -> 16 channels (the direct
-    // kernel 0.35 and 0.185), and wins from 16 -> 32 channels on (0.052 against 0.097 ms).  Those layers
-    // run the one-step dp4a kernel when the zero points let the operands enter shifted.
-    const long long red = (long long)L->C * L->Fh * L->Fw;
-    const bool ring_first = red > 32 || (L->C >= CB && L->K >= 32);
-    if (path != 2 && !(tensor_core && ring_first) && red <= 32 && (L->C < CB || (L->Fh == 1 && L->Fw == 1)) &&
-        a.zero_filt == -128 && (a.zero_in == 0 || a.zero_in == -128) && a.K <= 1024 &&
-        reinterpret_cast<uintptr_t>(in) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0)
+    if (path == 1 || (path == 0 && one_step_preferred(L)))
     {
-        const int words = (int)((red + 3) / 4);
-        const size_t smem = (size_t)(a.K / CB) * words * CB * sizeof(unsigned);
-        const long long total = (long long)a.N * a.Ho * a.Wo;
-        long long nb = (total + 255) / 256;
-        if (nb > (long long)num_sms() * 16)
-            nb = (long long)num_sms() * 16;
-        const unsigned blocks = (unsigned)nb;
-        const bool sgn = a.zero_in != 0, first = L->C < CB;
-        cudaStream_t st = as_stream(stream);
-        if (first && a.C == 3 && a.Fh == 3 && a.Fw == 3)
-            sgn ? conv2d_u8_onestep_kernel<true, true, true><<<blocks, 256, smem, st>>>(a, words, in, filt, bias, out)
-                : conv2d_u8_onestep_kernel<false, true, true><<<blocks, 256, smem, st>>>(a, words, in, filt, bias, out);
-        else if (first)
-            sgn ? conv2d_u8_onestep_kernel<true, true><<<blocks, 256, smem, st>>>(a, words, in, filt, bias, out)
-                : conv2d_u8_onestep_kernel<false, true><<<blocks, 256, smem, st>>>(a, words, in, filt, bias, out);
-        else
-            sgn ? conv2d_u8_onestep_kernel<true, false><<<blocks, 256, smem, st>>>(a, words, in, filt, bias, out)
-                : conv2d_u8_onestep_kernel<false, false><<<blocks, 256, smem, st>>>(a, words, in, filt, bias, out);
-        return launched("conv2d_u8_onestep_kernel");
+        const int one = conv2d_u8_onestep(L, a, in, filt, bias, out, as_stream(stream));
+        if (one >= 0)
+            return one;
     }
-    if (path == 2 || (tensor_core && ring_first))
+    if (tensor_core)
     {
         const int tc2 = conv2d_u8_ring(L, in, filt, bias, out, as_stream(stream));
         if (tc2 >= 0)

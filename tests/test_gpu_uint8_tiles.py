@@ -45,7 +45,8 @@ def test_depthwise_3x3_tiles(oracle, case, zp):
     assert want.min() < want.max()
 
 
-@pytest.mark.parametrize("case", [(32, 16, 8, 8, 5), (256, 256, 3, 3, 31), (64, 128, 6, 6, 8), (128, 32, 1, 2, 130), (96, 48, 5, 13, 4)],
+@pytest.mark.parametrize("case", [(32, 16, 8, 8, 5), (256, 256, 3, 3, 31), (64, 128, 6, 6, 8), (128, 32, 1, 2, 130), (96, 48, 5, 13, 4),
+                                  (32, 64, 12, 12, 17), (64, 32, 24, 24, 3), (32, 16, 3, 43, 140)],
                          ids=lambda c: "C{}_K{}_{}x{}_n{}".format(*c))
 @pytest.mark.parametrize("zp", [(0, -128), (-113, -121)], ids=lambda z: "zi{}_zf{}".format(*z))
 def test_pointwise_tiles_of_several_images(oracle, case, zp):
@@ -78,3 +79,29 @@ def test_global_average_pool_sizes(oracle, hw):
     S.AveragePool2D(H, W, 1, 0, 0, 0, 0, C, H, W, I, O, batch=N)
     want = np.stack([oracle.pool2d_u8(sh, q, x[n], average=True) for n in range(N)])
     assert np.array_equal(O.numpy().reshape(N, -1), want)
+
+
+@pytest.mark.parametrize("case", [
+    # C, K, H, W, Fh, Fw, stride, pads, batch
+    (16, 32, 24, 24, 1, 1, 1, (0, 0, 0, 0), 3),
+    (16, 128, 9, 9, 1, 1, 2, (1, 1, 1, 1), 2),
+    (16, 16, 300, 300, 1, 1, 1, (0, 0, 0, 0), 2),   # two pixels a thread, the last ones past the end
+    (32, 16, 7, 5, 1, 1, 1, (0, 0, 0, 0), 3),
+    (3, 16, 15, 17, 3, 3, 1, (1, 1, 1, 1), 3),
+    (3, 16, 400, 401, 3, 3, 2, (2, 3, 2, 3), 2),    # windows of nothing but padding
+    (2, 32, 11, 9, 3, 4, 1, (3, 0, 0, 3), 2),
+], ids=lambda c: "C{}_K{}_{}x{}_k{}x{}_s{}_p{}_n{}".format(*c))
+@pytest.mark.parametrize("zp", [(0, -128), (-113, -121), (-255, -250)], ids=lambda z: "zi{}_zf{}".format(*z))
+def test_reductions_of_one_step(oracle, case, zp):
+    C, K, H, W, Fh, Fw, s, pads, N = case
+    rng = np.random.default_rng(C + K + H)
+    q = _quant(rng, C * Fh * Fw, zp)
+    x = P.pack_activation(rng.integers(0, 256, (N, C, H, W)).astype(np.uint8))
+    w = P.pack_conv_filter(rng.integers(0, 256, (K, C, Fh, Fw)).astype(np.uint8))
+    sh = shape(C, K, H, W, Fh, Fw, s, pads, CB)
+    ho, wo = sh.out_hw()
+    I, F, O = qbuf(x, zp[0]), qbuf(w, zp[1]), _out(N * K * ho * wo, q)
+    S.Conv2D(Fh, Fw, s, *pads, K, C, H, W, I, F, O, batch=N, path="cuda_cores")
+    want = np.stack([oracle.conv2d_u8(sh, q, x[n], w) for n in range(N)])
+    assert np.array_equal(O.numpy().reshape(N, -1), want)
+    assert want.min() < want.max()
