@@ -42,7 +42,9 @@ struct RingArgs
     int cbs;      // input channel blocks (1 for a first layer)
     int steps;    // reduction steps of 32 bytes
     int tiles;    // ceil(N * Ho * Wo / 128)
-    int nblocks;  // K / NT
+    int nblocks;  // ceil(K / NT); the last one may have fewer channels
+    int jpairs;   // pairs of input channel blocks
+    FastDiv by_hw, by_Wo, by_fwc, by_C;
     int zero_in, zero_filt;
     int lshift, rshift, mult, k_zero;
 };
@@ -106,7 +108,9 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
                 const int tap = i / NT, k = i - tap * NT;
                 const int kg = nb * (NT / CB) + k / CB, k16 = k % CB;
                 int sum = 0;
-                if (FIRST)
+                if (kg * CB >= a.K)
+                    ;
+                else if (FIRST)
                     for (int c = 0; c < a.C; ++c)
                         sum += filt[((size_t)kg * kmax + (size_t)tap * a.C + c) * CB + k16];
                 else
@@ -121,7 +125,7 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
     tc_fence_after_sync();
     if (tid < NT)
     {
-        int c = a.k_zero + (bias ? bias[nb * NT + tid] : 0);
+        int c = a.k_zero + (bias && nb * NT + tid < a.K ? bias[nb * NT + tid] : 0);
         if (GENERAL && a.zero_in != 0)
         {
             int all = 0;
@@ -144,9 +148,9 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
             const int buf = i & 1;
             const long long g = (long long)tile * TILE_M + tid;
             const bool live = g < total_px;
-            const int n = live ? (int)(g / ((long long)a.Ho * a.Wo)) : 0;
-            const int px = live ? (int)(g - (long long)n * a.Ho * a.Wo) : 0;
-            const int oh = px / a.Wo, ow = px - oh * a.Wo;
+            const int n = live ? a.by_hw.div((int)g) : 0;
+            const int px = live ? (int)g - n * a.Ho * a.Wo : 0;
+            const int oh = a.by_Wo.div(px), ow = px - oh * a.Wo;
             const int ih0 = oh * a.row_stride - a.pad_t, iw0 = ow * a.stride - a.pad_l;
             const bool border = GENERAL && a.zero_in != 0 &&
                                 (ih0 < 0 || iw0 < 0 || ih0 + a.Fh > a.H || iw0 + a.Fw > a.W);
@@ -167,6 +171,8 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
 #pragma unroll
             for (int c0 = 0; c0 < NT; c0 += 16)
             {
+                if (nb * NT + c0 >= a.K)
+                    break;
                 uint32_t r[16];
                 tmem_ld16(lane_base + c0, r);
                 tmem_ld_wait();
@@ -208,19 +214,27 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
         // ---- producers: thread = (pixel row of the tile, which 16-byte chunk of the step)
         const int pt = tid - EPI_WARPS * 32;
         const int row = pt & (TILE_M - 1), half = pt >> 7;
-        const int jpairs = (a.cbs + 1) / 2;
         const unsigned flip_a = (!GENERAL && a.zero_in != 0) ? 0x80808080u : 0u;
         const unsigned flip_b = GENERAL ? 0u : 0x80808080u;
         // this thread's piece of the filter slice: 16-byte row `brow` of chunk `bhalf` of channel group `bgrp`
-        const bool has_b = pt < NT * 2;
         const int bgrp = pt >> 5, bhalf = (pt >> 4) & 1, brow = pt & 15;
+        const bool has_b = pt < NT * 2 && (nb * (NT / CB) + bgrp) * CB < a.K; // beyond K: whatever the stage holds, never stored
         bool ok = true;
         // The (tile, reduction step) pairs of this CTA form one sequence; a thread keeps the loads of
         // IN_FLIGHT consecutive pairs outstanding, across tile boundaries, before it stores any of them.
+        // Where a pair is follows from the one before it: divisions (by multiplication) only where a tile begins.
         const unsigned my_tiles = ((unsigned)a.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
         const unsigned units = my_tiles * (unsigned)a.steps;
-        const unsigned hw_out = (unsigned)(a.Ho * a.Wo);
-        const int fwc = a.Fw * a.C;
+        int tile = blockIdx.x, q = 0, kh = 0, kw = 0, j = 0; // of the next pair to load
+        bool live = false;
+        int ih0 = 0, iw0 = 0;
+        const uint8_t *img = in;
+        const uint8_t *brow_ptr = filt; // this thread's piece of the filter, at tap 0 and pair 0
+        if (has_b)
+            brow_ptr += FIRST ? ((size_t)(nb * (NT / CB) + bgrp) * kmax + bhalf * 16 + brow) * CB
+                              : ((size_t)(nb * (NT / CB) + bgrp) * a.cbs + bhalf) * taps * (CB * CB) + (size_t)brow * CB;
+        const long long plane = (long long)a.H * a.W * CB;
+        unsigned slot = 0, use = 0;
         for (unsigned w0 = 0; w0 < units && ok; w0 += IN_FLIGHT)
         {
             uint4 va[IN_FLIGHT], vb[IN_FLIGHT];
@@ -232,15 +246,16 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
                 const unsigned w = w0 + u;
                 if (w >= units)
                     continue;
-                const unsigned ti = w / (unsigned)a.steps;
-                const int q = (int)(w - ti * (unsigned)a.steps);
-                const unsigned g = (blockIdx.x + ti * gridDim.x) * TILE_M + row;
-                const bool live = g < total_px;
-                const unsigned n = live ? g / hw_out : 0u;
-                const unsigned px = live ? g - n * hw_out : 0u;
-                const int oh = (int)(px / (unsigned)a.Wo), ow = (int)px - oh * a.Wo;
-                const int ih0 = oh * a.row_stride - a.pad_t, iw0 = ow * a.stride - a.pad_l;
-                const uint8_t *img = in + (size_t)n * a.C * a.H * a.W;
+                if (q == 0)
+                {
+                    const unsigned g = (unsigned)tile * TILE_M + row;
+                    live = g < total_px;
+                    const int n = live ? a.by_hw.div((int)g) : 0, px = live ? (int)g - n * a.Ho * a.Wo : 0;
+                    const int oh = a.by_Wo.div(px), ow = px - oh * a.Wo;
+                    ih0 = oh * a.row_stride - a.pad_t; iw0 = ow * a.stride - a.pad_l;
+                    img = in + (size_t)n * a.C * a.H * a.W;
+                    kh = kw = j = 0;
+                }
                 if (FIRST)
                 {
                     // reduction index k = (kh * Fw + kw) * C + c, 16 of them per chunk; the three
@@ -249,9 +264,9 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
                     unsigned wv[4] = {0u, 0u, 0u, 0u};
                     if (live && k0 < kmax)
                     {
-                        int kh = k0 / fwc;
-                        const int r = k0 - kh * fwc;
-                        int kw = r / a.C, c = r - kw * a.C;
+                        int kh = a.by_fwc.div(k0);
+                        const int r = k0 - kh * a.Fw * a.C;
+                        int kw = a.by_C.div(r), c = r - kw * a.C;
 #pragma unroll
                         for (int b = 0; b < 16; ++b)
                         {
@@ -278,32 +293,33 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
                         const int k = q * 32 + bhalf * 16 + brow;
                         if (k < kmax) // filter [K/16][Fh*Fw*C rows][16]
                         {
-                            const uint4 v = *reinterpret_cast<const uint4 *>(
-                                filt + (((size_t)(nb * (NT / CB) + bgrp)) * kmax + k) * CB);
+                            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(brow_ptr + (size_t)q * 32 * CB));
                             vb[u] = make_uint4(v.x ^ flip_b, v.y ^ flip_b, v.z ^ flip_b, v.w ^ flip_b);
                         }
                     }
                 }
                 else
                 {
-                    const int tap = q / jpairs, j = q - tap * jpairs;
-                    const int kh = tap / a.Fw, kw = tap - kh * a.Fw;
                     const int cb = 2 * j + half;
                     const int ih = ih0 + kh, iw = iw0 + kw;
                     if (live && cb < a.cbs && ih >= 0 && ih < a.H && iw >= 0 && iw < a.W)
                     {
-                        const uint4 v = *reinterpret_cast<const uint4 *>(img + (((size_t)cb * a.H + ih) * a.W + iw) * CB);
+                        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(img + (cb * plane + ((long long)ih * a.W + iw) * CB)));
                         va[u] = make_uint4(v.x ^ flip_a, v.y ^ flip_a, v.z ^ flip_a, v.w ^ flip_a);
                     }
                     const int cbb = 2 * j + bhalf;
                     if (has_b && cbb < a.cbs) // filter [K/16][C/16][Fh][Fw][16 c][16 k]
                     {
-                        const uint4 v = *reinterpret_cast<const uint4 *>(
-                            filt + ((((size_t)(nb * (NT / CB) + bgrp)) * a.cbs + cbb) * taps + tap) * (CB * CB) +
-                            (size_t)brow * CB);
+                        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(brow_ptr + ((size_t)2 * j * taps + kh * a.Fw + kw) * (CB * CB)));
                         vb[u] = make_uint4(v.x ^ flip_b, v.y ^ flip_b, v.z ^ flip_b, v.w ^ flip_b);
                     }
+                    if (++j == a.jpairs)
+                    {
+                        j = 0;
+                        if (++kw == a.Fw) { kw = 0; ++kh; }
+                    }
                 }
+                if (++q == a.steps) { q = 0; tile += gridDim.x; }
             }
 #pragma unroll
             for (int u = 0; u < IN_FLIGHT; ++u)
@@ -311,7 +327,7 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
                 const unsigned w = w0 + u;
                 if (w >= units || !ok)
                     continue;
-                const unsigned s = w % STAGES, use = w / STAGES;
+                const unsigned s = slot;
                 if (use > 0) // every lane waits; the outcome is made the same for the whole warp
                     ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], (use - 1) & 1u, status, 32));
                 if (ok)
@@ -326,6 +342,7 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
                     if (lane == 0)
                         mbar_arrive(&full_bar[s]);
                 }
+                if (++slot == STAGES) { slot = 0; ++use; }
             }
         }
     }
@@ -440,8 +457,14 @@ int conv2d_u8_ring(const small_b200_layer *L, const uint8_t *in, const uint8_t *
     a.tiles = (int)((px + TILE_M - 1) / TILE_M);
     a.zero_in = L->zero_in; a.zero_filt = L->zero_filt;
     a.lshift = L->lshift; a.rshift = L->rshift; a.mult = L->multiplier; a.k_zero = L->k_zero;
-    const int nt = (L->K % 128 == 0) ? 128 : (L->K % 64 == 0) ? 64 : (L->K % 32 == 0) ? 32 : 16;
-    a.nblocks = L->K / nt;
+    // Every block of output channels gathers the pixels again, so: as few blocks as possible, then as few channels as those
+    // need (176 channels are two blocks of 128, not eleven of 16).
+    int nt = 128;
+    while (nt > 16 && (L->K + nt / 2 - 1) / (nt / 2) == (L->K + nt - 1) / nt)
+        nt /= 2;
+    a.nblocks = (L->K + nt - 1) / nt;
+    a.jpairs = (a.cbs + 1) / 2;
+    a.by_hw.set(a.Ho * a.Wo); a.by_Wo.set(a.Wo); a.by_fwc.set(a.Fw * a.C); a.by_C.set(a.C);
 #define SB_RING(NT_)                                                                                                  \
     (first ? (general ? launch_ring<NT_, true, true>(a, in, filt, bias, out, st)                                     \
                       : launch_ring<NT_, true, false>(a, in, filt, bias, out, st))                                   \
