@@ -14,12 +14,19 @@
 //   * filter zero point -128 with activation zero point 0 or -128 -- every quantised network here: the
 //     operands enter as signed / unsigned bytes already shifted, a tap outside the image is a zero byte,
 //     and the accumulator needs no correction at all;
-//   * anything else: both operands enter as unsigned bytes with zero bytes outside the image, so the MMA
-//     gives sum(a * b) over the valid taps.  zero_filt * sum(a) comes from sixteen extra accumulator
-//     columns whose filter column is all ones; zero_in * sum(b) + n * zero_in * zero_filt is a
-//     per-channel constant for interior pixels, and pixels at the border take away the per-tap channel
-//     sums (a table in shared memory, built once per CTA) of the taps they do not have.
+//   * anything else: both operands enter as unsigned bytes, so the MMA gives sum(a * b).  zero_filt * sum(a) comes from
+//     sixteen extra accumulator columns whose filter column is all ones; zero_in * sum(b) + n * zero_in * zero_filt is a
+//     per-channel constant.  A tap outside the image holds the byte -zero_in, whose (a + zero_in) is nothing; where that
+//     is no byte it holds zero, and pixels at the border take away the per-tap channel sums (a table in shared memory, built once
+//     per CTA) of the taps they do not have.
 // The int32 partial-sum form stays on the CUDA-core kernel.
+//
+// What bounds it: the producers (a step is 4 KB of pixels in 16-byte pieces, a load, a store and some thirty instructions
+// each) and, in layers of a few tiles an SM, the time from a load to its MMA.  Four loads are always on their way, replaced one
+// by one; zero points are folded in as late as the store, since an instruction on a loaded value waits for it.
+// us with six divisions per piece, loads in groups of four and a correction of every border pixel -> now: 3x3, 64 -> 64
+// channels at 41x41, 48 images 52 -> 29, with zero points -113 and -121 55 -> 34; 128 -> 128 at 14x14, 16 images 35 -> 20; one
+// image of 64 channels at 14x14 17.5 -> 10.5.
 //
 // First layers (1 to 3 channels, [H][W][C] activation, filter [K/16][1][Fh][Fw][C][16]) take the same
 // route with the reduction index running over (kernel row, kernel column, channel) byte by byte.
@@ -101,23 +108,42 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
             *reinterpret_cast<uint4 *>(smem + (size_t)st * G::STAGE + G::A_BYTES + (size_t)(NT / CB) * 2 * CB * CB + (size_t)r * CB) =
                 make_uint4(1u, 0u, 0u, 0u);
         }
-        // channel sums of the filter per tap, needed only where the activation zero point is not zero
+        // channel sums of the filter per tap, needed only where the activation zero point is not zero: a thread adds the rows
+        // of up to 16 channels, 16 output channels at a time
         if (a.zero_in != 0)
+        {
             for (int i = tid; i < taps * NT; i += THREADS)
+                tapsum[i] = 0;
+            __syncthreads();
+            const int parts = FIRST ? 1 : a.cbs, groups = min(NT / CB, a.K / CB - nb * (NT / CB));
+            for (int i = tid; i < taps * groups * parts; i += THREADS)
             {
-                const int tap = i / NT, k = i - tap * NT;
-                const int kg = nb * (NT / CB) + k / CB, k16 = k % CB;
-                int sum = 0;
-                if (kg * CB >= a.K)
-                    ;
-                else if (FIRST)
-                    for (int c = 0; c < a.C; ++c)
-                        sum += filt[((size_t)kg * kmax + (size_t)tap * a.C + c) * CB + k16];
-                else
-                    for (int c = 0; c < a.C; ++c)
-                        sum += filt[((((size_t)kg * a.cbs + c / CB) * taps) + tap) * (CB * CB) + (size_t)(c % CB) * CB + k16];
-                tapsum[i] = sum;
+                const int gp = i / taps, tap = i - gp * taps, grp = gp / parts, part = gp - grp * parts, kg = nb * (NT / CB) + grp;
+                const uint4 *w = reinterpret_cast<const uint4 *>(
+                    filt + (FIRST ? ((size_t)kg * kmax + (size_t)tap * a.C) * CB : (((size_t)kg * a.cbs + part) * taps + tap) * (CB * CB)));
+                unsigned even[4] = {0u, 0u, 0u, 0u}, odd[4] = {0u, 0u, 0u, 0u}; // pairs of sums of at most 16 bytes
+#pragma unroll
+                for (int c = 0; c < CB; ++c)
+                    if (!FIRST || c < a.C)
+                    {
+                        const uint4 v = __ldg(w + c);
+                        const unsigned x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                        {
+                            even[k] += x[k] & 0x00ff00ffu;
+                            odd[k] += (x[k] >> 8) & 0x00ff00ffu;
+                        }
+                    }
+                int *t = tapsum + tap * NT + grp * CB;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                {
+                    atomicAdd(t + 4 * k, (int)(even[k] & 0xffffu)); atomicAdd(t + 4 * k + 1, (int)(odd[k] & 0xffffu));
+                    atomicAdd(t + 4 * k + 2, (int)(even[k] >> 16)); atomicAdd(t + 4 * k + 3, (int)(odd[k] >> 16));
+                }
             }
+        }
         fence_proxy_async();
     }
     tc_fence_before_sync();
@@ -152,7 +178,7 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
             const int px = live ? (int)g - n * a.Ho * a.Wo : 0;
             const int oh = a.by_Wo.div(px), ow = px - oh * a.Wo;
             const int ih0 = oh * a.row_stride - a.pad_t, iw0 = ow * a.stride - a.pad_l;
-            const bool border = GENERAL && a.zero_in != 0 &&
+            const bool border = GENERAL && (a.zero_in > 0 || a.zero_in < -255) &&
                                 (ih0 < 0 || iw0 < 0 || ih0 + a.Fh > a.H || iw0 + a.Fw > a.W);
             ok = mbar_wait(&acc_full[buf], (i >> 1) & 1, status, 31);
             if (!ok)
@@ -216,6 +242,8 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
         const int row = pt & (TILE_M - 1), half = pt >> 7;
         const unsigned flip_a = (!GENERAL && a.zero_in != 0) ? 0x80808080u : 0u;
         const unsigned flip_b = GENERAL ? 0u : 0x80808080u;
+        // what a tap outside the image holds until it is stored
+        const unsigned outside = GENERAL ? (a.zero_in <= 0 && a.zero_in >= -255 ? (unsigned)-a.zero_in * 0x01010101u : 0u) : flip_a;
         // this thread's piece of the filter slice: 16-byte row `brow` of chunk `bhalf` of channel group `bgrp`
         const int bgrp = pt >> 5, bhalf = (pt >> 4) & 1, brow = pt & 15;
         const bool has_b = pt < NT * 2 && (nb * (NT / CB) + bgrp) * CB < a.K; // beyond K: whatever the stage holds, never stored
@@ -234,93 +262,94 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
             brow_ptr += FIRST ? ((size_t)(nb * (NT / CB) + bgrp) * kmax + bhalf * 16 + brow) * CB
                               : ((size_t)(nb * (NT / CB) + bgrp) * a.cbs + bhalf) * taps * (CB * CB) + (size_t)brow * CB;
         const long long plane = (long long)a.H * a.W * CB;
-        unsigned slot = 0, use = 0;
+        unsigned slot = 0, use = 0, loaded = 0;
+        auto load = [&](uint4 &x, uint4 &f) { // the next pair, if there is one
+            x = make_uint4(flip_a, flip_a, flip_a, flip_a); // zero once stored
+            f = make_uint4(flip_b, flip_b, flip_b, flip_b);
+            if (loaded >= units)
+                return;
+            ++loaded;
+            if (q == 0)
+            {
+                const unsigned g = (unsigned)tile * TILE_M + row;
+                live = g < total_px;
+                const int n = live ? a.by_hw.div((int)g) : 0, px = live ? (int)g - n * a.Ho * a.Wo : 0;
+                const int oh = a.by_Wo.div(px), ow = px - oh * a.Wo;
+                ih0 = oh * a.row_stride - a.pad_t; iw0 = ow * a.stride - a.pad_l;
+                img = in + (size_t)n * a.C * a.H * a.W;
+                kh = kw = j = 0;
+            }
+            if (FIRST)
+            {
+                // reduction index k = (kh * Fw + kw) * C + c, 16 of them per chunk; the three
+                // counters advance byte by byte
+                const int k0 = q * 32 + half * 16;
+                unsigned wv[4] = {flip_a, flip_a, flip_a, flip_a};
+                if (live && k0 < kmax)
+                {
+                    int kh = a.by_fwc.div(k0);
+                    const int r = k0 - kh * a.Fw * a.C;
+                    int kw = a.by_C.div(r), c = r - kw * a.C;
+#pragma unroll
+                    for (int b = 0; b < 16; ++b)
+                    {
+                        const int ih = ih0 + kh, iw = iw0 + kw;
+                        if (kh < a.Fh)
+                        {
+                            const unsigned v = ih >= 0 && ih < a.H && iw >= 0 && iw < a.W ? (unsigned)img[((size_t)ih * a.W + iw) * a.C + c]
+                                                                                          : outside & 0xffu;
+                            wv[b >> 2] = (wv[b >> 2] & ~(0xffu << (8 * (b & 3)))) | v << (8 * (b & 3));
+                        }
+                        if (++c == a.C)
+                        {
+                            c = 0;
+                            if (++kw == a.Fw)
+                            {
+                                kw = 0;
+                                ++kh;
+                            }
+                        }
+                    }
+                }
+                x = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+                if (has_b)
+                {
+                    const int k = q * 32 + bhalf * 16 + brow;
+                    if (k < kmax) // filter [K/16][Fh*Fw*C rows][16]
+                    {
+                        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(brow_ptr + (size_t)q * 32 * CB));
+                        f = v;
+                    }
+                }
+            }
+            else
+            {
+                const int cb = 2 * j + half;
+                const int ih = ih0 + kh, iw = iw0 + kw;
+                if (live && cb < a.cbs && ih >= 0 && ih < a.H && iw >= 0 && iw < a.W)
+                    x = __ldg(reinterpret_cast<const uint4 *>(img + (cb * plane + ((long long)ih * a.W + iw) * CB)));
+                else if (GENERAL && cb < a.cbs)
+                    x = make_uint4(outside, outside, outside, outside);
+                const int cbb = 2 * j + bhalf;
+                if (has_b && cbb < a.cbs) // filter [K/16][C/16][Fh][Fw][16 c][16 k]
+                {
+                    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(brow_ptr + ((size_t)2 * j * taps + kh * a.Fw + kw) * (CB * CB)));
+                    f = v;
+                }
+                if (++j == a.jpairs)
+                {
+                    j = 0;
+                    if (++kw == a.Fw) { kw = 0; ++kh; }
+                }
+            }
+            if (++q == a.steps) { q = 0; tile += gridDim.x; }
+        };
+        uint4 va[IN_FLIGHT], vb[IN_FLIGHT];
+#pragma unroll
+        for (int u = 0; u < IN_FLIGHT; ++u)
+            load(va[u], vb[u]);
         for (unsigned w0 = 0; w0 < units && ok; w0 += IN_FLIGHT)
         {
-            uint4 va[IN_FLIGHT], vb[IN_FLIGHT];
-#pragma unroll
-            for (int u = 0; u < IN_FLIGHT; ++u)
-            {
-                va[u] = make_uint4(0u, 0u, 0u, 0u);
-                vb[u] = make_uint4(0u, 0u, 0u, 0u);
-                const unsigned w = w0 + u;
-                if (w >= units)
-                    continue;
-                if (q == 0)
-                {
-                    const unsigned g = (unsigned)tile * TILE_M + row;
-                    live = g < total_px;
-                    const int n = live ? a.by_hw.div((int)g) : 0, px = live ? (int)g - n * a.Ho * a.Wo : 0;
-                    const int oh = a.by_Wo.div(px), ow = px - oh * a.Wo;
-                    ih0 = oh * a.row_stride - a.pad_t; iw0 = ow * a.stride - a.pad_l;
-                    img = in + (size_t)n * a.C * a.H * a.W;
-                    kh = kw = j = 0;
-                }
-                if (FIRST)
-                {
-                    // reduction index k = (kh * Fw + kw) * C + c, 16 of them per chunk; the three
-                    // counters advance byte by byte
-                    const int k0 = q * 32 + half * 16;
-                    unsigned wv[4] = {0u, 0u, 0u, 0u};
-                    if (live && k0 < kmax)
-                    {
-                        int kh = a.by_fwc.div(k0);
-                        const int r = k0 - kh * a.Fw * a.C;
-                        int kw = a.by_C.div(r), c = r - kw * a.C;
-#pragma unroll
-                        for (int b = 0; b < 16; ++b)
-                        {
-                            const int ih = ih0 + kh, iw = iw0 + kw;
-                            if (kh < a.Fh && ih >= 0 && ih < a.H && iw >= 0 && iw < a.W)
-                            {
-                                const unsigned v = (unsigned)img[((size_t)ih * a.W + iw) * a.C + c] ^ (flip_a & 0xffu);
-                                wv[b >> 2] |= v << (8 * (b & 3));
-                            }
-                            if (++c == a.C)
-                            {
-                                c = 0;
-                                if (++kw == a.Fw)
-                                {
-                                    kw = 0;
-                                    ++kh;
-                                }
-                            }
-                        }
-                    }
-                    va[u] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-                    if (has_b)
-                    {
-                        const int k = q * 32 + bhalf * 16 + brow;
-                        if (k < kmax) // filter [K/16][Fh*Fw*C rows][16]
-                        {
-                            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(brow_ptr + (size_t)q * 32 * CB));
-                            vb[u] = make_uint4(v.x ^ flip_b, v.y ^ flip_b, v.z ^ flip_b, v.w ^ flip_b);
-                        }
-                    }
-                }
-                else
-                {
-                    const int cb = 2 * j + half;
-                    const int ih = ih0 + kh, iw = iw0 + kw;
-                    if (live && cb < a.cbs && ih >= 0 && ih < a.H && iw >= 0 && iw < a.W)
-                    {
-                        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(img + (cb * plane + ((long long)ih * a.W + iw) * CB)));
-                        va[u] = make_uint4(v.x ^ flip_a, v.y ^ flip_a, v.z ^ flip_a, v.w ^ flip_a);
-                    }
-                    const int cbb = 2 * j + bhalf;
-                    if (has_b && cbb < a.cbs) // filter [K/16][C/16][Fh][Fw][16 c][16 k]
-                    {
-                        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(brow_ptr + ((size_t)2 * j * taps + kh * a.Fw + kw) * (CB * CB)));
-                        vb[u] = make_uint4(v.x ^ flip_b, v.y ^ flip_b, v.z ^ flip_b, v.w ^ flip_b);
-                    }
-                    if (++j == a.jpairs)
-                    {
-                        j = 0;
-                        if (++kw == a.Fw) { kw = 0; ++kh; }
-                    }
-                }
-                if (++q == a.steps) { q = 0; tile += gridDim.x; }
-            }
 #pragma unroll
             for (int u = 0; u < IN_FLIGHT; ++u)
             {
@@ -333,16 +362,19 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
                 if (ok)
                 {
                     uint8_t *st = smem + (size_t)s * G::STAGE;
-                    *reinterpret_cast<uint4 *>(st + (size_t)half * TILE_M * CB + (size_t)row * CB) = va[u];
+                    *reinterpret_cast<uint4 *>(st + (size_t)half * TILE_M * CB + (size_t)row * CB) =
+                        make_uint4(va[u].x ^ flip_a, va[u].y ^ flip_a, va[u].z ^ flip_a, va[u].w ^ flip_a);
                     if (has_b)
                         *reinterpret_cast<uint4 *>(st + G::A_BYTES + (size_t)bgrp * 2 * CB * CB + (size_t)bhalf * CB * CB +
-                                                   (size_t)brow * CB) = vb[u];
+                                                   (size_t)brow * CB) =
+                            make_uint4(vb[u].x ^ flip_b, vb[u].y ^ flip_b, vb[u].z ^ flip_b, vb[u].w ^ flip_b);
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0)
                         mbar_arrive(&full_bar[s]);
                 }
                 if (++slot == STAGES) { slot = 0; ++use; }
+                load(va[u], vb[u]);
             }
         }
     }

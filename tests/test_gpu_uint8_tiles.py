@@ -105,3 +105,27 @@ def test_reductions_of_one_step(oracle, case, zp):
     want = np.stack([oracle.conv2d_u8(sh, q, x[n], w) for n in range(N)])
     assert np.array_equal(O.numpy().reshape(N, -1), want)
     assert want.min() < want.max()
+
+
+@pytest.mark.parametrize("case", [
+    # C, K, H, W, Fh, Fw, stride, pads, batch
+    (48, 176, 9, 14, 3, 3, 1, (1, 1, 1, 1), 2),     # a second block of 48 channels of 128
+    (16, 80, 11, 7, 3, 3, 2, (0, 1, 0, 1), 3),      # one block of 80 of 128
+    (32, 48, 5, 5, 5, 3, 1, (2, 2, 1, 1), 12),      # one block of 48 of 64, several tiles
+    (3, 48, 9, 8, 5, 5, 2, (2, 2, 2, 2), 5),
+], ids=lambda c: "C{}_K{}_{}x{}_k{}x{}_s{}_p{}_n{}".format(*c))
+@pytest.mark.parametrize("zp", [(0, -128), (-113, -121), (4, -7)], ids=lambda z: "zi{}_zf{}".format(*z))
+def test_implicit_gemm_with_a_partial_block_of_channels(oracle, case, zp):
+    C, K, H, W, Fh, Fw, s, pads, N = case
+    rng = np.random.default_rng(C + K + H)
+    q = _quant(rng, C * Fh * Fw, zp)
+    x = P.pack_activation(rng.integers(0, 256, (N, C, H, W)).astype(np.uint8))
+    w = P.pack_conv_filter(rng.integers(0, 256, (K, C, Fh, Fw)).astype(np.uint8))
+    sh = shape(C, K, H, W, Fh, Fw, s, pads, CB)
+    ho, wo = sh.out_hw()
+    I, F, O = qbuf(x, zp[0]), qbuf(w, zp[1]), _out(N * K * ho * wo, q)
+    S.Conv2D(Fh, Fw, s, *pads, K, C, H, W, I, F, O, batch=N, path="tensor_core")
+    want = np.stack([oracle.conv2d_u8(sh, q, x[n], w) for n in range(N)])
+    assert _lib.device_status() == 0
+    assert np.array_equal(O.numpy().reshape(N, -1), want)
+    assert want.min() < want.max()
