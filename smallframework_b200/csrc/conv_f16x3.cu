@@ -522,12 +522,14 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                 }
             }
         }
-        else if (warp >= 1 && warp <= (PIXM ? 3 : 2) && lane == 0)
+        else if (warp >= 1 && warp <= (PIXM ? 3 : 2))
         {
             // ---------------- MMA issuers ----------------
             // All descriptor fields except the 16-byte-granular start address are fixed per CTA,
             // and a new operand position is one 64-bit add on a precomputed descriptor.  A = filter
             // tap (M = channels), B = patch shifted by the tap (N = pixels).
+            // The warps stay together and an elected lane issues: the operands then live in uniform registers, 42 cycles for
+            // an MMA of few columns where a lane on its own took 56 to 60 (ResNet-8 at 1024 images 440 -> 429 us).
             // Issuing one MMA costs a thread about as long as the tensor pipe needs for it
             // (measured: one thread sustains an N = 192 MMA every 122 cycles, the pipe takes 96;
             // two threads together reach the 96), and whatever the thread does between two groups
@@ -575,7 +577,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                 const uint64_t w_tap = (uint64_t)T.kv * 4, w_lo_off = (uint64_t)T.kv;
                 for (int cb = 0; cb < cbs_l && ok; ++cb)
                 {
-                    ok = mbar_wait(&x_ready[slot], xphase, status, 13);
+                    ok = __all_sync(0xffffffffu, mbar_wait(&x_ready[slot], xphase, status, 13));
                     if (!ok)
                         break;
                     uint64_t x_row = x_desc0 + x_slot_off; // patch position of tap (kh, 0)
@@ -590,87 +592,92 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                             ok = mbar_wait(&w_full[st], a.w_resident ? 0u : (uint32_t)wphase, status, 14);
                             if (ok && g > tb_mask)
                                 ok = mbar_wait(&t_empty[g & tb_mask], ((g >> tb_shift) - 1) & 1, status, 16);
+                            ok = __all_sync(0xffffffffu, ok);
                             if (!ok)
                                 break;
                             tc_fence_after_sync();
-                            uint64_t wh = w_desc0 + w_stage_off, xh = x_row;
-                            if (PIXM && MERGED)
+                            if (elect_one())
                             {
-                                // [W_hi | W_lo] is one operand of 2K columns: x_hi times it gives the hi*hi sums in
-                                // columns [0, K) and one cross term in [K, 2K), x_lo * W_hi adds the other cross
-                                // term there.  Two instructions per tap and 128 pixels instead of three, the 128-pixel
-                                // operand read from shared memory twice instead of three times, and the small terms
-                                // never meet a full-size accumulator; the accumulation warps add the two halves.
-                                const uint32_t d0 = tmem + (uint32_t)((g & tb_mask) * mtiles * 2 * a.K);
-                                int kw = 0;
-                                for (int tp = 0; tp < a.group; ++tp, wh += w_tap, xh += tap_step)
+                                uint64_t wh = w_desc0 + w_stage_off, xh = x_row;
+                                if (PIXM && MERGED)
                                 {
-                                    for (int mt = 0; mt < mtiles; ++mt)
+                                    // [W_hi | W_lo] is one operand of 2K columns: x_hi times it gives the hi*hi sums in
+                                    // columns [0, K) and one cross term in [K, 2K), x_lo * W_hi adds the other cross
+                                    // term there.  Two instructions per tap and 128 pixels instead of three, the 128-pixel
+                                    // operand read from shared memory twice instead of three times, and the small terms
+                                    // never meet a full-size accumulator; the accumulation warps add the two halves.
+                                    const uint32_t d0 = tmem + (uint32_t)((g & tb_mask) * mtiles * 2 * a.K);
+                                    int kw = 0;
+                                    for (int tp = 0; tp < a.group; ++tp, wh += w_tap, xh += tap_step)
                                     {
-                                        const uint64_t xa = xh + (uint64_t)mt * 512;
-                                        const uint32_t d = d0 + (uint32_t)(mt * 2 * a.K);
-                                        tc_mma_f16(d, xa, wh, idesc_wide, tp == 0 ? 0u : 1u);
-                                        tc_mma_f16(d + (uint32_t)a.K, xa + x_lo_off, wh, idesc, 1u);
+                                        for (int mt = 0; mt < mtiles; ++mt)
+                                        {
+                                            const uint64_t xa = xh + (uint64_t)mt * 512;
+                                            const uint32_t d = d0 + (uint32_t)(mt * 2 * a.K);
+                                            tc_mma_f16(d, xa, wh, idesc_wide, tp == 0 ? 0u : 1u);
+                                            tc_mma_f16(d + (uint32_t)a.K, xa + x_lo_off, wh, idesc, 1u);
+                                        }
+                                        if (++kw == a.Fw) // on to the next patch row (0 where a group is one row)
+                                        {
+                                            kw = 0;
+                                            xh += (uint64_t)a.row_skip;
+                                        }
                                     }
-                                    if (++kw == a.Fw) // on to the next patch row (0 where a group is one row)
+                                }
+                                else if (PIXM)
+                                {
+                                    const uint32_t d0 = tmem + (uint32_t)((g & tb_mask) * mtiles * a.K);
+                                    // The small cross terms of the whole group first, the hi*hi terms last: the
+                                    // tensor core adds into its accumulator with truncation, an error of one ulp OF
+                                    // THE ACCUMULATOR per MMA, so only the MMAs issued while it holds full-size sums
+                                    // (one per tap instead of three) contribute a full-size error.
+                                    uint64_t wh2 = wh, xh2 = xh;
+                                    int kw = 0, kw2 = 0;
+                                    for (int tp = 0; tp < a.group; ++tp, wh += w_tap, xh += tap_step)
                                     {
-                                        kw = 0;
-                                        xh += (uint64_t)a.row_skip;
+                                        const uint64_t wl = wh + w_lo_off;
+                                        for (int mt = 0; mt < mtiles; ++mt)
+                                        {
+                                            const uint64_t xa = xh + (uint64_t)mt * 512; // 128 pixels on
+                                            const uint32_t d = d0 + (uint32_t)(mt * a.K);
+                                            tc_mma_f16(d, xa, wl, idesc, tp == 0 ? 0u : 1u);
+                                            tc_mma_f16(d, xa + x_lo_off, wh, idesc, 1u);
+                                        }
+                                        if (++kw == a.Fw) { kw = 0; xh += (uint64_t)a.row_skip; }
                                     }
-                                }
-                            }
-                            else if (PIXM)
-                            {
-                                const uint32_t d0 = tmem + (uint32_t)((g & tb_mask) * mtiles * a.K);
-                                // The small cross terms of the whole group first, the hi*hi terms last: the
-                                // tensor core adds into its accumulator with truncation, an error of one ulp OF
-                                // THE ACCUMULATOR per MMA, so only the MMAs issued while it holds full-size sums
-                                // (one per tap instead of three) contribute a full-size error.
-                                uint64_t wh2 = wh, xh2 = xh;
-                                int kw = 0, kw2 = 0;
-                                for (int tp = 0; tp < a.group; ++tp, wh += w_tap, xh += tap_step)
-                                {
-                                    const uint64_t wl = wh + w_lo_off;
-                                    for (int mt = 0; mt < mtiles; ++mt)
+                                    for (int tp = 0; tp < a.group; ++tp, wh2 += w_tap, xh2 += tap_step)
                                     {
-                                        const uint64_t xa = xh + (uint64_t)mt * 512; // 128 pixels on
-                                        const uint32_t d = d0 + (uint32_t)(mt * a.K);
-                                        tc_mma_f16(d, xa, wl, idesc, tp == 0 ? 0u : 1u);
-                                        tc_mma_f16(d, xa + x_lo_off, wh, idesc, 1u);
+                                        for (int mt = 0; mt < mtiles; ++mt)
+                                            tc_mma_f16(d0 + (uint32_t)(mt * a.K), xh2 + (uint64_t)mt * 512, wh2, idesc, 1u);
+                                        if (++kw2 == a.Fw) { kw2 = 0; xh2 += (uint64_t)a.row_skip; }
                                     }
-                                    if (++kw == a.Fw) { kw = 0; xh += (uint64_t)a.row_skip; }
                                 }
-                                for (int tp = 0; tp < a.group; ++tp, wh2 += w_tap, xh2 += tap_step)
+                                else
                                 {
-                                    for (int mt = 0; mt < mtiles; ++mt)
-                                        tc_mma_f16(d0 + (uint32_t)(mt * a.K), xh2 + (uint64_t)mt * 512, wh2, idesc, 1u);
-                                    if (++kw2 == a.Fw) { kw2 = 0; xh2 += (uint64_t)a.row_skip; }
+                                    const uint32_t d = tmem + (uint32_t)((g & tb_mask) * a.NPX);
+                                    uint64_t wh2 = wh, xh2 = xh; // cross terms first, hi*hi last (see the pixel-major loop)
+                                    int kw = 0, kw2 = 0;
+                                    for (int tp = 0; tp < a.group; ++tp, wh += w_tap, xh += tap_step)
+                                    {
+                                        tc_mma_f16(d, wh + w_lo_off, xh, idesc, tp == 0 ? 0u : 1u);
+                                        tc_mma_f16(d, wh, xh + x_lo_off, idesc, 1u);
+                                        if (++kw == a.Fw) { kw = 0; xh += (uint64_t)a.row_skip; }
+                                    }
+                                    for (int tp = 0; tp < a.group; ++tp, wh2 += w_tap, xh2 += tap_step)
+                                    {
+                                        tc_mma_f16(d, wh2, xh2, idesc, 1u);
+                                        if (++kw2 == a.Fw) { kw2 = 0; xh2 += (uint64_t)a.row_skip; }
+                                    }
                                 }
+                                // the stage is free for the producer and the group's partial sums are
+                                // complete for the accumulation warps: one commit serves both while the
+                                // accumulator ring is no deeper than the filter ring (a waiter must not fall
+                                // two phases behind its barrier)
+                                tc_commit(&g_done[st]);
+                                if (own_t_full)
+                                    tc_commit(&t_full[g & tb_mask]);
                             }
-                            else
-                            {
-                                const uint32_t d = tmem + (uint32_t)((g & tb_mask) * a.NPX);
-                                uint64_t wh2 = wh, xh2 = xh; // cross terms first, hi*hi last (see the pixel-major loop)
-                                int kw = 0, kw2 = 0;
-                                for (int tp = 0; tp < a.group; ++tp, wh += w_tap, xh += tap_step)
-                                {
-                                    tc_mma_f16(d, wh + w_lo_off, xh, idesc, tp == 0 ? 0u : 1u);
-                                    tc_mma_f16(d, wh, xh + x_lo_off, idesc, 1u);
-                                    if (++kw == a.Fw) { kw = 0; xh += (uint64_t)a.row_skip; }
-                                }
-                                for (int tp = 0; tp < a.group; ++tp, wh2 += w_tap, xh2 += tap_step)
-                                {
-                                    tc_mma_f16(d, wh2, xh2, idesc, 1u);
-                                    if (++kw2 == a.Fw) { kw2 = 0; xh2 += (uint64_t)a.row_skip; }
-                                }
-                            }
-                            // the stage is free for the producer and the group's partial sums are
-                            // complete for the accumulation warps: one commit serves both while the
-                            // accumulator ring is no deeper than the filter ring (a waiter must not fall
-                            // two phases behind its barrier)
-                            tc_commit(&g_done[st]);
-                            if (own_t_full)
-                                tc_commit(&t_full[g & tb_mask]);
+                            __syncwarp();
                         }
                         if (++turn == NISS)
                             turn = 0;
@@ -678,7 +685,9 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                         w_stage_off += w_stage_step;
                         if (++st == a.w_stages) { st = 0; wphase ^= 1; w_stage_off = 0; }
                     }
-                    tc_commit(&x_empty[slot]); // both issuers: the slot is free once the MMAs of either are done
+                    if (elect_one())
+                        tc_commit(&x_empty[slot]); // all issuers: the slot is free once the MMAs of each are done
+                    __syncwarp();
                     x_slot_off += x_slot_step;
                     if (++slot == a.x_slots) { slot = 0; xphase ^= 1; x_slot_off = 0; }
                 }
