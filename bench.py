@@ -615,10 +615,16 @@ MEASURED_TRAFFIC = {
 def kernel_class(chain, i, L, dtype):
     """Which kernel runs layer i (with the layers it absorbs) and what bounds it."""
     follow = chain.absorbed(i)
+    if i in chain.tails:
+        return "pool_dense_softmax_f32_kernel", "stream"
     if L["op"] == "conv":
         if dtype == "f32":
+            if i in chain.small:
+                return "conv_small_f32_kernel (FFMA, latency)", "ffma"
             if chain.prepared[i] is not None:
-                return "conv_f16x3_kernel (tcgen05 kind::f16, two-word operands)" + (" + 2x2 max pool" if follow else ""), "tf32x3"
+                return "conv_f16x3_kernel (tcgen05 kind::f16, two-word operands)" + (" + 2x2 max pool" if follow else ""), "f16x3"
+            if L["stride"] > 1 and L["C"] >= 16:
+                return "conv_gather_f32_kernel (tcgen05 kind::tf32, two-word operands)", "tf32x3"
             name = "conv2d_first_f32_kernel (FFMA)" if L["C"] < 16 else "conv2d_f32_kernel (FFMA)"
             return name + (" + 2x2 max pool" if follow else ""), "ffma"
         if follow:
@@ -630,12 +636,14 @@ def kernel_class(chain, i, L, dtype):
         ho, wo = networks_out_hw(L)
         if L["C"] == 1 and L["Fw"] <= 4 and L["Fh"] <= 16 and ho * wo <= 128 and L["K"] <= 128:
             return "stem_u8_tc_kernel (im2col in shared memory + tcgen05 kind::i8)", "i8"
-        if L["C"] * L["Fh"] * L["Fw"] > 32 or (L["C"] >= 16 and L["K"] >= 32):
+        if L["C"] * L["Fh"] * L["Fw"] > 32 or (L["C"] >= 16 and L["K"] > 128):
             return "conv_u8_ring_kernel (implicit GEMM, tcgen05 kind::i8)", "i8"
         return "conv2d_u8_onestep_kernel (dp4a, streaming)", "stream"
     if L["op"] == "dwconv" and dtype == "u8":
-        rows = L["Fh"] == 3 and L["Fw"] == 3 and L["stride"] == 1
-        return ("dwconv3x3_u8_rows_kernel (dp4a)" if rows else "dwconv_u8_dp4a_kernel"), "stream"
+        tiles = L["Fh"] == 3 and L["Fw"] == 3 and L["stride"] == 1
+        return ("dwconv3x3_u8_tile_kernel (dp4a)" if tiles else "dwconv_u8_dp4a_kernel"), "stream"
+    if i in chain.blocks:
+        return "dwpw_f32_kernel (depthwise 3x3 + 1x1 on tcgen05 kind::tf32, two-word operands)", "tf32x3"
     return {"dwconv": "window_f32_kernel (depthwise)", "maxpool": "max pool", "avgpool": "average pool",
             "softmax": "softmax", "alias": "alias"}[L["op"]], "stream"
 
@@ -649,7 +657,8 @@ def per_layer_report(chain, layers, batch, wl, clocks, torch, pipes=None):
     """Times every launch of the step alone with CUDA events on the launching stream and charges it
     against its roofline: t_roof = max(flops / pipe peak, bytes / HBM peak).  Pipe peaks are MEASURED on
     this GPU (small_b200_peak_probe): the fp32 FMA pipe for CUDA-core convolutions, one third of the tf32
-    tensor rate for the 3xTF32 convolution (three MMAs per product), the i8 tensor rate for uint8
+    tensor rate where an fp32 result takes three tf32 MMAs per product and two thirds of it where it takes three of
+    kind::f16 (twice the tf32 rate), the i8 tensor rate for uint8
     tensor-core layers.  A launch that runs several layers (a producer and what it absorbs) is charged the
     flops of all of them and the bytes it has to move: the first layer's input, the last one's output, all
     the weights.  fp32 layers at their batch read inputs far larger than L2; the uint8 networks' layers are
@@ -658,7 +667,7 @@ def per_layer_report(chain, layers, batch, wl, clocks, torch, pipes=None):
     peaks = load_peaks()
     if pipes is None:
         pipes = measured_pipes(torch)
-    pipe_tops = {"ffma": pipes["ffma"], "tf32x3": pipes["tf32"] / 3.0, "i8": pipes["i8"],
+    pipe_tops = {"ffma": pipes["ffma"], "tf32x3": pipes["tf32"] / 3.0, "f16x3": pipes["tf32"] * 2.0 / 3.0, "i8": pipes["i8"],
                  "cuda_u8": pipes["ffma"], "stream": pipes["ffma"]}
     elt = chain.elt
     st = chain.stream.cuda_stream
@@ -701,7 +710,7 @@ def per_layer_report(chain, layers, batch, wl, clocks, torch, pipes=None):
         rows.append({"layer": "+".join(layers[k].get("name", layers[k]["op"]) for k in group), "kernel": kname,
                      "ms": round(ms, 4), "tflops": round(flops / (ms * 1e-3) / 1e12, 3),
                      "gbs": round(nbytes / (ms * 1e-3) / 1e9, 1),
-                     "bound": ("tensor" if kcls in ("tf32x3", "i8") else "fp32 pipe") if t_flop > t_mem else "hbm",
+                     "bound": ("tensor" if kcls in ("tf32x3", "f16x3", "i8") else "fp32 pipe") if t_flop > t_mem else "hbm",
                      "pipe": kcls, "roofline_frac": round(max(t_flop, t_mem) / (ms * 1e-3), 4)})
     top = max(range(len(rows)), key=lambda i: rows[i]["ms"])
     flops, nbytes = work[top]
@@ -717,6 +726,8 @@ def per_layer_report(chain, layers, batch, wl, clocks, torch, pipes=None):
                 "pipe": {"peak": pipe_tops[kcls], "frac": achieved / pipe_tops[kcls],
                          "note": {"tf32x3": "fp32 result from three tf32 MMAs per product: one third of the tf32 "
                                             "tensor rate measured on this GPU in this run",
+                                  "f16x3": "fp32 result from three kind::f16 MMAs per product: two thirds of the tf32 "
+                                           "tensor rate measured on this GPU in this run",
                                   "ffma": "fp32 FMA pipe measured on this GPU in this run",
                                   "i8": "i8 tensor rate measured on this GPU in this run"}.get(kcls, "")}}
     else:
