@@ -438,7 +438,12 @@ constexpr int FIRST_W_SLOTS = 4;
 constexpr int FIRST_W_FLOATS = 3 * 3 * 3 * CB;
 __constant__ float c_first_w[FIRST_W_SLOTS][FIRST_W_FLOATS];
 
-template <int C, int FH, int FW, bool POOL = true, int SLOT = -1>
+// S = 2 (POOL = false): the same for a stride of two, with blocks of 1x2 outputs (3 x 5 x 3 inputs; 2x2 blocks of 5 x 5 x 3
+// leave the SM three CTAs and took 188 us for the layer below).  Rows whose blocks start on 16 bytes
+// (no left padding, a width that is a multiple of 4) come as four 16-byte loads instead of 15 of four bytes, 48 bytes
+// apart from lane to lane either way.  One output pixel a thread with its filter from shared memory took 231 us for
+// 2048 images of 96x96 (81 at copy bandwidth), nearly all of it filter fetches; this takes 140.
+template <int C, int FH, int FW, bool POOL = true, int SLOT = -1, int S = 1>
 __global__ void __launch_bounds__(128)
 conv2d_first_pool_fixed_f32_kernel(const ConvArgs a, const float *__restrict__ in, const float *__restrict__ filt,
                                    const float *__restrict__ bias, float *__restrict__ out)
@@ -455,7 +460,8 @@ conv2d_first_pool_fixed_f32_kernel(const ConvArgs a, const float *__restrict__ i
         __syncthreads();
     }
     const float *w = SLOT < 0 ? w_s : c_first_w[SLOT < 0 ? 0 : SLOT];
-    const int Hp = a.Ho / 2, Wp = a.Wo / 2;
+    constexpr int BH = S == 1 ? 2 : 1, OUT = 2 * BH; // rows and outputs of a block
+    const int Hp = a.Ho / BH, Wp = a.Wo / 2;
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = p < Hp * Wp;
     if (!live)
@@ -466,15 +472,35 @@ conv2d_first_pool_fixed_f32_kernel(const ConvArgs a, const float *__restrict__ i
     }
     const int ph = p / Wp, pw = p - ph * Wp;
     const float *img = in + (size_t)n * C * a.H * a.W;
-    const int ih0 = 2 * ph - a.pad_t, iw0 = 2 * pw - a.pad_l;
-    float x[FH + 1][FW + 1][C];
+    const int ih0 = BH * S * ph - a.pad_t, iw0 = 2 * S * pw - a.pad_l;
+    constexpr int XH = FH + S * (BH - 1), XW = FW + S;
+    float x[XH][XW][C];
+    const bool quads = S == 2 && a.pad_l == 0 && a.W % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0;
 #pragma unroll
-    for (int dr = 0; dr <= FH; ++dr)
+    for (int dr = 0; dr < XH; ++dr)
     {
         const int ih = ih0 + dr;
         const bool rok = ih >= 0 && ih < a.H;
+        if (S == 2 && quads) // a block starts at a multiple of four pixels: the first four are in the row, the fifth perhaps not
+        {
+            const float4 *row = reinterpret_cast<const float4 *>(img + ((size_t)(rok ? ih : 0) * a.W + iw0) * C);
+            float v[4 * C + 4];
 #pragma unroll
-        for (int dc = 0; dc <= FW; ++dc)
+            for (int j = 0; j <= C; ++j)
+            {
+                const bool ok = rok && iw0 < a.W && (j < C || iw0 + 4 < a.W);
+                const float4 f = ok ? __ldg(row + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[4 * j] = f.x; v[4 * j + 1] = f.y; v[4 * j + 2] = f.z; v[4 * j + 3] = f.w;
+            }
+#pragma unroll
+            for (int dc = 0; dc < XW; ++dc)
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+                    x[dr][dc][c] = dc * C + c < 4 * C + 4 ? v[dc * C + c < 4 * C + 4 ? dc * C + c : 0] : 0.f;
+            continue;
+        }
+#pragma unroll
+        for (int dc = 0; dc < XW; ++dc)
         {
             const int iw = iw0 + dc;
             const bool ok = rok && iw >= 0 && iw < a.W;
@@ -484,12 +510,14 @@ conv2d_first_pool_fixed_f32_kernel(const ConvArgs a, const float *__restrict__ i
                 x[dr][dc][c] = ok ? __ldg(px + c) : 0.f; // a padded tap adds nothing
         }
     }
-    float acc[4][CB];
+    float acc[OUT][CB];
 #pragma unroll
     for (int k = 0; k < CB; ++k)
     {
         const float s = bias ? bias[kb * CB + k] : 0.f;
-        acc[0][k] = s; acc[1][k] = s; acc[2][k] = s; acc[3][k] = s;
+#pragma unroll
+        for (int o = 0; o < OUT; ++o)
+            acc[o][k] = s;
     }
 #pragma unroll
     for (int kh = 0; kh < FH; ++kh)
@@ -505,9 +533,9 @@ conv2d_first_pool_fixed_f32_kernel(const ConvArgs a, const float *__restrict__ i
                     const float4 wv = SLOT < 0 ? reinterpret_cast<const float4 *>(wt)[k4]
                                                : make_float4(wt[4 * k4], wt[4 * k4 + 1], wt[4 * k4 + 2], wt[4 * k4 + 3]);
 #pragma unroll
-                    for (int o = 0; o < 4; ++o)
+                    for (int o = 0; o < OUT; ++o)
                     {
-                        const float xv = x[(o >> 1) + kh][(o & 1) + kw][c];
+                        const float xv = x[(o >> 1) * S + kh][(o & 1) * S + kw][c];
                         float *ac = acc[o] + k4 * 4;
                         ac[0] = fmaf(xv, wv.x, ac[0]); ac[1] = fmaf(xv, wv.y, ac[1]);
                         ac[2] = fmaf(xv, wv.z, ac[2]); ac[3] = fmaf(xv, wv.w, ac[3]);
@@ -522,7 +550,7 @@ conv2d_first_pool_fixed_f32_kernel(const ConvArgs a, const float *__restrict__ i
         const float ns = act_neg_scale(a.act, a.slope);
         float *plane = out + ((size_t)n * (a.K / CB) + kb) * a.Ho * a.Wo * CB;
 #pragma unroll
-        for (int dr = 0; dr < 2; ++dr)
+        for (int dr = 0; dr < BH; ++dr)
         {
 #pragma unroll
             for (int dc = 0; dc < 2; ++dc)
@@ -545,23 +573,26 @@ conv2d_first_pool_fixed_f32_kernel(const ConvArgs a, const float *__restrict__ i
                 {
                     const int pht = pt / Wp, pwt = pt - pht * Wp;
                     const float4 v = *reinterpret_cast<const float4 *>(stage[warp] + t * 36 + piece * 4);
-                    *reinterpret_cast<float4 *>(plane + ((size_t)(2 * pht + dr) * a.Wo + 2 * pwt) * CB + piece * 4) = v;
+                    *reinterpret_cast<float4 *>(plane + ((size_t)(BH * pht + dr) * a.Wo + 2 * pwt) * CB + piece * 4) = v;
                 }
             }
             __syncwarp();
         }
         return;
     }
-    float *o = out + (((size_t)n * (a.K / CB) + kb) * Hp * Wp + p) * CB;
-#pragma unroll
-    for (int k4 = 0; k4 < CB; k4 += 4)
+    if constexpr (POOL)
     {
-        float v[4];
+        float *o = out + (((size_t)n * (a.K / CB) + kb) * Hp * Wp + p) * CB;
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            v[q] = fmaxf(fmaxf(apply_act_ns(acc[0][k4 + q], act_neg_scale(a.act, a.slope)), apply_act_ns(acc[1][k4 + q], act_neg_scale(a.act, a.slope))),
-                         fmaxf(apply_act_ns(acc[2][k4 + q], act_neg_scale(a.act, a.slope)), apply_act_ns(acc[3][k4 + q], act_neg_scale(a.act, a.slope))));
-        *reinterpret_cast<float4 *>(o + k4) = make_float4(v[0], v[1], v[2], v[3]);
+        for (int k4 = 0; k4 < CB; k4 += 4)
+        {
+            float v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                v[q] = fmaxf(fmaxf(apply_act_ns(acc[0][k4 + q], act_neg_scale(a.act, a.slope)), apply_act_ns(acc[1][k4 + q], act_neg_scale(a.act, a.slope))),
+                             fmaxf(apply_act_ns(acc[2][k4 + q], act_neg_scale(a.act, a.slope)), apply_act_ns(acc[3][k4 + q], act_neg_scale(a.act, a.slope))));
+            *reinterpret_cast<float4 *>(o + k4) = make_float4(v[0], v[1], v[2], v[3]);
+        }
     }
 }
 
@@ -611,7 +642,7 @@ int first_layer_slot(const float *filt)
     return -1;
 }
 
-template <bool POOL>
+template <bool POOL, int S = 1>
 int launch_first_fixed(const ConvArgs &a, dim3 grid, const float *in, const float *filt, const float *bias, float *out,
                        cudaStream_t st)
 {
@@ -621,11 +652,11 @@ int launch_first_fixed(const ConvArgs &a, dim3 grid, const float *in, const floa
                                         (size_t)slot * FIRST_W_FLOATS * sizeof(float), cudaMemcpyDeviceToDevice, st));
     switch (slot)
     {
-    case 0: conv2d_first_pool_fixed_f32_kernel<3, 3, 3, POOL, 0><<<grid, 128, 0, st>>>(a, in, filt, bias, out); break;
-    case 1: conv2d_first_pool_fixed_f32_kernel<3, 3, 3, POOL, 1><<<grid, 128, 0, st>>>(a, in, filt, bias, out); break;
-    case 2: conv2d_first_pool_fixed_f32_kernel<3, 3, 3, POOL, 2><<<grid, 128, 0, st>>>(a, in, filt, bias, out); break;
-    case 3: conv2d_first_pool_fixed_f32_kernel<3, 3, 3, POOL, 3><<<grid, 128, 0, st>>>(a, in, filt, bias, out); break;
-    default: conv2d_first_pool_fixed_f32_kernel<3, 3, 3, POOL><<<grid, 128, 0, st>>>(a, in, filt, bias, out); break;
+    case 0: conv2d_first_pool_fixed_f32_kernel<3, 3, 3, POOL, 0, S><<<grid, 128, 0, st>>>(a, in, filt, bias, out); break;
+    case 1: conv2d_first_pool_fixed_f32_kernel<3, 3, 3, POOL, 1, S><<<grid, 128, 0, st>>>(a, in, filt, bias, out); break;
+    case 2: conv2d_first_pool_fixed_f32_kernel<3, 3, 3, POOL, 2, S><<<grid, 128, 0, st>>>(a, in, filt, bias, out); break;
+    case 3: conv2d_first_pool_fixed_f32_kernel<3, 3, 3, POOL, 3, S><<<grid, 128, 0, st>>>(a, in, filt, bias, out); break;
+    default: conv2d_first_pool_fixed_f32_kernel<3, 3, 3, POOL, -1, S><<<grid, 128, 0, st>>>(a, in, filt, bias, out); break;
     }
     return launched(POOL ? "conv2d_first_pool_fixed_f32_kernel" : "conv2d_first_fixed_f32_kernel");
 }
@@ -674,12 +705,13 @@ int conv2d_f32_impl(const small_b200_layer *L, int pool, const float *in, const 
             conv2d_first_pool_f32_kernel<<<grid, 128, smem, st>>>(a, in, filt, bias, out);
             return launched("conv2d_first_pool_f32_kernel");
         }
-        if (L->C == 3 && L->Fh == 3 && L->Fw == 3 && L->stride == 1 && a.sh == 1 && !L->accumulate && a.Ho % 2 == 0 &&
-            a.Wo % 2 == 0 && a.Ho > 0 && a.Wo > 0)
+        if (L->C == 3 && L->Fh == 3 && L->Fw == 3 && a.sh == L->stride && L->stride <= 2 && !L->accumulate &&
+            (L->stride == 2 || a.Ho % 2 == 0) && a.Wo % 2 == 0 && a.Ho > 0 && a.Wo > 0)
         {
-            // 2x2 output blocks from a register patch, rows written through shared memory
-            dim3 grid(((a.Ho / 2) * (a.Wo / 2) + 127) / 128, a.K / CB, a.N);
-            return launch_first_fixed<false>(a, grid, in, filt, bias, out, st);
+            // 2x2 output blocks (stride 2: 1x2) from a register patch, rows written through shared memory
+            dim3 grid(((L->stride == 2 ? a.Ho : a.Ho / 2) * (a.Wo / 2) + 127) / 128, a.K / CB, a.N);
+            return L->stride == 1 ? launch_first_fixed<false>(a, grid, in, filt, bias, out, st)
+                                  : launch_first_fixed<false, 2>(a, grid, in, filt, bias, out, st);
         }
         dim3 grid((a.Ho * a.Wo + 255) / 256, a.K / CB, a.N);
         conv2d_first_f32_kernel<<<grid, 256, smem, st>>>(a, in, filt, bias, out);

@@ -1,4 +1,5 @@
-"""The gathering tensor-core kernel that small_b200_conv2d_f32 takes for strided windows, against the oracle."""
+"""The kernels that small_b200_conv2d_f32 takes for strided windows, the gathering tensor-core one and the first layer's, against
+the oracle."""
 import ctypes as C
 
 import numpy as np
@@ -20,6 +21,11 @@ CASES = [
     (48, 48, 19, 3, 3, 3, 2, "same", 60),       # 27 steps, images shorter than a tile
     (336, 64, 9, 9, 3, 3, 2, "same", 6),        # 189 of at most 192 steps
     (368, 32, 11, 11, 3, 3, 2, "same", 6),      # 207: the other kernel
+    # first layers, in blocks of 1x2 outputs
+    (3, 16, 96, 96, 3, 3, 2, "same", 8),        # rows by 16-byte loads
+    (3, 32, 95, 95, 3, 3, 2, (1, 1, 1, 1), 6),
+    (3, 16, 97, 95, 3, 3, 2, (1, 1, 1, 1), 8),  # an odd number of rows
+    (3, 16, 92, 92, 3, 3, 2, (2, 3, 0, 5), 9),  # blocks of nothing but padding
 ]
 
 
