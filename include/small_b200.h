@@ -156,15 +156,18 @@ int small_b200_conv2d_maxpool_f32(const small_b200_layer *conv, const small_b200
                                   const float *filt, const float *bias, float *out, void *stream);
 /* The same layer on the tensor cores (tcgen05 kind::f16 on pairs of half-precision words, fp32
  * accumulation in tensor memory), stride 1 only.  Each fp32 operand x enters the tensor core as
- * hi = half(x * 2^e) and lo = half(x * 2^e - hi), 22 bits like the two words of a 3xTF32 split (which
- * the functions are named after); the power of two belongs to the filter as a whole and to each patch
- * of 16 input channels of a tile, brings its largest magnitude to at least 2^6 and at most 65504, and is
+ * hi = half(x * 2^e) and lo = half((x * 2^e - hi) * 2^10), 22 bits like the two words of a 3xTF32 split
+ * (which the functions are named after).  The power of two belongs to the filter (or to one output
+ * channel, where that is 2^12 and more below the largest) and to each patch of 16 input channels of a
+ * tile: each pixel's values keep 22 bits of the largest of its 16, and each channel's weights 22 bits
+ * or 2^-35 of the largest of that channel, whatever the magnitudes beside them (tiles whose pixels lie
+ * 2^26 and more apart are computed on the FMA pipe, many times more slowly).  The scales are
  * undone in fp32.  The activations are split inside the kernel, in shared memory.  The caller
  * provides the filter re-laid for the tensor core:
  *   filt_prepared  small_b200_filter_prepare_tf32x3(filt), once per set of weights,
  *                  2 * K*C*Fh*Fw floats: per CTA tile and tap the hi and lo halves as
- *                  [c/8][hi k | lo k][8 c] (what the tensor core reads directly), then the inverse
- *                  of the filter's scale.  The layout depends on K alone; treat it as opaque.
+ *                  [c/8][hi k | lo k][8 c] (what the tensor core reads directly), then the inverses
+ *                  of the scales.  The layout depends on K alone; treat it as opaque.
  * ..._supported() says whether a shape is covered (1) or not (0).  The reference has no
  * counterpart of the preparation call (its filters are used as packed). */
 int small_b200_conv2d_f32_tf32x3_supported(const small_b200_layer *L);

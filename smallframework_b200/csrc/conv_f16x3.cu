@@ -1,11 +1,21 @@
 // conv_f16x3.cu -- fp32 dense convolution (stride 1) on the 5th-generation tensor cores, every fp32 operand as a
 // pair of half-precision words with a block scale.
 //
-// Arithmetic.  v * 2^e = hi + lo with hi = half(v * 2^e), lo = half(v * 2^e - hi), both truncated: 11 + 11 bits, the
-// very words of a 3xTF32 split (where the tensor core itself drops the low bits of a tf32 operand).  A product is a_lo*b_hi + a_hi*b_lo + a_hi*b_hi in fp32 tensor memory; the
-// dropped a_lo*b_lo is 2^-22 relative.  The power of two 2^e belongs to a block -- the whole filter, and a tile's patch
-// of 16 input channels -- and brings its largest magnitude to 2^13 or more, so the pair keeps its 22 bits down to 2^-16
-// of that magnitude and an absolute error below 2^-38 of it under that; it is undone in the FMA with which the
+// Arithmetic.  v * 2^e = hi + lo * 2^-10 with hi = half(v * 2^e), lo = half((v * 2^e - hi) * 2^10), both truncated: 11 + 11
+// bits, the very words of a 3xTF32 split (where the tensor core itself drops the low bits of a tf32 operand).  A product
+// is a_lo*b_hi + a_hi*b_lo + a_hi*b_hi in fp32 tensor memory; the dropped a_lo*b_lo is below 2^-20 of it.  The cross terms are
+// summed first, and the first a_hi*b_hi brings them down by 2^-10 (an operand of the instruction), or they have columns of
+// their own.  Half precision has a narrow range, so the power of two 2^e belongs to a block.
+//   * Filter: all of it, or one output channel where that is 2^12 and more below the largest.  A weight keeps its 22 bits
+//     down to 2^-14 of its channel's largest (2^-26 with a scale of its own) and an error below 2^-35 of that beneath.
+//   * Activations: a tile's patch of 16 input channels.  Every pixel's sixteen values keep 22 bits of the largest of them,
+//     however large the pixels beside it: the scale brings the patch's largest to 2^6 at least, 22 bits reach down
+//     to 2^-13, a patch with a pixel below that gets the scale that brings its largest to 2^13, and a tile with a patch where
+//     that does not do either is computed on the FMA pipe (plain_tile).
+// So an output channel, an image or a pixel is as good as if it stood alone: the words of a value that is in range do not
+// depend on the power of two.  (With lo stored as it is, 22 bits ended at 2^-3 and an error of 2^-24 remained: an output channel 2^-12 of
+// the largest kept half its digits.  The scaled second word costs 0.5 to 1.5 % of a layer: Tiny-YOLOv2 on 64 images 1.576
+// -> 1.597 ms, ResNet-8 on 1024 426 -> 432 us.)  Scales are undone in the FMA with which the
 // accumulation warps add a partial sum to their fp32 registers.  kind::f16 covers 16 channels per instruction where
 // kind::tf32 covers 8 at the same cost (N/2 cycles of the pipe, 128 + N operand rows of 32 bytes), so a layer needs half
 // the instructions, half the operand traffic in shared memory and half the filter bytes of the 3xTF32 form this
@@ -47,6 +57,7 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cstring>
 
 namespace
@@ -56,6 +67,7 @@ using namespace sb;
 constexpr int W_STAGES_MAX = 6; // filter stages, each one group of taps (a kernel row)
 constexpr int X_SLOTS_MAX = 3;
 constexpr int BOX_PX = 32; // widest box of a TMA load: 256 elements of 8 bytes
+constexpr int WIDE_WORDS = 32; // a CTA's tiles, a bit each: a launch has at most 1024 for every CTA
 constexpr int SCALE_RING = 16; // patches whose block scale is remembered: slots + unflushed accumulator buffers, rounded up
 
 struct TcArgs
@@ -120,45 +132,56 @@ struct TcArgs
 // convolution agree.
 __host__ __device__ inline int pick_mt(int K) { return K >= 128 ? 128 : 64; }
 
-// Largest magnitude of the filter (finite values; the sign bit cleared, floats compare like integers).
+// Largest magnitude of every output channel's filter, and behind those of all of them (finite values; the sign bit cleared, floats compare like integers).
+// blockIdx.y: block of 16 channels, n: its values [slab][16 c][16 k]; a thread stays with one channel.
 __global__ void __launch_bounds__(256) filter_max_kernel(long long n, const float *__restrict__ w, uint32_t *__restrict__ top)
 {
     uint32_t m = 0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    w += (long long)blockIdx.y * n;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256)
     {
         const uint32_t b = __float_as_uint(__ldg(w + i)) & 0x7fffffffu;
         m = max(m, b < 0x7f800000u ? b : 0u);
     }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0 && m)
-        atomicMax(top, m);
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+    if ((threadIdx.x & 31) < 16 && m)
+    {
+        atomicMax(top + blockIdx.y * CB + (threadIdx.x & 15), m);
+        atomicMax(top + gridDim.y * CB, m);
+    }
 }
 
+// The second word of a pair is stored 2^LO_SHIFT times its value.  It is below an ulp of the first, 2^-10 of a value that
+// half precision holds, so it stays below 65536 -- and keeps its 11 bits wherever the first word keeps its own.
+constexpr int LO_SHIFT = 10;
+constexpr float LO_UP = 1 << LO_SHIFT, LO_DOWN = 1.f / LO_UP;
+// A pair has its 22 bits from FAINT = 2^-13 on: its last bit is then 2^-34, the least that the second word can hold.
+constexpr float FAINT = 1.f / 8192;
+constexpr uint32_t FAINT_SEEN = 0x7fffffffu; // the splitters' word for a patch with a row below that
+
 // Block scale of a set of operands whose largest magnitude has the bits `top`: the power of two that brings it
-// into [2^13, 2^14), and its inverse.  Exponents are held to where both are normal numbers.
+// into [2^13, 2^14), and its inverse.  Exponents are held to where both, and LO_UP times the first, are normal numbers.
 __device__ __forceinline__ float scale_up(uint32_t top)
 {
-    const uint32_t e = max(top >> 23, 15u);
+    const uint32_t e = max(top >> 23, 30u);
     return __uint_as_float((267u - e) << 23);
 }
 __device__ __forceinline__ float scale_down(uint32_t top)
 {
-    const uint32_t e = max(top >> 23, 15u);
+    const uint32_t e = max(top >> 23, 30u);
     return __uint_as_float((e - 13u) << 23);
 }
 
 // packed filter [K/16][slab][16 c][16 k] -> half-precision pairs [K/MT][slab][c/8][hi kv | lo kv][8 c]; kv = MT
-// except in a last, partial tile (K % MT channels).  head[0] = the inverse of the filter's block scale.
+// except in a last, partial tile (K % MT channels).  down[k] = the inverse of channel k's block scale, down[2 K + 1] = 1 if
+// it isn't the same for all of them, down[2 K + 2] = the inverse of the filter's scale.
 __global__ void __launch_bounds__(256)
 prepare_filter_kernel(long long n, int slabs, int MT, int K, const float *__restrict__ w, const uint32_t *__restrict__ top,
-                      __half *__restrict__ pairs, float *__restrict__ head)
+                      __half *__restrict__ pairs, float *__restrict__ down)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    const uint32_t t0 = *top;
-    if (i == 0)
-        head[0] = scale_down(t0);
     const int k16 = (int)(i & 15), c = (int)((i >> 4) & 15);
     const long long t = i >> 8;            // kb16 * slabs + slab
     const int slab = (int)(t % slabs);
@@ -167,10 +190,24 @@ prepare_filter_kernel(long long n, int slabs, int MT, int K, const float *__rest
     const int kv = (K - tile * MT) < MT ? (K - tile * MT) : MT;
     const long long o = ((long long)tile * MT * slabs * 16 + (long long)slab * kv * 16) * 2 +
                         (long long)(c >> 3) * kv * 16 + (long long)(k - tile * MT) * 8 + (c & 7);
+    // The filter's scale, or the channel's own where the filter's would bring its largest weight below 2^1 (2^12 below the
+    // largest of all): at 2^1 a pair keeps its 22 bits down to 2^-14 of it, and loses no more than 2^-35 of it below that.
+    // Channels that share a scale cost the pixel-major kernel nothing; one that does not, a multiplication per output.
+    const uint32_t all = top[K];
+    const bool own = top[k] && top[k] + (12u << 23) < all;
+    const uint32_t t0 = own ? top[k] : all;
+    if (slab == 0 && c == 0)
+    {
+        down[k] = scale_down(t0);
+        if (own)
+            down[2 * K + 1] = 1.f;
+        if (k == 0)
+            down[2 * K + 2] = scale_down(all);
+    }
     const float v = w[i] * scale_up(t0);
     const __half h = __float2half_rz(v);
     pairs[o] = h;
-    pairs[o + (long long)kv * 8] = __float2half_rz(v - __half2float(h));
+    pairs[o + (long long)kv * 8] = __float2half_rz((v - __half2float(h)) * LO_UP);
 }
 
 // Tensor-core accumulation truncates: every MMA adds into the fp32 accumulator with
@@ -196,15 +233,20 @@ constexpr int SPLIT_THREADS = 128;
 constexpr int NUM_THREADS = 512;
 constexpr int COLS_PER_THREAD = 128;
 
-// Two fp32 values, already multiplied by their block scale, as a pair of half-precision words: hi = v,
-// lo = v - hi, both cut to 11 bits as a tf32 operand is.  (Rounded to nearest the 9216-term sums come out at 3.0e-7 of the
+// Two fp32 values times their block scale as two pairs of half-precision words: hi = v,
+// lo = (v - hi) * 2^LO_SHIFT, both cut to 11 bits as a tf32 operand is.  (Rounded to nearest the 9216-term sums come out at 3.0e-7 of the
 // largest instead of 5.2e-7, but then results drift from the 3xTF32 form's by more than either is off: 2.5e-5 of a
 // YOLO head, whose box sizes are exponentials, against 2e-6 with the same words.)
-__device__ __forceinline__ void split2(float a, float b, uint32_t &hi, uint32_t &lo)
+// up_lo = up * LO_UP.  (v - hi) * LO_UP in one fma on the half-precision word itself: as many instructions as without the factor.
+__device__ __forceinline__ void split2(float a, float b, float up, float up_lo, uint32_t &hi, uint32_t &lo)
 {
-    asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
-    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
-    asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(b - f.y), "f"(a - f.x));
+    static_assert(LO_SHIFT == 10, "0xE400 is -2^10 in half precision");
+    asm("{\n\t.reg .f32 x, y;\n\t.reg .f16 h, g, m;\n\t"
+        "mul.rn.f32 x, %2, %4;\n\tmul.rn.f32 y, %3, %4;\n\tcvt.rz.f16x2.f32 %0, y, x;\n\t"
+        "mov.b32 {h, g}, %0;\n\tmov.b16 m, 0xE400;\n\t"
+        "mul.rn.f32 x, %2, %5;\n\tmul.rn.f32 y, %3, %5;\n\tfma.rn.f32.f16 x, h, m, x;\n\tfma.rn.f32.f16 y, g, m, y;\n\t"
+        "cvt.rz.f16x2.f32 %1, y, x;\n\t}"
+        : "=&r"(hi), "=r"(lo) : "f"(a), "f"(b), "f"(up), "f"(up_lo));
 }
 __device__ __forceinline__ uint32_t finite_abs(float v)
 {
@@ -231,13 +273,14 @@ __device__ __forceinline__ uint32_t split_reduce(uint32_t m, uint32_t *words, in
 }
 // U pieces of 8 channels (piece u = half u & 1 of patch row u / 2; u, u + 128, ...) into hi and lo halves, in place.
 // Returns the largest magnitude of those that belong to the patch (`valid` rows of the first plane, `valid2` of the
-// second, `entries` further on).  Neither the reads nor the writes are predicated -- rows behind the patch hold whatever
+// second, `entries` further on); `least` becomes the least bits - 1 of a piece's largest magnitude (a piece of zeros: 2^32 - 1).  Neither the reads nor the writes are predicated -- rows behind the patch hold whatever
 // the slot held before and are never stored from -- because the predicates cost more than the work: 1090 cycles for
 // 256 rows by four warps one predicated piece at a time, 950 four at a time, 440 without the predicates (shared memory
 // delivers about 74 bytes per cycle to loads and stores, which makes 430 the floor).
 template <int U>
-__device__ __forceinline__ float split_pieces(float4 *piece, int u0, float up, uint32_t entries, int valid, int valid2)
+__device__ __forceinline__ float split_pieces(float4 *piece, int u0, float up, uint32_t entries, int valid, int valid2, uint32_t &least)
 {
+    const float up_lo = up * LO_UP;
     float4 v[U][2];
     float fm = 0.f;
 #pragma unroll
@@ -253,12 +296,14 @@ __device__ __forceinline__ float split_pieces(float4 *piece, int u0, float up, u
     {
         const int u = u0 + q * SPLIT_THREADS, sw = (u >> 2) & 3, late = sw & 1, h = u & 1, r = u >> 1;
         uint4 hi, lo; // of the chunks in the order they were read
-        split2(v[q][0].x * up, v[q][0].y * up, hi.x, lo.x);
-        split2(v[q][0].z * up, v[q][0].w * up, hi.y, lo.y);
-        split2(v[q][1].x * up, v[q][1].y * up, hi.z, lo.z);
-        split2(v[q][1].z * up, v[q][1].w * up, hi.w, lo.w);
-        const float top = fmaxf(max_abs(v[q][0]), max_abs(v[q][1]));
-        fm = fmaxf(fm, (r < valid || (uint32_t)(r - (int)entries) < (uint32_t)valid2) ? top : 0.f);
+        split2(v[q][0].x, v[q][0].y, up, up_lo, hi.x, lo.x);
+        split2(v[q][0].z, v[q][0].w, up, up_lo, hi.y, lo.y);
+        split2(v[q][1].x, v[q][1].y, up, up_lo, hi.z, lo.z);
+        split2(v[q][1].z, v[q][1].w, up, up_lo, hi.w, lo.w);
+        float top = fmaxf(max_abs(v[q][0]), max_abs(v[q][1]));
+        top = (r < valid || (uint32_t)(r - (int)entries) < (uint32_t)valid2) ? top : 0.f;
+        fm = fmaxf(fm, top);
+        least = __viaddmin_u32(__float_as_uint(top), 0xffffffffu, least);
         uint4 *row = reinterpret_cast<uint4 *>(piece + (2 * u & ~3));
         // late rows: chunks read in the other order, lo half written first
         row[(h + 2 * late) ^ sw] = late ? make_uint4(lo.z, lo.w, lo.x, lo.y) : hi;
@@ -316,10 +361,122 @@ __device__ __forceinline__ Tile decode_tile(const TcArgs &a, int t)
 #define SB_TILE_LOOP(cond_extra) \
     for (int t = first_tile, once_ = 0; (PERSIST ? (t < a.total_tiles) : (once_ == 0)) && (cond_extra); t += tile_step, ++once_)
 
+// Sums of two output channels k, k + 1 at four outputs (r, c) of image n over the channel blocks (or bundles) [cb0, cb1),
+// from the activations as they are and the filter's two words: fp32 products, sixteen to a sum, and those added up in fp64.
+__device__ __forceinline__ void plain_sums(const TcArgs &a, const float *in, const __half *filt, const float *filt_down, int n, int k,
+                                           const int *r, const int *c, int cb0, int cb1, float2 *out)
+{
+    const int kt = k / a.MT, kv = min(a.MT, a.K - kt * a.MT), taps = a.Fh * a.Fw;
+    const __half *wq = filt + ((long long)kt * a.MT * a.cbs * a.taps + (long long)cb0 * a.taps * kv) * 32 + (k - kt * a.MT) * 8;
+    const float2 down2 = __ldg(reinterpret_cast<const float2 *>(filt_down + k));
+    const float down[2] = {down2.x, down2.y};
+    double sum[4][2]; // [output][channel]
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        sum[i >> 1][i & 1] = 0.0;
+#pragma unroll 1
+    for (int step = 0; step < (cb1 - cb0) * a.taps; ++step, wq += kv * 32)
+    {
+        const int block = step / taps, tap = step - block * taps, kh = tap / a.Fw, kw = tap - kh * a.Fw;
+        const float *plane = in + (long long)((n * a.cbs + cb0) * a.cg + block) * a.x_plane;
+        const float4 *x[4];
+        float part[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            const int row = r[i] + kh - a.pad_t, col = c[i] + kw - a.pad_l;
+            const bool inside = (uint32_t)row < (uint32_t)a.H && (uint32_t)col < (uint32_t)a.W;
+            x[i] = inside ? reinterpret_cast<const float4 *>(plane + (long long)row * a.x_row + (long long)col * CB) : nullptr;
+            part[i][0] = part[i][1] = 0.f;
+        }
+#pragma unroll
+        for (int h = 0; h < 4; ++h) // four input channels
+        {
+            float4 v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                v[i] = x[i] ? __ldg(x[i] + h) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+            {
+                const uint2 *w = reinterpret_cast<const uint2 *>(wq + (h >> 1) * kv * 16 + q * 8 + (h & 1) * 4);
+                const uint2 hi = __ldg(w), lo = __ldg(w + kv * 2);
+                const float2 h0 = __half22float2(*reinterpret_cast<const __half2 *>(&hi.x)), h1 = __half22float2(*reinterpret_cast<const __half2 *>(&hi.y));
+                const float2 l0 = __half22float2(*reinterpret_cast<const __half2 *>(&lo.x)), l1 = __half22float2(*reinterpret_cast<const __half2 *>(&lo.y));
+                const float w0 = fmaf(l0.x, LO_DOWN, h0.x) * down[q], w1 = fmaf(l0.y, LO_DOWN, h0.y) * down[q];
+                const float w2 = fmaf(l1.x, LO_DOWN, h1.x) * down[q], w3 = fmaf(l1.y, LO_DOWN, h1.y) * down[q];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    part[i][q] = fmaf(v[i].w, w3, fmaf(v[i].z, w2, fmaf(v[i].y, w1, fmaf(v[i].x, w0, part[i][q]))));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (x[i]) // a tap in the padding adds nothing, whatever the filter holds
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    sum[i][q] += (double)part[i][q];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        out[i] = make_float2((float)sum[i][0], (float)sum[i][1]);
+}
+// The outputs of a tile that met a wide patch (see the splitters), by the accumulation warps on the FMA pipe: a thread makes two
+// channels of four GEMM columns, 32 apart, or of the four pixels of a pooled one.  Such a tile takes many times as long as
+// another one: images whose pixels are 2^26 apart within a tile are not what this kernel is for, but their results
+// are as good as any.  A launch with a split reduction leaves the sums of the CTA's channel blocks in its staging rows.
+template <bool SPLIT, bool POOL>
+__device__ __noinline__ void plain_tile(const TcArgs &a, const Tile T, const float *in, const __half *filt, const float *filt_down,
+                                           const float *bias, float *out, float act_ns, int warp, int lane, int cb0, int cb1, float *stage, int pitch)
+{
+    const int cols = POOL ? a.PW >> 1 : a.PW, px = POOL ? (a.TH >> 1) * cols : a.NPX, each = POOL ? 32 : 128;
+#pragma unroll 1
+    for (int k = warp * 2; k < T.kv; k += ACC_WARPS * 2)
+#pragma unroll 1
+        for (int p0 = 0; p0 < px; p0 += each)
+        {
+            const int kg = T.kt * a.MT + k;
+            int r[4], c[4];
+            bool live[4];
+            float2 v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                const int p = p0 + lane + (POOL ? 0 : 32 * i), ml = POOL ? p : T.m_local0 + p, rl = ml / cols, cl = ml - rl * cols;
+                r[i] = T.row_base + (POOL ? 2 * rl + (i >> 1) : rl);
+                c[i] = T.col_base + (POOL ? 2 * cl + (i & 1) : cl);
+                live[i] = p < px && c[i] - T.col_base < T.tw_valid && (POOL || rl < T.th_valid) && r[i] < a.Ho;
+                if (!live[i])
+                    c[i] = -0x8000; // outside the image for every tap
+            }
+            plain_sums(a, in, filt, filt_down, T.n, kg, r, c, cb0, cb1, v);
+            const float2 b = bias && cb0 == 0 ? __ldg(reinterpret_cast<const float2 *>(bias + kg)) : make_float2(0.f, 0.f);
+            if (POOL)
+                v[0] = make_float2(fmaxf(fmaxf(v[0].x, v[1].x), fmaxf(v[2].x, v[3].x)), fmaxf(fmaxf(v[0].y, v[1].y), fmaxf(v[2].y, v[3].y)));
+#pragma unroll
+            for (int i = 0; i < (POOL ? 1 : 4); ++i)
+                if (live[i])
+                {
+                    float2 y = make_float2(v[i].x + b.x, v[i].y + b.y);
+                    float2 *o = reinterpret_cast<float2 *>(stage + (size_t)(p0 + lane + 32 * i) * pitch + k);
+                    if (!SPLIT)
+                    {
+                        o = reinterpret_cast<float2 *>(out + ((long long)T.n * (a.K / CB) + kg / CB) * a.o_kb_stride +
+                                                       (long long)(POOL ? r[i] >> 1 : r[i]) * a.o_row_stride +
+                                                       (long long)(POOL ? c[i] >> 1 : c[i]) * CB + kg % CB);
+                        if (a.accumulate)
+                            y = make_float2(y.x + o->x, y.y + o->y);
+                        y = make_float2(apply_act_ns(y.x, act_ns), apply_act_ns(y.y, act_ns));
+                    }
+                    *o = y;
+                }
+        }
+}
+
 template <bool PERSIST, bool SPLIT, bool PIXM = false, int MERGED = 0, bool POOL = false> // MERGED: 1 merged operand, 2 with whole-window groups
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restrict__ in, const __half *__restrict__ filt,
-                  const float *__restrict__ filt_scale, const TcArgs a, const float *__restrict__ bias, float *__restrict__ out, int *status)
+                  const float *__restrict__ filt_down, const __grid_constant__ TcArgs a, const float *__restrict__ bias, float *__restrict__ out, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t x_full[X_SLOTS_MAX], x_ready[X_SLOTS_MAX], x_empty[X_SLOTS_MAX];
@@ -329,6 +486,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     __shared__ uint32_t tmem_base_s;
     __shared__ __align__(8) uint64_t x_redo;   // a patch fetched again because its block scale did not fit
     __shared__ float patch_down[SCALE_RING];   // inverse of the block scale of each patch in flight
+    __shared__ uint32_t wide_tiles[WIDE_WORDS]; // bit i: the CTA's tile i has a wide patch (see the splitters)
     __shared__ __align__(16) uint32_t split_top[3][4];      // the splitter warps' maxima of the patch at hand
     __shared__ int acc_failed; // an accumulation warp gave up on a wait: all eight leave at the same tile
 
@@ -424,6 +582,8 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
         tmem_alloc(&tmem_base_s, tmem_cols);
         tmem_relinquish();
     }
+    if (tid >= NUM_THREADS - WIDE_WORDS)
+        wide_tiles[tid - (NUM_THREADS - WIDE_WORDS)] = 0;
     tc_fence_before_sync();
     if (split)
         cluster_sync_all(); // the peer's barriers exist before anybody can arrive on them
@@ -436,20 +596,10 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     {
         // The launch has 512 x 128 registers; the roles' shares add up to that at most (setmaxnreg draws on nothing else):
         // 128 x 88 + 256 x 168 + 128 x 88, pixel-major tiles 128 x 88 + 256 x 144 + 128 x 112.
-        if (warp < FIRST_ACC_WARP)
-        {
-            if (PIXM)
-                asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-            else
-                asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-        }
+        if (PIXM && warp >= FIRST_SPLIT_WARP)
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");
         else
-        {
-            if (PIXM)
-                asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");
-            else
-                asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-        }
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
         if (warp == 0 && lane == 0)
         {
             // ---------------- producer ----------------
@@ -645,11 +795,15 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                                         }
                                         if (++kw == a.Fw) { kw = 0; xh += (uint64_t)a.row_skip; }
                                     }
-                                    for (int tp = 0; tp < a.group; ++tp, wh2 += w_tap, xh2 += tap_step)
+                                    // the cross terms are 2^LO_SHIFT times too large: the first of the others mends that
+                                    for (int mt = 0; mt < mtiles; ++mt)
+                                        tc_mma_f16_rescaled<LO_SHIFT>(d0 + (uint32_t)(mt * a.K), xh2 + (uint64_t)mt * 512, wh2, idesc);
+                                    for (int tp = 1; tp < a.group; ++tp)
                                     {
+                                        wh2 += w_tap; xh2 += tap_step;
+                                        if (++kw2 == a.Fw) { kw2 = 0; xh2 += (uint64_t)a.row_skip; }
                                         for (int mt = 0; mt < mtiles; ++mt)
                                             tc_mma_f16(d0 + (uint32_t)(mt * a.K), xh2 + (uint64_t)mt * 512, wh2, idesc, 1u);
-                                        if (++kw2 == a.Fw) { kw2 = 0; xh2 += (uint64_t)a.row_skip; }
                                     }
                                 }
                                 else
@@ -663,10 +817,12 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                                         tc_mma_f16(d, wh, xh + x_lo_off, idesc, 1u);
                                         if (++kw == a.Fw) { kw = 0; xh += (uint64_t)a.row_skip; }
                                     }
-                                    for (int tp = 0; tp < a.group; ++tp, wh2 += w_tap, xh2 += tap_step)
+                                    tc_mma_f16_rescaled<LO_SHIFT>(d, wh2, xh2, idesc);
+                                    for (int tp = 1; tp < a.group; ++tp)
                                     {
-                                        tc_mma_f16(d, wh2, xh2, idesc, 1u);
+                                        wh2 += w_tap; xh2 += tap_step;
                                         if (++kw2 == a.Fw) { kw2 = 0; xh2 += (uint64_t)a.row_skip; }
+                                        tc_mma_f16(d, wh2, xh2, idesc, 1u);
                                     }
                                 }
                                 // the stage is free for the producer and the group's partial sums are
@@ -704,7 +860,10 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             // The block scale: a CTA starts from its first patch's largest magnitude (brought to 2^13..2^14) and keeps the
             // power of two as long as every patch's largest scaled magnitude stays in [2^6, 65504); the pass that converts
             // also finds that magnitude.  (Finding it first took as long as the conversion: a second pass over shared
-            // memory and a barrier in front of every patch.)  A patch outside the range is fetched and converted again.
+            // memory and a barrier in front of every patch.)  A patch outside the range is fetched and converted again, and so is
+            // one with a faint piece, whose largest magnitude is not zero but below FAINT when scaled (pieces, not whole
+            // rows: a row is two lanes').  Then rows are looked at: a patch with a faint row at the scale that is its
+            // own, one 2^-26 of its largest, makes its tile a wide one.
             const int sid = tid - FIRST_SPLIT_WARP * 32;
             bool ok = true, known = false;
             int slot = 0, scale_at = 0;
@@ -729,23 +888,35 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                     {
                         if (!known)
                         {
+                            uint32_t least_row = 0xffffffffu;
                             for (int u = sid; u < total; u += SPLIT_THREADS)
+                            {
+                                uint32_t row = max(finite_max(piece[2 * u]), finite_max(piece[2 * u + 1]));
+                                row = max(row, __shfl_xor_sync(0xffffffffu, row, 1));
                                 if ((u >> 1) < valid || (uint32_t)((u >> 1) - (int)entries) < (uint32_t)valid2)
-                                    m = max(m, max(finite_max(piece[2 * u]), finite_max(piece[2 * u + 1])));
+                                {
+                                    m = max(m, row);
+                                    least_row = min(least_row, row - 1u);
+                                }
+                            }
                             m = split_reduce(m, split_top[2], warp - FIRST_SPLIT_WARP, lane);
                             up = scale_up(m);
                             down = scale_down(m);
+                            if (least_row != 0xffffffffu && __uint_as_float(least_row + 1u) * up < FAINT)
+                                atomicOr(&wide_tiles[once_ >> 5], 1u << (once_ & 31));
                         }
                         float fm = 0.f;
+                        uint32_t least = 0xffffffffu;
                         int base = sid;
                         for (; base + 3 * SPLIT_THREADS < total; base += 4 * SPLIT_THREADS)
-                            fm = fmaxf(fm, split_pieces<4>(piece, base, up, entries, valid, valid2));
+                            fm = fmaxf(fm, split_pieces<4>(piece, base, up, entries, valid, valid2, least));
                         for (; base < total; base += SPLIT_THREADS)
-                            fm = fmaxf(fm, split_pieces<1>(piece, base, up, entries, valid, valid2));
+                            fm = fmaxf(fm, split_pieces<1>(piece, base, up, entries, valid, valid2, least));
                         fence_proxy_async();
-                        m = split_reduce(__float_as_uint(fm * up), split_top[turn], warp - FIRST_SPLIT_WARP, lane);
+                        const bool faint = least != 0xffffffffu && __uint_as_float(least + 1u) * up < FAINT;
+                        m = split_reduce(faint ? FAINT_SEEN : __float_as_uint(fm * up), split_top[turn], warp - FIRST_SPLIT_WARP, lane);
                         // 0: all zero; not below 65504: would have overflowed (or an infinity in the input, which no
-                        // scale helps: it stays one)
+                        // scale helps: it stays one), or a faint row was seen
                         if (!known || m == 0 || (m >= 0x42800000u && m < 0x477fe000u))
                             break;
                         if (sid == 0)
@@ -776,8 +947,10 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
         else
             asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
-        const float w_down = __ldg(filt_scale);             // inverse of the filter's block scale
         const float act_ns = act_neg_scale(a.act, a.slope); // activation: v > 0 ? v : v * act_ns
+        // Whether tile i of this CTA is wide; known when its last sums are.  What is stored for such a tile is overwritten at
+        // the end, so it matters here only where the output is also an input.
+        auto is_wide = [&](int i) { return ((*reinterpret_cast<volatile uint32_t *>(&wide_tiles[i >> 5]) >> (i & 31)) & 1u) != 0; };
         if (PIXM)
         {
             // ---------------- accumulation + epilogue, pixel-major ----------------
@@ -785,6 +958,8 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             // the running sums need 64 registers, a flush is one or two loads, and the epilogue
             // writes 64 contiguous bytes per channel block straight from the registers (a warp
             // covers 32 consecutive pixels: no transposition through shared memory, no barrier).
+            const bool own_scales = __ldg(filt_down + 2 * a.K + 1) != 0.f;
+            const float w_down = own_scales ? 1.f : __ldg(filt_down + 2 * a.K + 2);
             const int quarter = warp & 3, mt = (warp - FIRST_ACC_WARP) >> 2;
             const int mtiles = a.NPX >> 7;
             const bool active = mt < mtiles;
@@ -794,14 +969,14 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             for (int t = first_tile, once_ = 0; (PERSIST ? (t < a.total_tiles) : (once_ == 0)) && ok; t += tile_step, ++once_, ++pc)
             {
                 const Tile T = decode_tile(a, t);
-                // the bias seeds the sums (these loads overlap the wait for the first group)
+                // the bias seeds the sums (these loads overlap the wait for the first group), unless channels have scales of their own
                 constexpr int ACC = MERGED ? 32 : 64; // output channels a thread can hold
                 float acc[ACC];
 #pragma unroll
                 for (int c4 = 0; c4 < ACC / 4; ++c4)
                 {
-                    const float4 b = (bias && c4 * 4 < a.K) ? __ldg(reinterpret_cast<const float4 *>(bias) + c4)
-                                                            : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 b = (bias && !own_scales && c4 * 4 < a.K) ? __ldg(reinterpret_cast<const float4 *>(bias) + c4)
+                                                                           : make_float4(0.f, 0.f, 0.f, 0.f);
                     acc[4 * c4] = b.x; acc[4 * c4 + 1] = b.y; acc[4 * c4 + 2] = b.z; acc[4 * c4 + 3] = b.w;
                 }
                 int in_cb = 0;
@@ -830,7 +1005,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                             {
 #pragma unroll
                                 for (int e = 0; e < 16; ++e)
-                                    acc[e] = fmaf(__uint_as_float(v[e]) + __uint_as_float(v[16 + e]), down, acc[e]);
+                                    acc[e] = fmaf(fmaf(__uint_as_float(v[16 + e]), LO_DOWN, __uint_as_float(v[e])), down, acc[e]);
                             }
                             else
                             {
@@ -841,7 +1016,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                                 tmem_ld_wait();
 #pragma unroll
                                 for (int e = 0; e < 32; ++e)
-                                    acc[e] = fmaf(__uint_as_float(v[e]), down, acc[e]);
+                                    acc[e] = fmaf(__uint_as_float(v[e]), down * LO_DOWN, acc[e]);
                             }
                         }
                         else // K = 64
@@ -864,6 +1039,16 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                     if (lane == 0)
                         mbar_arrive(&t_empty[tb]);
                 }
+                if (own_scales)
+#pragma unroll
+                    for (int c4 = 0; c4 < ACC / 4; ++c4)
+                        if (c4 * 4 < a.K)
+                        {
+                            const float4 b = bias ? __ldg(reinterpret_cast<const float4 *>(bias) + c4) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            const float4 d = __ldg(reinterpret_cast<const float4 *>(filt_down) + c4);
+                            acc[4 * c4] = fmaf(acc[4 * c4], d.x, b.x); acc[4 * c4 + 1] = fmaf(acc[4 * c4 + 1], d.y, b.y);
+                            acc[4 * c4 + 2] = fmaf(acc[4 * c4 + 2], d.z, b.z); acc[4 * c4 + 3] = fmaf(acc[4 * c4 + 3], d.w, b.w);
+                        }
                 if (POOL)
                 {
                     // 2x2 max pool, stride 2, on the sums in registers (K = 32 or 64: a thread holds ACC = K
@@ -927,7 +1112,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                         }
                     }
                 }
-                else if (ok && active)
+                else if (ok && active && !(a.accumulate && is_wide(once_)))
                 {
                     const int ml = T.m_local0 + mt * 128 + quarter * 32 + lane;
                     const int rl = a.by_PW.div(ml), cl = ml - rl * a.PW;
@@ -984,7 +1169,9 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
         {
             const Tile T = decode_tile(a, t);
             // the bias of this thread's channel seeds its sums (rank 0 only when several CTAs share a tile)
-            const float seed = (bias && crank == 0 && lane_has_row && k_local < T.kv) ? __ldg(bias + T.kt * a.MT + k_local) : 0.f;
+            const bool has_channel = lane_has_row && k_local < T.kv;
+            const float seed = (bias && crank == 0 && has_channel) ? __ldg(bias + T.kt * a.MT + k_local) : 0.f;
+            const float w_down = has_channel ? __ldg(filt_down + T.kt * a.MT + k_local) : 0.f;
             float acc[COLS_PER_THREAD];
 #pragma unroll
             for (int c = 0; c < COLS_PER_THREAD; ++c)
@@ -1051,6 +1238,12 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                     }
                 }
                 asm volatile("bar.sync 1, 256;" ::: "memory"); // the eight accumulation warps
+                if (split && ok && is_wide(0))
+                {
+                    // this CTA's part of the sums, in place of what it staged (each wide CTA of the cluster its own)
+                    plain_tile<true, false>(a, T, in, filt, filt_down, bias, out, act_ns, warp - FIRST_ACC_WARP, lane, cb_begin, cb_begin + cbs_l, stage, pitch);
+                    __syncwarp();
+                }
                 if (split)
                 {
                     // Every warp tells every CTA of the cluster that its sums are staged; when all have, the units of the
@@ -1102,7 +1295,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                     __syncwarp();
                     mbar_wait_cluster(&peer_done, 0, status, 21);
                 }
-                else if (ok)
+                else if (ok && !(a.accumulate && is_wide(0)))
                 {
                     for (int pg = warp - FIRST_ACC_WARP; pg < a.NPX / 8; pg += ACC_WARPS)
                     {
@@ -1164,7 +1357,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                     asm volatile("bar.sync 1, 256;" ::: "memory"); // the eight accumulation warps
                     if (*reinterpret_cast<volatile int *>(&acc_failed))
                         ok = false;
-                    if (ok)
+                    if (ok && !(a.accumulate && is_wide(once_)))
                     {
                         // staged row s holds pixel (s / 32) * my_cols + piece * 32 + s % 32 of the tile
                         const int s_row = (warp - FIRST_ACC_WARP) * 8 + psub;
@@ -1204,6 +1397,20 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     __syncthreads();
     if (warp == 0)
         tmem_dealloc(tmem, tmem_cols);
+    // Wide tiles, when everything else is done: nobody waits for these warps any more, and in the middle of the tile loop the
+    // code for them costs every other tile registers (ResNet-8 at 1024 images 426 us without it, 432 with a call here, 464
+    // with it in the loop).
+    if (!split && __any_sync(0xffffffffu, lane < WIDE_WORDS ? wide_tiles[lane] : 0u) && warp >= FIRST_ACC_WARP && warp < FIRST_SPLIT_WARP)
+    {
+        const float act_ns = act_neg_scale(a.act, a.slope);
+        for (int i = 0, t = first_tile; i < WIDE_WORDS * 32 && t < a.total_tiles; ++i, t += tile_step)
+        {
+            if (wide_tiles[i >> 5] >> (i & 31) & 1u)
+                plain_tile<false, POOL>(a, decode_tile(a, t), in, filt, filt_down, bias, out, act_ns, warp - FIRST_ACC_WARP, lane, 0, a.cbs, nullptr, 0);
+            if (!PERSIST)
+                break;
+        }
+    }
 }
 
 // Picks ring depths for the patch / filter sizes already in `a`.  Narrow layers run persistent (one
@@ -1500,11 +1707,12 @@ int small_b200_filter_prepare_tf32x3(const small_b200_layer *L, const float *fil
     if (!L || L->C % CB != 0 || L->K % CB != 0 || L->C <= 0 || L->K <= 0 || L->Fh <= 0 || L->Fw <= 0)
         return fail(SMALL_B200_INVALID_ARGUMENT, "Conv2D<float> (3xTF32) ERROR: shape not covered by the tensor-core path.");
     const long long n = (long long)L->K * L->C * L->Fh * L->Fw;
-    // [0, n) floats: the half-precision pairs; behind them the inverse of the block scale and the largest magnitude
-    uint32_t *top = reinterpret_cast<uint32_t *>(prepared + n + 1);
-    SB_CUDA(cudaMemsetAsync(top, 0, sizeof(uint32_t), as_stream(stream)));
-    const long long blocks = (n + 255) / 256;
-    filter_max_kernel<<<(unsigned)(blocks < 1024 ? blocks : 1024), 256, 0, as_stream(stream)>>>(n, filt, top);
+    // [0, n) floats: the half-precision pairs; behind them, for each output channel, the inverse of its block scale and its
+    // largest magnitude, then that of all, and what prepare_filter_kernel says (n is 16 K at least, and the caller provides 2 n)
+    uint32_t *top = reinterpret_cast<uint32_t *>(prepared + n + L->K);
+    SB_CUDA(cudaMemsetAsync(top, 0, ((size_t)L->K + 2) * sizeof(uint32_t), as_stream(stream)));
+    const long long blocks = (n + 255) / 256, per_block = n / L->K * CB, max_blocks = (per_block + 1023) / 1024;
+    filter_max_kernel<<<dim3((unsigned)(max_blocks < 64 ? max_blocks : 64), (unsigned)(L->K / CB)), 256, 0, as_stream(stream)>>>(per_block, filt, top);
     if (int rc = launched("filter_max_kernel"))
         return rc;
     prepare_filter_kernel<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(
@@ -1683,7 +1891,7 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
     a.ksplit = (a.pixm || a.persistent) ? 1 : cut.split;
     blocks *= a.ksplit;
     const __half *filt = reinterpret_cast<const __half *>(filt_prepared);
-    const float *filt_scale = filt_prepared + (size_t)a.K * a.C * a.Fh * a.Fw;
+    const float *filt_down = filt_prepared + (size_t)a.K * a.C * a.Fh * a.Fw;
     auto launch_split = [&](const TcArgs &ta, long long nblocks) -> int {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)nblocks); cfg.blockDim = dim3(NUM_THREADS);
@@ -1692,7 +1900,7 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = (unsigned)ta.ksplit; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
-        SB_CUDA(cudaLaunchKernelEx(&cfg, conv_f16x3_kernel<false, true>, mx, in, filt, filt_scale, ta, bias, out, status));
+        SB_CUDA(cudaLaunchKernelEx(&cfg, conv_f16x3_kernel<false, true>, mx, in, filt, filt_down, ta, bias, out, status));
         return SMALL_B200_OK;
     };
     if (!a.pixm && !a.persistent && cut.rem_split)
@@ -1700,7 +1908,7 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         const long long full = tiles / num_sms() * num_sms(), rem = tiles - full;
         TcArgs a1 = a;
         a1.tile_base = 0;
-        conv_f16x3_kernel<false, false><<<(unsigned)full, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_scale, a1, bias, out, status);
+        conv_f16x3_kernel<false, false><<<(unsigned)full, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a1, bias, out, status);
         if (int rc = launched("conv_f16x3_kernel"))
             return rc;
         TcArgs a2 = a;
@@ -1710,9 +1918,14 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         return launched("conv_f16x3_kernel");
     }
     const bool whole = a.merged && a.cg == 1 && a.group != a.Fw; // whole-window groups (TcArgs::row_skip)
+    const long long room = a.persistent ? blocks * WIDE_WORDS * 32 : tiles; // tiles of a launch (wide_tiles)
+    for (long long base = 0; base < tiles; base += room)
+    {
+    a.tile_base = (int)base; a.total_tiles = (int)std::min(tiles, base + room);
+    const unsigned grid = (unsigned)(a.persistent ? std::min(blocks, tiles - base) : blocks);
 #define SB_LAUNCH_PIXM(M, P) \
-    conv_f16x3_kernel<true, false, true, M, P><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(\
-        mx, in, filt, filt_scale, a, bias, out, status)
+    conv_f16x3_kernel<true, false, true, M, P><<<grid, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(\
+        mx, in, filt, filt_down, a, bias, out, status)
     if (a.pool && whole)
         SB_LAUNCH_PIXM(2, true);
     else if (a.pool && a.merged)
@@ -1725,17 +1938,20 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         SB_LAUNCH_PIXM(1, false);
 #undef SB_LAUNCH_PIXM
     else if (a.pixm)
-        conv_f16x3_kernel<true, false, true><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_scale, a, bias, out, status);
+        conv_f16x3_kernel<true, false, true><<<grid, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
     else if (a.persistent)
-        conv_f16x3_kernel<true, false><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_scale, a, bias, out, status);
+        conv_f16x3_kernel<true, false><<<grid, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
     else if (a.ksplit > 1)
     {
         if (int rc = launch_split(a, blocks))
             return rc;
     }
     else
-        conv_f16x3_kernel<false, false><<<(unsigned)blocks, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_scale, a, bias, out, status);
-    return launched("conv_f16x3_kernel");
+        conv_f16x3_kernel<false, false><<<grid, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
+    if (int rc = launched("conv_f16x3_kernel"))
+        return rc;
+    }
+    return SMALL_B200_OK;
 }
 } // namespace
 

@@ -261,6 +261,16 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uin
                  ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
                  : "memory");
 }
+// The same with D = A * B + D * 2^-DOWN: what the accumulator holds is brought to another scale on the way.
+template <int DOWN>
+__device__ __forceinline__ void tc_mma_f16_rescaled(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc)
+{
+    static_assert(DOWN >= 0 && DOWN <= 15, "a four-bit field");
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n\t}"
+                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(DOWN)
+                 : "memory");
+}
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp gets lane (base lane + i).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *r)
 {
