@@ -12,6 +12,8 @@
 //     however large the pixels beside it: the scale brings the patch's largest to 2^6 at least, 22 bits reach down
 //     to 2^-13, a patch with a pixel below that gets the scale that brings its largest to 2^13, and a tile with a patch where
 //     that does not do either is computed on the FMA pipe (plain_tile).
+//   * An infinity is no pair (inf - inf): a tile with one in a patch goes the same way, and with one in the filter, or a NaN
+//     (which the zeros of the padding must not meet), the layer does.  A NaN in the activations is its own pair.
 // So an output channel, an image or a pixel is as good as if it stood alone: the words of a value that is in range do not
 // depend on the power of two.  (With lo stored as it is, 22 bits ended at 2^-3 and an error of 2^-24 remained: an output channel 2^-12 of
 // the largest kept half its digits.  The scaled second word costs 0.5 to 1.5 % of a layer: Tiny-YOLOv2 on 64 images 1.576
@@ -132,6 +134,9 @@ struct TcArgs
 // convolution agree.
 __host__ __device__ inline int pick_mt(int K) { return K >= 128 ? 128 : 64; }
 
+// What the word behind the largest magnitudes says: channels have scales of their own; sums are to be made on the FMA pipe.
+constexpr uint32_t OWN_SCALES = 1, PLAIN_FILTER = 2;
+
 // Largest magnitude of every output channel's filter, and behind those of all of them (finite values; the sign bit cleared, floats compare like integers).
 // blockIdx.y: block of 16 channels, n: its values [slab][16 c][16 k]; a thread stays with one channel.
 __global__ void __launch_bounds__(256) filter_max_kernel(long long n, const float *__restrict__ w, uint32_t *__restrict__ top)
@@ -141,7 +146,10 @@ __global__ void __launch_bounds__(256) filter_max_kernel(long long n, const floa
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256)
     {
         const uint32_t b = __float_as_uint(__ldg(w + i)) & 0x7fffffffu;
-        m = max(m, b < 0x7f800000u ? b : 0u);
+        if (b >= 0x7f800000u)
+            top[gridDim.y * CB + 1] = PLAIN_FILTER;
+        else
+            m = max(m, b);
     }
     m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
     if ((threadIdx.x & 31) < 16 && m)
@@ -173,8 +181,8 @@ __device__ __forceinline__ float scale_down(uint32_t top)
 }
 
 // packed filter [K/16][slab][16 c][16 k] -> half-precision pairs [K/MT][slab][c/8][hi kv | lo kv][8 c]; kv = MT
-// except in a last, partial tile (K % MT channels).  down[k] = the inverse of channel k's block scale, down[2 K + 1] = 1 if
-// it isn't the same for all of them, down[2 K + 2] = the inverse of the filter's scale.
+// except in a last, partial tile (K % MT channels).  down[k] = the inverse of channel k's block scale, down[2 K + 1] holds
+// OWN_SCALES if it isn't the same for all of them (beside PLAIN_FILTER, set before), down[2 K + 2] = the inverse of the filter's scale.
 __global__ void __launch_bounds__(256)
 prepare_filter_kernel(long long n, int slabs, int MT, int K, const float *__restrict__ w, const uint32_t *__restrict__ top,
                       __half *__restrict__ pairs, float *__restrict__ down)
@@ -200,14 +208,14 @@ prepare_filter_kernel(long long n, int slabs, int MT, int K, const float *__rest
     {
         down[k] = scale_down(t0);
         if (own)
-            down[2 * K + 1] = 1.f;
+            atomicOr(reinterpret_cast<uint32_t *>(down) + 2 * K + 1, OWN_SCALES);
         if (k == 0)
             down[2 * K + 2] = scale_down(all);
     }
     const float v = w[i] * scale_up(t0);
     const __half h = __float2half_rz(v);
     pairs[o] = h;
-    pairs[o + (long long)kv * 8] = __float2half_rz((v - __half2float(h)) * LO_UP);
+    pairs[o + (long long)kv * 8] = fabsf(v) <= 65504.f ? __float2half_rz((v - __half2float(h)) * LO_UP) : __float2half_rz(0.f);
 }
 
 // Tensor-core accumulation truncates: every MMA adds into the fp32 accumulator with
@@ -248,14 +256,27 @@ __device__ __forceinline__ void split2(float a, float b, float up, float up_lo, 
         "cvt.rz.f16x2.f32 %1, y, x;\n\t}"
         : "=&r"(hi), "=r"(lo) : "f"(a), "f"(b), "f"(up), "f"(up_lo));
 }
-__device__ __forceinline__ uint32_t finite_abs(float v)
+// Largest magnitude (as bits) of the finite ones among eight values; `inf` is set if there is an infinity among them.
+__device__ __forceinline__ uint32_t finite_max(const float4 *v, bool &inf)
 {
-    const uint32_t b = __float_as_uint(v) & 0x7fffffffu;
-    return b < 0x7f800000u ? b : 0u;
-}
-__device__ __forceinline__ uint32_t finite_max(const float4 v)
-{
-    return max(max(finite_abs(v.x), finite_abs(v.y)), max(finite_abs(v.z), finite_abs(v.w)));
+    const uint4 a = *reinterpret_cast<const uint4 *>(v), b = *reinterpret_cast<const uint4 *>(v + 1);
+    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        m = max(m, w[i] & 0x7fffffffu);
+    if (m >= 0x7f800000u)
+    {
+        m = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+        {
+            const uint32_t u = w[i] & 0x7fffffffu;
+            inf = inf || u == 0x7f800000u;
+            m = max(m, u < 0x7f800000u ? u : 0u);
+        }
+    }
+    return m;
 }
 __device__ __forceinline__ float max_abs(const float4 v)
 {
@@ -310,6 +331,26 @@ __device__ __forceinline__ float split_pieces(float4 *piece, int u0, float up, u
         row[(h + 2 - 2 * late) ^ sw] = late ? make_uint4(hi.z, hi.w, hi.x, hi.y) : lo;
     }
     return fm;
+}
+
+// What the rows (a pixel's sixteen channels) of a patch hold that are this thread's to look at: the largest finite
+// magnitude, and the least bits - 1 of a row's largest one (2^32 - 1: none but zeros; 0 where there is an infinity, so that the
+// row counts as faint).  Once per CTA, and for patches that do not fit the scale at hand.
+__device__ __forceinline__ uint2 look_at_rows(const float4 *piece, int sid, int total, uint32_t entries, int valid, int valid2)
+{
+    uint2 seen = make_uint2(0u, 0xffffffffu);
+    for (int u = sid; u < total; u += SPLIT_THREADS)
+    {
+        bool inf = false;
+        uint32_t row = finite_max(piece + 2 * u, inf);
+        row = max(row, __shfl_xor_sync(0xffffffffu, row, 1)); // the row's other piece
+        if ((u >> 1) < valid || (uint32_t)((u >> 1) - (int)entries) < (uint32_t)valid2)
+        {
+            seen.x = max(seen.x, row);
+            seen.y = min(seen.y, inf ? 0u : row - 1u);
+        }
+    }
+    return seen;
 }
 
 // One tile of work: an image, a range of pixels and a block of MT output channels.
@@ -486,6 +527,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     __shared__ uint32_t tmem_base_s;
     __shared__ __align__(8) uint64_t x_redo;   // a patch fetched again because its block scale did not fit
     __shared__ float patch_down[SCALE_RING];   // inverse of the block scale of each patch in flight
+    static_assert(WIDE_WORDS == 32, "a lane each");
     __shared__ uint32_t wide_tiles[WIDE_WORDS]; // bit i: the CTA's tile i has a wide patch (see the splitters)
     __shared__ __align__(16) uint32_t split_top[3][4];      // the splitter warps' maxima of the patch at hand
     __shared__ int acc_failed; // an accumulation warp gave up on a wait: all eight leave at the same tile
@@ -888,21 +930,12 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                     {
                         if (!known)
                         {
-                            uint32_t least_row = 0xffffffffu;
-                            for (int u = sid; u < total; u += SPLIT_THREADS)
-                            {
-                                uint32_t row = max(finite_max(piece[2 * u]), finite_max(piece[2 * u + 1]));
-                                row = max(row, __shfl_xor_sync(0xffffffffu, row, 1));
-                                if ((u >> 1) < valid || (uint32_t)((u >> 1) - (int)entries) < (uint32_t)valid2)
-                                {
-                                    m = max(m, row);
-                                    least_row = min(least_row, row - 1u);
-                                }
-                            }
+                            const uint2 seen = look_at_rows(piece, sid, total, entries, valid, valid2);
+                            m = seen.x;
                             m = split_reduce(m, split_top[2], warp - FIRST_SPLIT_WARP, lane);
                             up = scale_up(m);
                             down = scale_down(m);
-                            if (least_row != 0xffffffffu && __uint_as_float(least_row + 1u) * up < FAINT)
+                            if (seen.y != 0xffffffffu && __uint_as_float(seen.y + 1u) * up < FAINT)
                                 atomicOr(&wide_tiles[once_ >> 5], 1u << (once_ & 31));
                         }
                         float fm = 0.f;
@@ -950,6 +983,11 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
         const float act_ns = act_neg_scale(a.act, a.slope); // activation: v > 0 ? v : v * act_ns
         // Whether tile i of this CTA is wide; known when its last sums are.  What is stored for such a tile is overwritten at
         // the end, so it matters here only where the output is also an input.
+        if (__ldg(reinterpret_cast<const uint32_t *>(filt_down) + 2 * a.K + 1) & PLAIN_FILTER)
+        {
+            wide_tiles[lane] = 0xffffffffu; // all of them; every warp for itself
+            __syncwarp();
+        }
         auto is_wide = [&](int i) { return ((*reinterpret_cast<volatile uint32_t *>(&wide_tiles[i >> 5]) >> (i & 31)) & 1u) != 0; };
         if (PIXM)
         {
@@ -958,7 +996,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             // the running sums need 64 registers, a flush is one or two loads, and the epilogue
             // writes 64 contiguous bytes per channel block straight from the registers (a warp
             // covers 32 consecutive pixels: no transposition through shared memory, no barrier).
-            const bool own_scales = __ldg(filt_down + 2 * a.K + 1) != 0.f;
+            const bool own_scales = __ldg(reinterpret_cast<const uint32_t *>(filt_down) + 2 * a.K + 1) & OWN_SCALES;
             const float w_down = own_scales ? 1.f : __ldg(filt_down + 2 * a.K + 2);
             const int quarter = warp & 3, mt = (warp - FIRST_ACC_WARP) >> 2;
             const int mtiles = a.NPX >> 7;
@@ -1400,7 +1438,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     // Wide tiles, when everything else is done: nobody waits for these warps any more, and in the middle of the tile loop the
     // code for them costs every other tile registers (ResNet-8 at 1024 images 426 us without it, 432 with a call here, 464
     // with it in the loop).
-    if (!split && __any_sync(0xffffffffu, lane < WIDE_WORDS ? wide_tiles[lane] : 0u) && warp >= FIRST_ACC_WARP && warp < FIRST_SPLIT_WARP)
+    if (!split && __any_sync(0xffffffffu, wide_tiles[lane]) && warp >= FIRST_ACC_WARP && warp < FIRST_SPLIT_WARP)
     {
         const float act_ns = act_neg_scale(a.act, a.slope);
         for (int i = 0, t = first_tile; i < WIDE_WORDS * 32 && t < a.total_tiles; ++i, t += tile_step)
