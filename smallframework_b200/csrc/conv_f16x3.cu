@@ -165,6 +165,11 @@ constexpr int LO_SHIFT = 10;
 constexpr float LO_UP = 1 << LO_SHIFT, LO_DOWN = 1.f / LO_UP;
 // A pair has its 22 bits from FAINT = 2^-13 on: its last bit is then 2^-34, the least that the second word can hold.
 constexpr float FAINT = 1.f / 8192;
+// Magnitudes up to which a sum of 2^20 products stays finite, and with it what the tensor core makes of it: 2^45 for the
+// filter, a scale of 2^-48 (magnitudes of 2^61 at least) for a patch.
+constexpr uint32_t LARGE_FILTER = (127u + 45) << 23;
+constexpr float LARGE_DOWN = 281474976710656.f; // 2^48
+constexpr float LEAST_DOWN = 1.f / (1 << 30);
 constexpr uint32_t FAINT_SEEN = 0x7fffffffu; // the splitters' word for a patch with a row below that
 
 // Block scale of a set of operands whose largest magnitude has the bits `top`: the power of two that brings it
@@ -207,8 +212,12 @@ prepare_filter_kernel(long long n, int slabs, int MT, int K, const float *__rest
     if (slab == 0 && c == 0)
     {
         down[k] = scale_down(t0);
-        if (own)
+        // What the two scales are together has to be a number, and what the sums are: channels so small (2^-17) have theirs
+        // undone apart from the patch's, and a filter so large (2^45) is left to the FMA pipe.
+        if (own || (top[k] && down[k] < LEAST_DOWN))
             atomicOr(reinterpret_cast<uint32_t *>(down) + 2 * K + 1, OWN_SCALES);
+        if (top[k] >= LARGE_FILTER)
+            atomicOr(reinterpret_cast<uint32_t *>(down) + 2 * K + 1, PLAIN_FILTER);
         if (k == 0)
             down[2 * K + 2] = scale_down(all);
     }
@@ -911,6 +920,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             int slot = 0, scale_at = 0;
             uint32_t phase = 0, turn = 0;
             uint32_t redone = 0;
+            uint32_t limit = 0;
             float up = 1.f, down = 1.f;
             SB_TILE_LOOP(ok)
             {
@@ -935,7 +945,8 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                             m = split_reduce(m, split_top[2], warp - FIRST_SPLIT_WARP, lane);
                             up = scale_up(m);
                             down = scale_down(m);
-                            if (seen.y != 0xffffffffu && __uint_as_float(seen.y + 1u) * up < FAINT)
+                            limit = down >= LARGE_DOWN ? 0u : 0xffffffffu;
+                            if (!limit || (seen.y != 0xffffffffu && __uint_as_float(seen.y + 1u) * up < FAINT))
                                 atomicOr(&wide_tiles[once_ >> 5], 1u << (once_ & 31));
                         }
                         float fm = 0.f;
@@ -961,7 +972,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                         known = false;
                         m = 0;
                     }
-                    known = m != 0; // an all-zero patch says nothing about the next one
+                    known = m - 1u < limit; // an all-zero patch says nothing about the next one; a large one's scale is not kept
                     if (sid == 0)
                     {
                         patch_down[scale_at] = down;
@@ -1213,7 +1224,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             float acc[COLS_PER_THREAD];
 #pragma unroll
             for (int c = 0; c < COLS_PER_THREAD; ++c)
-                acc[c] = seed;
+                acc[c] = 0.f;
             int in_cb = 0;
             for (int g = 0; g < groups && ok; ++g, ++gc)
             {
@@ -1230,7 +1241,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                 if (!ok)
                     break;
                 tc_fence_after_sync();
-                const float down = *reinterpret_cast<volatile float *>(&patch_down[pc % SCALE_RING]) * w_down;
+                const float down = *reinterpret_cast<volatile float *>(&patch_down[pc % SCALE_RING]);
                 const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(tb * a.NPX + col0);
 #pragma unroll
                 for (int piece = 0; piece < COLS_PER_THREAD / 32; ++piece)
@@ -1265,14 +1276,14 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
 #pragma unroll
                         for (int e = 0; e < COLS_PER_THREAD; ++e)
                             if (e < my_cols)
-                                srow[e * 144] = acc[e];
+                                srow[e * 144] = fmaf(acc[e], w_down, seed);
                     }
                     else
                     {
 #pragma unroll
                         for (int e = 0; e < COLS_PER_THREAD; ++e)
                             if (e < my_cols)
-                                srow[e * 80] = acc[e];
+                                srow[e * 80] = fmaf(acc[e], w_down, seed);
                     }
                 }
                 asm volatile("bar.sync 1, 256;" ::: "memory"); // the eight accumulation warps
@@ -1378,13 +1389,13 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                         {
 #pragma unroll
                             for (int e = 0; e < 32; ++e)
-                                srow[e * 144] = acc[piece * 32 + e];
+                                srow[e * 144] = fmaf(acc[piece * 32 + e], w_down, seed);
                         }
                         else
                         {
 #pragma unroll
                             for (int e = 0; e < 32; ++e)
-                                srow[e * 80] = acc[piece * 32 + e];
+                                srow[e * 80] = fmaf(acc[piece * 32 + e], w_down, seed);
                         }
                     }
                     // The give-up decision is made for the CTA, not per warp: the named barrier below

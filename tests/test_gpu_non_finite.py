@@ -83,6 +83,16 @@ def test_infinities_in_the_activations(oracle, case):
     _same(oracle, case, x, w)
 
 
+@pytest.mark.parametrize("case", CASES, ids=IDS)
+def test_products_past_the_largest_number(oracle, case):
+    """Finite operands whose products are not, beside zeros, which stay nothing whatever the scales are."""
+    C, K, H, W, f, s, N, _ = case
+    x, w = _operands(case)
+    x = np.abs(x) * 1e38
+    x[N // 2, :, H // 3:] = 0
+    _same(oracle, case, x, (np.abs(w) + 0.01) * 1e12)
+
+
 @pytest.mark.parametrize("case", NO_POOL, ids=NO_POOL_IDS)
 def test_nan_in_the_activations(oracle, case):
     C, K, H, W, f, s, N, _ = case

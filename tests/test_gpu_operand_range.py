@@ -109,6 +109,21 @@ def test_pixels_far_apart(case, bits):
            _signed(rng, (N, K, H, W)) * 2.0 ** -bits)
 
 
+# magnitudes of activations and filter that the tensor core is not given, or whose scales are far apart
+EXTREMES = [(3e37, 1e-20), (1e-30, 1e30), (1e-18, 1e-16), (1e-35, 1e3)]
+
+
+@pytest.mark.parametrize("scales", EXTREMES, ids=lambda s: "x{:g}_w{:g}".format(*s))
+@pytest.mark.parametrize("case", CASES, ids=IDS)
+def test_extreme_magnitudes(case, scales):
+    C, K, H, W, f, N, what = case
+    rng = np.random.default_rng(C + K + H)
+    x = _signed(rng, (N, C, H, W)) * scales[0]
+    x[N // 2, :, H // 2:] = 0
+    out = scales[0] * scales[1]
+    _check(case, x, _signed(rng, (K, C, f, f)) * scales[1], _signed(rng, K) * out, _signed(rng, (N, K, H, W)) * out)
+
+
 def test_wide_tiles_past_the_tiles_of_one_launch():
     """A launch has at most 1024 tiles a CTA: images of one tile each, more than 148 CTAs take in one launch, a few of them wide."""
     C = K = 16
