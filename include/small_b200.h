@@ -157,11 +157,12 @@ int small_b200_conv2d_maxpool_f32(const small_b200_layer *conv, const small_b200
 /* The same layer on the tensor cores (tcgen05 kind::f16 on pairs of half-precision words, fp32
  * accumulation in tensor memory), stride 1 only.  Each fp32 operand x enters the tensor core as
  * hi = half(x * 2^e) and lo = half((x * 2^e - hi) * 2^10), 22 bits like the two words of a 3xTF32 split
- * (which the functions are named after).  The power of two belongs to the filter (or to one output
- * channel, where that is 2^12 and more below the largest) and to each patch of 16 input channels of a
- * tile: each pixel's values keep 22 bits of the largest of its 16, and each channel's weights 22 bits
- * or 2^-35 of the largest of that channel, whatever the magnitudes beside them (tiles whose pixels lie
- * 2^26 and more apart are computed on the FMA pipe, many times more slowly).  The scales are
+ * (which the functions are named after).  The power of two belongs to the filter, or to one output
+ * channel that would lose digits by that, and to each patch of 16 input channels of a tile.  Whatever the
+ * magnitudes beside them, a pixel's 16 values keep 22 bits of the largest of them (tiles whose pixels lie 2^26
+ * and more apart are computed on the FMA pipe, many times more slowly, and so are those with an
+ * infinity), and a tap's 16 weights 22 bits of the largest of them down to 2^-26 of the largest of the
+ * output channel (beneath that, an error of 2^-47 of the latter).  The scales are
  * undone in fp32.  The activations are split inside the kernel, in shared memory.  The caller
  * provides the filter re-laid for the tensor core:
  *   filt_prepared  small_b200_filter_prepare_tf32x3(filt), once per set of weights,

@@ -6,8 +6,9 @@
 // is a_lo*b_hi + a_hi*b_lo + a_hi*b_hi in fp32 tensor memory; the dropped a_lo*b_lo is below 2^-20 of it.  The cross terms are
 // summed first, and the first a_hi*b_hi brings them down by 2^-10 (an operand of the instruction), or they have columns of
 // their own.  Half precision has a narrow range, so the power of two 2^e belongs to a block.
-//   * Filter: all of it, or one output channel where that is 2^12 and more below the largest.  A weight keeps its 22 bits
-//     down to 2^-14 of its channel's largest (2^-26 with a scale of its own) and an error below 2^-35 of that beneath.
+//   * Filter: all of it, or one output channel where the filter's scale would take digits from one of its rows (a tap's
+//     sixteen input channels).  A row keeps 22 bits of its largest weight, down to 2^-26 of the channel's largest; beneath
+//     that an error below 2^-47 of the channel's largest is left.
 //   * Activations: a tile's patch of 16 input channels.  Every pixel's sixteen values keep 22 bits of the largest of them,
 //     however large the pixels beside it: the scale brings the patch's largest to 2^6 at least, 22 bits reach down
 //     to 2^-13, a patch with a pixel below that gets the scale that brings its largest to 2^13, and a tile with a patch where
@@ -137,25 +138,35 @@ __host__ __device__ inline int pick_mt(int K) { return K >= 128 ? 128 : 64; }
 // What the word behind the largest magnitudes says: channels have scales of their own; sums are to be made on the FMA pipe.
 constexpr uint32_t OWN_SCALES = 1, PLAIN_FILTER = 2;
 
-// Largest magnitude of every output channel's filter, and behind those of all of them (finite values; the sign bit cleared, floats compare like integers).
-// blockIdx.y: block of 16 channels, n: its values [slab][16 c][16 k]; a thread stays with one channel.
-__global__ void __launch_bounds__(256) filter_max_kernel(long long n, const float *__restrict__ w, uint32_t *__restrict__ top)
+// Magnitudes of the filter's finite values as bits (without the sign, floats compare like integers): of every output channel the
+// largest, behind those the largest of all, the word above, a place for the filter's scale, and of every channel the
+// least of a row's largest (a row: a slab's sixteen input channels; ones of zeros do not count), complemented: 0 is none.
+// blockIdx.y: block of 16 channels, its values [slab][16 c][16 k]; a thread takes rows of one channel.
+__global__ void __launch_bounds__(256) filter_max_kernel(int slabs, const float *__restrict__ w, uint32_t *__restrict__ top)
 {
-    uint32_t m = 0;
-    w += (long long)blockIdx.y * n;
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256)
+    const int K = gridDim.y * CB, k = blockIdx.y * CB + (threadIdx.x & 15);
+    uint32_t m = 0, least = 0;
+    for (int slab = blockIdx.x * 16 + (threadIdx.x >> 4); slab < slabs; slab += gridDim.x * 16)
     {
-        const uint32_t b = __float_as_uint(__ldg(w + i)) & 0x7fffffffu;
-        if (b >= 0x7f800000u)
-            top[gridDim.y * CB + 1] = PLAIN_FILTER;
-        else
-            m = max(m, b);
+        const float *row = w + ((long long)blockIdx.y * slabs + slab) * CB * CB + (threadIdx.x & 15);
+        uint32_t r = 0;
+#pragma unroll
+        for (int c = 0; c < CB; ++c)
+        {
+            const uint32_t b = __float_as_uint(__ldg(row + c * CB)) & 0x7fffffffu;
+            if (b >= 0x7f800000u)
+                top[K + 1] = PLAIN_FILTER;
+            else
+                r = max(r, b);
+        }
+        m = max(m, r);
+        least = max(least, r ? ~r : 0u);
     }
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
-    if ((threadIdx.x & 31) < 16 && m)
+    if (m)
     {
-        atomicMax(top + blockIdx.y * CB + (threadIdx.x & 15), m);
-        atomicMax(top + gridDim.y * CB, m);
+        atomicMax(top + k, m);
+        atomicMax(top + K, m);
+        atomicMax(top + K + 3 + k, least);
     }
 }
 
@@ -203,11 +214,10 @@ prepare_filter_kernel(long long n, int slabs, int MT, int K, const float *__rest
     const int kv = (K - tile * MT) < MT ? (K - tile * MT) : MT;
     const long long o = ((long long)tile * MT * slabs * 16 + (long long)slab * kv * 16) * 2 +
                         (long long)(c >> 3) * kv * 16 + (long long)(k - tile * MT) * 8 + (c & 7);
-    // The filter's scale, or the channel's own where the filter's would bring its largest weight below 2^1 (2^12 below the
-    // largest of all): at 2^1 a pair keeps its 22 bits down to 2^-14 of it, and loses no more than 2^-35 of it below that.
-    // Channels that share a scale cost the pixel-major kernel nothing; one that does not, a multiplication per output.
-    const uint32_t all = top[K];
-    const bool own = top[k] && top[k] + (12u << 23) < all;
+    // The filter's scale, or the channel's own where one of its rows would be faint at the filter's.  Channels that share a
+    // scale cost the pixel-major kernel nothing; one that does not, a multiplication per output.
+    const uint32_t all = top[K], least = ~top[K + 3 + k];
+    const bool own = top[k] && __uint_as_float(least) * scale_up(all) < FAINT;
     const uint32_t t0 = own ? top[k] : all;
     if (slab == 0 && c == 0)
     {
@@ -1757,15 +1767,16 @@ int small_b200_filter_prepare_tf32x3(const small_b200_layer *L, const float *fil
         return fail(SMALL_B200_INVALID_ARGUMENT, "Conv2D<float> (3xTF32) ERROR: shape not covered by the tensor-core path.");
     const long long n = (long long)L->K * L->C * L->Fh * L->Fw;
     // [0, n) floats: the half-precision pairs; behind them, for each output channel, the inverse of its block scale and its
-    // largest magnitude, then that of all, and what prepare_filter_kernel says (n is 16 K at least, and the caller provides 2 n)
+    // largest magnitude, then what filter_max_kernel says (n is 16 K at least, and the caller provides 2 n)
     uint32_t *top = reinterpret_cast<uint32_t *>(prepared + n + L->K);
-    SB_CUDA(cudaMemsetAsync(top, 0, ((size_t)L->K + 2) * sizeof(uint32_t), as_stream(stream)));
-    const long long blocks = (n + 255) / 256, per_block = n / L->K * CB, max_blocks = (per_block + 1023) / 1024;
-    filter_max_kernel<<<dim3((unsigned)(max_blocks < 64 ? max_blocks : 64), (unsigned)(L->K / CB)), 256, 0, as_stream(stream)>>>(per_block, filt, top);
+    SB_CUDA(cudaMemsetAsync(top, 0, (2 * (size_t)L->K + 3) * sizeof(uint32_t), as_stream(stream)));
+    const long long blocks = (n + 255) / 256;
+    const int slabs = (L->C / CB) * L->Fh * L->Fw, max_blocks = (slabs + 63) / 64;
+    filter_max_kernel<<<dim3((unsigned)(max_blocks < 64 ? max_blocks : 64), (unsigned)(L->K / CB)), 256, 0, as_stream(stream)>>>(slabs, filt, top);
     if (int rc = launched("filter_max_kernel"))
         return rc;
     prepare_filter_kernel<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(
-        n, (L->C / CB) * L->Fh * L->Fw, pick_mt(L->K), L->K, filt, top, reinterpret_cast<__half *>(prepared), prepared + n);
+        n, slabs, pick_mt(L->K), L->K, filt, top, reinterpret_cast<__half *>(prepared), prepared + n);
     return launched("prepare_filter_kernel");
 }
 

@@ -87,6 +87,19 @@ def test_output_channels_far_apart(case):
            _signed(rng, (N, K, H, W)) * own[None, :, 0])
 
 
+@pytest.mark.parametrize("case", [c for c in CASES if c[0] > 16], ids=[i for c, i in zip(CASES, IDS) if c[0] > 16])
+def test_weights_of_a_channel_far_apart(case):
+    """Half of the blocks of input channels 2^24 larger than the others, their weights as much smaller, in output channels
+    2^11 below the largest: either half matters as much as the other."""
+    C, K, H, W, f, N, _ = case
+    rng = np.random.default_rng(C + K + H)
+    block = np.repeat(np.where(np.arange(C // 16) % 2, 2.0 ** 24, 1.0), 16)
+    own = np.full((K, 1, 1, 1), 2.0 ** -11)
+    own[K // 2] = 1
+    _check(case, _signed(rng, (N, C, H, W)) * block[:, None, None], _signed(rng, (K, C, f, f)) * own / block[:, None, None],
+           _signed(rng, K) * own[:, 0, 0, 0], _signed(rng, (N, K, H, W)) * own[None, :, 0])
+
+
 @pytest.mark.parametrize("bits", [20, 80], ids=lambda b: f"{b}bits")
 @pytest.mark.parametrize("case", CASES, ids=IDS)
 def test_images_far_apart(case, bits):
