@@ -397,7 +397,7 @@ dwconv_u8_dp4a_kernel(const QArgs a, const uint8_t *__restrict__ in, const uint8
 }
 
 // Depthwise 3x3, stride 1, through shared memory.  A tile is whole planes (an image's channel block) where they are small,
-// else a run of rows of one plane; CTAs are persistent and fetch the next tile before they compute one.  Pixels are copied 16
+// else a run of rows of one plane, or of pieces of its rows where two whole rows don't fit (COLS); CTAs are persistent and fetch the next tile before they compute one.  Pixels are copied 16
 // bytes a thread (a bulk copy a row took some 50 cycles each, more than all else for rows of 3 or 6 pixels) into a pitch
 // that has room for the padding, which holds the byte -zero_in, whose contribution (a + zero_in) * w is nothing: every tap is
 // inside.  A thread computes 2 rows x TW pixels of 4 channels.  The four rows a kernel column covers for the two output
@@ -412,6 +412,9 @@ dwconv_u8_dp4a_kernel(const QArgs a, const uint8_t *__restrict__ in, const uint8
 // was bound by L1 wavefronts, with twice the transposes.  2048 images, us before -> now: 16 channels at 48x48 102 -> 70, 32 at
 // 24x24 52 -> 36, 64 at 12x12 29 -> 22, 128 at 6x6 16.5 -> 13.6, 256 at 3x3 9.2 -> 10.9 (half the rows of its last pairs
 // are nothing); a whole MobileNet's 13 layers 330 -> 285.
+// Pieces of rows (from a width of some 380 on; the layer ran one pixel a thread, dwconv_u8_dp4a_kernel, at zero points that kernel
+// takes, else tap by tap), 16 channels, us: 416x416, 64 images 367 -> 159, 1080x1920, 8 images 545 -> 241; at zero points
+// -113 / -121 477 -> 200 and 710 -> 280.  A row's output is a bulk copy of its own, by a lane of its own.
 // TW is odd: eight strips, TW * 16 bytes apart, times four quarters of a pixel then touch all 32 banks.
 constexpr int DW_THREADS = 256;
 struct DwTile
@@ -420,14 +423,15 @@ struct DwTile
     int planes;    // planes per tile (more than one only when a tile covers all rows)
     int rows, row_tiles; // output rows per tile (even, or all of them), tiles down a plane
     int strips, pairs, pitch, in_rows; // pitch and in_rows in pixels and rows of shared memory
+    int cols, col_tiles; // output columns per tile (COLS: a row is cut into several)
     int zero_in, sum_a;  // sum_a: 128 + zero_filt
     int lshift, rshift, mult, k_zero;
     int tiles;
     unsigned in_bytes, out_bytes, out_at, w_at; // bytes of a stage; offsets
-    FastDiv by_row_tiles, by_cbs, by_strips, by_pairs, by_pitch, by_in_rows, by_copy_rows, by_W;
+    FastDiv by_row_tiles, by_col_tiles, by_cbs, by_strips, by_pairs, by_pitch, by_in_rows, by_copy_rows, by_W;
 };
 
-template <int TW, bool SUM_A>
+template <int TW, bool SUM_A, bool COLS>
 __global__ void __launch_bounds__(DW_THREADS, 3)
 dwconv3x3_u8_tile_kernel(const DwTile a, const uint8_t *__restrict__ in, const uint8_t *__restrict__ filt,
                          const int32_t *__restrict__ bias, uint8_t *__restrict__ out)
@@ -436,8 +440,8 @@ dwconv3x3_u8_tile_kernel(const DwTile a, const uint8_t *__restrict__ in, const u
     const int tid = threadIdx.x, first = blockIdx.x, step = gridDim.x;
     // padding: columns, and the rows that are padding in every tile, once for both stages
     const unsigned pad = (unsigned)(-a.zero_in & 255) * 0x01010101u;
-    const bool whole = a.row_tiles == 1;
-    for (int st = 0; st < 2 && first + st * step < a.tiles; ++st)
+    const bool whole = !COLS && a.row_tiles == 1;
+    for (int st = 0; !COLS && st < 2 && first + st * step < a.tiles; ++st)
         for (int i = tid; i < a.planes * a.in_rows * a.pitch; i += DW_THREADS)
         {
             const int lr = a.by_pitch.div(i), x = i - lr * a.pitch - a.pad_l, r = lr - a.by_in_rows.div(lr) * a.in_rows - a.pad_t;
@@ -466,10 +470,32 @@ dwconv3x3_u8_tile_kernel(const DwTile a, const uint8_t *__restrict__ in, const u
         }
         words[(cb * 4 + 3) * CB + ch] = (unsigned)(a.k_zero + (bias ? bias[cb * CB + ch] : 0) + a.zero_in * sum);
     }
+    // Where a tile lies: its first plane, how many, its first output row and column.
+    struct Place { int plane0, planes, oh0, ow0; };
+    auto place = [&](int tile) {
+        const int t = COLS ? a.by_col_tiles.div(tile) : tile, unit = a.by_row_tiles.div(t);
+        return Place{unit * a.planes, min(a.planes, a.N * a.cbs - unit * a.planes), (t - unit * a.row_tiles) * a.rows,
+                     COLS ? (tile - t * a.col_tiles) * a.cols : 0};
+    };
     // A tile's rows: copies of those of the image; rows that are padding (in runs of rows only) are written.
     auto fetch = [&](int tile, int st) {
-        const int unit = a.by_row_tiles.div(tile), oh0 = (tile - unit * a.row_tiles) * a.rows, plane0 = unit * a.planes;
-        const int planes = min(a.planes, a.N * a.cbs - plane0), top = oh0 - a.pad_t;
+        const Place p = place(tile);
+        const int plane0 = p.plane0, planes = p.planes, top = p.oh0 - a.pad_t;
+        if (COLS) // padding on any side: a byte of its own for every pixel outside
+        {
+            const int left = p.ow0 - a.pad_l;
+            const uint8_t *from = in + ((size_t)plane0 * a.H * a.W + left) * CB;
+            for (int i = tid; i < a.in_rows * a.pitch; i += DW_THREADS)
+            {
+                const int lr = a.by_pitch.div(i), x = i - lr * a.pitch, r = lr + top;
+                uint8_t *at = smem + st * a.in_bytes + (size_t)i * CB;
+                if ((unsigned)r < (unsigned)a.H && (unsigned)(x + left) < (unsigned)a.W)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(at)), "l"(from + ((long long)r * a.W + x) * CB) : "memory");
+                else
+                    *reinterpret_cast<uint4 *>(at) = make_uint4(pad, pad, pad, pad);
+            }
+            return;
+        }
         const int r_lo = max(top, 0), r_hi = min(top + a.in_rows, a.H), count = max(r_hi - r_lo, 0);
         uint8_t *stage = smem + st * a.in_bytes;
         const uint32_t to = smem_u32(stage) + (uint32_t)(((r_lo - top) * a.pitch + a.pad_l) * CB);
@@ -489,11 +515,17 @@ dwconv3x3_u8_tile_kernel(const DwTile a, const uint8_t *__restrict__ in, const u
                     *reinterpret_cast<uint4 *>(stage + (size_t)i * CB) = make_uint4(pad, pad, pad, pad);
             }
     };
-    auto store = [&](int tile, int st) { // by one thread, after all of them have fenced and met
-        const int unit = a.by_row_tiles.div(tile), oh0 = (tile - unit * a.row_tiles) * a.rows, plane0 = unit * a.planes;
-        const int planes = min(a.planes, a.N * a.cbs - plane0), rows = min(a.rows, a.Ho - oh0);
-        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out + ((size_t)plane0 * a.Ho + oh0) * a.Wo * CB),
-                     "r"(smem_u32(smem + a.out_at + st * a.out_bytes)), "r"((unsigned)(planes * rows * a.Wo * CB))
+    // By the storing threads, after all of them have fenced and met: one copy, or (COLS) one for each row.
+    const bool storer = COLS ? tid < a.rows : tid == 0;
+    auto store = [&](int tile, int st) {
+        const Place p = place(tile);
+        const int rows = min(a.rows, a.Ho - p.oh0);
+        if (COLS && tid >= rows)
+            return;
+        const int r = COLS ? tid : 0;
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out + (((size_t)p.plane0 * a.Ho + p.oh0 + r) * a.Wo + p.ow0) * CB),
+                     "r"(smem_u32(smem + a.out_at + st * a.out_bytes) + (unsigned)(r * a.cols * CB)),
+                     "r"((unsigned)(COLS ? min(a.cols, a.Wo - p.ow0) * CB : p.planes * rows * a.Wo * CB))
                      : "memory");
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     };
@@ -508,15 +540,16 @@ dwconv3x3_u8_tile_kernel(const DwTile a, const uint8_t *__restrict__ in, const u
         // go, its stage be filled again), and the output before that one has been read.
         asm volatile("cp.async.wait_all;" ::: "memory");
         fence_proxy_async();
-        if (tid == 0)
+        if (storer)
             asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         __syncthreads();
-        if (tid == 0 && tile != first)
+        if (storer && tile != first)
             store(tile - step, st ^ 1);
         if (tile + step < a.tiles)
             fetch(tile + step, st ^ 1);
-        const int unit = a.by_row_tiles.div(tile), oh0 = (tile - unit * a.row_tiles) * a.rows, plane0 = unit * a.planes;
-        const int planes = min(a.planes, a.N * a.cbs - plane0), rows = min(a.rows, a.Ho - oh0);
+        const Place p = place(tile);
+        const int plane0 = p.plane0, planes = p.planes, rows = min(a.rows, a.Ho - p.oh0);
+        const int pitch_out = COLS ? a.cols : a.Wo, cols = COLS ? min(a.cols, a.Wo - p.ow0) : a.Wo;
         const uint8_t *sI = smem + st * a.in_bytes;
         uint8_t *sO = smem + a.out_at + st * a.out_bytes;
         for (int i = tid; i < planes * per_plane * 4; i += DW_THREADS)
@@ -581,12 +614,12 @@ dwconv3x3_u8_tile_kernel(const DwTile a, const uint8_t *__restrict__ in, const u
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 seeds[j] = requant_seed(seed[j], a.mult);
-            unsigned *dst = reinterpret_cast<unsigned *>(sO + ((size_t)(pl * a.rows + r) * a.Wo + ow0) * CB) + q;
+            unsigned *dst = reinterpret_cast<unsigned *>(sO + ((size_t)(pl * a.rows + r) * pitch_out + ow0) * CB) + q;
 #pragma unroll
             for (int h = 0; h < 2; ++h)
 #pragma unroll
                 for (int o = 0; o < TW; ++o)
-                    if (ow0 + o < a.Wo && r + h < rows)
+                    if (ow0 + o < cols && r + h < rows)
                     {
                         unsigned v;
                         if (fast)
@@ -600,14 +633,14 @@ dwconv3x3_u8_tile_kernel(const DwTile a, const uint8_t *__restrict__ in, const u
                         else
                             v = requant_pack4_general(acc[h][o][0] + seed[0], acc[h][o][1] + seed[1], acc[h][o][2] + seed[2],
                                                       acc[h][o][3] + seed[3], a.lshift, a.rshift, a.mult);
-                        dst[(h * a.Wo + o) * 4] = v;
+                        dst[(h * pitch_out + o) * 4] = v;
                     }
         }
         st ^= 1;
     }
     fence_proxy_async();
     __syncthreads();
-    if (tid == 0)
+    if (storer)
     {
         store(first + (a.tiles - 1 - first) / step * step, st ^ 1);
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -1089,59 +1122,87 @@ int launch_dw_tile(const small_b200_layer *L, const QArgs &q, const uint8_t *in,
     // accumulators of 5 would not fit the registers.
     auto cost = [&](int tw) { return (q.Wo + tw - 1) / tw * (tw * 76 + (tw + 2) * 14); };
     const int tw = !a.sum_a && cost(5) <= cost(3) ? 5 : 3;
-    a.strips = (q.Wo + tw - 1) / tw;
-    a.pitch = (a.strips * tw + 2) | 1; // odd: row pairs, two pitches apart, use different banks
-    if (q.W + q.pad_l > a.pitch || q.W > 4096 || q.H > 0x10000)
-        return -1;
+    const long long cap = 72 * 1024, room = 3LL * num_sms(); // three CTAs an SM, what the registers leave
+    const int total_strips = (q.Wo + tw - 1) / tw;
+    auto width = [&](int strips) { // of a tile
+        a.strips = strips; a.cols = strips == total_strips ? q.Wo : strips * tw;
+        a.pitch = (strips * tw + 2) | 1; // odd: row pairs, two pitches apart, use different banks
+    };
     auto bytes = [&](int planes, int rows) {
         const int in_rows = (rows + 1) / 2 * 2 + 2;
         a.in_bytes = (unsigned)((planes * in_rows * a.pitch * CB + 127) & ~127);
-        a.out_bytes = (unsigned)((planes * rows * q.Wo * CB + 127) & ~127);
+        a.out_bytes = (unsigned)((planes * rows * a.cols * CB + 127) & ~127);
         a.out_at = 2 * a.in_bytes;
         a.w_at = a.out_at + 2 * a.out_bytes;
         return (long long)a.w_at + a.cbs * 4 * CB * 4;
     };
     // The tile: the one with the shortest estimated time, rounds of a CTA's threads plus about half a round for a tile's
-    // barrier and copies, at three CTAs an SM (what the registers leave; so many hide each other's waits).
-    const long long cap = 72 * 1024, room = 3LL * num_sms();
-    int best_planes = 0, best_rows = 0;
+    // barrier and copies, with three CTAs an SM, which hide each other's waits.
+    int best_planes = 0, best_rows = 0, best_strips = total_strips;
     double best = 1e30;
-    auto consider = [&](int planes, int rows) {
+    auto consider = [&](int planes, int rows, double copies) {
         const long long items = (long long)planes * ((rows + 1) / 2) * a.strips * 4;
-        const long long tiles = (total_planes + planes - 1) / planes * ((q.Ho + rows - 1) / rows);
-        const double time = (double)((tiles + room - 1) / room) * ((double)((items + DW_THREADS - 1) / DW_THREADS) + 0.5);
-        if (time < best) { best = time; best_planes = planes; best_rows = rows; }
+        const long long tiles = (total_planes + planes - 1) / planes * ((q.Ho + rows - 1) / rows) * ((total_strips + a.strips - 1) / a.strips);
+        const double time = (double)((tiles + room - 1) / room) * ((double)((items + DW_THREADS - 1) / DW_THREADS) + 0.5 + copies);
+        if (time < best) { best = time; best_planes = planes; best_rows = rows; best_strips = a.strips; }
     };
-    for (int planes = 1; planes <= 256 && planes <= total_planes && bytes(planes, q.Ho) <= cap; ++planes)
-        consider(planes, q.Ho);
-    for (int rows = 2; rows < q.Ho && bytes(1, rows) <= cap; rows += 2)
-        consider(1, rows);
+    if (q.W <= 4096 && q.H <= 0x10000)
+    {
+        width(total_strips);
+        if (q.W + q.pad_l <= a.pitch)
+        {
+            for (int planes = 1; planes <= 256 && planes <= total_planes && bytes(planes, q.Ho) <= cap; ++planes)
+                consider(planes, q.Ho, 0.0);
+            for (int rows = 2; rows < q.Ho && bytes(1, rows) <= cap; rows += 2)
+                consider(1, rows, 0.0);
+        }
+    }
+    // Rows that don't fit as a whole, four in and two out, twice (192 bytes a pixel: from a width of some 380 on, less with many
+    // channels), are cut.  Whole rows are as fast up to there: 16 channels, 64 images, 376 wide 158 us, 416 wide in pieces 159.
+    // Tiles of 4 to 32 rows then, so that few of the rows are copied twice; a sixteenth of a round for a pixel a thread copies.
+    const bool cut = !best_planes;
+    if (cut)
+        for (int pieces = 2; pieces <= total_strips; ++pieces)
+        {
+            const int strips = (total_strips + pieces - 1) / pieces;
+            if (strips == a.strips || strips > 128)
+                continue;
+            width(strips);
+            for (int rows = std::min(4, q.Ho); rows <= std::min(32, q.Ho) && bytes(1, rows) <= cap; rows += rows < q.Ho ? std::min(2, q.Ho - rows) : 1)
+                consider(1, rows, ((rows + 1) / 2 * 2 + 2) * a.pitch / (16.0 * DW_THREADS));
+            if (strips <= 8)
+                break;
+        }
     if (!best_planes)
         return -1;
+    width(best_strips);
+    a.col_tiles = (total_strips + a.strips - 1) / a.strips;
     a.planes = best_planes; a.rows = best_rows;
     a.row_tiles = (q.Ho + a.rows - 1) / a.rows;
     a.pairs = (a.rows + 1) / 2; a.in_rows = 2 * a.pairs + 2;
     const size_t smem = (size_t)bytes(a.planes, a.rows);
-    const long long tiles = (total_planes + a.planes - 1) / a.planes * a.row_tiles;
+    const long long tiles = (total_planes + a.planes - 1) / a.planes * a.row_tiles * a.col_tiles;
     if (tiles > 0x3fffffffLL || total_planes > 0x3fffffffLL)
         return -1;
     a.tiles = (int)tiles;
     const unsigned blocks = (unsigned)(tiles < room ? tiles : room);
-    const int copy_rows = std::min(a.H, a.in_rows - a.pad_t); // rows of the image in a tile of whole planes
+    const int copy_rows = cut ? 1 : std::min(a.H, a.in_rows - a.pad_t); // rows of the image in a tile of whole planes
     if (copy_rows <= 0)
         return -1;
-    a.by_row_tiles.set(a.row_tiles); a.by_cbs.set(a.cbs); a.by_strips.set(a.strips); a.by_pairs.set(a.pairs);
+    a.by_row_tiles.set(a.row_tiles); a.by_col_tiles.set(a.col_tiles); a.by_cbs.set(a.cbs); a.by_strips.set(a.strips); a.by_pairs.set(a.pairs);
     a.by_pitch.set(a.pitch); a.by_in_rows.set(a.in_rows); a.by_copy_rows.set(copy_rows); a.by_W.set(a.W);
     static PerDeviceOnce configured;
     int dev;
     if (configured.needed(&dev))
     {
-        SB_CUDA(cudaFuncSetAttribute(dwconv3x3_u8_tile_kernel<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
-        SB_CUDA(cudaFuncSetAttribute(dwconv3x3_u8_tile_kernel<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
-        SB_CUDA(cudaFuncSetAttribute(dwconv3x3_u8_tile_kernel<5, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+        for (auto k : {dwconv3x3_u8_tile_kernel<3, true, false>, dwconv3x3_u8_tile_kernel<3, false, false>, dwconv3x3_u8_tile_kernel<5, false, false>,
+                       dwconv3x3_u8_tile_kernel<3, true, true>, dwconv3x3_u8_tile_kernel<3, false, true>, dwconv3x3_u8_tile_kernel<5, false, true>})
+            SB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
         configured.mark(dev);
     }
-    auto kern = a.sum_a ? dwconv3x3_u8_tile_kernel<3, true> : tw == 5 ? dwconv3x3_u8_tile_kernel<5, false> : dwconv3x3_u8_tile_kernel<3, false>;
+    auto kern = a.sum_a ? (cut ? dwconv3x3_u8_tile_kernel<3, true, true> : dwconv3x3_u8_tile_kernel<3, true, false>)
+              : tw == 5 ? (cut ? dwconv3x3_u8_tile_kernel<5, false, true> : dwconv3x3_u8_tile_kernel<5, false, false>)
+                        : (cut ? dwconv3x3_u8_tile_kernel<3, false, true> : dwconv3x3_u8_tile_kernel<3, false, false>);
     kern<<<blocks, DW_THREADS, smem, st>>>(a, in, filt, bias, out);
     return launched("dwconv3x3_u8_tile_kernel");
 }

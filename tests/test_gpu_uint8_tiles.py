@@ -45,6 +45,41 @@ def test_depthwise_3x3_tiles(oracle, case, zp):
     assert want.min() < want.max()
 
 
+# rows that do not fit a tile as a whole: a last piece of one strip, of few columns and of one; runs of rows with an odd
+# one at the end; a single row; columns of nothing but padding; the widest
+WIDE_CASES = [
+    (16, 37, 416, None, 2), (16, 5, 700, None, 1), (48, 34, 1001, None, 1), (16, 1, 900, None, 2), (16, 9, 511, (0, 0, 0, 0), 2),
+    (32, 6, 640, (2, 4, 3, 1), 1), (2048, 3, 190, None, 1), (16, 3, 5003, None, 1),
+]
+
+
+@pytest.mark.parametrize("case", WIDE_CASES, ids=lambda c: "C{}_{}x{}_p{}_n{}".format(*c))
+@pytest.mark.parametrize("zp", [(0, -128), (-113, -121), (-255, -250)], ids=lambda z: "zi{}_zf{}".format(*z))
+def test_depthwise_3x3_tiles_of_wide_images(oracle, case, zp):
+    test_depthwise_3x3_tiles(oracle, case, zp)
+
+
+@pytest.mark.parametrize("zp", [(-128, -128), (-113, -121)], ids=lambda z: "zi{}_zf{}".format(*z))
+def test_depthwise_3x3_of_wide_images_is_as_fast_as_of_narrow_ones(zp):
+    """A pixel of a row that does not fit a tile takes no longer than one of a row that does (0.9 of its time; 2.1 to 2.3
+    on the kernel for any window): half as long again is left for the clock."""
+    import torch
+
+    def us(W):
+        C, H, N = 16, 416, 64
+        x = qbuf(np.random.default_rng(W).integers(0, 256, N * C * H * W), zp[0])
+        w, o = qbuf(np.arange(C * 9) % 256, zp[1]), _out(N * C * H * W, Quant(*zp, 0, 8, 1 << 30, 0))
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(7)]
+        for e in ev:
+            for _ in range(10):
+                S.DepthwiseConv2D(3, 3, 1, 1, 1, 1, 1, C, H, W, x, w, o, batch=N)
+            e.record()
+        torch.cuda.synchronize()
+        return min(a.elapsed_time(b) for a, b in zip(ev, ev[1:])) / W
+
+    assert us(416) <= 1.5 * us(368)
+
+
 @pytest.mark.parametrize("case", [(32, 16, 8, 8, 5), (256, 256, 3, 3, 31), (64, 128, 6, 6, 8), (128, 32, 1, 2, 130), (96, 48, 5, 13, 4),
                                   (32, 64, 12, 12, 17), (64, 32, 24, 24, 3), (32, 16, 3, 43, 140)],
                          ids=lambda c: "C{}_K{}_{}x{}_n{}".format(*c))
