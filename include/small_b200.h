@@ -178,6 +178,10 @@ int small_b200_conv2d_f32_tf32x3_supported(const small_b200_layer *L);
  * of at least 256 pixels in all), else 0.  The C++ platform headers and the Python executor both
  * ask here, so they pick the same kernel for the same call. */
 int small_b200_conv2d_f32_tf32x3_preferred(const small_b200_layer *L);
+/* How the current device's launch cuts a covered layer: cut[0] the widest tile in pixels, cut[1] how many CTAs of a
+ * cluster share the reduction of a tile, cut[2] the same for the tiles of a last, partial wave where those are a
+ * launch of their own (0: they are not).  For tests and reports; the convolution asks itself. */
+int small_b200_conv2d_f32_tf32x3_cut(const small_b200_layer *L, int *cut);
 int small_b200_filter_prepare_tf32x3(const small_b200_layer *L, const float *filt, float *prepared, void *stream);
 int small_b200_conv2d_f32_tf32x3(const small_b200_layer *L, const float *in, const float *filt_prepared,
                                  const float *bias, float *out, void *stream);

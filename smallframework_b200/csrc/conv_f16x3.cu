@@ -1824,6 +1824,25 @@ struct Cut
 {
     int npx_cap, split, rem_split;
 };
+int configure()
+{
+    static PerDeviceOnce configured;
+    int dev;
+    if (configured.needed(&dev))
+    {
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        configured.mark(dev);
+    }
+    return SMALL_B200_OK;
+}
 // Clusters of S such CTAs (one per SM) that the current device runs at a time: they may not cross the borders of its
 // groups of SMs (148 SMs: 74 pairs, 33 clusters of 4, 22 of 6, 15 of 8).
 int resident_clusters(int S)
@@ -1902,21 +1921,8 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
 {
     if (int rc = check_window_layer(L, "Conv2D<float>", true, 2))
         return rc;
-    static PerDeviceOnce configured;
-    int dev;
-    if (configured.needed(&dev))
-    {
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        configured.mark(dev);
-    }
+    if (int rc = configure())
+        return rc;
     TcArgs a;
     const Cut cut = pool ? Cut{256, 1, 0} : choose_cut(L);
     if (pool ? !plan_pooled(L, pool, a) : !plan(L, a, cut.npx_cap))
@@ -2014,6 +2020,17 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
     return SMALL_B200_OK;
 }
 } // namespace
+
+extern "C" int small_b200_conv2d_f32_tf32x3_cut(const small_b200_layer *L, int *cut)
+{
+    if (!L || !cut || !small_b200_conv2d_f32_tf32x3_supported(L))
+        return fail(SMALL_B200_INVALID_ARGUMENT, "Conv2D<float> (3xTF32) ERROR: shape not covered by the tensor-core path.");
+    if (int rc = configure()) // the clusters that fit are counted with the kernel's shared memory
+        return rc;
+    const Cut c = choose_cut(L);
+    cut[0] = c.npx_cap; cut[1] = c.split; cut[2] = c.rem_split;
+    return SMALL_B200_OK;
+}
 
 // ---------------------------------------------------------------------------------------------
 // The same tensor-core convolution for callers that must not allocate device memory.

@@ -1,8 +1,8 @@
 """Parity at the sizes the benchmark runs, layer by layer, against the oracle (which is
 bit-identical to the reference's REF build): Tiny-YOLOv2 at 416x416 on both fp32 paths (two
-images alone, and two sampled images of a 64-image launch, which is what takes the persistent
-multi-tile loops, the wide-image tiling and the two-CTA split reduction through several
-waves), the 13 YOLOv3-tiny convolutions at 416x416, DS-CNN uint8 at batch 4096 and
+images alone, where most layers' tiles are shared by the CTAs of a cluster, and three sampled images of a
+64-image launch, which is what takes the persistent multi-tile loops, the wide-image tiling and a launch
+for the last, partial wave of tiles at their real sizes), the 13 YOLOv3-tiny convolutions at 416x416, DS-CNN uint8 at batch 4096 and
 MobileNet-v1 x0.25 uint8 at batch 2048 with sampled images, bit-exact.
 
 Every layer is compared on the input the device kernel itself read, so the 1e-5 gate
@@ -15,6 +15,7 @@ import torch
 from smallframework_b200 import _lib, networks
 from smallframework_b200 import packing as P
 from tests.gpu_util import oracle_chain, rel_max_err, run_layers_checked
+from tests.test_gpu_cluster_cuts import cut_of
 
 pytestmark = pytest.mark.gpu
 
@@ -53,8 +54,8 @@ def test_tiny_yolov2_416_two_images_per_layer(oracle, tensor_core):
 
 @pytest.mark.parametrize("tensor_core", [False, "auto"])
 def test_tiny_yolov2_416_batch64_sampled_images(oracle, tensor_core):
-    """The launch the benchmark times: 64 images per GPU.  conv8 then is 512 tiles = 1024 CTAs in
-    clusters of two over several waves, conv2/conv3 walk many tiles per persistent CTA."""
+    """The launch the benchmark times: 64 images per GPU.  conv8 then is 512 tiles of one CTA each in whole waves and the rest in a
+    launch of clusters of two, conv2/conv3 walk many tiles per persistent CTA."""
     layers = networks.tiny_yolov2(seed=4, size=416)
     N = 64
     g = torch.Generator(device="cuda").manual_seed(41)
@@ -84,8 +85,10 @@ def test_yolov3_tiny_layer_416(oracle, idx):
 
 
 def test_conv_1024_to_1024_13x13_many_clusters(oracle):
-    """The split reduction (two CTAs per tile) with far more clusters than SMs: 40 images x 8
-    channel tiles = 320 tiles = 640 CTAs."""
+    """40 images x 8 channel tiles = 320 tiles: two whole waves of one CTA a tile and 24 tiles in clusters of three.  (Cuts over a
+    whole layer: tests/test_gpu_cluster_cuts.py.)"""
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert cut_of(1024, 1024, 13, 13, 3, 40) == (1, 3)
     L = dict(op="conv", name="deep", C=1024, K=1024, H=13, W=13, Fh=3, Fw=3, stride=1, pads=(1, 1, 1, 1),
              act=2, slope=0.1)
     rng = np.random.default_rng(77)
