@@ -604,12 +604,17 @@ def run_layer_sweep(args):
         "clocks": clk.summary(), "layers": rows}), flush=True)
 
 
-# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of a layer's launch from a one-pass ncu
-# capture at the bench size: (layer, batch) -> (bytes, summary under profiles/, date of the capture).
-# A capture belongs to the kernel as it was that day; the line reports the provenance with the number.
+# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of a layer's launches from a one-pass ncu
+# capture at the bench size: (layer, batch, kernel) -> (bytes, summary under profiles/, date of the capture).
+# The kernel's name is part of the key: another kernel's bytes say nothing about the one that runs.
 MEASURED_TRAFFIC = {
-    ("conv8", 64): (210.6e6, "conv_tf32x3_kernel_conv8_batch16.md", "2026-11-25"),
+    ("conv8", 64, "conv_f16x3_kernel"): (186.6e6, "convolution_kernels_small_cases.md", "2026-12-02"),
 }
+
+
+def measured_traffic(layer, batch, kernel):
+    """The captured traffic of this kernel on this layer at this batch, or None."""
+    return MEASURED_TRAFFIC.get((layer, batch, kernel.split()[0]))
 
 
 def kernel_class(chain, i, L, dtype):
@@ -715,7 +720,7 @@ def per_layer_report(chain, layers, batch, wl, clocks, torch, pipes=None):
     top = max(range(len(rows)), key=lambda i: rows[i]["ms"])
     flops, nbytes = work[top]
     kcls = rows[top]["pipe"]
-    traffic = MEASURED_TRAFFIC.get((rows[top]["layer"], batch))
+    traffic = measured_traffic(rows[top]["layer"], batch, rows[top]["kernel"])
     src = None if traffic is None else {"profile": "profiles/" + traffic[1], "captured": traffic[2]}
     if rows[top]["bound"] != "hbm":
         achieved = flops / (rows[top]["ms"] * 1e-3) / 1e12
