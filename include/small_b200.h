@@ -160,7 +160,7 @@ int small_b200_conv2d_maxpool_f32(const small_b200_layer *conv, const small_b200
  * (which the functions are named after).  The power of two belongs to the filter, or to one output
  * channel that would lose digits by that, and to each patch of 16 input channels of a tile.  Whatever the
  * magnitudes beside them, a pixel's 16 values keep 22 bits of the largest of them (tiles whose pixels lie 2^26
- * and more apart are computed on the FMA pipe, many times more slowly, and so are those with an
+ * and more apart are computed on the FMA pipe, 8 to 140 times more slowly, and so are those with an
  * infinity), and a tap's 16 weights 22 bits of the largest of them down to 2^-26 of the largest of the
  * output channel (beneath that, an error of 2^-47 of the latter).  The scales are
  * undone in fp32.  The activations are split inside the kernel, in shared memory.  The caller

@@ -9,8 +9,9 @@
 // hi*hi terms in up to six accumulators in turn, because the tensor core truncates when it adds.  Against fp64 the largest error is a half to a third of the FFMA kernel's (3.1e-7 to 4.7e-7 of
 // the largest output against 5.2e-7 to 1.5e-6).
 //
-// What bounds it: shared memory.  A step of 64 output channels writes 24 KB of words and the MMAs read some 36 KB: 570 to 590
-// cycles, of which the MMAs alone would need 250.  Copies by cp.async to shared memory with the split there took 760, one
+// What bounds it: no unit (32 -> 64 channels 3x3 at 16x16, 1024 images: L1 and shared memory 66 % of their peak, issue 46 %, the
+// unit that feeds the tensor pipe 34 %) but the chain of a step, loads above all.  A step of 64 output channels writes 24 KB of
+// words and the MMAs read some 36 KB: 570 to 590 cycles, of which the MMAs alone would need 250.  Copies by cp.async to shared memory with the split there took 760, one
 // step at a time in all pixel warps 1200, eight pairs of pixel warps (64 registers a thread) 660.  With 16 input channels it
 // is the latency of the loads: 680 cycles, whatever the number of output channels.
 // Stride 2, us, FFMA kernel -> this one: 96 -> 192 channels 3x3 at 57x57, 32 images 346 -> 95; 32 -> 64 3x3 at 16x16, 1024

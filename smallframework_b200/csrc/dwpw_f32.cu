@@ -1,10 +1,13 @@
 // dwpw_f32.cu -- fp32 depthwise 3x3 convolution and the 1x1 convolution behind it (a depthwise-separable block,
 // include/small/models/MobileNetTiny.hpp) as one kernel: the activation between the two never leaves the SM.
 //
-// What bounds it: memory.  A block moves its input and its output once; as two layers the activation between them is
+// A block moves its input and its output once; as two layers the activation between them is
 // written and read again, and the 1x1 layer alone ran at 2 to 3 TB/s because its patches went through shared memory three
 // times (bulk copy, operand split, tensor core).  Here what the depthwise warps write to shared memory IS the tensor
 // core's operand.
+// What bounds it: no unit (16 channels at 48x48, 256 images: issue 37 % of its peak, loads and stores of shared memory 23 %,
+// tensor pipe 3 %, DRAM 10 %) but the depthwise warps' chain of reads, sums and stores, 3.6 times the block's bytes at copy
+// bandwidth there.
 //
 // A tile is NI images x TH x TW <= 128 output pixels times KT <= 128 output channels.  Roles of a persistent CTA:
 //   * one thread keeps patches of 16 channels on their way, one TMA box each (rows of the image are contiguous in it, zeros
@@ -12,8 +15,8 @@
 //     trips to memory per strip: 385 us for the block of 16 channels at 48x48 on 2048 images.)
 //   * eight warps compute the depthwise layer, each one 16-channel block of a tile at a time and on its own (they meet
 //     nowhere): a thread owns four channels of a block of R x 3 outputs, reads every input of that block once (2.5 reads
-//     per output with R = 4, 4.5 with one row: shared memory, not the FMA pipe, is what these warps press on), and writes
-//     every value as it is (hi: the tensor core ignores the 13 low mantissa bits of a tf32 operand) and as v - trunc(v)
+//     per output with R = 4, 4.5 with one row) and the filter's nine 16-byte words again for every output row (up to three per
+//     output more: 68 of the 96 registers hold sums and inputs), and writes every value as it is (hi: the tensor core ignores the 13 low mantissa bits of a tf32 operand) and as v - trunc(v)
 //     (lo) into rows of 64 bytes in the 64-byte swizzle.  Neighbouring blocks are three pixels apart, an odd number, so the
 //     reads of eight lanes fall into different banks (stride 1);
 //   * one warp issues the MMAs, kind::tf32, M = 128 pixels: x_hi * [W_hi | W_lo] and x_lo * W_hi.  The cross terms have
@@ -23,6 +26,10 @@
 // tf32 words rather than the block-scaled half-precision ones of conv_f16x3.cu: they need no scale, so a thread can write
 // its operands without knowing its neighbours' magnitudes, and the tensor pipe has time to spare (128 -> 128 channels:
 // 3072 cycles per tile against 2980 for the tile's bytes).
+// An infinity has no second word (inf - inf): outputs whose products sum to an infinity are NaN here.  Making such sums
+// again from the products, as conv_gather_f32.cu and conv_f16x3.cu do, was taken back: the code for it, never run, in the
+// epilogue, behind a call or behind the last barrier, costs every block 3.5 to 6 % (MobileNet at 2048 images 1092 -> 1130
+// to 1160 us).
 #include "tc_common.cuh"
 
 namespace sb

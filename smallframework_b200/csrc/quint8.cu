@@ -407,8 +407,8 @@ dwconv_u8_dp4a_kernel(const QArgs a, const uint8_t *__restrict__ in, const uint8
 //   sum (a + zI)(w + zF) = sum a w' + (128 + zF) sum a + zI sum (w + zF)
 // with the last term in the seed of the requantisation and the second one (SUM_A: another three dp4a a column) only
 // where zF != -128.  The output goes back through shared memory as one bulk copy.
-// What bounds it: the integer pipes (three dp4a, two or three instructions of transposes and loads, four and a half of
-// requantisation per output byte).  Reading strips of a row straight from global memory, 96 bytes apart from lane to lane,
+// What bounds it: instructions (three dp4a, two or three of transposes and loads, four and a half of requantisation per output
+// byte): 62 % of the issue slots and 42 % of the ALU at 256 images of 48x48.  Reading strips of a row straight from global memory, 96 bytes apart from lane to lane,
 // was bound by L1 wavefronts, with twice the transposes.  2048 images, us before -> now: 16 channels at 48x48 102 -> 70, 32 at
 // 24x24 52 -> 36, 64 at 12x12 29 -> 22, 128 at 6x6 16.5 -> 13.6, 256 at 3x3 9.2 -> 10.9 (half the rows of its last pairs
 // are nothing); a whole MobileNet's 13 layers 330 -> 285.
@@ -1312,7 +1312,7 @@ int launch_onestep(const OneArgs &a, const uint8_t *in, const uint8_t *filt, con
     const size_t smem = (size_t)a.K * (WORDS + 1) * 4; // at most 36 KB
     constexpr int PX = 2;
     const long long sms = num_sms(), many = (long long)PX * 256;
-    if (a.total >= sms * many) // four pixels a thread once that leaves a CTA for every SM
+    if (a.total >= sms * many) // two pixels a thread once that leaves a CTA for every SM
     {
         const long long nb = std::min((a.total + many - 1) / many, sms * 8);
         conv2d_u8_onestep_kernel<WORDS, KIND, PX><<<(unsigned)nb, 256, smem, st>>>(a, in, filt, bias, out);

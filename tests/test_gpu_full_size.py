@@ -54,8 +54,8 @@ def test_tiny_yolov2_416_two_images_per_layer(oracle, tensor_core):
 
 @pytest.mark.parametrize("tensor_core", [False, "auto"])
 def test_tiny_yolov2_416_batch64_sampled_images(oracle, tensor_core):
-    """The launch the benchmark times: 64 images per GPU.  conv8 then is 512 tiles of one CTA each in whole waves and the rest in a
-    launch of clusters of two, conv2/conv3 walk many tiles per persistent CTA."""
+    """The launch the benchmark times: 64 images per GPU.  conv8 then is 512 tiles, 444 in three whole waves of one CTA each and 68 in
+    a launch of clusters of two, conv2/conv3 walk many tiles per persistent CTA."""
     layers = networks.tiny_yolov2(seed=4, size=416)
     N = 64
     g = torch.Generator(device="cuda").manual_seed(41)
