@@ -656,8 +656,10 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     if (warp < FIRST_ACC_WARP || warp >= FIRST_SPLIT_WARP)
     {
         // The launch has 512 x 128 registers; the roles' shares add up to that at most (setmaxnreg draws on nothing else):
-        // 128 x 88 + 256 x 168 + 128 x 88, pixel-major tiles 128 x 88 + 256 x 144 + 128 x 112.
-        if (PIXM && warp >= FIRST_SPLIT_WARP)
+        // 128 x 88 + 256 x 168 + 128 x 88, pixel-major tiles 128 x 112 + 256 x 144 + 128 x 112.  (The least share also bounds
+        // the function that is called for wide tiles: with 88 for the issuing warps it and its callers spilled, 16 -> 32 channels at
+        // 208x208 with the pool 186 us, 168 with 112.)
+        if (PIXM)
             asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");
         else
             asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
