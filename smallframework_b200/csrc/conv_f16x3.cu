@@ -17,14 +17,14 @@
 //     (which the zeros of the padding must not meet), the layer does.  A NaN in the activations is its own pair.
 // So an output channel, an image or a pixel is as good as if it stood alone: the words of a value that is in range do not
 // depend on the power of two.  (With lo stored as it is, 22 bits ended at 2^-3 and an error of 2^-24 remained: an output channel 2^-12 of
-// the largest kept half its digits.  The scaled second word costs 0.5 to 1.5 % of a layer: Tiny-YOLOv2 on 64 images 1.576
-// -> 1.597 ms, ResNet-8 on 1024 426 -> 432 us.)  Scales are undone in the FMA with which the
+// the largest kept half its digits.  All of this costs 0.5 to 1.5 %: Tiny-YOLOv2 on 64 images 1.625
+// -> 1.635 ms, ResNet-8 on 1024 429 -> 435 us.)  Scales are undone in the FMA with which the
 // accumulation warps add a partial sum to their fp32 registers.  kind::f16 covers 16 channels per instruction where
 // kind::tf32 covers 8 at the same cost (N/2 cycles of the pipe, 128 + N operand rows of 32 bytes), so a layer needs half
 // the instructions, half the operand traffic in shared memory and half the filter bytes of the 3xTF32 form this
-// replaced: 1024 -> 1024 channels 3x3 on 64 images of 13x13 0.800 -> 0.464 ms, 16 -> 32 at 208x208 with the max
-// pool 0.198 -> 0.162, 128 -> 256 at 26x26 0.122 -> 0.075.  Against fp64 the 9216-term sums of the first are off by
-// 5.2e-7 of the largest (3xTF32: 7.3e-7; the fp32 loop nest of include/small/abstract_layer.hpp:1368-1823, whose
+// replaced: 1024 -> 1024 channels 3x3 on 64 images of 13x13 0.800 -> 0.439 ms, 16 -> 32 at 208x208 with the max
+// pool 0.198 -> 0.168, 128 -> 256 at 26x26 0.122 -> 0.078.  Against fp64 the 9216-term sums of the first are off by
+// 5.3e-7 of the largest (3xTF32: 7.3e-7; the fp32 loop nest of include/small/abstract_layer.hpp:1368-1823, whose
 // FLOAT_CONV_TILE_C this replaces: 5.7e-6).
 //
 // GEMM orientation: D[k][pixel] = sum_c W[k][c] * X[pixel][c].  The output channels are the
@@ -262,7 +262,7 @@ constexpr int COLS_PER_THREAD = 128;
 
 // Two fp32 values times their block scale as two pairs of half-precision words: hi = v,
 // lo = (v - hi) * 2^LO_SHIFT, both cut to 11 bits as a tf32 operand is.  (Rounded to nearest the 9216-term sums come out at 3.0e-7 of the
-// largest instead of 5.2e-7, but then results drift from the 3xTF32 form's by more than either is off: 2.5e-5 of a
+// largest instead of 5.3e-7, but then results drift from the 3xTF32 form's by more than either is off: 2.5e-5 of a
 // YOLO head, whose box sizes are exponentials, against 2e-6 with the same words.)
 // up_lo = up * LO_UP.  (v - hi) * LO_UP in one fma on the half-precision word itself: as many instructions as without the factor.
 __device__ __forceinline__ void split2(float a, float b, float up, float up_lo, uint32_t &hi, uint32_t &lo)
