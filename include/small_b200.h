@@ -197,7 +197,7 @@ int small_b200_conv2d_maxpool_f32_tf32x3(const small_b200_layer *conv, const sma
 /* The tensor-core convolution above for callers that cannot allocate device memory (code
  * running where cudaMalloc is forbidden or would stall the device, plug-ins that are handed
  * nothing but their input and output pointers).  It takes the PACKED filter as the reference
- * lays it out and keeps its scratch -- the re-laid filter and its lo copy -- in a fixed 16 MiB
+ * lays it out and keeps its scratch -- the re-laid filter and its scales -- in a fixed 16 MiB
  * array inside the library, so it calls no allocator of any kind.  Limits and rules:
  *   - 2*K*C*Fh*Fw floats must fit in 4 Mi floats; larger calls are
  *     refused with SMALL_B200_INVALID_ARGUMENT and a message that states both sizes;
