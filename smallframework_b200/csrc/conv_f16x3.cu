@@ -384,11 +384,11 @@ struct Tile
 __device__ __forceinline__ Tile decode_tile(const TcArgs &a, int t)
 {
     // Pixel tile fastest, then the image, channel tile slowest.  The CTAs that run at the same time then
-    // share one or two filter slices (a slice of a 1024 -> 1024 3x3 layer is 9.4 MB with its lo copy),
+    // share one or two filter slices (a slice of a 1024 -> 1024 3x3 layer is 4.7 MB),
     // which stay in L2 while every image's tiles pass over them, and the activations of the whole batch
     // (44 MB there) stay in L2 from one slice to the next; neighbouring tiles of an image, whose patches
     // share their halo rows, still run side by side.  With the channel tile fastest, every 9 images streamed
-    // all 75 MB of filter again: 541 MB of DRAM reads per launch for 126 MB of algorithmic bytes (176 MB
+    // all of the filter again (with tf32 words, 541 MB of DRAM reads for 126 MB of algorithmic bytes; 166 MB
     // now, and the layer 3 % faster).
     Tile T;
     const int t1 = a.by_px_tiles.div(t), pt = t - t1 * a.px_tiles;
@@ -1659,7 +1659,7 @@ bool plan_as_g(const small_b200_layer *L, TcArgs &a, bool pixm, bool pool, bool 
     const int gran = a.pixm ? 128 : 64;
     int npx_first = ((m_img + tiles_cap - 1) / tiles_cap + gran - 1) / gran * gran;
     // First pass: only plans that keep two patches in flight (a layer with few channel blocks
-    // per CTA otherwise waits for every patch's load and lo copy), even at a narrower tile;
+    // per CTA otherwise waits for every patch's load and split), even at a narrower tile;
     // second pass: anything that fits.
     for (int pass = 0; pass < 2; ++pass)
         for (int npx = npx_first; npx >= (pass == 0 ? 128 : gran); npx -= gran)
@@ -2038,7 +2038,7 @@ extern "C" int small_b200_conv2d_f32_tf32x3_cut(const small_b200_layer *L, int *
 // The same tensor-core convolution for callers that must not allocate device memory.
 //
 // small_b200_conv2d_f32_tf32x3 needs scratch from its caller: the filter re-laid for the tensor
-// core, with its lo copy.  Some callers cannot provide it: code that runs inside
+// core, with its scales.  Some callers cannot provide it: code that runs inside
 // a region where cudaMalloc is forbidden or would synchronise the device (a real-time loop, a
 // plug-in that only ever receives its input and output pointers, a host that has handed all of
 // its device memory to another allocator).  For them the scratch lives in this fixed array
@@ -2079,7 +2079,7 @@ extern "C" int small_b200_conv2d_f32_tf32x3_noalloc(const small_b200_layer *L, c
         return fail(SMALL_B200_INVALID_ARGUMENT,
                     "Conv2D<float> (3xTF32, no-alloc) ERROR: shape not covered by the tensor-core path.");
     const size_t filt_elems = (size_t)L->K * L->C * L->Fh * L->Fw;
-    const size_t need = 2 * filt_elems; // the re-laid filter and its lo copy
+    const size_t need = 2 * filt_elems; // what small_b200_filter_prepare_tf32x3 asks for
     if (need > STATIC_SCRATCH_FLOATS)
         return fail(SMALL_B200_INVALID_ARGUMENT,
                     "Conv2D<float> (3xTF32, no-alloc) ERROR: this call needs " + std::to_string(need * 4) +
