@@ -380,6 +380,18 @@ int small_b200_conv2d_avgpool_dense_u8(const small_b200_layer *conv, const small
                                        const small_b200_layer *dense, const uint8_t *in, const uint8_t *conv_filt,
                                        const int32_t *conv_bias, const uint8_t *dense_filt, const int32_t *dense_bias,
                                        uint8_t *out, void *stream);
+/* The whole keyword-spotting network (include/small/models/DSCNNTiny.hpp) as one kernel: layers[0] the first
+ * layer (1 -> 64 channels, windows up to 16x4), then up to six pairs of a 3x3 stride-1 'same' depthwise and a 1x1 convolution of 64
+ * channels, then a global average pool and a dense layer (K <= 128): n = 2 * pairs + 3 layers, images of at most 128 pixels behind the
+ * first layer.  ..._prepare() lays the weights out once per set of weights in ..._prepared_bytes() bytes (0: not covered; opaque, 16-byte
+ * aligned): filts[i] / biases[i] are layer i's device pointers (NULL for the pool; biases, or any of them, may be NULL), and the layers'
+ * quantisers and zero points are those of the call.  `out` holds [N][layers[n - 1].K] bytes.  Bit-identical to the n calls. */
+int small_b200_separable_network_u8_supported(const small_b200_layer *layers, int32_t n);
+size_t small_b200_separable_network_u8_prepared_bytes(const small_b200_layer *layers, int32_t n);
+int small_b200_separable_network_u8_prepare(const small_b200_layer *layers, int32_t n, const uint8_t *const *filts,
+                                            const int32_t *const *biases, void *prepared, void *stream);
+int small_b200_separable_network_u8(const small_b200_layer *layers, int32_t n, const void *prepared, const uint8_t *in, uint8_t *out,
+                                    void *stream);
 /* small::DepthwiseConv2D<QUInt8Buffer> (:1059); with L->accumulate = 1 PartialDepthwiseConv2D (:1194)
  * under the conditions of the partial convolution above (C = 16, N = 1, bias = NULL). */
 int small_b200_dwconv2d_u8(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt,

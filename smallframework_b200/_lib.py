@@ -107,13 +107,17 @@ SIGNATURES = {
     "small_b200_conv2d_dwconv2d_u8": [_LP, _LP, _VP, _VP, _VP, _VP, _VP, _VP, _VP],
     "small_b200_conv2d_avgpool_dense_u8_supported": [_LP, _LP, _LP],
     "small_b200_conv2d_avgpool_dense_u8": [_LP, _LP, _LP, _VP, _VP, _VP, _VP, _VP, _VP, _VP],
+    "small_b200_separable_network_u8_supported": [_LP, _I32],
+    "small_b200_separable_network_u8_prepare": [_LP, _I32, C.POINTER(_VP), C.POINTER(_VP), _VP, _VP],
+    "small_b200_separable_network_u8": [_LP, _I32, _VP, _VP, _VP, _VP],
     "small_b200_groupconv2d_u8": [_LP, C.c_int32, _VP, _VP, _VP, _VP, _VP],
     "small_b200_maxpool2d_u8": [_LP, _VP, _VP, _VP],
     "small_b200_avgpool2d_u8": [_LP, _VP, _VP, _VP],
     "small_b200_relu_u8": [_I64, _LP, _VP, _VP, _VP],
 }
 OTHER = {"small_b200_last_error": ([], C.c_char_p), "small_b200_launch_count": ([], C.c_uint64),
-         "small_b200_nms_scratch_bytes": ([C.c_int32], C.c_size_t)}
+         "small_b200_nms_scratch_bytes": ([C.c_int32], C.c_size_t),
+         "small_b200_separable_network_u8_prepared_bytes": ([_LP, C.c_int32], C.c_size_t)}
 
 
 def exported_names():

@@ -328,7 +328,8 @@ class Chain:
         producer and enqueue_layer() does nothing for it.  fuse_u8: a uint8 convolution followed by a
         3x3 depthwise convolution (the reference's Conv2D_ReLU_DepthwiseConv2D_ReLU pairing), or by the
         global average pool and the dense layer that end the keyword-spotting network, runs as one kernel
-        where the library covers the shapes; the absorbed layers are entered in `fused_into` likewise.
+        where the library covers the shapes; the absorbed layers are entered in `fused_into` likewise; a keyword-spotting network
+        that the library covers whole (small_b200_separable_network_u8_supported) is one kernel.
         "auto" also runs layers of a few million multiply-adds in the latency kernel
         (small_b200_conv2d_f32_small_preferred) and a global average pool with the dense layer and the softmax behind it as
         one kernel.  fuse_dw: an fp32 depthwise convolution followed by a 1x1 convolution (a depthwise-separable block) runs as
@@ -424,7 +425,19 @@ class Chain:
                     continue
                 if lib().small_b200_conv2d_maxpool_f32_supported(C.byref(dc), C.byref(dp)):
                     self.fused_into[i + 1] = i
-        if dtype == "u8" and fuse_u8:
+        self.whole = None  # the list is one kernel: its weights, laid out once
+        if dtype == "u8" and fuse_u8 and not any("src" in L for L in layers):
+            descs = self._desc_array()
+            nbytes = lib().small_b200_separable_network_u8_prepared_bytes(descs, len(layers))
+            if nbytes:
+                self.whole = torch.empty(nbytes, dtype=torch.uint8, device=self.dev)
+                ptrs = lambda k: (C.c_void_p * len(layers))(*[None if t[k] is None else t[k].data_ptr() for t in self.params])
+                check(lib().small_b200_separable_network_u8_prepare(descs, len(layers), ptrs(0), ptrs(1), self.whole.data_ptr(),
+                                                                    torch.cuda.current_stream().cuda_stream))
+                torch.cuda.synchronize()
+        if self.whole is not None:
+            self.fused_into = {i: 0 for i in range(1, len(layers))}
+        elif dtype == "u8" and fuse_u8:
             i = 0
             while i < len(layers) - 1:
                 L = layers[i]
@@ -482,6 +495,10 @@ class Chain:
                      q.get("zero_in", 0), q.get("zero_filt", 0), q.get("lshift", 0),
                      q.get("rshift", 0), q.get("multiplier", 0), 0)
 
+    def _desc_array(self):
+        return (Layer * len(self.layers))(*[self._desc(L, L["C"] if i == 0 else padded(L["C"]))
+                                            for i, L in enumerate(self.layers)])
+
     def enqueue_layer(self, i, src, dst, stream):
         L = self.layers[i]
         wt, bs = self.params[i]
@@ -493,7 +510,9 @@ class Chain:
         if i in self.fused_into:
             return  # computed by its producer
         follow = self.absorbed(i)
-        if i in self.tails:
+        if self.whole is not None:
+            check(l.small_b200_separable_network_u8(self._desc_array(), len(self.layers), p(self.whole), p(src), p(dst), stream))
+        elif i in self.tails:
             D = self.layers[i + 1]
             w2, b2 = self.params[i + 1]
             check(l.small_b200_avgpool_dense_f32(C.byref(d), C.byref(self._desc(D, padded(D["C"]))), int(len(follow) > 1), p(src),

@@ -1,0 +1,106 @@
+"""A keyword-spotting network as one kernel (csrc/net_u8_tc.cu) against the oracle's layer-by-layer result, bit-exact: both
+splits of a CTA's warps over images (up to two images a CTA, up to four; several rounds), images up to the 128-pixel limit and down to one
+pixel, windows of one to four chunks of the reduction, signed and unsigned operands, constants too large for the
+in-accumulator form, quantisers outside the common form."""
+import numpy as np
+import pytest
+import torch
+
+from smallframework_b200 import _lib, networks
+from smallframework_b200 import packing as P
+from smallframework_b200.packing import calc_padding, output_dim
+from tests.gpu_util import oracle_chain
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # H, W, Fh, Fw, stride, blocks, batch, zero_in, zero_mid, classes, biases, quantiser
+    (49, 10, 10, 4, 2, 4, 1, -128, 0, 12, 1024, "common"),
+    (49, 10, 10, 4, 2, 4, 3, -128, 0, 12, 1024, "common"),
+    (49, 10, 10, 4, 2, 4, 200, -128, 0, 12, 1024, "common"),     # two images a CTA
+    (49, 10, 10, 4, 2, 4, 301, -128, 0, 12, 1024, "common"),     # four, some CTAs with fewer
+    (49, 10, 10, 4, 2, 4, 1400, -128, 0, 12, 1024, "common"),    # several rounds
+    (16, 8, 3, 3, 1, 1, 5, 0, 0, 128, 1024, "common"),           # 128 pixels
+    (11, 11, 16, 1, 1, 2, 450, 0, -128, 16, 1024, "common"),     # one column of sixteen taps, signed intermediates
+    (1, 1, 1, 1, 1, 1, 600, -128, 0, 3, 0, "common"),            # one pixel, no biases
+    (9, 1, 5, 2, 1, 6, 7, -128, -128, 12, 1024, "common"),       # one column, six blocks
+    (1, 40, 2, 4, 3, 5, 170, 0, 0, 12, 3_000_000, "common"),     # one row; constants beyond the digits
+    (20, 12, 10, 4, 2, 2, 310, -128, 0, 12, 1024, "left shift"),
+    (20, 12, 10, 4, 2, 2, 2, -128, -128, 12, 3_000_000, "small right shift"),
+]
+
+
+def _same(H, W, Fh, Fw, s):
+    return (*calc_padding(H, Fh, s), *calc_padding(W, Fw, s))
+
+
+def _layers(rng, H, W, Fh, Fw, s, blocks, zi, zm, classes, top, quantiser):
+    """Random weights; multipliers calibrated on two images so that every layer's bytes spread over 0..255."""
+    cur = rng.integers(0, 256, (2, 1, H, W)).astype(np.uint8)
+    L = []
+
+    def add(op, name, C, K, H, W, Fh, Fw, s, pads, zero):
+        nonlocal cur
+        dw = op == "dwconv"
+        w = rng.integers(0, 256, (K, Fh, Fw) if dw else (K, C, Fh, Fw)).astype(np.uint8)
+        b = rng.integers(-top, top + 1, K).astype(np.int32) if top else np.zeros(K, np.int32)
+        acc = networks._calibrate(cur, w, b, zero, -128, s, pads, dw)
+        scale = 255.0 / max(float(np.percentile(acc, 99)), 1.0)
+        ls, rs, mult = networks._requant_params(scale)
+        if quantiser == "left shift":
+            ls, rs = 1, rs + 1
+        elif quantiser == "small right shift":
+            rs, mult = 1, max(int(round(scale * 2.0 ** 32)), 1)
+        L.append(dict(op=op, name=name, C=C, K=K, H=H, W=W, Fh=Fh, Fw=Fw, stride=s, pads=pads, act=0, slope=0.0, w=w,
+                      b=b if top else None, q=dict(zero_in=zero, zero_filt=-128, lshift=ls, rshift=rs, multiplier=mult)))
+        cur = np.clip(np.rint(acc * scale), 0, 255).astype(np.uint8)
+
+    pads = _same(H, W, Fh, Fw, s)
+    h, v = output_dim(H, pads[0], pads[1], Fh, s), output_dim(W, pads[2], pads[3], Fw, s)
+    add("conv", "stem", 1, 64, H, W, Fh, Fw, s, pads, zi)
+    for i in range(blocks):
+        add("dwconv", f"dw{i}", 64, 64, h, v, 3, 3, 1, (1, 1, 1, 1), zm)
+        add("conv", f"pw{i}", 64, 64, h, v, 1, 1, 1, (0, 0, 0, 0), int(rng.integers(-20, 20)) if zm else 0)
+    ls, rs, mult = networks._requant_params(1.0 / (h * v))
+    L.append(dict(op="avgpool", name="pool", C=64, K=64, H=h, W=v, Fh=h, Fw=v, stride=1, pads=(0, 0, 0, 0),
+                  q=dict(zero_in=0, zero_filt=0, lshift=ls, rshift=rs, multiplier=mult)))
+    cur = np.clip(np.rint(cur.astype(np.float64).mean(axis=(2, 3), keepdims=True)), 0, 255).astype(np.uint8)
+    add("conv", "dense", 64, classes, 1, 1, 1, 1, 1, (0, 0, 0, 0), 0)
+    return L
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "{}x{}_k{}x{}_s{}_b{}_n{}_zi{}_zm{}_Kd{}_{}_{}".format(*c).replace(" ", ""))
+def test_network_is_one_kernel(oracle, case):
+    H, W, Fh, Fw, s, blocks, N, zi, zm, classes, top, quantiser = case
+    rng = np.random.default_rng(H * 1000 + W * 10 + N)
+    layers = _layers(rng, H, W, Fh, Fw, s, blocks, zi, zm, classes, top, quantiser)
+    chain = networks.Chain(layers, N, "u8")
+    x = P.pack_activation(rng.integers(0, 256, (N, 1, H, W), dtype=np.uint8))
+    chain.x.copy_(torch.from_numpy(x.ravel()))
+    chain.capture()
+    for _ in range(2):
+        chain.launch()
+    chain.stream.synchronize()
+    assert _lib.device_status() == 0
+    assert chain.kernels_per_step == 1
+    got = chain.y.cpu().numpy().reshape(N, -1)
+    for n in sorted(set([0, N // 3, N // 2, N - 1])):
+        want = oracle_chain(oracle, layers, x[n], "u8")
+        assert np.array_equal(got[n], want), (n, got[n], want)
+    assert len(np.unique(got[:, :classes])) > 1
+
+
+def test_networks_outside_the_one_kernel_form_run_layer_by_layer(oracle):
+    """144 pixels do not fit a tile: the same list runs as its layers, with the same bytes."""
+    rng = np.random.default_rng(5)
+    layers = _layers(rng, 12, 12, 3, 3, 1, 1, -128, 0, 12, 1024, "common")
+    chain = networks.Chain(layers, 2, "u8")
+    assert chain.whole is None
+    x = P.pack_activation(rng.integers(0, 256, (2, 1, 12, 12), dtype=np.uint8))
+    chain.x.copy_(torch.from_numpy(x.ravel()))
+    chain.capture()
+    chain.launch()
+    chain.stream.synchronize()
+    got = chain.y.cpu().numpy().reshape(2, -1)
+    for n in range(2):
+        assert np.array_equal(got[n], oracle_chain(oracle, layers, x[n], "u8"))
