@@ -1284,6 +1284,9 @@ int conv2d_u8_tensor_core(const small_b200_layer *L, const uint8_t *in, const ui
                           const int32_t *bias, uint8_t *out, cudaStream_t st);
 int conv2d_u8_one_channel_tc(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt,
                              const int32_t *bias, uint8_t *out, cudaStream_t st);
+// Defined in conv_u8_patch.cu: windows of more than one tap on blocks of channels, for zero points whose padding is a byte.
+int conv2d_u8_patch(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
+                    uint8_t *out, cudaStream_t st);
 // Defined in conv_u8_ring.cu: every other window / stride / channel count as an implicit GEMM on the
 // tensor core, for the zero points it covers; -1 otherwise.
 int conv2d_u8_ring(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
@@ -1403,6 +1406,12 @@ int conv2d_u8_dispatch(const small_b200_layer *L, const uint8_t *in, const uint8
         const int one = conv2d_u8_onestep(L, a, in, filt, bias, out, as_stream(stream));
         if (one >= 0)
             return one;
+    }
+    if (tensor_core)
+    {
+        const int tc2 = conv2d_u8_patch(L, in, filt, bias, out, as_stream(stream));
+        if (tc2 >= 0)
+            return tc2;
     }
     if (tensor_core)
     {

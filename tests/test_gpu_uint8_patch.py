@@ -1,0 +1,55 @@
+"""The uint8 convolution that fetches its pixels once (csrc/conv_u8_patch.cu) against the oracle, bit-exact: rows cut into
+parts, ragged last tiles, several whole images a tile, strides of two with odd sizes, windows other than 3x3, odd numbers of
+channel blocks, filters that stay in shared memory and filters that travel with the pixels, partial blocks of output channels,
+and the zero points whose padding is a byte."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_uint8 import _case_id, _check_conv, _quant
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # C, K, H, W, Fh, Fw, stride, pads, batch
+    (64, 64, 45, 37, 3, 3, 1, "same", 5),       # three rows of the full width a tile
+    (64, 128, 45, 37, 3, 3, 2, "same", 3),
+    (32, 16, 33, 37, 3, 3, 1, "same", 45),      # several tiles a CTA
+    (64, 128, 45, 37, 3, 3, 2, "same", 38),     # ... with two stages
+    (144, 32, 20, 20, 3, 3, 1, "same", 112),    # ... in chunks of the channels
+    (16, 16, 112, 112, 3, 3, 1, "same", 2),     # one block of channels: nine slabs, an odd step
+    (16, 32, 11, 130, 3, 3, 1, "same", 1),      # wider than a tile
+    (48, 48, 7, 7, 3, 3, 1, "same", 40),        # whole images a tile, odd blocks
+    (32, 64, 3, 3, 3, 3, 1, "same", 37),        # many of them, the last tile partial
+    (32, 32, 1, 1, 3, 3, 1, "same", 9),         # every tap but one outside
+    (256, 256, 20, 19, 3, 3, 1, "same", 2),     # the filter travels
+    (256, 128, 20, 19, 3, 3, 1, "same", 38),    # ... through several tiles a CTA
+    (208, 336, 9, 10, 3, 3, 2, "same", 3),      # odd blocks, a partial block of output channels
+    (256, 512, 14, 13, 3, 3, 2, "same", 2),
+    (512, 64, 10, 6, 3, 3, 1, "same", 1),
+    (32, 48, 9, 14, 5, 5, 1, "same", 2),
+    (16, 16, 30, 9, 7, 7, 1, "same", 2),
+    (80, 16, 17, 5, 2, 4, 2, "valid", 3),
+    (64, 32, 6, 40, 1, 3, 1, "same", 2),
+    (32, 32, 40, 6, 3, 1, 2, "same", 2),
+    (16, 16, 3, 3, 7, 7, 1, (3, 3, 3, 3), 4),   # windows that cover the image
+    (32, 64, 57, 57, 3, 3, 1, (1, 0, 0, 1), 1),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=_case_id)
+@pytest.mark.parametrize("zp", [(0, -128), (-113, -121), (-255, -130)], ids=lambda z: "zi{}_zf{}".format(*z))
+def test_conv2d_u8_patch(oracle, case, zp):
+    from oracle.bindings import same_pads
+    C, K, H, W, Fh, Fw, s, pm, N = case
+    pads = same_pads(H, W, Fh, Fw, s) if pm == "same" else (0, 0, 0, 0) if pm == "valid" else pm
+    rng = np.random.default_rng(C * 100 + H * 10 + W + zp[0] + 1000)
+    _check_conv(oracle, case, pads, _quant(rng, C * Fh * Fw, zp), rng, zp[0] != 0, None)
+
+
+@pytest.mark.parametrize("shift", [0, 1], ids=lambda r: f"rshift{r}")
+def test_quantisers_outside_the_common_form(oracle, shift):
+    from oracle.bindings import Quant, same_pads
+    case = (32, 32, 9, 11, 3, 3, 1, "same", 2)
+    rng = np.random.default_rng(3)
+    q = Quant(-3, -120, 2 - 2 * shift, shift, 1 << 14, 0)
+    _check_conv(oracle, case, same_pads(9, 11, 3, 3, 1), q, rng, True, None)
