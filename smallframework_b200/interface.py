@@ -13,6 +13,7 @@ non-CUDA buffer raises.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 
 import numpy as np
@@ -95,8 +96,14 @@ def _to_device(data, dtype, device):
     return torch.from_numpy(np.ascontiguousarray(data, dtype=np_dtype).reshape(-1)).to(device)
 
 
+_raw_stream, _device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream(stream):
     if stream is None:
+        # the handle itself: a Stream object takes 3.3 us of a layer call's 10 to 13, the handle 0.2
+        if _raw_stream is not None and torch.cuda.is_initialized():
+            return _raw_stream(_device())
         return torch.cuda.current_stream().cuda_stream
     return getattr(stream, "cuda_stream", stream)
 
@@ -126,6 +133,22 @@ def _layer(batch, C_, K, H, W, Fh, Fw, stride, t, b, l, r, accumulate=0, act=ACT
     return L
 
 
+@functools.lru_cache(maxsize=1024, typed=True)
+def _described(*fields):
+    """A descriptor as the library takes it and the layer's output height and width, kept by value: a program calls the same
+    few layers again and again, and building one takes 2 us.  Nobody writes to a descriptor."""
+    L = Layer(*fields)
+    return (C.byref(L), *L.out_hw())
+
+
+def _desc(batch, C_, K, H, W, Fh, Fw, stride, t, b, l, r, accumulate, act, slope, inp, filt, out):
+    if not isinstance(out, QUInt8Buffer):
+        return _described(batch, C_, K, H, W, Fh, Fw, stride, t, b, l, r, accumulate, act, slope, 0, 0, 0, 0, 0, 0)
+    return _described(batch, C_, K, H, W, Fh, Fw, stride, t, b, l, r, accumulate, act, slope,
+                      inp.zero() if isinstance(inp, QUInt8Buffer) else 0, filt.zero() if isinstance(filt, QUInt8Buffer) else 0,
+                      out.lshift, out.rshift, out.multiplier, 0)
+
+
 def _need(buf, elems, what):
     if buf.size() < elems:
         raise ValueError(f"{what}: buffer holds {buf.size()} elements, {elems} needed")
@@ -134,8 +157,7 @@ def _need(buf, elems, what):
 # --------------------------------------------------------------------------- dense conv
 def _conv(name, partial, kh, kw, stride, t, b, l, r, K, C_, H, W, inp, filt, out, bias, act,
           slope, batch, stream, path=None):
-    L = _layer(batch, C_, K, H, W, kh, kw, stride, t, b, l, r, int(partial), act, slope, inp, filt, out)
-    ho, wo = L.out_hw()
+    L, ho, wo = _desc(batch, C_, K, H, W, kh, kw, stride, t, b, l, r, int(partial), act, slope, inp, filt, out)
     if C_ % CB == 0 or C_ in (1, 2, 3):
         _need(inp, batch * C_ * H * W, name + " input")
         _need(filt, K * C_ * kh * kw, name + " filter")
@@ -143,11 +165,11 @@ def _conv(name, partial, kh, kw, stride, t, b, l, r, K, C_, H, W, inp, filt, out
         # the quint8 partial form finds its int32 partial sums in the output buffer
         _need(out, (4 if partial and _is_q(out) else 1) * batch * K * ho * wo, name + " output")
     if _is_q(out):
-        fn = {None: lib().small_b200_conv2d_u8, "cuda_cores": lib().small_b200_conv2d_u8_cuda_cores,
-              "tensor_core": lib().small_b200_conv2d_u8_tensor_core}[path]
+        fn = lib().small_b200_conv2d_u8 if path is None else {
+            "cuda_cores": lib().small_b200_conv2d_u8_cuda_cores, "tensor_core": lib().small_b200_conv2d_u8_tensor_core}[path]
     else:
         fn = lib().small_b200_conv2d_f32
-    check(fn(C.byref(L), _ptr(inp), _ptr(filt), _ptr(bias), _ptr(out), _stream(stream)))
+    check(fn(L, _ptr(inp), _ptr(filt), _ptr(bias), _ptr(out), _stream(stream)))
 
 
 def Conv2D(kernel_height, kernel_width, stride, t_pad, b_pad, l_pad, r_pad,
@@ -236,16 +258,15 @@ def Conv2D_Bias_Activation_Maxpool2D(conv_kernel_height, conv_kernel_width, conv
 # --------------------------------------------------------------------------- per-channel windows
 def _window(fn_f32, fn_u8, name, has_filter, kh, kw, stride, t, b, l, r, C_, H, W, inp, filt, out,
             bias, partial, act, slope, batch, stream):
-    L = _layer(batch, C_, C_, H, W, kh, kw, stride, t, b, l, r, int(partial), act, slope, inp, filt, out)
-    ho, wo = L.out_hw()
+    L, ho, wo = _desc(batch, C_, C_, H, W, kh, kw, stride, t, b, l, r, int(partial), act, slope, inp, filt, out)
     if C_ % CB == 0:
         _need(inp, batch * C_ * H * W, name + " input")
         _need(out, (4 if partial and _is_q(out) else 1) * batch * C_ * ho * wo, name + " output")
     fn = getattr(lib(), fn_u8 if _is_q(out) else fn_f32)
     if has_filter:
-        check(fn(C.byref(L), _ptr(inp), _ptr(filt), _ptr(bias), _ptr(out), _stream(stream)))
+        check(fn(L, _ptr(inp), _ptr(filt), _ptr(bias), _ptr(out), _stream(stream)))
     else:
-        check(fn(C.byref(L), _ptr(inp), _ptr(out), _stream(stream)))
+        check(fn(L, _ptr(inp), _ptr(out), _stream(stream)))
 
 
 def DepthwiseConv2D(kernel_height, kernel_width, stride, t_pad, b_pad, l_pad, r_pad,
@@ -349,9 +370,9 @@ def ReLUActivation(input_channels, input_height, input_width, input_buf, output_
     n = batch * input_channels * input_height * input_width
     if _is_q(output_buf):
         _chan_check("ReLUActivation<quint8>", input_channels)
-        L = _layer(batch, input_channels, input_channels, input_height, input_width, 1, 1, 1,
-                   0, 0, 0, 0, inp=input_buf, out=output_buf)
-        check(lib().small_b200_relu_u8(n, C.byref(L), _ptr(input_buf), _ptr(output_buf), _stream(stream)))
+        L, _, _ = _desc(batch, input_channels, input_channels, input_height, input_width, 1, 1, 1, 0, 0, 0, 0, 0, ACT_NONE, 0.0,
+                        input_buf, None, output_buf)
+        check(lib().small_b200_relu_u8(n, L, _ptr(input_buf), _ptr(output_buf), _stream(stream)))
     else:
         _chan_check("ReLUActivation<float>", input_channels)
         check(lib().small_b200_relu_f32(n, _ptr(input_buf), _ptr(output_buf), _stream(stream)))
@@ -457,9 +478,9 @@ def Conv2D_3xTF32(kernel_height, kernel_width, stride, t_pad, b_pad, l_pad, r_pa
                   partial=False, activation=ACT_NONE, negative_slope=0.0, batch=1, stream=None):
     """small::Conv2D / PartialConv2D<FloatBuffer> (+ bias / activation) on the tensor cores;
     prepared_filter_buf = prepare_filter_3xTF32(filter)."""
-    L = _layer(batch, input_channels, output_channels, input_height, input_width, kernel_height,
-               kernel_width, stride, t_pad, b_pad, l_pad, r_pad, int(partial), activation, negative_slope)
-    check(lib().small_b200_conv2d_f32_tf32x3(C.byref(L), _ptr(input_buf),
+    L, _, _ = _desc(batch, input_channels, output_channels, input_height, input_width, kernel_height, kernel_width, stride, t_pad,
+                    b_pad, l_pad, r_pad, int(partial), activation, negative_slope, None, None, None)
+    check(lib().small_b200_conv2d_f32_tf32x3(L, _ptr(input_buf),
                                              _ptr(prepared_filter_buf), _ptr(bias_buf),
                                              _ptr(output_buf), _stream(stream)))
 
