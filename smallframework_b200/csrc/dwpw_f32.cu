@@ -7,7 +7,7 @@
 // core's operand.
 // What bounds it: no unit (16 channels at 48x48, 256 images: issue 37 % of its peak, loads and stores of shared memory 23 %,
 // tensor pipe 3 %, DRAM 10 %) but the depthwise warps' chain of reads, sums and stores, 3.6 times the block's bytes at copy
-// bandwidth there.
+// bandwidth there.  Blocks of so few channels run on the FMA pipe (dwpw_direct_f32.cu, where the rule stands).
 //
 // A tile is NI images x TH x TW <= 128 output pixels times KT <= 128 output channels.  Roles of a persistent CTA:
 //   * one thread keeps patches of 16 channels on their way, one TMA box each (rows of the image are contiguous in it, zeros
@@ -36,6 +36,9 @@ namespace sb
 {
 bool conv_small_preferred(const small_b200_layer *L); // conv_small_f32.cu
 double conv_small_us(const small_b200_layer *L);
+// dwpw_direct_f32.cu: blocks of few channels on the FMA pipe; -1 where it leaves them to this kernel
+int dwpw_direct_f32(const small_b200_layer *D, const small_b200_layer *L, const float *in, const float *dwf, const float *b1, const float *pwf,
+                    const float *b2, float *out, cudaStream_t st);
 } // namespace sb
 
 namespace
@@ -636,6 +639,9 @@ int small_b200_dwconv2d_conv2d_f32(const small_b200_layer *dw, const small_b200_
     a.ns2 = pw->act == SMALL_B200_ACT_RELU ? 0.f : pw->act == SMALL_B200_ACT_LEAKY ? pw->slope : 1.f;
     a.has_b1 = dw_bias != nullptr; a.has_b2 = pw_bias != nullptr;
     cudaStream_t st = as_stream(stream);
+    const int direct = dwpw_direct_f32(dw, pw, in, dw_filt, dw_bias, pw_prepared, pw_bias, out, st);
+    if (direct >= 0)
+        return direct;
     CUtensorMap mx; // [N][C/16][H][W x 8 elements of 8 bytes]
     {
         const uint64_t dims[4] = {(uint64_t)a.W * 8, (uint64_t)a.H, (uint64_t)a.cbs, (uint64_t)a.N};
