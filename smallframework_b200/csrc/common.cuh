@@ -234,6 +234,24 @@ __device__ __forceinline__ uint4 requant_pack16(const int32_t *acc, int32_t lshi
 }
 #endif
 
+#ifdef __CUDACC__
+// Eight floats to memory, as one 32-byte store where the buffer's alignment allows it.  A thread that owns a pixel writes 64 bytes, 64
+// from the next thread's: 16 bytes at a time that is half a sector a lane and four times the ideal number of passes.
+__device__ __forceinline__ bool whole_sectors(const float *buffer) { return (reinterpret_cast<uintptr_t>(buffer) & 31) == 0; }
+__device__ __forceinline__ void store8(float *p, const float *v, bool sectors)
+{
+    if (sectors)
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]),
+                     "f"(v[5]), "f"(v[6]), "f"(v[7])
+                     : "memory");
+    else
+    {
+        reinterpret_cast<float4 *>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<float4 *>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+}
+#endif
+
 __device__ __forceinline__ float apply_act(float v, int act, float slope)
 {
     if (act == SMALL_B200_ACT_RELU)

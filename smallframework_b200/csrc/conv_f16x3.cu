@@ -1023,7 +1023,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             const float w_down = own_scales ? 1.f : __ldg(filt_down + 2 * a.K + 2);
             const int quarter = warp & 3, mt = (warp - FIRST_ACC_WARP) >> 2;
             const int mtiles = a.NPX >> 7;
-            const bool active = mt < mtiles;
+            const bool active = mt < mtiles, sectors = whole_sectors(out);
             const size_t plane = (size_t)a.o_kb_stride;
             bool ok = true;
             int gc = 0, pc = 0; // groups flushed, patches they came from
@@ -1164,11 +1164,12 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                             for (int j = 0; j < HALF / 4; ++j)
                             {
                                 const float4 y = reinterpret_cast<const float4 *>(xrow)[j]; // row rl + 1 shares the slot
-                                float4 x = make_float4(fmaxf(keep[4 * j], y.x), fmaxf(keep[4 * j + 1], y.y),
-                                                       fmaxf(keep[4 * j + 2], y.z), fmaxf(keep[4 * j + 3], y.w));
-                                x.x = apply_act_ns(x.x, act_ns); x.y = apply_act_ns(x.y, act_ns);
-                                x.z = apply_act_ns(x.z, act_ns); x.w = apply_act_ns(x.w, act_ns);
-                                *(reinterpret_cast<float4 *>(o + (size_t)(j >> 2) * plane) + (j & 3)) = x;
+                                keep[4 * j] = apply_act_ns(fmaxf(keep[4 * j], y.x), act_ns);
+                                keep[4 * j + 1] = apply_act_ns(fmaxf(keep[4 * j + 1], y.y), act_ns);
+                                keep[4 * j + 2] = apply_act_ns(fmaxf(keep[4 * j + 2], y.z), act_ns);
+                                keep[4 * j + 3] = apply_act_ns(fmaxf(keep[4 * j + 3], y.w), act_ns);
+                                if (j & 1)
+                                    store8(o + (size_t)(j >> 2) * plane + (j & 2) * 4, keep + 4 * j - 4, sectors);
                             }
                         }
                     }
@@ -1188,17 +1189,17 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
 #pragma unroll
                                 for (int j = 0; j < 4; ++j)
                                 {
-                                    float4 x = make_float4(acc[kb * 16 + 4 * j], acc[kb * 16 + 4 * j + 1], acc[kb * 16 + 4 * j + 2],
-                                                           acc[kb * 16 + 4 * j + 3]);
-                                    float4 *op = reinterpret_cast<float4 *>(o + (size_t)kb * plane) + j;
+                                    float *x = acc + kb * 16 + 4 * j, *op = o + (size_t)kb * plane + 4 * j;
                                     if (a.accumulate)
                                     {
-                                        const float4 s4 = *op;
-                                        x.x += s4.x; x.y += s4.y; x.z += s4.z; x.w += s4.w;
+                                        const float4 s4 = *reinterpret_cast<const float4 *>(op);
+                                        x[0] += s4.x; x[1] += s4.y; x[2] += s4.z; x[3] += s4.w;
                                     }
-                                    x.x = apply_act_ns(x.x, act_ns); x.y = apply_act_ns(x.y, act_ns);
-                                    x.z = apply_act_ns(x.z, act_ns); x.w = apply_act_ns(x.w, act_ns);
-                                    *op = x;
+#pragma unroll
+                                    for (int e = 0; e < 4; ++e)
+                                        x[e] = apply_act_ns(x[e], act_ns);
+                                    if (j & 1)
+                                        store8(op - 4, x - 4, sectors);
                                 }
                             }
                     }

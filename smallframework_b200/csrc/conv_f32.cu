@@ -583,15 +583,16 @@ conv2d_first_pool_fixed_f32_kernel(const ConvArgs a, const float *__restrict__ i
     if constexpr (POOL)
     {
         float *o = out + (((size_t)n * (a.K / CB) + kb) * Hp * Wp + p) * CB;
+        const bool sectors = whole_sectors(out);
 #pragma unroll
-        for (int k4 = 0; k4 < CB; k4 += 4)
+        for (int k8 = 0; k8 < CB; k8 += 8)
         {
-            float v[4];
+            float v[8];
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                v[q] = fmaxf(fmaxf(apply_act_ns(acc[0][k4 + q], act_neg_scale(a.act, a.slope)), apply_act_ns(acc[1][k4 + q], act_neg_scale(a.act, a.slope))),
-                             fmaxf(apply_act_ns(acc[2][k4 + q], act_neg_scale(a.act, a.slope)), apply_act_ns(acc[3][k4 + q], act_neg_scale(a.act, a.slope))));
-            *reinterpret_cast<float4 *>(o + k4) = make_float4(v[0], v[1], v[2], v[3]);
+            for (int q = 0; q < 8; ++q)
+                v[q] = fmaxf(fmaxf(apply_act_ns(acc[0][k8 + q], act_neg_scale(a.act, a.slope)), apply_act_ns(acc[1][k8 + q], act_neg_scale(a.act, a.slope))),
+                             fmaxf(apply_act_ns(acc[2][k8 + q], act_neg_scale(a.act, a.slope)), apply_act_ns(acc[3][k8 + q], act_neg_scale(a.act, a.slope))));
+            store8(o + k8, v, sectors);
         }
     }
 }

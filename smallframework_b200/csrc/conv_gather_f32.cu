@@ -302,6 +302,7 @@ conv_gather_f32_kernel(const GArgs a, const float *__restrict__ in, const float 
     {
         // ---------------- sums, bias, activation, stores ----------------
         const int quarter = warp & 3, half = (warp - FIRST_EPI_WARP) >> 2, m = quarter * 32 + lane, hw = a.Ho * a.Wo;
+        const bool sectors = whole_sectors(out);
         bool ok = true;
         int buf = 0, odd_start = 0;
         uint32_t phase = 0;
@@ -357,9 +358,11 @@ conv_gather_f32_kernel(const GArgs a, const float *__restrict__ in, const float 
                             const float4 r = dst[j];
                             b.x += r.x; b.y += r.y; b.z += r.z; b.w += r.w;
                         }
-                        dst[j] = make_float4(apply_act_ns(y[4 * j] + b.x, a.ns), apply_act_ns(y[4 * j + 1] + b.y, a.ns),
-                                             apply_act_ns(y[4 * j + 2] + b.z, a.ns), apply_act_ns(y[4 * j + 3] + b.w, a.ns));
+                        y[4 * j] = apply_act_ns(y[4 * j] + b.x, a.ns); y[4 * j + 1] = apply_act_ns(y[4 * j + 1] + b.y, a.ns);
+                        y[4 * j + 2] = apply_act_ns(y[4 * j + 2] + b.z, a.ns); y[4 * j + 3] = apply_act_ns(y[4 * j + 3] + b.w, a.ns);
                     }
+                    store8(reinterpret_cast<float *>(dst), y, sectors);
+                    store8(reinterpret_cast<float *>(dst + 2), y + 8, sectors);
                 }
             }
             tc_fence_before_sync();

@@ -52,14 +52,6 @@ __device__ __forceinline__ float2 parts(pair a)
     return d;
 }
 
-// Whole sectors: 16 bytes a lane, 64 apart, took four times the ideal number of passes.
-__device__ __forceinline__ void store8(float *p, const float *v)
-{
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]),
-                 "f"(v[6]), "f"(v[7])
-                 : "memory");
-}
-
 template <int K, int S>
 __global__ void __launch_bounds__(MAX_THREADS, CTAS)
 dwpw_direct_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ DirectArgs a, const float *__restrict__ dwf,
@@ -189,7 +181,7 @@ dwpw_direct_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
                         const float2 s = parts(acc[v][kb * 8 + 4 * q + e]);
                         y[2 * e] = apply_act_ns(s.x, a.ns2); y[2 * e + 1] = apply_act_ns(s.y, a.ns2);
                     }
-                    store8(o + ((size_t)kb * a.Ho + v) * a.Wo * CB + q * 8, y);
+                    store8(o + ((size_t)kb * a.Ho + v) * a.Wo * CB + q * 8, y, true);
                 }
 }
 

@@ -408,6 +408,7 @@ dwpw_f32_kernel(const __grid_constant__ CUtensorMap map_x, const DpArgs a, const
         const int hw = a.Ho * a.Wo;
         const int m = quarter * 32 + lane, rr = a.by_TW.div(m), ni = a.by_TH.div(rr);
         const int r = rr - ni * a.TH, c = m - rr * a.TW; // this lane's pixel of a tile
+        const bool sectors = whole_sectors(out);
         bool ok = true;
         int buf = 0;
         uint32_t phase = 0;
@@ -457,9 +458,11 @@ dwpw_f32_kernel(const __grid_constant__ CUtensorMap map_x, const DpArgs a, const
                     {
                         const float4 b = a.has_b2 ? __ldg(reinterpret_cast<const float4 *>(b2 + kt * a.KT + kb * CB) + j)
                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
-                        dst[j] = make_float4(apply_act_ns(y[4 * j] + b.x, a.ns2), apply_act_ns(y[4 * j + 1] + b.y, a.ns2),
-                                             apply_act_ns(y[4 * j + 2] + b.z, a.ns2), apply_act_ns(y[4 * j + 3] + b.w, a.ns2));
+                        y[4 * j] = apply_act_ns(y[4 * j] + b.x, a.ns2); y[4 * j + 1] = apply_act_ns(y[4 * j + 1] + b.y, a.ns2);
+                        y[4 * j + 2] = apply_act_ns(y[4 * j + 2] + b.z, a.ns2); y[4 * j + 3] = apply_act_ns(y[4 * j + 3] + b.w, a.ns2);
                     }
+                    store8(reinterpret_cast<float *>(dst), y, sectors);
+                    store8(reinterpret_cast<float *>(dst + 2), y + 8, sectors);
                 }
             }
             tc_fence_before_sync();
