@@ -45,7 +45,7 @@
 //   For one image and one block of 16 input channels, TMA copies a patch of the packed
 //   activations [rows][PW columns][16 ch] (64 bytes per pixel) into shared memory.
 //   PW = W + max(pad_l, pad_r): the zero column(s) that TMA's out-of-bounds fill produces at the
-//   left edge of every row also serve as the right padding of the row above.  Four splitter warps turn every
+//   left edge of every row also serve as the right padding of the row above.  Splitter warps turn every
 //   64-byte row into its 32 bytes of hi and 32 bytes of lo halves, in place and in the 64-byte swizzle, and that IS a
 //   K-major operand of the tensor core: rows of 64 bytes, 8-pixel groups 512 bytes apart; the hardware applies the
 //   swizzle to absolute shared-memory addresses, so a descriptor may start at any pixel.  Output pixel (r, c) is GEMM
@@ -68,7 +68,7 @@ namespace
 using namespace sb;
 
 constexpr int W_STAGES_MAX = 6; // filter stages, each one group of taps (a kernel row)
-constexpr int X_SLOTS_MAX = 3;
+__host__ __device__ constexpr int x_slots_max(int merged) { return merged ? 4 : 3; }
 constexpr int BOX_PX = 32; // widest box of a TMA load: 256 elements of 8 bytes
 constexpr int WIDE_WORDS = 32; // a CTA's tiles, a bit each: a launch has at most 1024 for every CTA
 constexpr int SCALE_RING = 16; // patches whose block scale is remembered: slots + unflushed accumulator buffers, rounded up
@@ -248,16 +248,21 @@ prepare_filter_kernel(long long n, int slabs, int MT, int K, const float *__rest
 //
 // warp 0: TMA producer, warps 1..2 (pixel-major 1..3): MMA issuers, warps 4..11: accumulation +
 // epilogue (lane quarter = warp % 4, pixel half = (warp - 4) / 4), warps 12..15: operand
-// splitters.
+// splitters, and in the MERGED kernels with two sets of them warps 16..19 (below).
 //
 // The unit of the filter pipeline is a GROUP of taps: one bulk copy and one
 // tcgen05.commit, which frees the filter stage for the producer and hands the partial sums to
 // the accumulation warps.
+//
+//
+// MERGED kernels (16 or 32 output channels) can have a second set of splitters, warps 16..19: the sets take the patches in turn.  A
+// set takes 2100 to 3700 cycles a patch, a chain of a few hundred instructions, where the MMAs of a tile need 1400 to 2000:
+// with one set it was the splitters that such a layer waited for.
 constexpr int ACC_WARPS = 8;
 constexpr int FIRST_ACC_WARP = 4;
 constexpr int FIRST_SPLIT_WARP = 12;
 constexpr int SPLIT_THREADS = 128;
-constexpr int NUM_THREADS = 512;
+__host__ __device__ constexpr int num_threads(int split_sets) { return split_sets == 2 ? 640 : 512; }
 constexpr int COLS_PER_THREAD = 128;
 
 // Two fp32 values times their block scale as two pairs of half-precision words: hi = v,
@@ -302,12 +307,16 @@ __device__ __forceinline__ float max_abs(const float4 v)
     return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 }
 // Largest of the splitter threads' values; `words` is used again only after another call.
-__device__ __forceinline__ uint32_t split_reduce(uint32_t m, uint32_t *words, int w, int lane)
+template <int SPLIT_SETS>
+__device__ __forceinline__ uint32_t split_reduce(uint32_t m, uint32_t *words, int w, int lane, int set)
 {
     m = __reduce_max_sync(0xffffffffu, m);
     if (lane == 0)
         words[w] = m;
-    asm volatile("bar.sync 2, 128;" ::: "memory");
+    if (SPLIT_SETS == 1)
+        asm volatile("bar.sync 2, 128;" ::: "memory");
+    else
+        asm volatile("bar.sync %0, 128;" ::"r"(2 + set) : "memory");
     const uint4 t = *reinterpret_cast<const uint4 *>(words);
     return max(max(t.x, t.y), max(t.z, t.w));
 }
@@ -533,22 +542,24 @@ __device__ __noinline__ void plain_tile(const TcArgs &a, const Tile T, const flo
         }
 }
 
-template <bool PERSIST, bool SPLIT, bool PIXM = false, int MERGED = 0, bool POOL = false> // MERGED: 1 merged operand, 2 with whole-window groups
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+// MERGED: 1 merged operand, 2 with whole-window groups
+template <bool PERSIST, bool SPLIT, bool PIXM = false, int MERGED = 0, bool POOL = false, int SPLIT_SETS = 1>
+__global__ void __launch_bounds__(num_threads(SPLIT_SETS), 1)
 conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restrict__ in, const __half *__restrict__ filt,
                   const float *__restrict__ filt_down, const __grid_constant__ TcArgs a, const float *__restrict__ bias, float *__restrict__ out, int *status)
 {
+    constexpr int NUM_THREADS = num_threads(SPLIT_SETS), X_SLOTS_MAX = x_slots_max(MERGED);
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t x_full[X_SLOTS_MAX], x_ready[X_SLOTS_MAX], x_empty[X_SLOTS_MAX];
     __shared__ __align__(8) uint64_t w_full[W_STAGES_MAX], g_done[W_STAGES_MAX];
     __shared__ __align__(8) uint64_t t_full[4], t_empty[4];
     __shared__ __align__(8) uint64_t peer_staged, peer_done; // split reduction: hand-over between the two CTAs
     __shared__ uint32_t tmem_base_s;
-    __shared__ __align__(8) uint64_t x_redo;   // a patch fetched again because its block scale did not fit
+    __shared__ __align__(8) uint64_t x_redo[SPLIT_SETS]; // a patch fetched again because its block scale did not fit
     __shared__ float patch_down[SCALE_RING];   // inverse of the block scale of each patch in flight
     static_assert(WIDE_WORDS == 32, "a lane each");
     __shared__ uint32_t wide_tiles[WIDE_WORDS]; // bit i: the CTA's tile i has a wide patch (see the splitters)
-    __shared__ __align__(16) uint32_t split_top[3][4];      // the splitter warps' maxima of the patch at hand
+    __shared__ __align__(16) uint32_t split_top[SPLIT_SETS][3][4];      // the splitter warps' maxima of the patch at hand
     __shared__ int acc_failed; // an accumulation warp gave up on a wait: all eight leave at the same tile
 
     const uint32_t entries = (uint32_t)a.PR * a.PW;
@@ -606,8 +617,8 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
         }
     };
     auto issue_patch = [&](const Tile &T, int cb, int slot) { fetch_patch(T, cb, slot, &x_full[slot]); };
-    auto reload_patch = [&](const Tile &, int t, int cb, int slot) {
-        fetch_patch(decode_tile(a, t), cb, slot, &x_redo);
+    auto reload_patch = [&](const Tile &, int t, int cb, int slot, uint64_t *redo) {
+        fetch_patch(decode_tile(a, t), cb, slot, redo);
     };
     auto issue_filter = [&](const Tile &T, int g, int st) {
         // the group's taps are contiguous, [tap][c/8][hi kv | lo kv][8 c]: one run; a partial last tile (kv < MT)
@@ -631,7 +642,9 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                 mbar_init(&w_full[i], 1); mbar_init(&g_done[i], 1);
             }
             for (int i = 0; i < 4; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], ACC_WARPS); }
-            mbar_init(&x_redo, 1); mbar_init(&peer_staged, ACC_WARPS * S); mbar_init(&peer_done, ACC_WARPS * S);
+            for (int i = 0; i < SPLIT_SETS; ++i)
+                mbar_init(&x_redo[i], 1);
+            mbar_init(&peer_staged, ACC_WARPS * S); mbar_init(&peer_done, ACC_WARPS * S);
             fence_barrier_init();
             // The first patch and the first filter stage only need their barriers: their round
             // trip to memory overlaps the tensor-memory allocation and the CTA-wide barrier.
@@ -659,7 +672,11 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
         // 128 x 88 + 256 x 168 + 128 x 88, pixel-major tiles 128 x 112 + 256 x 144 + 128 x 112.  (The least share also bounds
         // the function that is called for wide tiles: with 88 for the issuing warps it and its callers spilled, 16 -> 32 channels at
         // 208x208 with the pool 186 us, 168 with 112.)
-        if (PIXM)
+        if (SPLIT_SETS == 2 && warp >= FIRST_SPLIT_WARP)
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+        else if (SPLIT_SETS == 2)
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+        else if (PIXM)
             asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");
         else
             asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
@@ -927,9 +944,12 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             // one with a faint piece, whose largest magnitude is not zero but below FAINT when scaled (pieces, not whole
             // rows: a row is two lanes').  Then rows are looked at: a patch with a faint row at the scale that is its
             // own, one 2^-26 of its largest, makes its tile a wide one.
-            const int sid = tid - FIRST_SPLIT_WARP * 32;
-            bool ok = true, known = false;
-            int slot = 0, scale_at = 0;
+            // Two sets take the patches in turn, each with a scale of its own; a slot is always the same set's, or, where their number is
+            // odd, one set takes all patches.
+            const int set = SPLIT_SETS > 1 ? (warp - FIRST_SPLIT_WARP) >> 2 : 0, sid = tid - (FIRST_SPLIT_WARP + 4 * set) * 32;
+            const bool in_turn = SPLIT_SETS > 1 && !(a.x_slots & 1);
+            bool ok = set == 0 || in_turn, known = false;
+            int slot = 0, scale_at = 0, whose = 0;
             uint32_t phase = 0, turn = 0;
             uint32_t redone = 0;
             uint32_t limit = 0;
@@ -943,6 +963,17 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                 const int total = (int)(x_part >> 5); // pieces, whole passes of the warps: the slot has room for them
                 for (int cb = 0; cb < cbs_l && ok; ++cb)
                 {
+                    if (in_turn)
+                    {
+                        const bool mine = whose == set;
+                        whose ^= 1;
+                        if (!mine)
+                        {
+                            scale_at = (scale_at + 1) % SCALE_RING;
+                            if (++slot == a.x_slots) { slot = 0; phase ^= 1; }
+                            continue;
+                        }
+                    }
                     ok = mbar_wait(&x_full[slot], phase, status, 17);
                     if (!ok)
                         break;
@@ -954,7 +985,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                         {
                             const uint2 seen = look_at_rows(piece, sid, total, entries, valid, valid2);
                             m = seen.x;
-                            m = split_reduce(m, split_top[2], warp - FIRST_SPLIT_WARP, lane);
+                            m = split_reduce<SPLIT_SETS>(m, split_top[set][2], warp - FIRST_SPLIT_WARP - 4 * set, lane, set);
                             up = scale_up(m);
                             down = scale_down(m);
                             limit = down >= LARGE_DOWN ? 0u : 0xffffffffu;
@@ -964,20 +995,21 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                         float fm = 0.f;
                         uint32_t least = 0xffffffffu;
                         int base = sid;
-                        for (; base + 3 * SPLIT_THREADS < total; base += 4 * SPLIT_THREADS)
-                            fm = fmaxf(fm, split_pieces<4>(piece, base, up, entries, valid, valid2, least));
+                        constexpr int AT_ONCE = SPLIT_SETS == 2 ? 2 : 4; // (registers: two sets of splitters have 72 a thread)
+                        for (; base + (AT_ONCE - 1) * SPLIT_THREADS < total; base += AT_ONCE * SPLIT_THREADS)
+                            fm = fmaxf(fm, split_pieces<AT_ONCE>(piece, base, up, entries, valid, valid2, least));
                         for (; base < total; base += SPLIT_THREADS)
                             fm = fmaxf(fm, split_pieces<1>(piece, base, up, entries, valid, valid2, least));
                         fence_proxy_async();
                         const bool faint = least != 0xffffffffu && __uint_as_float(least + 1u) * up < FAINT;
-                        m = split_reduce(faint ? FAINT_SEEN : __float_as_uint(fm * up), split_top[turn], warp - FIRST_SPLIT_WARP, lane);
+                        m = split_reduce<SPLIT_SETS>(faint ? FAINT_SEEN : __float_as_uint(fm * up), split_top[set][turn], warp - FIRST_SPLIT_WARP - 4 * set, lane, set);
                         // 0: all zero; not below 65504: would have overflowed (or an infinity in the input, which no
                         // scale helps: it stays one), or a faint row was seen
                         if (!known || m == 0 || (m >= 0x42800000u && m < 0x477fe000u))
                             break;
                         if (sid == 0)
-                            reload_patch(T, t, cb, slot);
-                        ok = mbar_wait(&x_redo, redone & 1, status, 18);
+                            reload_patch(T, t, cb, slot, &x_redo[set]);
+                        ok = mbar_wait(&x_redo[set], redone & 1, status, 18);
                         ++redone;
                         if (!ok)
                             break;
@@ -1001,8 +1033,10 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     {
         if (!PIXM)
             asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
-        else
+        else if (SPLIT_SETS == 1)
             asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+        else
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 128;");
         const float act_ns = act_neg_scale(a.act, a.slope); // activation: v > 0 ? v : v * act_ns
         // Whether tile i of this CTA is wide; known when its last sums are.  What is stored for such a tile is overwritten at
         // the end, so it matters here only where the output is also an input.
@@ -1040,6 +1074,23 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                                                                            : make_float4(0.f, 0.f, 0.f, 0.f);
                     acc[4 * c4] = b.x; acc[4 * c4 + 1] = b.y; acc[4 * c4 + 2] = b.z; acc[4 * c4 + 3] = b.w;
                 }
+                // This thread's pixel.
+                const int ml = T.m_local0 + mt * 128 + quarter * 32 + lane;
+                const int rl = a.by_PW.div(ml), cl = ml - rl * a.PW, r = T.row_base + rl, c = T.col_base + cl;
+                const bool live = !POOL && active && cl < T.tw_valid && rl < T.th_valid && r < a.Ho;
+                float *o = out + (size_t)T.n * (a.K / CB) * plane + (size_t)r * a.o_row_stride + (size_t)c * CB;
+                auto add_old = [&]() {
+#pragma unroll
+                    for (int c4 = 0; c4 < ACC / 4; ++c4)
+                        if (c4 * 4 < a.K)
+                        {
+                            const float4 old = *(reinterpret_cast<const float4 *>(o + (size_t)(c4 >> 2) * plane) + (c4 & 3));
+                            acc[4 * c4] += old.x; acc[4 * c4 + 1] += old.y; acc[4 * c4 + 2] += old.z; acc[4 * c4 + 3] += old.w;
+                        }
+                };
+                if (!POOL && a.accumulate && live) // on its way to L2 while the sums are made (87 -> 80 us, see the launch)
+                    for (int kb = 0; kb * CB < a.K; ++kb)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(o + (size_t)kb * plane));
                 int in_cb = 0;
                 for (int g = 0; g < groups && ok; ++g, ++gc)
                 {
@@ -1126,8 +1177,6 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                     // Every warp comes to the first barrier at every tile; a warp whose wait ran out says so
                     // before it and all leave together (see the channel-major epilogue).
                     constexpr int HALF = ACC / 2;
-                    const int ml = mt * 128 + quarter * 32 + lane; // tiled plans: m_local0 = 0
-                    const int rl = a.by_PW.div(ml), cl = ml - rl * a.PW;
                     const int upper = lane & 1;
                     float *xrow = reinterpret_cast<float *>(smem + a.stage_off) +
                                   ((size_t)(rl >> 1) * (a.PW >> 1) + (cl >> 1)) * (ACC + 4) + upper * HALF;
@@ -1155,11 +1204,11 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                             }
                         }
                         asm volatile("bar.sync 1, 256;" ::: "memory");
-                        const int r = T.row_base + rl, c = T.col_base + (cl & ~1);
+                        const int c0 = T.col_base + (cl & ~1);
                         if (active && !(rl & 1) && (cl & ~1) < T.tw_valid && rl < a.TH && r < a.Ho)
                         {
                             float *o = out + ((size_t)T.n * (a.K / CB) + (size_t)upper * (HALF / CB)) * plane +
-                                       (size_t)(r >> 1) * a.o_row_stride + (size_t)(c >> 1) * CB;
+                                       (size_t)(r >> 1) * a.o_row_stride + (size_t)(c0 >> 1) * CB;
 #pragma unroll
                             for (int j = 0; j < HALF / 4; ++j)
                             {
@@ -1174,35 +1223,19 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                         }
                     }
                 }
-                else if (ok && active && !(a.accumulate && is_wide(once_)))
+                else if (ok && live && !(a.accumulate && is_wide(once_)))
                 {
-                    const int ml = T.m_local0 + mt * 128 + quarter * 32 + lane;
-                    const int rl = a.by_PW.div(ml), cl = ml - rl * a.PW;
-                    const int r = T.row_base + rl, c = T.col_base + cl;
-                    if (cl < T.tw_valid && rl < T.th_valid && r < a.Ho)
-                    {
-                        float *o = out + (size_t)T.n * (a.K / CB) * plane + (size_t)r * a.o_row_stride + (size_t)c * CB;
+                    if (a.accumulate)
+                        add_old();
 #pragma unroll
-                        for (int kb = 0; kb < ACC / 16; ++kb)
-                            if (kb * CB < a.K)
-                            {
+                    for (int k8 = 0; k8 < ACC / 8; ++k8)
+                        if (k8 * 8 < a.K)
+                        {
 #pragma unroll
-                                for (int j = 0; j < 4; ++j)
-                                {
-                                    float *x = acc + kb * 16 + 4 * j, *op = o + (size_t)kb * plane + 4 * j;
-                                    if (a.accumulate)
-                                    {
-                                        const float4 s4 = *reinterpret_cast<const float4 *>(op);
-                                        x[0] += s4.x; x[1] += s4.y; x[2] += s4.z; x[3] += s4.w;
-                                    }
-#pragma unroll
-                                    for (int e = 0; e < 4; ++e)
-                                        x[e] = apply_act_ns(x[e], act_ns);
-                                    if (j & 1)
-                                        store8(op - 4, x - 4, sectors);
-                                }
-                            }
-                    }
+                            for (int e = 0; e < 8; ++e)
+                                acc[8 * k8 + e] = apply_act_ns(acc[8 * k8 + e], act_ns);
+                            store8(o + (size_t)(k8 >> 1) * plane + (k8 & 1) * 8, acc + 8 * k8, sectors);
+                        }
                 }
             }
         }
@@ -1503,7 +1536,7 @@ bool fit_rings(TcArgs &a, bool need_two)
     {
         const int stages = a.cbs * (a.taps / a.group);
         if (stages <= W_STAGES_MAX)
-            for (int xs = 3; xs >= 2; --xs)
+            for (int xs = a.merged ? 4 : 3; xs >= 2; xs -= a.merged ? 2 : 1) // (two sets of splitters: an even number)
             {
                 const size_t ops = (size_t)xs * x_part + (size_t)stages * w_part;
                 const size_t smem = ops + pool_rows;
@@ -1515,10 +1548,13 @@ bool fit_rings(TcArgs &a, bool need_two)
                 }
             }
     }
+    for (int any = a.merged ? 0 : 1; any < 2; ++any) // two sets of splitters want an even number of slots
     for (int persistent = (a.MT == 64 ? 1 : 0); persistent >= (a.pixm ? 1 : 0); --persistent)
         for (const auto &p : pref)
         {
             const int xs = p[0] < a.cbs || persistent ? p[0] : a.cbs;
+            if (!any && (xs & 1))
+                continue;
             if (need_two && xs < 2 && a.cbs >= 2)
                 continue;
             const size_t ops = (size_t)xs * x_part + (size_t)p[1] * w_part;
@@ -1840,6 +1876,10 @@ int configure()
         SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         configured.mark(dev);
@@ -1862,7 +1902,7 @@ int resident_clusters(int S)
     if (S > 1)
     {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)S); cfg.blockDim = dim3(NUM_THREADS);
+        cfg.gridDim = dim3((unsigned)S); cfg.blockDim = dim3(num_threads(1));
         cfg.dynamicSmemBytes = 226 * 1024;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1963,7 +2003,7 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
     const float *filt_down = filt_prepared + (size_t)a.K * a.C * a.Fh * a.Fw;
     auto launch_split = [&](const TcArgs &ta, long long nblocks) -> int {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)nblocks); cfg.blockDim = dim3(NUM_THREADS);
+        cfg.gridDim = dim3((unsigned)nblocks); cfg.blockDim = dim3(num_threads(1));
         cfg.dynamicSmemBytes = ta.smem_bytes; cfg.stream = as_stream(stream);
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1977,7 +2017,7 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
         const long long full = tiles / num_sms() * num_sms(), rem = tiles - full;
         TcArgs a1 = a;
         a1.tile_base = 0;
-        conv_f16x3_kernel<false, false><<<(unsigned)full, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a1, bias, out, status);
+        conv_f16x3_kernel<false, false><<<(unsigned)full, num_threads(1), a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a1, bias, out, status);
         if (int rc = launched("conv_f16x3_kernel"))
             return rc;
         TcArgs a2 = a;
@@ -1992,31 +2032,48 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
     {
     a.tile_base = (int)base; a.total_tiles = (int)std::min(tiles, base + room);
     const unsigned grid = (unsigned)(a.persistent ? std::min(blocks, tiles - base) : blocks);
-#define SB_LAUNCH_PIXM(M, P) \
-    conv_f16x3_kernel<true, false, true, M, P><<<grid, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(\
+    // Two sets of splitters where the conversion of the patches sets the pace: more than three patches a CTA, one after the
+    // other (16 -> 32 channels at 208x208, 32 images: 86.4 us with one set, 81.6 with two; 64 -> 32 at 52x52, 64 images 41.4
+    // and 37.3; with two patches a CTA, 16 -> 16 at 32x32, 32 images, 8.3 and 8.6).  One set, whose kernel leaves the accumulation
+    // warps more registers, where those also read what is there (16 -> 16 at 32x32, 1024 images onto the shortcut: 80 and
+    // 85), and before a pool, which makes them the slower ones while the input comes from L2 (16 -> 32 at 208x208, 16 images
+    // 43.2 and 44.6; 64 images, 177 MB from memory, 152.2 and 146.6).
+    constexpr size_t L2_BYTES = (size_t)126 << 20;
+    const bool two = a.merged && !a.accumulate && (a.cbs > 1 || tiles > 3 * blocks) &&
+                     (!a.pool || (size_t)L->N * L->C * L->H * L->W * sizeof(float) > L2_BYTES);
+#define SB_LAUNCH_PIXM(M, P, SETS) \
+    conv_f16x3_kernel<true, false, true, M, P, SETS><<<grid, num_threads(SETS), a.smem_bytes, as_stream(stream)>>>(\
         mx, in, filt, filt_down, a, bias, out, status)
-    if (a.pool && whole)
-        SB_LAUNCH_PIXM(2, true);
+    if (a.pool && whole && two)
+        SB_LAUNCH_PIXM(2, true, 2);
+    else if (a.pool && whole)
+        SB_LAUNCH_PIXM(2, true, 1);
+    else if (a.pool && two)
+        SB_LAUNCH_PIXM(1, true, 2);
     else if (a.pool && a.merged)
-        SB_LAUNCH_PIXM(1, true);
+        SB_LAUNCH_PIXM(1, true, 1);
     else if (a.pool)
-        SB_LAUNCH_PIXM(0, true);
+        SB_LAUNCH_PIXM(0, true, 1);
+    else if (whole && two)
+        SB_LAUNCH_PIXM(2, false, 2);
     else if (whole)
-        SB_LAUNCH_PIXM(2, false);
+        SB_LAUNCH_PIXM(2, false, 1);
+    else if (two)
+        SB_LAUNCH_PIXM(1, false, 2);
     else if (a.merged)
-        SB_LAUNCH_PIXM(1, false);
+        SB_LAUNCH_PIXM(1, false, 1);
 #undef SB_LAUNCH_PIXM
     else if (a.pixm)
-        conv_f16x3_kernel<true, false, true><<<grid, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
+        conv_f16x3_kernel<true, false, true><<<grid, num_threads(1), a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
     else if (a.persistent)
-        conv_f16x3_kernel<true, false><<<grid, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
+        conv_f16x3_kernel<true, false><<<grid, num_threads(1), a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
     else if (a.ksplit > 1)
     {
         if (int rc = launch_split(a, blocks))
             return rc;
     }
     else
-        conv_f16x3_kernel<false, false><<<grid, NUM_THREADS, a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
+        conv_f16x3_kernel<false, false><<<grid, num_threads(1), a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
     if (int rc = launched("conv_f16x3_kernel"))
         return rc;
     }

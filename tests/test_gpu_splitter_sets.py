@@ -1,0 +1,43 @@
+"""16 and 32 output channels on the tensor cores with one and two sets of operand splitters (csrc/conv_f16x3.cu), to either side of
+the line between them: images of magnitudes apart, so that a patch converted with another one's scale shows."""
+import numpy as np
+import pytest
+
+from oracle.bindings import same_pads, shape
+from smallframework_b200 import _lib
+from smallframework_b200 import interface as S
+from smallframework_b200 import packing as P
+from tests.gpu_util import CB, fbuf, oracle_conv_batch, rel_max_err
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # C, K, H, W, kernel, images, pool: a 16x16 or 32x32 image gives two and eight patches of 16 channels and 128 pixels
+    (16, 16, 32, 32, 3, 16, False), (16, 16, 32, 32, 3, 47, False), (16, 16, 32, 32, 3, 90, False), (16, 32, 16, 16, 3, 301, False),
+    (32, 32, 16, 16, 3, 1, False), (48, 16, 20, 20, 3, 7, False), (80, 32, 9, 20, 3, 131, False), (128, 16, 7, 7, 1, 40, False),
+    (16, 32, 70, 90, 5, 9, False), (48, 32, 40, 130, 3, 4, True), (16, 32, 208, 208, 3, 5, True), (16, 32, 208, 208, 3, 51, True),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "C{}_K{}_{}x{}_k{}_n{}{}".format(*c[:6], "_pool" if c[6] else ""))
+def test_against_the_oracle(oracle, case):
+    c, k, h, w, f, n, pool = case
+    pads = same_pads(h, w, f, f, 1)
+    rng = np.random.default_rng(c + k + h + n)
+    x = rng.uniform(-1, 1, (n, c, h, w)).astype(np.float32) * (8.0 ** (np.arange(n) % 5 - 2)).astype(np.float32)[:, None, None, None]
+    x, wt = P.pack_activation(x), P.pack_conv_filter(rng.normal(0, np.sqrt(2.0 / (c * f * f)), (k, c, f, f)).astype(np.float32))
+    I, F = fbuf(x), fbuf(wt)
+    Fp, O = S.FloatBuffer(2 * F.size()), S.FloatBuffer(n * k * h * w // (4 if pool else 1))
+    S.prepare_filter_3xTF32(f, f, k, c, F, Fp)
+    if pool:
+        S.Conv2D_Maxpool2D_3xTF32(f, f, pads, k, c, h, w, I, Fp, None, O, batch=n)
+    else:
+        S.Conv2D_3xTF32(f, f, 1, *pads, k, c, h, w, I, Fp, None, O, batch=n)
+    got = O.numpy().reshape(n, -1)
+    assert _lib.device_status() == 0
+    some = np.unique(np.linspace(0, n - 1, 12).astype(int))
+    want = oracle_conv_batch(oracle, shape(c, k, h, w, f, f, 1, pads, CB), x[some], wt)
+    for i, ref in zip(some, want):
+        if pool:
+            ref = oracle.pool2d_f32(shape(k, k, h, w, 2, 2, 2, (0, 0, 0, 0), CB), ref)
+        assert rel_max_err(got[i], ref) <= 1e-5  # pairs of 11-bit words: a product is off by 2^-21 at most, the rest is fp32 sums
