@@ -1287,6 +1287,9 @@ int conv2d_u8_one_channel_tc(const small_b200_layer *L, const uint8_t *in, const
 // Defined in conv_u8_patch.cu: windows of more than one tap on blocks of channels, for zero points whose padding is a byte.
 int conv2d_u8_patch(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
                     uint8_t *out, cudaStream_t st);
+// Defined in conv_u8_rgb.cu: first layers on many pixels of three channels, where conv2d_u8_onestep would take them; -1 otherwise.
+int conv2d_u8_rgb(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
+                  uint8_t *out, cudaStream_t st);
 // Defined in conv_u8_ring.cu: every other window / stride / channel count as an implicit GEMM on the
 // tensor core, for the zero points it covers; -1 otherwise.
 int conv2d_u8_ring(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
@@ -1400,6 +1403,12 @@ int conv2d_u8_dispatch(const small_b200_layer *L, const uint8_t *in, const uint8
         const int tc1 = conv2d_u8_one_channel_tc(L, in, filt, bias, out, as_stream(stream));
         if (tc1 >= 0)
             return tc1;
+    }
+    if (path == 0 && one_step_preferred(L))
+    {
+        const int rgb = conv2d_u8_rgb(L, in, filt, bias, out, as_stream(stream));
+        if (rgb >= 0)
+            return rgb;
     }
     if (path == 1 || (path == 0 && one_step_preferred(L)))
     {
