@@ -1290,6 +1290,9 @@ int conv2d_u8_patch(const small_b200_layer *L, const uint8_t *in, const uint8_t 
 // Defined in conv_u8_rgb.cu: first layers on many pixels of three channels, where conv2d_u8_onestep would take them; -1 otherwise.
 int conv2d_u8_rgb(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
                   uint8_t *out, cudaStream_t st);
+// Defined in conv_u8_thin.cu: pointwise layers on many pixels of 16 or 32 channels; -1 otherwise.
+int conv2d_u8_thin(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
+                   uint8_t *out, cudaStream_t st);
 // Defined in conv_u8_ring.cu: every other window / stride / channel count as an implicit GEMM on the
 // tensor core, for the zero points it covers; -1 otherwise.
 int conv2d_u8_ring(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
@@ -1304,9 +1307,9 @@ bool one_step_covers(const small_b200_layer *L)
     return (long long)L->C * L->Fh * L->Fw <= 32 && (L->C < CB || (L->Fh == 1 && L->Fw == 1)) && L->zero_in <= 0 && L->zero_in >= -255 &&
            L->K <= 1024;
 }
-// ... and which the kernel does faster than the tensor cores.  2048 images, us, this kernel and those: 16 -> 32 channels at
-// 24x24 27 and 49, 16 -> 64 48 and 68, 16 -> 128 at 12x12 25 and 29; but 32 -> 32 at 24x24 37 and 34, and a few images of 32
-// channels 5 and 4.
+// ... and which the kernel does faster than conv_u8_tc.cu (what conv_u8_rgb.cu and conv_u8_thin.cu do faster never gets here).  2048
+// images, us, this kernel and that one: 16 -> 32 channels at 24x24 27 and 49, 16 -> 64 48 and 68, 16 -> 128 at 12x12 25 and 29; but
+// 32 -> 32 at 24x24 37 and 34, and a few images of 32 channels 5 and 4.
 bool one_step_preferred(const small_b200_layer *L)
 {
     return one_step_covers(L) && (L->C < CB || (L->C == CB && L->K <= 128));
@@ -1389,6 +1392,12 @@ int conv2d_u8_dispatch(const small_b200_layer *L, const uint8_t *in, const uint8
     QArgs a; fill(L, a, true);
     if (a.N == 0 || a.Ho == 0 || a.Wo == 0)
         return SMALL_B200_OK;
+    if (path == 0)
+    {
+        const int thin = conv2d_u8_thin(L, in, filt, bias, out, as_stream(stream));
+        if (thin >= 0)
+            return thin;
+    }
     if (path == 0 && L->C >= CB && one_step_preferred(L))
     {
         const int one = conv2d_u8_onestep(L, a, in, filt, bias, out, as_stream(stream));

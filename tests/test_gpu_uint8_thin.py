@@ -1,0 +1,38 @@
+"""uint8 pointwise layers on 16 and 32 channels as one MMA a tile (csrc/conv_u8_thin.cu) against the oracle, bit-exact: tiles across
+images, ragged last tiles, several blocks and parts of output channels, more tiles a CTA than stages, any zero points."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_uint8 import _case_id, _check_conv, _quant
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # C, K, H, W, Fh, Fw, stride, pads, batch
+    (16, 16, 48, 48, 1, 1, 1, "valid", 320),
+    (16, 64, 1, 1, 1, 1, 1, "valid", 1),
+    (16, 32, 24, 24, 1, 1, 1, "valid", 240),
+    (16, 64, 37, 7, 1, 1, 1, "valid", 133),    # parts of the output channels
+    (16, 48, 5, 5, 1, 1, 1, "valid", 3600),    # many images a tile
+    (32, 32, 24, 24, 1, 1, 1, "valid", 200),   # four and a half tiles an image
+    (32, 16, 16, 8, 1, 1, 1, "valid", 601),
+    (32, 64, 16, 8, 1, 1, 1, "valid", 64),
+    (32, 64, 31, 33, 1, 1, 1, "valid", 90),
+    (32, 128, 111, 113, 1, 1, 1, "valid", 2),
+    (32, 48, 23, 45, 1, 1, 1, "valid", 60),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=_case_id)
+@pytest.mark.parametrize("zp", [(0, -128), (-113, -121), (-255, -130)], ids=lambda z: "zi{}_zf{}".format(*z))
+def test_conv2d_u8_thin(oracle, case, zp):
+    rng = np.random.default_rng(case[0] + case[1] + case[2] + zp[0] + 1000)
+    _check_conv(oracle, case, (0, 0, 0, 0), _quant(rng, case[0], zp), rng, zp[0] != 0, None)
+
+
+@pytest.mark.parametrize("C", [16, 32])
+@pytest.mark.parametrize("shift", [0, 1], ids=lambda r: f"rshift{r}")
+def test_quantisers_outside_the_common_form(oracle, shift, C):
+    from oracle.bindings import Quant
+    rng = np.random.default_rng(3)
+    _check_conv(oracle, (C, 32, 32, 32, 1, 1, 1, "valid", 130), (0, 0, 0, 0), Quant(-3, -120, 2 - 2 * shift, shift, 1 << 19, 0), rng, True, None)
