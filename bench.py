@@ -619,6 +619,8 @@ def measured_traffic(layer, batch, kernel):
 
 def kernel_class(chain, i, L, dtype):
     """Which kernel runs layer i (with the layers it absorbs) and what bounds it."""
+    if chain.whole is not None:
+        return "net_u8_tc_kernel (tcgen05 kind::i8, the whole network)", "i8"
     follow = chain.absorbed(i)
     if i in chain.tails:
         return "pool_dense_softmax_f32_kernel", "stream"
@@ -635,19 +637,32 @@ def kernel_class(chain, i, L, dtype):
         if follow:
             tail = "depthwise 3x3 on tcgen05" if len(follow) == 1 else "global average pool + dense"
             return f"block_u8_tc_kernel (tcgen05 kind::i8 {'im2col first layer' if L['C'] == 1 else '1x1'} -> {tail})", "i8"
+        ho, wo = networks_out_hw(L)
+        outputs = chain.batch * ho * wo
+        thin = L["Fh"] == 1 and L["Fw"] == 1 and L["stride"] == 1 and L["K"] <= 128
+        if thin and L["C"] == 16 and (L["K"] >= 64 or outputs * L["K"] >= 4 << 20) or \
+                thin and L["C"] == 32 and outputs >= 8192 and -(-ho * wo // 128) * 512 <= ho * wo * 5:
+            return "conv_u8_thin_kernel (tcgen05 kind::i8)", "i8"
         pw = (L["Fh"] == 1 and L["Fw"] == 1 and L["stride"] == 1 and L["C"] % 32 == 0 and L["C"] <= 256)
         if pw:
             return "pw_u8_tc_kernel (tcgen05 kind::i8)", "i8"
-        ho, wo = networks_out_hw(L)
         if L["C"] == 1 and L["Fw"] <= 4 and L["Fh"] <= 16 and ho * wo <= 128 and L["K"] <= 128:
             return "stem_u8_tc_kernel (im2col in shared memory + tcgen05 kind::i8)", "i8"
         if L["C"] * L["Fh"] * L["Fw"] > 32 or (L["C"] >= 16 and L["K"] > 128):
-            return "conv_u8_ring_kernel (implicit GEMM, tcgen05 kind::i8)", "i8"
+            return ("conv_u8_patch_kernel (tcgen05 kind::i8)" if L["C"] % 16 == 0 and L["Fh"] * L["Fw"] > 1 else
+                    "conv_u8_ring_kernel (implicit GEMM, tcgen05 kind::i8)"), "i8"
+        if L["C"] == 3 and outputs >= 200000 and L["Fw"] <= (6 if L["stride"] == 2 else 5):
+            return "conv_u8_rgb_kernel (tcgen05 kind::i8)", "i8"
         return "conv2d_u8_onestep_kernel (dp4a, streaming)", "stream"
     if L["op"] == "dwconv" and dtype == "u8":
         tiles = L["Fh"] == 3 and L["Fw"] == 3 and L["stride"] == 1
         return ("dwconv3x3_u8_tile_kernel (dp4a)" if tiles else "dwconv_u8_dp4a_kernel"), "stream"
     if i in chain.blocks:
+        ho, wo = networks_out_hw(L)
+        K, outputs = chain.layers[i + 1]["K"], chain.batch * ho * wo
+        if K in (16, 32) and ((L["stride"] == 1 and (L["C"] <= 16 or L["C"] <= 32 and outputs >= 16384)) or
+                              (L["stride"] == 2 and L["C"] == 16 and K == 32 and outputs <= 131072)):
+            return "dwpw_direct_f32_kernel (depthwise 3x3 + 1x1, FFMA)", "ffma"
         return "dwpw_f32_kernel (depthwise 3x3 + 1x1 on tcgen05 kind::tf32, two-word operands)", "tf32x3"
     return {"dwconv": "window_f32_kernel (depthwise)", "maxpool": "max pool", "avgpool": "average pool",
             "softmax": "softmax", "alias": "alias"}[L["op"]], "stream"
