@@ -639,9 +639,10 @@ def kernel_class(chain, i, L, dtype):
             return f"block_u8_tc_kernel (tcgen05 kind::i8 {'im2col first layer' if L['C'] == 1 else '1x1'} -> {tail})", "i8"
         ho, wo = networks_out_hw(L)
         outputs = chain.batch * ho * wo
-        thin = L["Fh"] == 1 and L["Fw"] == 1 and L["stride"] == 1 and L["K"] <= 128
-        if thin and L["C"] == 16 and (L["K"] >= 64 or outputs * L["K"] >= 4 << 20) or \
-                thin and L["C"] == 32 and outputs >= 8192 and -(-ho * wo // 128) * 512 <= ho * wo * 5:
+        C, K = L["C"] if i == 0 else networks_padded(L["C"]), networks_padded(L["K"])
+        thin = L["Fh"] == 1 and L["Fw"] == 1 and L["stride"] == 1 and K <= 128
+        if thin and C == 16 and (K >= 64 or outputs * K >= 4 << 20) or \
+                thin and C == 32 and outputs >= 8192 and -(-ho * wo // 128) * 512 <= ho * wo * 5:
             return "conv_u8_thin_kernel (tcgen05 kind::i8)", "i8"
         pw = (L["Fh"] == 1 and L["Fw"] == 1 and L["stride"] == 1 and L["C"] % 32 == 0 and L["C"] <= 256)
         if pw:
@@ -659,13 +660,18 @@ def kernel_class(chain, i, L, dtype):
         return ("dwconv3x3_u8_tile_kernel (dp4a)" if tiles else "dwconv_u8_dp4a_kernel"), "stream"
     if i in chain.blocks:
         ho, wo = networks_out_hw(L)
-        K, outputs = chain.layers[i + 1]["K"], chain.batch * ho * wo
+        K, outputs = networks_padded(chain.layers[i + 1]["K"]), chain.batch * ho * wo
         if K in (16, 32) and ((L["stride"] == 1 and (L["C"] <= 16 or L["C"] <= 32 and outputs >= 16384)) or
-                              (L["stride"] == 2 and L["C"] == 16 and K == 32 and outputs <= 131072)):
+                              (L["stride"] == 2 and L["C"] <= 16 and K == 32 and outputs <= 131072)):
             return "dwpw_direct_f32_kernel (depthwise 3x3 + 1x1, FFMA)", "ffma"
         return "dwpw_f32_kernel (depthwise 3x3 + 1x1 on tcgen05 kind::tf32, two-word operands)", "tf32x3"
     return {"dwconv": "window_f32_kernel (depthwise)", "maxpool": "max pool", "avgpool": "average pool",
             "softmax": "softmax", "alias": "alias"}[L["op"]], "stream"
+
+
+def networks_padded(channels):
+    from smallframework_b200.networks import padded
+    return padded(channels)
 
 
 def networks_out_hw(L):

@@ -11,8 +11,9 @@
 // Roles: 16 epilogue warps (sets of four, an accumulator each), 12 producer warps (a tile each, from global memory through registers and a
 // table of the patch's chunks), 2 issuing warps (tiles in turn: what one spends on a tile's MMAs and waits is 600 cycles and more).
 //
-// What bounds it: instructions.  A tile of 256 outputs of 16 channels takes 1100 of the epilogue's warps (five and a half per
-// 32 results, half of them on the half-rate integer pipe) and 350 of the producer's; the three MMAs take 132 cycles.  The CUDA cores' form
+// What bounds it: instructions.  A tile of 256 outputs of 16 channels takes 2000 warp instructions (five and a half per 32
+// results, half of them on the half-rate integer pipe, some 35 a chunk of four pixels), at 57 % of the issue slots and 39 % of the ALU (512
+// images of 96x96); its three MMAs take 132 cycles.  The CUDA cores' form
 // has seven dp4a and the gather of the window beside the same requantisation.  us, that form -> this: 3 -> 16
 // channels at 96x96 with a stride of two, 2048 images 98.8 -> 53.4 (19 at the rate of a copy of its bytes), 3 -> 32 149.7 -> 82;
 // at 32x32, stride 1, 4096 images 84 -> 48; at 416x416, 16 images 53 -> 25.7.  On the way: one issuing warp in a rolled loop 76 (1150

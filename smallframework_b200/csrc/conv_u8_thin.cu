@@ -9,7 +9,7 @@
 // Roles: 24 epilogue warps (six sets of four, an accumulator each), a producing and two issuing warps (tiles in turn).
 //
 // What bounds it: the epilogue's instructions, five and a half per 32 results, half of them on the half-rate integer pipe: a tile of 256
-// pixels and 16 channels takes 580 cycles, of which its MMA 44.  us, 2048 images, before (see the rule below) -> this: 16 -> 16 at
+// pixels and 16 channels takes 1450 warp instructions and 580 cycles, its MMA 44 of them.  us, 2048 images, before (see the rule below) -> this: 16 -> 16 at
 // 48x48 55.9 -> 38.0 (23 at the rate of a copy of its bytes), 16 -> 32 at 24x24 26.3 -> 17.4, 16 -> 128 88.9 -> 58.8, 32 -> 32 32.2 -> 22.4,
 // 32 -> 16 25.8 -> 18.1; 32 -> 64 at 112x112, 16 images 11.7 -> 8.2.
 #include "tc_common.cuh"
