@@ -642,7 +642,7 @@ def kernel_class(chain, i, L, dtype):
         C, K = L["C"] if i == 0 else networks_padded(L["C"]), networks_padded(L["K"])
         thin = L["Fh"] == 1 and L["Fw"] == 1 and L["stride"] == 1 and K <= 128
         if thin and C == 16 and (K >= 64 or outputs * K >= 4 << 20) or \
-                thin and C == 32 and outputs >= 8192 and -(-ho * wo // 128) * 512 <= ho * wo * 5:
+                thin and C in (32, 64) and outputs >= 30000 and ho * wo >= 64:
             return "conv_u8_thin_kernel (tcgen05 kind::i8)", "i8"
         pw = (L["Fh"] == 1 and L["Fw"] == 1 and L["stride"] == 1 and L["C"] % 32 == 0 and L["C"] <= 256)
         if pw:

@@ -1290,7 +1290,7 @@ int conv2d_u8_patch(const small_b200_layer *L, const uint8_t *in, const uint8_t 
 // Defined in conv_u8_rgb.cu: first layers on many pixels of three channels, where conv2d_u8_onestep would take them; -1 otherwise.
 int conv2d_u8_rgb(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
                   uint8_t *out, cudaStream_t st);
-// Defined in conv_u8_thin.cu: pointwise layers on many pixels of 16 or 32 channels; -1 otherwise.
+// Defined in conv_u8_thin.cu: pointwise layers on many pixels of 16, 32 or 64 channels; -1 otherwise.
 int conv2d_u8_thin(const small_b200_layer *L, const uint8_t *in, const uint8_t *filt, const int32_t *bias,
                    uint8_t *out, cudaStream_t st);
 // Defined in conv_u8_ring.cu: every other window / stride / channel count as an implicit GEMM on the

@@ -1,4 +1,4 @@
-"""uint8 pointwise layers on 16 and 32 channels as one MMA a tile (csrc/conv_u8_thin.cu) against the oracle, bit-exact: tiles across
+"""uint8 pointwise layers on 16, 32 and 64 channels as one or two MMAs a tile (csrc/conv_u8_thin.cu) against the oracle, bit-exact: tiles across
 images, ragged last tiles, several blocks and parts of output channels, more tiles a CTA than stages, any zero points."""
 import numpy as np
 import pytest
@@ -16,10 +16,15 @@ CASES = [
     (16, 48, 5, 5, 1, 1, 1, "valid", 3600),    # many images a tile
     (32, 32, 24, 24, 1, 1, 1, "valid", 200),   # four and a half tiles an image
     (32, 16, 16, 8, 1, 1, 1, "valid", 601),
-    (32, 64, 16, 8, 1, 1, 1, "valid", 64),
+    (32, 64, 16, 8, 1, 1, 1, "valid", 240),
     (32, 64, 31, 33, 1, 1, 1, "valid", 90),
-    (32, 128, 111, 113, 1, 1, 1, "valid", 2),
+    (32, 128, 111, 113, 1, 1, 1, "valid", 3),
     (32, 48, 23, 45, 1, 1, 1, "valid", 60),
+    (32, 64, 12, 12, 1, 1, 1, "valid", 231),   # tiles across images: two or three of them a tile
+    (32, 16, 13, 5, 1, 1, 1, "valid", 827),
+    (64, 64, 12, 12, 1, 1, 1, "valid", 1999),  # two reduction steps
+    (64, 48, 8, 8, 1, 1, 1, "valid", 1320),
+    (64, 128, 17, 4, 1, 1, 1, "valid", 1150),
 ]
 
 
@@ -30,7 +35,7 @@ def test_conv2d_u8_thin(oracle, case, zp):
     _check_conv(oracle, case, (0, 0, 0, 0), _quant(rng, case[0], zp), rng, zp[0] != 0, None)
 
 
-@pytest.mark.parametrize("C", [16, 32])
+@pytest.mark.parametrize("C", [16, 32, 64])
 @pytest.mark.parametrize("shift", [0, 1], ids=lambda r: f"rshift{r}")
 def test_quantisers_outside_the_common_form(oracle, shift, C):
     from oracle.bindings import Quant
