@@ -174,8 +174,10 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
     constexpr int GW = 4 * PARTS, GT = GW * 32, CBW = KB / PARTS, MAX_GROUPS = WARPS / GW;
     constexpr int PPARTS = GW / KB; // warps that share the pixels of a channel block in the pool
     extern __shared__ __align__(1024) uint8_t smem[];
-    // A group's operand is complete; its sums are: of a depthwise layer the first half of the channels, of any layer all.
-    __shared__ __align__(8) uint64_t loaded, ready[MAX_GROUPS], half_done[MAX_GROUPS], done[MAX_GROUPS];
+    // A group's operand is complete; its sums are: of a depthwise layer the first half of the channels and the second, of another
+    // layer all.  A wait by parity cannot tell a phase from the one two further on, so whoever waits on a barrier has to see
+    // each of its phases; warps that need the first half alone wait for `half_done` in every depthwise layer and for `rest_done` in none.
+    __shared__ __align__(8) uint64_t loaded, ready[MAX_GROUPS], half_done[MAX_GROUPS], rest_done[MAX_GROUPS], done[MAX_GROUPS];
     __shared__ uint32_t tmem_base_s;
     __shared__ int failed[MAX_GROUPS];
     __shared__ int4 quant[MAX_STAGES]; // multiplier, bit, shift, 0: not the common quantiser
@@ -204,7 +206,7 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
             mbar_init(&loaded, 1);
             for (int g = 0; g < MAX_GROUPS; ++g)
             {
-                mbar_init(&ready[g], GW); mbar_init(&half_done[g], 1); mbar_init(&done[g], 1);
+                mbar_init(&ready[g], GW); mbar_init(&half_done[g], 1); mbar_init(&rest_done[g], 1); mbar_init(&done[g], 1);
                 failed[g] = 0;
             }
             fence_barrier_init();
@@ -291,8 +293,7 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                                     tc_mma_i8(d0 + (uint32_t)(cb * CB), d_pair[p] + at + (uint64_t)(cb * a.E), b + (uint64_t)((p * KB + cb) * 32),
                                               idesc, p == 0 ? seeded : 1u);
                             // the epilogue of the first half runs under the MMAs of the second
-                            if (h == 0)
-                                tc_commit(&half_done[g]);
+                            tc_commit(h == 0 ? &half_done[g] : &rest_done[g]);
                         }
                     }
                     else
@@ -304,8 +305,8 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                         tc_mma_i8(d0, d_mid + at, b, idesc, seeded); // 32 bytes of the reduction each
                         if (!stem || a.Fh > 8)
                             tc_mma_i8(d0, d_mid + at + (uint64_t)(2 * a.E), b + (uint64_t)b_step, idesc, 1u);
+                        tc_commit(&done[g]);
                     }
-                    tc_commit(&done[g]);
                 }
                 __syncwarp();
             }
@@ -333,7 +334,7 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                 }
             }
         };
-        uint32_t phase = 0, half_phase = 0;
+        uint32_t phase = 0, dw_phase = 0; // of `done`; of `half_done` and `rest_done`
         bool ok = mbar_wait(&loaded, 0, status, 50);
         const uint32_t big = *reinterpret_cast<const uint32_t *>(smem + a.o_big);
         if (first < a.N)
@@ -387,9 +388,12 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                     if (three && to_right)
                         *reinterpret_cast<uint4 *>(p1 + copy_bytes - CB) = o; // copy kw = 2, entry q + W - 1
                 };
-                // (A warp that waits for the first half alone is behind the second one when it comes to the next stage's barrier.)
-                const bool early = dw && cb0 * 2 < KB;
-                ok = early ? mbar_wait(&half_done[group], half_phase, status, 51) : mbar_wait(&done[group], phase, status, 52);
+                // its channels' sums: a depthwise layer's first half, second half or (a group of four warps) both in turn
+                // its channels' sums: a depthwise layer's first half, second half or (a group of four warps) both in turn.  (One wait on
+                // a barrier chosen beforehand: 4096 images 139.5 us.)
+                const bool late = PARTS > 1 && cb0 * 2 >= KB;
+                ok = !dw ? mbar_wait(&done[group], phase, status, 52)
+                         : late ? mbar_wait(&rest_done[group], dw_phase, status, 54) : mbar_wait(&half_done[group], dw_phase, status, 51);
                 tc_fence_after_sync();
                 if (rq.w && !((big >> s) & 1u))
                 {
@@ -403,7 +407,7 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                         {
                             if (PARTS == 1 && i + 1 == KB / 2 && dw)
                             {
-                                ok = mbar_wait(&done[group], phase, status, 52) && ok;
+                                ok = mbar_wait(&rest_done[group], dw_phase, status, 54) && ok;
                                 tc_fence_after_sync();
                             }
                             tmem_ld16(d + (uint32_t)((i + 1) * CB), r[(i + 1) & 1]);
@@ -415,15 +419,18 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                 }
                 else
                 {
-                    ok = mbar_wait(&done[group], phase, status, 52) && ok;
-                    tc_fence_after_sync();
+                    if (PARTS == 1 && dw)
+                    {
+                        ok = mbar_wait(&rest_done[group], dw_phase, status, 54) && ok;
+                        tc_fence_after_sync();
+                    }
 #pragma unroll 1
                     for (int i = 0; i < CBW; ++i)
                         put(cb0 + i, requant16_any(d + (uint32_t)(i * CB),
                                                    ((big >> s) & 1u) ? reinterpret_cast<const int *>(smem + a.o_corr) + s * K + (cb0 + i) * CB : nullptr, a.q[s]));
                 }
-                phase ^= 1;
-                half_phase ^= dw;
+                phase ^= !dw;
+                dw_phase ^= dw;
                 if (s == 0)
                     store_image(); // everybody's im2col of this image is done
             }

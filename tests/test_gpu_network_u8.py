@@ -90,6 +90,28 @@ def test_network_is_one_kernel(oracle, case):
     assert len(np.unique(got[:, :classes])) > 1
 
 
+@pytest.mark.parametrize("N", [1, 147, 149, 200, 296, 297], ids=lambda n: f"n{n}")
+def test_every_image_of_a_batch(oracle, N):
+    """All images, several batches one behind the other: groups of eight warps at one and at two images a CTA, where a warp may begin with
+    half of a depthwise layer's sums, and the first batch of groups of four."""
+    rng = np.random.default_rng(77)
+    layers = _layers(rng, 25, 10, 4, 4, 2, 3, -128, 0, 12, 1024, "common")
+    chain = networks.Chain(layers, N, "u8")
+    chain.capture()
+    for batch in range(3):
+        x = P.pack_activation(rng.integers(0, 256, (N, 1, 25, 10), dtype=np.uint8))
+        chain.stream.synchronize()
+        chain.x.copy_(torch.from_numpy(x.ravel()))
+        torch.cuda.current_stream().synchronize()
+        for _ in range(5):
+            chain.launch()
+        chain.stream.synchronize()
+        assert _lib.device_status() == 0
+        got = chain.y.cpu().numpy().reshape(N, -1)
+        want = np.stack([oracle_chain(oracle, layers, x[n], "u8") for n in range(N)])
+        assert np.array_equal(got, want.reshape(N, -1)), np.flatnonzero((got != want.reshape(N, -1)).any(axis=1))
+
+
 def test_networks_outside_the_one_kernel_form_run_layer_by_layer(oracle):
     """144 pixels do not fit a tile: the same list runs as its layers, with the same bytes."""
     rng = np.random.default_rng(5)
