@@ -88,7 +88,7 @@ conv_gather_f32_kernel(const GArgs a, const float *__restrict__ in, const float 
                        float *__restrict__ out, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[]; // [slot][pixels hi | pixels lo | filter]
-    __shared__ __align__(8) uint64_t full[SLOTS], empty[SLOTS], d_full[2], d_empty[2];
+    __shared__ __align__(8) uint64_t full[SLOTS], empty[SLOTS], d_full[2], d_empty[2], w_all; // w_all: a resident filter's every step is there
     __shared__ uint32_t tmem_base_s;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     uint32_t tmem_cols = 32;
@@ -100,6 +100,7 @@ conv_gather_f32_kernel(const GArgs a, const float *__restrict__ in, const float 
         {
             for (int i = 0; i < SLOTS; ++i) { mbar_init(&full[i], 3); mbar_init(&empty[i], 1); }
             for (int i = 0; i < 2; ++i) { mbar_init(&d_full[i], MMA_WARPS); mbar_init(&d_empty[i], EPI_WARPS); }
+            mbar_init(&w_all, (uint32_t)a.steps);
             fence_barrier_init();
         }
         __syncwarp();
@@ -131,6 +132,10 @@ conv_gather_f32_kernel(const GArgs a, const float *__restrict__ in, const float 
             const uint32_t d0 = tmem + (uint32_t)(buf * a.d_cols + warp * a.groups * kv), dx = d0 + (uint32_t)kv;
             if (used >= a.d_bufs)
                 ok = __all_sync(0xffffffffu, mbar_wait(&d_empty[buf], d_phase, status, 50));
+            // A resident filter's step comes with the pixels of its first use.  With an odd number of steps the warps trade steps from
+            // one tile to the next, and what the other one has waited for says nothing here.
+            if (a.w_resident && used == 1)
+                ok = __all_sync(0xffffffffu, ok && mbar_wait(&w_all, 0, status, 55));
             uint32_t dh = d0;
             int in_sum = 0, sum = 0, s = s0;
             for (; s < a.steps && ok; s += MMA_WARPS)
@@ -294,7 +299,11 @@ conv_gather_f32_kernel(const GArgs a, const float *__restrict__ in, const float 
             }
             __syncwarp();
             if (lane == 0)
+            {
+                if (a.w_resident && i < a.steps)
+                    mbar_arrive(&w_all);
                 mbar_arrive(&full[slot]);
+            }
             load();
         }
     }

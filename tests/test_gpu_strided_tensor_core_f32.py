@@ -4,6 +4,7 @@ import ctypes as C
 
 import numpy as np
 import pytest
+import torch
 
 from oracle.bindings import same_pads, shape
 from smallframework_b200 import interface as S
@@ -57,6 +58,33 @@ def run(oracle, case, bias, part, x_edit=None):
 def test_strided_convolution(oracle, case, mode):
     got, want = run(oracle, case, mode != "plain", mode != "plain")
     assert rel_max_err(got, want) <= 1e-5
+
+
+# C, K, H, W, window, images: filters that stay in shared memory, of 1, 2, 3, 4 and 9 steps, and three tiles or more an SM
+RESIDENT = [(16, 32, 64, 64, 1, 60), (32, 64, 49, 51, 1, 100), (48, 16, 64, 64, 1, 60), (64, 64, 40, 40, 1, 150), (16, 64, 64, 64, 3, 60)]
+
+
+@pytest.mark.parametrize("case", RESIDENT, ids=lambda c: "C{}_K{}_{}x{}_k{}_n{}".format(*c))
+def test_resident_filters_through_many_tiles(case):
+    """Every image, against fp64, of launches whose filters differ.  With an odd number of steps a step is issued by one warp in a CTA's
+    first tile and by the other in its second.  (Bound: the fp32 gate of the other tests.)"""
+    c, k, h, w, f, n = case
+    pads = same_pads(h, w, f, f, 2)
+    rng = np.random.default_rng(c + k + f)
+    ho, wo = shape(c, k, h, w, f, f, 2, pads, CB).out_hw()
+    assert n * ho * wo > 3 * 148 * 128
+    x = rng.uniform(-1, 1, (n, c, h, w)).astype(np.float32)
+    X, O = fbuf(P.pack_activation(x)), S.FloatBuffer(n * k * ho * wo)
+    L = Layer(n, c, k, h, w, f, f, 2, *pads, 0, 0, 0.1, 0, 0, 0, 0, 0, 0)
+    xp = torch.nn.functional.pad(torch.from_numpy(x.astype(np.float64)), (pads[2], pads[3], pads[0], pads[1]))
+    for _ in range(4):
+        wt = rng.normal(0, np.sqrt(2.0 / (c * f * f)), (k, c, f, f)).astype(np.float32)
+        W = fbuf(P.pack_conv_filter(wt))
+        check(lib().small_b200_conv2d_f32(C.byref(L), X.ptr(), W.ptr(), None, O.ptr(), S._stream(None)))
+        got = P.unpack_activation(O.numpy().reshape(n, -1), k, ho, wo)
+        assert device_status() == 0
+        want = torch.nn.functional.conv2d(xp, torch.from_numpy(wt.astype(np.float64)), stride=2).numpy()
+        assert rel_max_err(got, want) <= 1e-5
 
 
 def test_values_outside_the_words_range(oracle):
