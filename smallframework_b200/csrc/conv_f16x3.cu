@@ -180,7 +180,9 @@ constexpr float FAINT = 1.f / 8192;
 // filter, a scale of 2^-48 (magnitudes of 2^61 at least) for a patch.
 constexpr uint32_t LARGE_FILTER = (127u + 45) << 23;
 constexpr float LARGE_DOWN = 281474976710656.f; // 2^48
-constexpr float LEAST_DOWN = 1.f / (1 << 30);
+// The least inverse scale of a channel that is undone in one factor with the patch's (2^-110 at least): 2^-30, and 2^-20 with 32 output
+// channels, where cross terms are added by a factor of their own, LO_DOWN times that product.
+__device__ __forceinline__ float least_down(int K) { return K == 32 ? LO_UP / (1 << 30) : 1.f / (1 << 30); }
 constexpr uint32_t FAINT_SEEN = 0x7fffffffu; // the splitters' word for a patch with a row below that
 
 // Block scale of a set of operands whose largest magnitude has the bits `top`: the power of two that brings it
@@ -222,9 +224,9 @@ prepare_filter_kernel(long long n, int slabs, int MT, int K, const float *__rest
     if (slab == 0 && c == 0)
     {
         down[k] = scale_down(t0);
-        // What the two scales are together has to be a number, and what the sums are: channels so small (2^-17) have theirs
+        // What the two scales are together has to be a number, and what the sums are: channels so small (2^-17, or 2^-7) have theirs
         // undone apart from the patch's, and a filter so large (2^45) is left to the FMA pipe.
-        if (own || (top[k] && down[k] < LEAST_DOWN))
+        if (own || (top[k] && down[k] < least_down(K)))
             atomicOr(reinterpret_cast<uint32_t *>(down) + 2 * K + 1, OWN_SCALES);
         if (top[k] >= LARGE_FILTER)
             atomicOr(reinterpret_cast<uint32_t *>(down) + 2 * K + 1, PLAIN_FILTER);

@@ -122,8 +122,9 @@ def test_pixels_far_apart(case, bits):
            _signed(rng, (N, K, H, W)) * 2.0 ** -bits)
 
 
-# magnitudes of activations and filter that the tensor core is not given, or whose scales are far apart
-EXTREMES = [(3e37, 1e-20), (1e-30, 1e30), (1e-18, 1e-16), (1e-35, 1e3)]
+# magnitudes of activations and filter that the tensor core is not given, or whose scales are far apart, or whose inverse scales
+# (2^-110 and, as the kernel has it, 2^-30 or 2^-20 at least) multiply to next to nothing
+EXTREMES = [(3e37, 1e-20), (1e-30, 1e30), (1e-18, 1e-16), (1e-35, 1e3), (1e-30, 1e-5), (1e-30, 1.25e-2)]
 
 
 @pytest.mark.parametrize("scales", EXTREMES, ids=lambda s: "x{:g}_w{:g}".format(*s))
