@@ -266,6 +266,7 @@ constexpr int FIRST_SPLIT_WARP = 12;
 constexpr int SPLIT_THREADS = 128;
 __host__ __device__ constexpr int num_threads(int split_sets) { return split_sets == 2 ? 640 : 512; }
 constexpr int COLS_PER_THREAD = 128;
+__host__ __device__ constexpr int num_issuers(bool pixm) { return pixm ? 3 : 2; } // they take groups in turn
 
 // Two fp32 values times their block scale as two pairs of half-precision words: hi = v,
 // lo = (v - hi) * 2^LO_SHIFT, both cut to 11 bits as a tf32 operand is.  (Rounded to nearest the 9216-term sums come out at 3.0e-7 of the
@@ -771,7 +772,7 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
             // busy.  The groups are independent sums, so the two threads need no order between them.
             // Pixel-major tiles (PIXM: M = 128 pixels, N = all 32 or 64 output channels) have cheap
             // MMAs (N/2 cycles each), so a third thread joins to keep up with the pipe.
-            constexpr int NISS = PIXM ? 3 : 2;
+            constexpr int NISS = num_issuers(PIXM);
             const int me = warp - 1; // this thread issues the groups with g % NISS == me
             int turn = 0;            // g % NISS
             const bool own_t_full = PIXM || a.tbufs > a.w_stages;
@@ -1524,6 +1525,7 @@ bool fit_rings(TcArgs &a, bool need_two)
     const size_t staging = (size_t)64 * (a.MT + 16) * 4; // 32 pixels of each half of the tile
     // {patch slots, filter stages (>= 2: a commit serves both rings)}
     static const int pref[][2] = {{3, 6}, {3, 4}, {3, 3}, {2, 3}, {3, 2}, {2, 2}, {1, 3}, {1, 2}};
+    const int issuers = num_issuers(a.pixm);
     // persistent where it pays and fits: narrow layers (64-channel tiles: small filter stages and
     // staging rows, little work per tile); wide ones need the shared memory for deeper rings
     // Pixel-major persistent tiles whose whole filter fits: one stage per group of a tile, loaded once
@@ -1554,6 +1556,12 @@ bool fit_rings(TcArgs &a, bool need_two)
     for (int persistent = (a.MT == 64 ? 1 : 0); persistent >= (a.pixm ? 1 : 0); --persistent)
         for (const auto &p : pref)
         {
+            // A wait by parity takes a phase two further on for done, so an issuer has to see every fill of a stage it waits
+            // on: a stage is always the same issuer's.  (Waiting for the MMAs of a stage's last fill as well lets any number serve, but
+            // 64 -> 64 channels 7x7 at 28x28, 64 images, then takes 99.6 us instead of 90.6, 256 -> 256 at 14x14 118 instead of 105,
+            // and ResNet-8 on 1024 images 2 % longer for the test alone.)
+            if (p[1] % issuers)
+                continue;
             const int xs = p[0] < a.cbs || persistent ? p[0] : a.cbs;
             if (!any && (xs & 1))
                 continue;
