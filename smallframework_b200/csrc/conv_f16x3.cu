@@ -120,6 +120,7 @@ struct TcArgs
     // 16 or 32 output channels: a pixel-major MMA takes [W_hi | W_lo] (the rows lie one behind the other in every
     // 8-channel chunk) as ONE operand of 2K columns (the MERGED kernel, see its issuer).
     int merged;
+    int split_sets;      // sets of splitters, 1 or 2 (see want_two_sets); with two the number of patch slots is even
     // Windows of at most nine taps are summed WHOLE in tensor memory where the stages fit (group = taps: at most nine
     // full-size accumulations, as many as one kernel row of two-word tf32 operands used to need): one flush and
     // one round of hand-overs per patch instead of one per kernel row.  row_skip: descriptor units from the last
@@ -1511,6 +1512,22 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
     }
 }
 
+// Two sets of splitters where the conversion of the patches sets the pace: more than three patches a CTA, one after the
+// other (16 -> 32 channels at 208x208, 32 images: 86.4 us with one set, 81.6 with two; 64 -> 32 at 52x52, 64 images 41.4
+// and 37.3; with two patches a CTA, 16 -> 16 at 32x32, 32 images, 8.3 and 8.6).  One set, whose patch slots need not be an even number
+// (three for two: 128 -> 32 with the pool at 112x112, 16 images 130.5 -> 111.0, 64 -> 32 5x5 with the pool at 64x64, 64 images
+// 154.7 -> 147.1, 32 -> 16 1x1 onto what is there at 112x112, 16 images 17.2 -> 16.8) and whose kernel leaves the accumulation
+// warps more registers, where those also read what is there (16 -> 16 at 32x32, 1024 images onto the shortcut: 80 and
+// 85), and before a pool, which makes them the slower ones while the input comes from L2 (16 -> 32 at 208x208, 16 images
+// 43.2 and 44.6; 64 images, 177 MB from memory, 152.2 and 146.6).
+bool want_two_sets(const TcArgs &a)
+{
+    constexpr long long L2_BYTES = 126ll << 20;
+    const long long tiles = (long long)a.N * a.px_tiles * a.k_tiles, blocks = std::min<long long>(tiles, num_sms());
+    return a.merged && !a.accumulate && (a.cbs > 1 || tiles > 3 * blocks) &&
+           (!a.pool || (long long)a.N * a.C * a.H * a.W * (long long)sizeof(float) > L2_BYTES);
+}
+
 // Picks ring depths for the patch / filter sizes already in `a`.  Narrow layers run persistent (one
 // CTA per SM walks over the tiles, roles overlap across tiles), which needs the output staging rows
 // next to the operand buffers; the others keep the deepest rings and let the staging alias them.  need_two: only accept plans with two patches in flight.
@@ -1521,6 +1538,7 @@ bool fit_rings(TcArgs &a, bool need_two)
     const int entries = a.PR * a.PW;
     const size_t x_part = ((size_t)entries * 64 * a.cg + 4095) & ~(size_t)4095;
     a.WR = a.pixm ? a.K : a.MT;
+    a.split_sets = want_two_sets(a) ? 2 : 1; // (pixel-major tiles: always persistent)
     const size_t w_part = (size_t)a.WR * 64 * a.group; // one filter stage
     const size_t staging = (size_t)64 * (a.MT + 16) * 4; // 32 pixels of each half of the tile
     // {patch slots, filter stages (>= 2: a commit serves both rings)}
@@ -1540,7 +1558,7 @@ bool fit_rings(TcArgs &a, bool need_two)
     {
         const int stages = a.cbs * (a.taps / a.group);
         if (stages <= W_STAGES_MAX)
-            for (int xs = a.merged ? 4 : 3; xs >= 2; xs -= a.merged ? 2 : 1) // (two sets of splitters: an even number)
+            for (int xs = x_slots_max(a.merged); xs >= 2; xs -= a.split_sets)
             {
                 const size_t ops = (size_t)xs * x_part + (size_t)stages * w_part;
                 const size_t smem = ops + pool_rows;
@@ -1552,7 +1570,7 @@ bool fit_rings(TcArgs &a, bool need_two)
                 }
             }
     }
-    for (int any = a.merged ? 0 : 1; any < 2; ++any) // two sets of splitters want an even number of slots
+    for (int any = a.split_sets == 2 ? 0 : 1; any < 2; ++any) // two sets of splitters want an even number of slots
     for (int persistent = (a.MT == 64 ? 1 : 0); persistent >= (a.pixm ? 1 : 0); --persistent)
         for (const auto &p : pref)
         {
@@ -2042,15 +2060,7 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
     {
     a.tile_base = (int)base; a.total_tiles = (int)std::min(tiles, base + room);
     const unsigned grid = (unsigned)(a.persistent ? std::min(blocks, tiles - base) : blocks);
-    // Two sets of splitters where the conversion of the patches sets the pace: more than three patches a CTA, one after the
-    // other (16 -> 32 channels at 208x208, 32 images: 86.4 us with one set, 81.6 with two; 64 -> 32 at 52x52, 64 images 41.4
-    // and 37.3; with two patches a CTA, 16 -> 16 at 32x32, 32 images, 8.3 and 8.6).  One set, whose kernel leaves the accumulation
-    // warps more registers, where those also read what is there (16 -> 16 at 32x32, 1024 images onto the shortcut: 80 and
-    // 85), and before a pool, which makes them the slower ones while the input comes from L2 (16 -> 32 at 208x208, 16 images
-    // 43.2 and 44.6; 64 images, 177 MB from memory, 152.2 and 146.6).
-    constexpr size_t L2_BYTES = (size_t)126 << 20;
-    const bool two = a.merged && !a.accumulate && (a.cbs > 1 || tiles > 3 * blocks) &&
-                     (!a.pool || (size_t)L->N * L->C * L->H * L->W * sizeof(float) > L2_BYTES);
+    const bool two = a.split_sets == 2;
 #define SB_LAUNCH_PIXM(M, P, SETS) \
     conv_f16x3_kernel<true, false, true, M, P, SETS><<<grid, num_threads(SETS), a.smem_bytes, as_stream(stream)>>>(\
         mx, in, filt, filt_down, a, bias, out, status)
