@@ -68,7 +68,7 @@ namespace
 using namespace sb;
 
 constexpr int W_STAGES_MAX = 6; // filter stages, each one group of taps (a kernel row)
-__host__ __device__ constexpr int x_slots_max(int merged) { return merged ? 4 : 3; }
+__host__ __device__ constexpr int x_slots_max(bool merged) { return merged ? 4 : 3; }
 constexpr int BOX_PX = 32; // widest box of a TMA load: 256 elements of 8 bytes
 constexpr int WIDE_WORDS = 32; // a CTA's tiles, a bit each: a launch has at most 1024 for every CTA
 constexpr int SCALE_RING = 16; // patches whose block scale is remembered: slots + unflushed accumulator buffers, rounded up
@@ -546,8 +546,7 @@ __device__ __noinline__ void plain_tile(const TcArgs &a, const Tile T, const flo
         }
 }
 
-// MERGED: 1 merged operand, 2 with whole-window groups
-template <bool PERSIST, bool SPLIT, bool PIXM = false, int MERGED = 0, bool POOL = false, int SPLIT_SETS = 1>
+template <bool PERSIST, bool SPLIT, bool PIXM = false, bool MERGED = false, bool POOL = false, int SPLIT_SETS = 1>
 __global__ void __launch_bounds__(num_threads(SPLIT_SETS), 1)
 conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restrict__ in, const __half *__restrict__ filt,
                   const float *__restrict__ filt_down, const __grid_constant__ TcArgs a, const float *__restrict__ bias, float *__restrict__ out, int *status)
@@ -1897,19 +1896,17 @@ int configure()
     int dev;
     if (configured.needed(&dev))
     {
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 1, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<true, false, true, 2, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+#define SB_SMEM(...) SB_CUDA(cudaFuncSetAttribute(conv_f16x3_kernel<__VA_ARGS__>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024))
+        SB_SMEM(true, false);
+        SB_SMEM(true, false, true);
+        SB_SMEM(true, false, true, false, true);
+        SB_SMEM(true, false, true, true);
+        SB_SMEM(true, false, true, true, true);
+        SB_SMEM(true, false, true, true, false, 2);
+        SB_SMEM(true, false, true, true, true, 2);
+        SB_SMEM(false, false);
+        SB_SMEM(false, true);
+#undef SB_SMEM
         configured.mark(dev);
     }
     return SMALL_B200_OK;
@@ -2054,7 +2051,6 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
             return rc;
         return launched("conv_f16x3_kernel");
     }
-    const bool whole = a.merged && a.cg == 1 && a.group != a.Fw; // whole-window groups (TcArgs::row_skip)
     const long long room = a.persistent ? blocks * WIDE_WORDS * 32 : tiles; // tiles of a launch (wide_tiles)
     for (long long base = 0; base < tiles; base += room)
     {
@@ -2064,27 +2060,19 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
 #define SB_LAUNCH_PIXM(M, P, SETS) \
     conv_f16x3_kernel<true, false, true, M, P, SETS><<<grid, num_threads(SETS), a.smem_bytes, as_stream(stream)>>>(\
         mx, in, filt, filt_down, a, bias, out, status)
-    if (a.pool && whole && two)
-        SB_LAUNCH_PIXM(2, true, 2);
-    else if (a.pool && whole)
-        SB_LAUNCH_PIXM(2, true, 1);
-    else if (a.pool && two)
-        SB_LAUNCH_PIXM(1, true, 2);
+    if (a.pool && two)
+        SB_LAUNCH_PIXM(true, true, 2);
     else if (a.pool && a.merged)
-        SB_LAUNCH_PIXM(1, true, 1);
+        SB_LAUNCH_PIXM(true, true, 1);
     else if (a.pool)
-        SB_LAUNCH_PIXM(0, true, 1);
-    else if (whole && two)
-        SB_LAUNCH_PIXM(2, false, 2);
-    else if (whole)
-        SB_LAUNCH_PIXM(2, false, 1);
+        SB_LAUNCH_PIXM(false, true, 1);
     else if (two)
-        SB_LAUNCH_PIXM(1, false, 2);
+        SB_LAUNCH_PIXM(true, false, 2);
     else if (a.merged)
-        SB_LAUNCH_PIXM(1, false, 1);
-#undef SB_LAUNCH_PIXM
+        SB_LAUNCH_PIXM(true, false, 1);
     else if (a.pixm)
-        conv_f16x3_kernel<true, false, true><<<grid, num_threads(1), a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
+        SB_LAUNCH_PIXM(false, false, 1);
+#undef SB_LAUNCH_PIXM
     else if (a.persistent)
         conv_f16x3_kernel<true, false><<<grid, num_threads(1), a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);
     else if (a.ksplit > 1)
