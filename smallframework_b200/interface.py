@@ -15,6 +15,7 @@ from __future__ import annotations
 import ctypes as C
 import functools
 import math
+import struct
 
 import numpy as np
 import torch
@@ -133,12 +134,27 @@ def _layer(batch, C_, K, H, W, Fh, Fw, stride, t, b, l, r, accumulate=0, act=ACT
     return L
 
 
-@functools.lru_cache(maxsize=1024, typed=True)
-def _described(*fields):
-    """A descriptor as the library takes it and the layer's output height and width, kept by value: a program calls the same
-    few layers again and again, and building one takes 2 us.  Nobody writes to a descriptor."""
-    L = Layer(*fields)
+# The fields of a descriptor but the last, which stays 0.
+_pack_fields = struct.Struct("=14if6i4x").pack
+assert struct.calcsize("=14if6i4x") == C.sizeof(Layer)
+
+
+@functools.lru_cache(maxsize=1024)
+def _from_bytes(key):
+    L = Layer.from_buffer_copy(key)
     return (C.byref(L), *L.out_hw())
+
+
+def _described(*fields):
+    """A descriptor as the library takes it and the layer's output height and width, kept by its own bytes (a slope of -0.0 is
+    another one than 0.0, and a dimension counts as what it is worth now): a program calls the same few layers again and
+    again, and building one takes 2 us.  Nobody writes to a descriptor."""
+    try:
+        key = _pack_fields(*fields)
+    except (struct.error, OverflowError):  # what a descriptor refuses, or takes in its own way
+        L = Layer(*fields)
+        return (C.byref(L), *L.out_hw())
+    return _from_bytes(key)
 
 
 def _desc(batch, C_, K, H, W, Fh, Fw, stride, t, b, l, r, accumulate, act, slope, inp, filt, out):
