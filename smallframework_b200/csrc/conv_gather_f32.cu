@@ -100,7 +100,7 @@ conv_gather_f32_kernel(const GArgs a, const float *__restrict__ in, const float 
         {
             for (int i = 0; i < SLOTS; ++i) { mbar_init(&full[i], 3); mbar_init(&empty[i], 1); }
             for (int i = 0; i < 2; ++i) { mbar_init(&d_full[i], MMA_WARPS); mbar_init(&d_empty[i], EPI_WARPS); }
-            mbar_init(&w_all, (uint32_t)a.steps);
+            mbar_init(&w_all, (uint32_t)a.steps * 32);
             fence_barrier_init();
         }
         __syncwarp();
@@ -296,14 +296,12 @@ conv_gather_f32_kernel(const GArgs a, const float *__restrict__ in, const float 
                         o[kv] = split(v[j], o);
                     }
                 fence_proxy_async();
+                if (a.w_resident)
+                    mbar_arrive(&w_all);
             }
             __syncwarp();
             if (lane == 0)
-            {
-                if (a.w_resident && i < a.steps)
-                    mbar_arrive(&w_all);
                 mbar_arrive(&full[slot]);
-            }
             load();
         }
     }
