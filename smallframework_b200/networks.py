@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import operator
 
 import numpy as np
 import torch
@@ -311,6 +312,18 @@ def algorithmic_work(L, elt):
 
 
 # --------------------------------------------------------------------------- executor
+def _upload(arrays, device):
+    """Arrays (or None) as tensors on the device, views of one tensor: one copy, and one count of writes."""
+    starts = np.cumsum([0] + [0 if a is None else -(-a.nbytes // 256) * 256 for a in arrays])
+    host = np.zeros(int(starts[-1]), np.uint8)
+    for a, at in zip(arrays, starts):
+        if a is not None:
+            host[at:at + a.nbytes] = np.ascontiguousarray(a).view(np.uint8).ravel()
+    whole = torch.from_numpy(host).to(device)
+    return [None if a is None else whole[at:at + a.nbytes].view(torch.from_numpy(a[:0]).dtype)
+            for a, at in zip(arrays, starts.tolist())]
+
+
 class Chain:
     """A layer list bound to device memory for a fixed batch.
 
@@ -329,7 +342,9 @@ class Chain:
         3x3 depthwise convolution (the reference's Conv2D_ReLU_DepthwiseConv2D_ReLU pairing), or by the
         global average pool and the dense layer that end the keyword-spotting network, runs as one kernel
         where the library covers the shapes; the absorbed layers are entered in `fused_into` likewise; a keyword-spotting network
-        that the library covers whole (small_b200_separable_network_u8_supported) is one kernel.
+        that the library covers whole (small_b200_separable_network_u8_supported) is one kernel, with a copy of `params` that
+        is laid out again when a launch finds them written to (see prepare_whole).
+        fp32 filters laid out for the tensor cores are copies made here, once.
         "auto" also runs layers of a few million multiply-adds in the latency kernel
         (small_b200_conv2d_f32_small_preferred) and a global average pool with the dense layer and the softmax behind it as
         one kernel.  fuse_dw: an fp32 depthwise convolution followed by a 1x1 convolution (a depthwise-separable block) runs as
@@ -344,21 +359,17 @@ class Chain:
         c, h, w = input_shape(layers)
         self.x = torch.zeros(batch * c * h * w, dtype=self.tdtype, device=self.dev)
         max_act = 0
-        self.params = []
+        host = []
         for L in layers:
             ho, wo = _out_hw(L)
             kp = padded(L["K"])
             max_act = max(max_act, batch * kp * ho * wo)
-            if L["op"] == "alias":
-                self.params.append((None, None))
-                continue
-            wt = bs = None
-            if L["op"] in ("conv", "dwconv"):
-                w_np, b_np = padded_params(L, len(self.params) == 0, dtype)
-                wt = torch.from_numpy(w_np).to(self.dev)
-                if b_np is not None:
-                    bs = torch.from_numpy(b_np).to(self.dev)
-            self.params.append((wt, bs))
+            host.append(padded_params(L, len(host) == 0, dtype) if L["op"] in ("conv", "dwconv") else (None, None))
+        if dtype == "u8":
+            flat = iter(_upload([a for pair in host for a in pair], self.dev))
+            self.params = list(zip(flat, flat))
+        else:
+            self.params = [tuple(None if a is None else torch.from_numpy(a).to(self.dev) for a in pair) for pair in host]
         self.bufs = [torch.zeros(max_act, dtype=self.tdtype, device=self.dev) for _ in range(2)]
         # layers that name their buffers (a small DAG, e.g. residual stages) get one tensor per name
         self.named = {"in": self.x}
@@ -426,14 +437,13 @@ class Chain:
                 if lib().small_b200_conv2d_maxpool_f32_supported(C.byref(dc), C.byref(dp)):
                     self.fused_into[i + 1] = i
         self.whole = None  # the list is one kernel: its weights, laid out once
+        self._counted = ()  # what they were made from, and torch's counts of the writes to it then
         if dtype == "u8" and fuse_u8 and not any("src" in L for L in layers):
             descs = self._desc_array()
             nbytes = lib().small_b200_separable_network_u8_prepared_bytes(descs, len(layers))
             if nbytes:
                 self.whole = torch.empty(nbytes, dtype=torch.uint8, device=self.dev)
-                ptrs = lambda k: (C.c_void_p * len(layers))(*[None if t[k] is None else t[k].data_ptr() for t in self.params])
-                check(lib().small_b200_separable_network_u8_prepare(descs, len(layers), ptrs(0), ptrs(1), self.whole.data_ptr(),
-                                                                    torch.cuda.current_stream().cuda_stream))
+                self.prepare_whole(torch.cuda.current_stream().cuda_stream)
                 torch.cuda.synchronize()
         if self.whole is not None:
             self.fused_into = {i: 0 for i in range(1, len(layers))}
@@ -499,6 +509,22 @@ class Chain:
         return (Layer * len(self.layers))(*[self._desc(L, L["C"] if i == 0 else padded(L["C"]))
                                             for i, L in enumerate(self.layers)])
 
+    def prepare_whole(self, stream=None):
+        """Lays the weights of a network that is one kernel out, on `stream` (the chain's own by default).  launch() does it when torch
+        has counted a write to what the graph was recorded with, capture() and enqueue() also when `params` holds other tensors.  To be called
+        after a write that torch does not count (through `.data`, to inference tensors, or from outside torch)."""
+        self._whole_of = list(self.params)
+        tensors = [t for pair in self.params for t in pair if t is not None and not t.is_inference()]
+        bases = {id(b): b for b in (t if t._base is None else t._base for t in tensors)}.values()  # a view counts with its base
+        self._counted = [(b, b._version) for b in bases]
+        ptrs = lambda k: (C.c_void_p * len(self.layers))(*[None if t[k] is None else t[k].data_ptr() for t in self.params])
+        check(lib().small_b200_separable_network_u8_prepare(self._desc_array(), len(self.layers), ptrs(0), ptrs(1), self.whole.data_ptr(),
+                                                            self.stream.cuda_stream if stream is None else stream))
+
+    def _whole_is_current(self):
+        return all(b._version == v for b, v in self._counted) and len(self.params) == len(self._whole_of) and \
+            all(map(operator.is_, self.params, self._whole_of))
+
     def enqueue_layer(self, i, src, dst, stream):
         L = self.layers[i]
         wt, bs = self.params[i]
@@ -511,6 +537,8 @@ class Chain:
             return  # computed by its producer
         follow = self.absorbed(i)
         if self.whole is not None:
+            if not self._whole_is_current():
+                self.prepare_whole(stream)
             check(l.small_b200_separable_network_u8(self._desc_array(), len(self.layers), p(self.whole), p(src), p(dst), stream))
         elif i in self.tails:
             D = self.layers[i + 1]
@@ -606,6 +634,8 @@ class Chain:
         for xin in (inputs if inputs is not None else [self.x]):
             saved, self.x = self.x, xin
             self.named["in"] = xin
+            if self.whole is not None and not self._whole_is_current():
+                self.prepare_whole()  # (not into the graph)
             self.stream.synchronize()
             gp = C.c_void_p()
             check(l.small_b200_graph_begin(self.stream.cuda_stream))
@@ -622,6 +652,10 @@ class Chain:
     def launch(self, k=0):
         if self.graph is None:
             self.capture()
+        for base, version in self._counted:
+            if base._version != version:
+                self.prepare_whole()
+                break
         check(lib().small_b200_graph_launch(self.graphs[k % len(self.graphs)], self.stream.cuda_stream))
 
     def __del__(self):

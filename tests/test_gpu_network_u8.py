@@ -112,6 +112,51 @@ def test_every_image_of_a_batch(oracle, N):
         assert np.array_equal(got, want.reshape(N, -1)), np.flatnonzero((got != want.reshape(N, -1)).any(axis=1))
 
 
+@pytest.mark.parametrize("how", ["written", "replaced", "replaced, then written", "untracked"])
+def test_weights_changed_after_the_recording(oracle, how):
+    """A launch computes with what the tensors of `params` hold then, as a network that runs layer by layer does."""
+    rng = np.random.default_rng(11)
+    old, new = (_layers(np.random.default_rng(s), 25, 10, 4, 4, 2, 2, -128, 0, 12, 1024, "common") for s in (1, 2))
+    new = [dict(a, **{k: b[k] for k in ("w", "b") if k in b}) for a, b in zip(old, new)]  # other weights, the same quantisers
+    chain = networks.Chain(old, 3, "u8")
+    x = P.pack_activation(rng.integers(0, 256, (3, 1, 25, 10), dtype=np.uint8))
+    chain.x.copy_(torch.from_numpy(x.ravel()))
+    chain.capture()
+
+    def run():
+        torch.cuda.synchronize()
+        chain.launch()
+        chain.stream.synchronize()
+        return chain.y.cpu().numpy().reshape(3, -1)
+
+    want_old, want_new = (np.stack([oracle_chain(oracle, L, x[n], "u8") for n in range(3)]).reshape(3, -1) for L in (old, new))
+    assert not np.array_equal(want_old, want_new)
+    assert np.array_equal(run(), want_old)
+    other = networks.Chain(new, 1, "u8").params
+    if how.startswith("replaced"):
+        chain.params[:] = [tuple(None if t is None else t.clone() for t in pair) for pair in other]
+        chain.capture()
+        assert np.array_equal(run(), want_new)
+        if "written" in how:
+            for mine, theirs in zip(chain.params, networks.Chain(old, 1, "u8").params):
+                for a, b in zip(mine, theirs):
+                    if a is not None:
+                        a.copy_(b)
+            assert np.array_equal(run(), want_old)
+        return
+    for mine, theirs in zip(chain.params, other):
+        for a, b in zip(mine, theirs):
+            if a is not None:
+                (a.data if how == "untracked" else a).copy_(b)
+    if how == "untracked":
+        torch.cuda.synchronize()
+        chain.prepare_whole()
+    assert np.array_equal(run(), want_new)
+    y = chain.enqueue()  # layer calls instead of the graph
+    chain.stream.synchronize()
+    assert np.array_equal(y.cpu().numpy().reshape(3, -1), want_new)
+
+
 def test_networks_outside_the_one_kernel_form_run_layer_by_layer(oracle):
     """144 pixels do not fit a tile: the same list runs as its layers, with the same bytes."""
     rng = np.random.default_rng(5)
