@@ -181,7 +181,7 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
             const int ih0 = oh * a.row_stride - a.pad_t, iw0 = ow * a.stride - a.pad_l;
             const bool border = GENERAL && (a.zero_in > 0 || a.zero_in < -255) &&
                                 (ih0 < 0 || iw0 < 0 || ih0 + a.Fh > a.H || iw0 + a.Fw > a.W);
-            ok = mbar_wait(&acc_full[buf], (i >> 1) & 1, status, 31);
+            ok = mbar_wait(&acc_full[buf], (i >> 1) & 1, status, 56);
             if (!ok)
                 break;
             tc_fence_after_sync();
@@ -359,7 +359,7 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
                     continue;
                 const unsigned s = slot;
                 if (use > 0) // every lane waits; the outcome is made the same for the whole warp
-                    ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], (use - 1) & 1u, status, 32));
+                    ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[s], (use - 1) & 1u, status, 57));
                 if (ok)
                 {
                     uint8_t *st = smem + (size_t)s * G::STAGE;
@@ -391,14 +391,14 @@ conv_u8_ring_kernel(const RingArgs a, const uint8_t *__restrict__ in, const uint
         {
             const int buf = i & 1;
             if (i >= 2)
-                ok = mbar_wait(&acc_empty[buf], ((i >> 1) - 1) & 1, status, 33);
+                ok = mbar_wait(&acc_empty[buf], ((i >> 1) - 1) & 1, status, 58);
             if (!ok)
                 break;
             tc_fence_after_sync();
             for (int q = 0; q < a.steps && ok; ++q, ++consumed)
             {
                 const unsigned s = consumed % STAGES;
-                ok = mbar_wait(&full_bar[s], (consumed / STAGES) & 1u, status, 34);
+                ok = mbar_wait(&full_bar[s], (consumed / STAGES) & 1u, status, 59);
                 if (!ok)
                     break;
                 tc_fence_after_sync();

@@ -83,7 +83,7 @@ dwpw_direct_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
     if (tid < K)
         s_b2[tid] = b2 ? __ldg(b2 + tid) : 0.f;
     __syncthreads();
-    if (!mbar_wait(&full, 0, status, 81))
+    if (!mbar_wait(&full, 0, status, 85))
         return;
     const int strip = a.by_TW.div(tid), x = tid - strip * a.TW, row = strip * V;
     if (row >= a.TH || c0 + x >= a.Wo)

@@ -237,7 +237,7 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
     if (!worker)
     {
         // ---------------- issuers: each the MMAs of every other group ----------------
-        bool ok = __all_sync(0xffffffffu, mbar_wait(&loaded, 0, status, 50));
+        bool ok = __all_sync(0xffffffffu, mbar_wait(&loaded, 0, status, 71));
         const uint32_t big = __shfl_sync(0xffffffffu, *reinterpret_cast<const uint32_t *>(smem + a.o_big), 0), mem = smem_u32(smem + a.o_group);
         const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base_s, 0);
         const uint64_t d_ones = make_smem_desc(smem_u32(smem + a.o_ones), BM * CB, 8 * CB, 0);
@@ -271,7 +271,7 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                 const int block = s >> 1;
                 const uint32_t seeded = ((big >> s) & 1u) ^ 1u, sgn = (a.signed_in >> s) & 1u, d0 = tmem + (uint32_t)(g * K);
                 const uint64_t at = (uint64_t)((uint32_t)g * (a.group_bytes >> 4));
-                ok = __all_sync(0xffffffffu, mbar_wait(&ready[g], phase, status, 53));
+                ok = __all_sync(0xffffffffu, mbar_wait(&ready[g], phase, status, 74));
                 if (!ok)
                     break;
                 tc_fence_after_sync();
@@ -335,7 +335,7 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
             }
         };
         uint32_t phase = 0, dw_phase = 0; // of `done`; of `half_done` and `rest_done`
-        bool ok = mbar_wait(&loaded, 0, status, 50);
+        bool ok = mbar_wait(&loaded, 0, status, 71);
         const uint32_t big = *reinterpret_cast<const uint32_t *>(smem + a.o_big);
         if (first < a.N)
         {
@@ -392,8 +392,8 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                 // its channels' sums: a depthwise layer's first half, second half or (a group of four warps) both in turn.  (One wait on
                 // a barrier chosen beforehand: 4096 images 139.5 us.)
                 const bool late = PARTS > 1 && cb0 * 2 >= KB;
-                ok = !dw ? mbar_wait(&done[group], phase, status, 52)
-                         : late ? mbar_wait(&rest_done[group], dw_phase, status, 54) : mbar_wait(&half_done[group], dw_phase, status, 51);
+                ok = !dw ? mbar_wait(&done[group], phase, status, 73)
+                         : late ? mbar_wait(&rest_done[group], dw_phase, status, 75) : mbar_wait(&half_done[group], dw_phase, status, 72);
                 tc_fence_after_sync();
                 if (rq.w && !((big >> s) & 1u))
                 {
@@ -407,7 +407,7 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                         {
                             if (PARTS == 1 && i + 1 == KB / 2 && dw)
                             {
-                                ok = mbar_wait(&rest_done[group], dw_phase, status, 54) && ok;
+                                ok = mbar_wait(&rest_done[group], dw_phase, status, 75) && ok;
                                 tc_fence_after_sync();
                             }
                             tmem_ld16(d + (uint32_t)((i + 1) * CB), r[(i + 1) & 1]);
@@ -421,7 +421,7 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                 {
                     if (PARTS == 1 && dw)
                     {
-                        ok = mbar_wait(&rest_done[group], dw_phase, status, 54) && ok;
+                        ok = mbar_wait(&rest_done[group], dw_phase, status, 75) && ok;
                         tc_fence_after_sync();
                     }
 #pragma unroll 1
