@@ -617,61 +617,36 @@ def measured_traffic(layer, batch, kernel):
     return MEASURED_TRAFFIC.get((layer, batch, kernel.split()[0]))
 
 
-def kernel_class(chain, i, L, dtype):
-    """Which kernel runs layer i (with the layers it absorbs) and what bounds it."""
-    if chain.whole is not None:
-        return "net_u8_tc_kernel (tcgen05 kind::i8, the whole network)", "i8"
-    follow = chain.absorbed(i)
-    if i in chain.tails:
-        return "pool_dense_softmax_f32_kernel", "stream"
-    if L["op"] == "conv":
-        if dtype == "f32":
-            if i in chain.small:
-                return "conv_small_f32_kernel (FFMA, latency)", "ffma"
-            if chain.prepared[i] is not None:
-                return "conv_f16x3_kernel (tcgen05 kind::f16, two-word operands)" + (" + 2x2 max pool" if follow else ""), "f16x3"
-            if L["stride"] > 1 and L["C"] >= 16:
-                return "conv_gather_f32_kernel (tcgen05 kind::tf32, two-word operands)", "tf32x3"
-            name = "conv2d_first_f32_kernel (FFMA)" if L["C"] < 16 else "conv2d_f32_kernel (FFMA)"
-            return name + (" + 2x2 max pool" if follow else ""), "ffma"
-        if follow:
-            tail = "depthwise 3x3 on tcgen05" if len(follow) == 1 else "global average pool + dense"
-            return f"block_u8_tc_kernel (tcgen05 kind::i8 {'im2col first layer' if L['C'] == 1 else '1x1'} -> {tail})", "i8"
-        ho, wo = networks_out_hw(L)
-        outputs = chain.batch * ho * wo
-        C, K = L["C"] if i == 0 else networks_padded(L["C"]), networks_padded(L["K"])
-        thin = L["Fh"] == 1 and L["Fw"] == 1 and L["stride"] == 1 and K <= 128
-        if thin and C == 16 and (K >= 64 or outputs * K >= 4 << 20) or \
-                thin and C in (32, 64) and outputs >= 30000 and ho * wo >= 64:
-            return "conv_u8_thin_kernel (tcgen05 kind::i8)", "i8"
-        pw = (L["Fh"] == 1 and L["Fw"] == 1 and L["stride"] == 1 and L["C"] % 32 == 0 and L["C"] <= 256)
-        if pw:
-            return "pw_u8_tc_kernel (tcgen05 kind::i8)", "i8"
-        if L["C"] == 1 and L["Fw"] <= 4 and L["Fh"] <= 16 and ho * wo <= 128 and L["K"] <= 128:
-            return "stem_u8_tc_kernel (im2col in shared memory + tcgen05 kind::i8)", "i8"
-        if L["C"] * L["Fh"] * L["Fw"] > 32 or (L["C"] >= 16 and L["K"] > 128):
-            return ("conv_u8_patch_kernel (tcgen05 kind::i8)" if L["C"] % 16 == 0 and L["Fh"] * L["Fw"] > 1 else
-                    "conv_u8_ring_kernel (implicit GEMM, tcgen05 kind::i8)"), "i8"
-        if L["C"] == 3 and outputs >= 200000 and L["Fw"] <= (6 if L["stride"] == 2 else 5):
-            return "conv_u8_rgb_kernel (tcgen05 kind::i8)", "i8"
-        return "conv2d_u8_onestep_kernel (dp4a, streaming)", "stream"
-    if L["op"] == "dwconv" and dtype == "u8":
-        tiles = L["Fh"] == 3 and L["Fw"] == 3 and L["stride"] == 1
-        return ("dwconv3x3_u8_tile_kernel (dp4a)" if tiles else "dwconv_u8_dp4a_kernel"), "stream"
-    if i in chain.blocks:
-        ho, wo = networks_out_hw(L)
-        K, outputs = networks_padded(chain.layers[i + 1]["K"]), chain.batch * ho * wo
-        if K in (16, 32) and ((L["stride"] == 1 and (L["C"] <= 16 or L["C"] <= 32 and outputs >= 16384)) or
-                              (L["stride"] == 2 and L["C"] <= 16 and K == 32 and outputs <= 131072)):
-            return "dwpw_direct_f32_kernel (depthwise 3x3 + 1x1, FFMA)", "ffma"
-        return "dwpw_f32_kernel (depthwise 3x3 + 1x1 on tcgen05 kind::tf32, two-word operands)", "tf32x3"
-    return {"dwconv": "window_f32_kernel (depthwise)", "maxpool": "max pool", "avgpool": "average pool",
-            "softmax": "softmax", "alias": "alias"}[L["op"]], "stream"
+# What bounds a kernel, by the name the library gives it; others stream.
+KERNELS = {
+    "net_u8_tc_kernel": ("tcgen05 kind::i8, the whole network", "i8"),
+    "block_u8_tc_kernel": ("tcgen05 kind::i8", "i8"),
+    "pw_u8_tc_kernel": ("tcgen05 kind::i8", "i8"),
+    "stem_u8_tc_kernel": ("im2col in shared memory + tcgen05 kind::i8", "i8"),
+    "conv_u8_thin_kernel": ("tcgen05 kind::i8", "i8"),
+    "conv_u8_rgb_kernel": ("tcgen05 kind::i8", "i8"),
+    "conv_u8_patch_kernel": ("tcgen05 kind::i8", "i8"),
+    "conv_u8_ring_kernel": ("implicit GEMM, tcgen05 kind::i8", "i8"),
+    "conv2d_u8_onestep_kernel": ("dp4a, streaming", "stream"),
+    "dwconv3x3_u8_tile_kernel": ("dp4a", "stream"),
+    "conv_f16x3_kernel": ("tcgen05 kind::f16, two-word operands", "f16x3"),
+    "conv_gather_f32_kernel": ("tcgen05 kind::tf32, two-word operands", "tf32x3"),
+    "dwpw_f32_kernel": ("depthwise 3x3 + 1x1 on tcgen05 kind::tf32, two-word operands", "tf32x3"),
+    "dwpw_direct_f32_kernel": ("depthwise 3x3 + 1x1, FFMA", "ffma"),
+    "conv_small_f32_kernel": ("FFMA, latency", "ffma"),
+    "conv_first_small_f32_kernel": ("FFMA, latency", "ffma"),
+    "conv2d_f32_kernel": ("FFMA", "ffma"),
+    "conv2d_first_f32_kernel": ("FFMA", "ffma"),
+    "conv2d_first_fixed_f32_kernel": ("FFMA", "ffma"),
+    "conv2d_first_pool_f32_kernel": ("FFMA", "ffma"),
+    "conv2d_first_pool_fixed_f32_kernel": ("FFMA", "ffma"),
+}
 
 
-def networks_padded(channels):
-    from smallframework_b200.networks import padded
-    return padded(channels)
+def kernel_class(name, follow=()):
+    """(kernel, pipe) of the kernel of this name that ran a layer and, in its epilogue, the layers `follow`."""
+    note, pipe = KERNELS.get(name, ("", "stream"))
+    return name + (f" ({note})" if note else "") + "".join(" + " + f for f in follow), pipe
 
 
 def networks_out_hw(L):
@@ -689,7 +664,7 @@ def per_layer_report(chain, layers, batch, wl, clocks, torch, pipes=None):
     flops of all of them and the bytes it has to move: the first layer's input, the last one's output, all
     the weights.  fp32 layers at their batch read inputs far larger than L2; the uint8 networks' layers are
     L2-resident here as they are inside a step (see config.l2)."""
-    from smallframework_b200 import networks
+    from smallframework_b200 import _lib, networks
     peaks = load_peaks()
     if pipes is None:
         pipes = measured_pipes(torch)
@@ -730,7 +705,10 @@ def per_layer_report(chain, layers, batch, wl, clocks, torch, pipes=None):
         flops *= batch
         nbytes = abytes * batch + wbytes
         work[len(rows)] = (flops, nbytes)
-        kname, kcls = kernel_class(chain, i, L, wl["dtype"])
+        chain.enqueue_layer(i, src, dst, st)
+        chain.stream.synchronize()
+        inside = () if chain.whole is not None else [layers[k]["op"] for k in group[1:]]
+        kname, kcls = kernel_class(_lib.last_kernel(), inside)
         t_flop = flops / (pipe_tops[kcls] * 1e12)
         t_mem = nbytes / (peaks["hbm"] * 1e9)
         rows.append({"layer": "+".join(layers[k].get("name", layers[k]["op"]) for k in group), "kernel": kname,

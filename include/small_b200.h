@@ -110,6 +110,8 @@ int small_b200_selftest_bounded_wait(uint32_t polls, void *stream);
 int small_b200_peak_probe(int kind, double *tera_ops);
 /* Number of kernels this library has launched in this process since it was loaded. */
 uint64_t small_b200_launch_count(void);
+/* Name of the kernel that the calling thread launched last ("" before its first launch): which of a layer's kernels a call took. */
+const char *small_b200_last_kernel(void);
 
 /* ---- memory (the platform's alloc_buffer/free_buffer,
  *      include/small/platforms/reference/Buffer.hpp:36-61, FloatBuffer.hpp:59-77) ------- */

@@ -115,7 +115,7 @@ SIGNATURES = {
     "small_b200_avgpool2d_u8": [_LP, _VP, _VP, _VP],
     "small_b200_relu_u8": [_I64, _LP, _VP, _VP, _VP],
 }
-OTHER = {"small_b200_last_error": ([], C.c_char_p), "small_b200_launch_count": ([], C.c_uint64),
+OTHER = {"small_b200_last_error": ([], C.c_char_p), "small_b200_last_kernel": ([], C.c_char_p), "small_b200_launch_count": ([], C.c_uint64),
          "small_b200_nms_scratch_bytes": ([C.c_int32], C.c_size_t),
          "small_b200_separable_network_u8_prepared_bytes": ([_LP, C.c_int32], C.c_size_t)}
 
@@ -166,3 +166,8 @@ def device_status() -> int:
 
 def launch_count() -> int:
     return int(lib().small_b200_launch_count())
+
+
+def last_kernel() -> str:
+    """Name of the kernel that this thread launched last."""
+    return lib().small_b200_last_kernel().decode()

@@ -15,6 +15,7 @@ namespace sb
 constexpr int CB = SMALL_B200_CB;
 
 extern thread_local std::string g_last_error;
+extern thread_local const char *g_last_kernel;
 extern std::atomic<uint64_t> g_launches;
 
 inline int fail(int code, const std::string &msg)
@@ -37,10 +38,11 @@ inline int cuda_fail(cudaError_t e, const char *what)
             return sb::cuda_fail(e_, #call);        \
     } while (0)
 
-// Call after every kernel launch: counts it and turns a launch error into a return code.
+// Call after every kernel launch: counts it, keeps its name (a literal) and turns a launch error into a return code.
 inline int launched(const char *name)
 {
     g_launches.fetch_add(1, std::memory_order_relaxed);
+    g_last_kernel = name;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return cuda_fail(e, name);

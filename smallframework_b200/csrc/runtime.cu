@@ -6,6 +6,7 @@
 namespace sb
 {
 thread_local std::string g_last_error;
+thread_local const char *g_last_kernel = "";
 std::atomic<uint64_t> g_launches{0};
 
 int check_window_layer(const small_b200_layer *L, const char *name, bool dense, int max_stride)
@@ -45,6 +46,7 @@ int small_b200_set_device(int device)
 }
 
 uint64_t small_b200_launch_count(void) { return g_launches.load(); }
+const char *small_b200_last_kernel(void) { return g_last_kernel; }
 
 int small_b200_malloc(size_t bytes, void **ptr)
 {
