@@ -438,7 +438,10 @@ class Chain:
                     self.fused_into[i + 1] = i
         self.whole = None  # the list is one kernel: its weights, laid out once
         self._counted = ()  # what they were made from, and torch's counts of the writes to it then
-        if dtype == "u8" and fuse_u8 and not any("src" in L for L in layers):
+        # (a descriptor does not say whether a layer is dense or depthwise, or which pool it is)
+        pairs = max(0, (len(layers) - 3) // 2)
+        if dtype == "u8" and fuse_u8 and not any("src" in L for L in layers) and \
+                [L["op"] for L in layers] == ["conv"] + ["dwconv", "conv"] * pairs + ["avgpool", "conv"]:
             descs = self._desc_array()
             nbytes = lib().small_b200_separable_network_u8_prepared_bytes(descs, len(layers))
             if nbytes:

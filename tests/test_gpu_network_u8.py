@@ -171,3 +171,24 @@ def test_networks_outside_the_one_kernel_form_run_layer_by_layer(oracle):
     got = chain.y.cpu().numpy().reshape(2, -1)
     for n in range(2):
         assert np.array_equal(got[n], oracle_chain(oracle, layers, x[n], "u8"))
+
+
+@pytest.mark.parametrize("which", ["dense 3x3", "max pool"])
+def test_other_operations_of_the_same_shapes_run_layer_by_layer(oracle, which):
+    """A dense 3x3 layer has the descriptor of a depthwise one, a global max pool that of an average pool."""
+    rng = np.random.default_rng(6)
+    layers = _layers(rng, 25, 10, 4, 4, 2, 2, -128, 0, 12, 1024, "common")
+    if which == "dense 3x3":
+        layers[3].update(op="conv", w=rng.integers(0, 256, (64, 64, 3, 3)).astype(np.uint8))
+    else:
+        layers[-2] = {**layers[-2], "op": "maxpool"}
+    chain = networks.Chain(layers, 2, "u8")
+    assert chain.whole is None
+    x = P.pack_activation(rng.integers(0, 256, (2, 1, 25, 10), dtype=np.uint8))
+    chain.x.copy_(torch.from_numpy(x.ravel()))
+    chain.capture()
+    chain.launch()
+    chain.stream.synchronize()
+    got = chain.y.cpu().numpy().reshape(2, -1)
+    for n in range(2):
+        assert np.array_equal(got[n], oracle_chain(oracle, layers, x[n], "u8"))
