@@ -146,7 +146,7 @@ conv_u8_thin_kernel(const __grid_constant__ ThinArgs a, const uint8_t *__restric
 #pragma unroll
                 for (int g = 0; g < G; ++g)
                 {
-                        const int px = tile * G * BM + g * BM + m;
+                    const int px = tile * G * BM + g * BM + m;
                     live[g] = px < a.total;
                     const int n = a.by_P.div(live[g] ? px : 0), p = px - n * a.P;
                     o[g] = out + ((size_t)n * kbs + kb0) * plane + (long long)p * CB;
@@ -214,10 +214,10 @@ conv_u8_thin_kernel(const __grid_constant__ ThinArgs a, const uint8_t *__restric
             }
             else
             {
-                // a lane a plane and image: the pixels of at most three images
+                // a lane a plane and image: the pixels of at most three images (a.P >= 64); seg * a.P fits in 31 bits
                 const int n = a.by_P.div(px0), p = px0 - n * a.P;
-                const int row0 = seg ? seg * a.P - p : 0, rows = min(seg ? a.P : a.P - p, left - row0);
-                if (rows > 0)
+                const int row0 = seg ? min(seg, 2) * a.P - p : 0, rows = min(seg ? a.P : a.P - p, left - row0);
+                if (seg < 3 && rows > 0)
                     tma_load_1d(dst + cb * HALF + row0 * CB, in + (((size_t)(n + seg) * a.chunks + cb) * a.P + (seg ? 0 : p)) * CB, (uint32_t)rows * CB,
                                 &full[st]);
             }
