@@ -506,18 +506,22 @@ bool plan(const small_b200_layer *L, int n, NetArgs &a)
         return false;
     a = NetArgs{};
     const small_b200_layer &c = L[0];
-    if (c.N < 0 || c.C != 1 || c.K != K || c.zero_filt != -128 || (c.zero_in != 0 && c.zero_in != -128) || !quant_ok(c) || c.Fh < 1 ||
+    // (images are counted in 32 bits, with a round of the CTAs' groups on top)
+    if (c.N < 0 || c.N > 0x7fff0000 || c.H < 1 || c.W < 1 || c.C != 1 || c.K != K || c.zero_filt != -128 || (c.zero_in != 0 && c.zero_in != -128) || !quant_ok(c) || c.Fh < 1 ||
         c.Fh > 16 || c.Fw < 1 || c.Fw > 4 || c.stride < 1 || c.pad_t < 0 || c.pad_b < 0 || c.pad_l < 0 || c.pad_r < 0)
+        return false;
+    const long long tall = (long long)c.H + c.pad_t + c.pad_b, wide = (long long)c.W + c.pad_l + c.pad_r; // the padded image
+    if ((long long)c.H * c.W > IMAGE_BYTES * 128 || tall > SMEM_LIMIT || wide > SMEM_LIMIT || tall * wide > SMEM_LIMIT)
         return false;
     a.N = c.N;
     a.H = out_dim(c.H, c.pad_t, c.pad_b, c.Fh, c.stride);
     a.W = out_dim(c.W, c.pad_l, c.pad_r, c.Fw, c.stride);
     a.HW = a.H * a.W;
-    if (a.H <= 0 || a.W <= 0 || a.HW > BM || c.H * c.W > IMAGE_BYTES * 128)
+    if (a.H <= 0 || a.W <= 0 || a.HW > BM)
         return false;
     a.H0 = c.H; a.W0 = c.W; a.Fh = c.Fh; a.Fw = c.Fw; a.stride = c.stride; a.pad_t = c.pad_t; a.pad_l = c.pad_l;
-    a.pitch = ((c.W + c.pad_l + c.pad_r + 12) + 3) & ~3; // room for the unaligned window read
-    a.img_bytes = ((c.H + c.pad_t + c.pad_b + 1) * a.pitch + 127) & ~127;
+    a.pitch = (((int)wide + 12) + 3) & ~3; // room for the unaligned window read
+    a.img_bytes = (((int)tall + 1) * a.pitch + 127) & ~127;
     a.E = (BM + 2 * a.W + 7) & ~7;
     a.q[0] = quant(c); a.zero_in[0] = c.zero_in;
     a.signed_in = c.zero_in != 0;
@@ -537,7 +541,8 @@ bool plan(const small_b200_layer *L, int n, NetArgs &a)
             a.signed_in |= 1u << s;
     }
     const small_b200_layer &pl = L[n - 2], &dn = L[n - 1];
-    if (pl.N != a.N || pl.C != K || pl.H != a.H || pl.W != a.W || pl.Fh != a.H || pl.Fw != a.W || !no_pads(pl) || !quant_ok(pl))
+    if (pl.N != a.N || pl.C != K || pl.H != a.H || pl.W != a.W || pl.Fh != a.H || pl.Fw != a.W || pl.stride < 1 || pl.stride > 3 ||
+        !no_pads(pl) || !quant_ok(pl))
         return false;
     if (dn.N != a.N || dn.C != K || dn.H != 1 || dn.W != 1 || dn.Fh != 1 || dn.Fw != 1 || dn.stride != 1 || !no_pads(dn) ||
         dn.K <= 0 || dn.K % CB != 0 || dn.K > 128 || !quant_ok(dn) || dn.zero_filt != -128)

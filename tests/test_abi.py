@@ -72,3 +72,26 @@ def test_shape_queries_need_no_gpu():
     assert fused(conv, _layer(16, 16, 416, 416, 2, 2, 2, (0, 0, 0, 0), 4))
     assert not fused(conv, _layer(16, 16, 416, 416, 2, 2, 1, (0, 1, 0, 1), 4))   # stride-1 pool
     assert not fused(conv, _layer(16, 16, 208, 208, 2, 2, 2, (0, 0, 0, 0), 4))   # pool of another tensor
+
+
+def _network(N=3, H=49, W=10, stride=2, pads=(4, 5, 1, 1), pool_stride=1):
+    """Descriptors of a keyword-spotting network: a 10x4 first layer, two blocks, average pool, dense layer."""
+    t, b, l, r = pads
+    h, w = (H + t + b - 10) // stride + 1, (W + l + r - 4) // stride + 1
+    q = (0, -128, 0, 10, 1 << 30, 0)
+    make = lambda c, k, h, w, fh, fw, s, p: _lib.Layer(N, c, k, h, w, fh, fw, s, *p, 0, 0, 0.0, *q)
+    none, one = (0, 0, 0, 0), (1, 1, 1, 1)
+    block = [make(64, 64, h, w, 3, 3, 1, one), make(64, 64, h, w, 1, 1, 1, none)]
+    layers = [make(1, 64, H, W, 10, 4, stride, pads), *block, *block, make(64, 64, h, w, h, w, pool_stride, none),
+              make(64, 16, 1, 1, 1, 1, 1, none)]
+    return (_lib.Layer * len(layers))(*layers), len(layers)
+
+
+def test_whole_network_sizes_are_not_cut_to_32_bits():
+    """Padded images whose bytes, input pixels or images are more than an int holds are not covered."""
+    covered = lambda **k: bool(_lib.lib().small_b200_separable_network_u8_supported(*_network(**k)))
+    assert covered() and covered(N=0x7fff0000)
+    assert not covered(N=0x7fffffff)                                                             # an image more than a round below 2^31
+    assert not covered(stride=8192, pads=(32742, 32744, 32757, 32757))                           # 65536 rows of 65536 bytes
+    assert not covered(H=65536, W=65536, stride=16384, pads=(0, 0, 0, 0))                        # 2^32 pixels
+    assert not covered(pool_stride=0)                                                            # refused as a layer too
