@@ -500,6 +500,9 @@ bool fit(PatchArgs &a, int NT)
 {
     const uint32_t block = (uint32_t)(a.planes * a.E * CB), slab_run = (uint32_t)(a.taps * SLAB), groups = NT / CB + 1;
     auto plan = [&](bool resident, int cc, int stages) {
+        const unsigned long long filter = (unsigned long long)groups * slab_run * (resident ? a.cbs : cc);
+        if (filter > SMEM_LIMIT || (unsigned long long)block * cc > SMEM_LIMIT) // (what follows is in 32 bits)
+            return false;
         a.resident = resident; a.cc = cc; a.stages = stages; a.chunks = (a.cbs + cc - 1) / cc;
         a.run = slab_run * (uint32_t)(resident ? a.cbs : cc);
         a.patch_bytes = block * cc;
@@ -560,7 +563,8 @@ int conv2d_u8_patch(const small_b200_layer *L, const uint8_t *in, const uint8_t 
         if (TW > BM)
             continue;
         const int rows = (BM - TW) / PW + 1, TH = std::min(rows, a.Ho), RI = TH + more_r;
-        const int ni = parts == 1 && TH == a.Ho ? std::min((rows - TH) / RI + 1, a.N) : 1;
+        int ni = parts == 1 && TH == a.Ho ? std::min((rows - TH) / RI + 1, a.N) : 1;
+        ni = (int)std::min<long long>(ni, 0xffffffffll / ((long long)a.C * a.H * a.W)); // 32-bit offsets inside a tile's images
         const int tx = (a.Wo + TW - 1) / TW, ty = (a.Ho + TH - 1) / TH;
         const long long tiles = (long long)tx * ty * ((a.N + ni - 1) / ni);
         if (best >= 0 && tiles >= best)

@@ -2,9 +2,14 @@
 parts, ragged last tiles, several whole images a tile, strides of two with odd sizes, windows other than 3x3, odd numbers of
 channel blocks, filters that stay in shared memory and filters that travel with the pixels, partial blocks of output channels,
 and the zero points whose padding is a byte."""
+import ctypes
+
 import numpy as np
 import pytest
+import torch
 
+from oracle.bindings import shape
+from smallframework_b200 import _lib
 from tests.test_gpu_uint8 import _case_id, _check_conv, _quant
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +58,30 @@ def test_quantisers_outside_the_common_form(oracle, shift):
     rng = np.random.default_rng(3)
     q = Quant(-3, -120, 2 - 2 * shift, shift, 1 << 14, 0)
     _check_conv(oracle, case, same_pads(9, 11, 3, 3, 1), q, rng, True, None)
+
+
+@pytest.mark.parametrize("case", [
+    # C, H, W, Fh, Fw, stride, images: a filter and a patch whose bytes wrap to next to nothing in 32 bits; tiles of more than 2^32 bytes
+    (139811 * 16, 7, 7, 7, 7, 1, 1),
+    (838860 * 16, 8, 10, 1, 2, 2, 6),
+], ids=["filter", "tile"])
+def test_sizes_beyond_32_bits(oracle, case):
+    """Millions of channels, of which three blocks have pixels other than zero."""
+    C, H, W, Fh, Fw, s, N = case
+    blocks, taps, used = C // 16, Fh * Fw, [0, C // 48, C // 16 - 1]
+    ho, wo = (H - Fh) // s + 1, (W - Fw) // s + 1
+    gen = torch.Generator("cuda").manual_seed(5)
+    x = torch.zeros(N, blocks, H * W * 16, dtype=torch.uint8, device="cuda")
+    x[:, used] = torch.randint(0, 256, (N, 3, H * W * 16), dtype=torch.uint8, device="cuda", generator=gen)
+    w = torch.randint(0, 256, (blocks, taps * 256), dtype=torch.uint8, device="cuda", generator=gen)
+    out = torch.empty(N, ho * wo * 16, dtype=torch.uint8, device="cuda")
+    q = _quant(np.random.default_rng(5), 48 * taps, (0, -121))
+    L = _lib.Layer(N, C, 16, H, W, Fh, Fw, s, 0, 0, 0, 0, 0, 0, 0.0, q.zero_in, q.zero_filt, q.lshift, q.rshift, q.multiplier, q.k_zero)
+    stream = torch.cuda.current_stream()
+    _lib.check(_lib.lib().small_b200_conv2d_u8(ctypes.byref(L), x.data_ptr(), w.data_ptr(), None, out.data_ptr(), stream.cuda_stream))
+    stream.synchronize()
+    assert _lib.device_status() == 0 and _lib.last_kernel() == "conv_u8_patch_kernel"
+    sh = shape(48, 16, H, W, Fh, Fw, s, (0, 0, 0, 0), 16)
+    few, xs = w[used].cpu().numpy().ravel(), x[:, used].cpu().numpy()
+    want = np.stack([oracle.conv2d_u8(sh, q, xs[n].ravel(), few) for n in range(N)])
+    assert np.array_equal(out.cpu().numpy(), want.reshape(N, -1)) and want.min() < want.max()
