@@ -257,7 +257,6 @@ prepare_filter_kernel(long long n, int slabs, int MT, int K, const float *__rest
 // tcgen05.commit, which frees the filter stage for the producer and hands the partial sums to
 // the accumulation warps.
 //
-//
 // MERGED kernels (16 or 32 output channels) can have a second set of splitters, warps 16..19: the sets take the patches in turn.  A
 // set takes 2100 to 3700 cycles a patch, a chain of a few hundred instructions, where the MMAs of a tile need 1400 to 2000:
 // with one set it was the splitters that such a layer waited for.
@@ -546,7 +545,8 @@ __device__ __noinline__ void plain_tile(const TcArgs &a, const Tile T, const flo
         }
 }
 
-template <bool PERSIST, bool SPLIT, bool PIXM = false, bool MERGED = false, bool POOL = false, int SPLIT_SETS = 1>
+// LATE: the accumulation warps work out where their pixel goes behind the sums, and fetch nothing ahead (see the launch).
+template <bool PERSIST, bool SPLIT, bool PIXM = false, bool MERGED = false, bool POOL = false, int SPLIT_SETS = 1, bool LATE = false>
 __global__ void __launch_bounds__(num_threads(SPLIT_SETS), 1)
 conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__restrict__ in, const __half *__restrict__ filt,
                   const float *__restrict__ filt_down, const __grid_constant__ TcArgs a, const float *__restrict__ bias, float *__restrict__ out, int *status)
@@ -1077,23 +1077,22 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                                                                            : make_float4(0.f, 0.f, 0.f, 0.f);
                     acc[4 * c4] = b.x; acc[4 * c4 + 1] = b.y; acc[4 * c4 + 2] = b.z; acc[4 * c4 + 3] = b.w;
                 }
-                // This thread's pixel.
-                const int ml = T.m_local0 + mt * 128 + quarter * 32 + lane;
-                const int rl = a.by_PW.div(ml), cl = ml - rl * a.PW, r = T.row_base + rl, c = T.col_base + cl;
-                const bool live = !POOL && active && cl < T.tw_valid && rl < T.th_valid && r < a.Ho;
-                float *o = out + (size_t)T.n * (a.K / CB) * plane + (size_t)r * a.o_row_stride + (size_t)c * CB;
-                auto add_old = [&]() {
-#pragma unroll
-                    for (int c4 = 0; c4 < ACC / 4; ++c4)
-                        if (c4 * 4 < a.K)
-                        {
-                            const float4 old = *(reinterpret_cast<const float4 *>(o + (size_t)(c4 >> 2) * plane) + (c4 & 3));
-                            acc[4 * c4] += old.x; acc[4 * c4 + 1] += old.y; acc[4 * c4 + 2] += old.z; acc[4 * c4 + 3] += old.w;
-                        }
+                int rl, cl, r, c; // this thread's pixel, of the patch and of the output
+                bool live;
+                float *o;
+                auto locate = [&]() {
+                    const int ml = T.m_local0 + mt * 128 + quarter * 32 + lane;
+                    rl = a.by_PW.div(ml); cl = ml - rl * a.PW; r = T.row_base + rl; c = T.col_base + cl;
+                    live = !POOL && active && cl < T.tw_valid && rl < T.th_valid && r < a.Ho;
+                    o = out + (size_t)T.n * (a.K / CB) * plane + (size_t)r * a.o_row_stride + (size_t)c * CB;
                 };
-                if (!POOL && a.accumulate && live) // on its way to L2 while the sums are made (87 -> 80 us, see the launch)
-                    for (int kb = 0; kb * CB < a.K; ++kb)
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(o + (size_t)kb * plane));
+                if (!LATE)
+                {
+                    locate();
+                    if (!POOL && a.accumulate && live) // on its way to L2 while the sums are made
+                        for (int kb = 0; kb * CB < a.K; ++kb)
+                            asm volatile("prefetch.global.L2 [%0];" ::"l"(o + (size_t)kb * plane));
+                }
                 int in_cb = 0;
                 for (int g = 0; g < groups && ok; ++g, ++gc)
                 {
@@ -1154,6 +1153,8 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                     if (lane == 0)
                         mbar_arrive(&t_empty[tb]);
                 }
+                if (LATE)
+                    locate();
                 if (own_scales)
 #pragma unroll
                     for (int c4 = 0; c4 < ACC / 4; ++c4)
@@ -1229,7 +1230,13 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
                 else if (ok && live && !(a.accumulate && is_wide(once_)))
                 {
                     if (a.accumulate)
-                        add_old();
+#pragma unroll
+                        for (int c4 = 0; c4 < ACC / 4; ++c4)
+                            if (c4 * 4 < a.K)
+                            {
+                                const float4 old = *(reinterpret_cast<const float4 *>(o + (size_t)(c4 >> 2) * plane) + (c4 & 3));
+                                acc[4 * c4] += old.x; acc[4 * c4 + 1] += old.y; acc[4 * c4 + 2] += old.z; acc[4 * c4 + 3] += old.w;
+                            }
 #pragma unroll
                     for (int k8 = 0; k8 < ACC / 8; ++k8)
                         if (k8 * 8 < a.K)
@@ -1541,7 +1548,7 @@ bool fit_rings(TcArgs &a, bool need_two)
     const size_t w_part = (size_t)a.WR * 64 * a.group; // one filter stage
     const size_t staging = (size_t)64 * (a.MT + 16) * 4; // 32 pixels of each half of the tile
     // {patch slots, filter stages (>= 2: a commit serves both rings)}
-    static const int pref[][2] = {{3, 6}, {3, 4}, {3, 3}, {2, 3}, {3, 2}, {2, 2}, {1, 3}, {1, 2}};
+    static const int pref[][2] = {{4, 6}, {4, 3}, {3, 6}, {3, 4}, {3, 3}, {2, 3}, {3, 2}, {2, 2}, {1, 3}, {1, 2}};
     const int issuers = num_issuers(a.pixm);
     // persistent where it pays and fits: narrow layers (64-channel tiles: small filter stages and
     // staging rows, little work per tile); wide ones need the shared memory for deeper rings
@@ -1578,6 +1585,12 @@ bool fit_rings(TcArgs &a, bool need_two)
             // 64 -> 64 channels 7x7 at 28x28, 64 images, then takes 99.6 us instead of 90.6, 256 -> 256 at 14x14 118 instead of 105,
             // and ResNet-8 on 1024 images 2 % longer for the test alone.)
             if (p[1] % issuers)
+                continue;
+            // Four slots serve two sets of splitters, each with its next patch on the way while the MMAs read its last one (two
+            // slots and four, us: 256 -> 32 channels 3x3 at 94x23, 128 images 330 and 280; 64 -> 32 7x7 at 135x96, 64 images 667 and 624; 128 -> 16
+            // 1x1 at 22x184, 32 images 29.3 and 24.0).  Six filter stages beside them only where a group is a whole window: 128 -> 32 3x3
+            // at 8x13, 128 images 17.4 with six and 17.9 with three, but 256 -> 16 5x5 at 81x92, 64 images 851 and 742.
+            if (p[0] == 4 && (a.split_sets != 2 || any || (p[1] == 6 && a.group != a.taps)))
                 continue;
             const int xs = p[0] < a.cbs || persistent ? p[0] : a.cbs;
             if (!any && (xs & 1))
@@ -1904,6 +1917,8 @@ int configure()
         SB_SMEM(true, false, true, true, true);
         SB_SMEM(true, false, true, true, false, 2);
         SB_SMEM(true, false, true, true, true, 2);
+        SB_SMEM(true, false, true, true, false, 1, true);
+        SB_SMEM(true, false, true, true, false, 2, true);
         SB_SMEM(false, false);
         SB_SMEM(false, true);
 #undef SB_SMEM
@@ -2056,22 +2071,29 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
     {
     a.tile_base = (int)base; a.total_tiles = (int)std::min(tiles, base + room);
     const unsigned grid = (unsigned)(a.persistent ? std::min(blocks, tiles - base) : blocks);
-    const bool two = a.split_sets == 2;
-#define SB_LAUNCH_PIXM(M, P, SETS) \
-    conv_f16x3_kernel<true, false, true, M, P, SETS><<<grid, num_threads(SETS), a.smem_bytes, as_stream(stream)>>>(\
+    // Tiles of many patches: LATE, since what the other form keeps in registers over the sums costs more in every group than the
+    // epilogue then gains.  us, the other form and this: onto what is there 256 -> 16 channels 3x3 at 162x43, 64 images 428 and 414, 128 -> 16
+    // at 30x52, one image 20.4 and 19.1; but 16 -> 16 at 112x112, 256 images 178 and 207, 64 -> 64 1x1 at 32x32, 1024 images 133 and 159.
+    const bool two = a.split_sets == 2, late = a.cg == 1 && a.cbs > 4;
+#define SB_LAUNCH_PIXM(M, P, SETS, LATE) \
+    conv_f16x3_kernel<true, false, true, M, P, SETS, LATE><<<grid, num_threads(SETS), a.smem_bytes, as_stream(stream)>>>(\
         mx, in, filt, filt_down, a, bias, out, status)
     if (a.pool && two)
-        SB_LAUNCH_PIXM(true, true, 2);
+        SB_LAUNCH_PIXM(true, true, 2, false);
     else if (a.pool && a.merged)
-        SB_LAUNCH_PIXM(true, true, 1);
+        SB_LAUNCH_PIXM(true, true, 1, false);
     else if (a.pool)
-        SB_LAUNCH_PIXM(false, true, 1);
+        SB_LAUNCH_PIXM(false, true, 1, false);
+    else if (two && late)
+        SB_LAUNCH_PIXM(true, false, 2, true);
     else if (two)
-        SB_LAUNCH_PIXM(true, false, 2);
+        SB_LAUNCH_PIXM(true, false, 2, false);
+    else if (a.merged && late)
+        SB_LAUNCH_PIXM(true, false, 1, true);
     else if (a.merged)
-        SB_LAUNCH_PIXM(true, false, 1);
+        SB_LAUNCH_PIXM(true, false, 1, false);
     else if (a.pixm)
-        SB_LAUNCH_PIXM(false, false, 1);
+        SB_LAUNCH_PIXM(false, false, 1, false);
 #undef SB_LAUNCH_PIXM
     else if (a.persistent)
         conv_f16x3_kernel<true, false><<<grid, num_threads(1), a.smem_bytes, as_stream(stream)>>>(mx, in, filt, filt_down, a, bias, out, status);

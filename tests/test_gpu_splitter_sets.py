@@ -41,3 +41,31 @@ def test_against_the_oracle(oracle, case):
         if pool:
             ref = oracle.pool2d_f32(shape(k, k, h, w, 2, 2, 2, (0, 0, 0, 0), CB), ref)
         assert rel_max_err(got[i], ref) <= 1e-5  # pairs of 11-bit words: a product is off by 2^-21 at most, the rest is fp32 sums
+
+
+TRAVELLING = [
+    # C, K, H, W, kernel, images, onto what is there: more patches than filter stages, two tiles a CTA and more
+    (128, 32, 26, 35, 3, 90, False), (144, 16, 26, 35, 3, 90, False), (96, 16, 20, 60, 5, 70, False), (64, 32, 16, 60, 7, 70, False),
+    (256, 16, 30, 33, 1, 90, False), (128, 16, 26, 35, 3, 90, True), (112, 32, 26, 35, 3, 2, True),
+]
+
+
+@pytest.mark.parametrize("case", TRAVELLING, ids=lambda c: "C{}_K{}_{}x{}_k{}_n{}{}".format(*c[:6], "_onto" if c[6] else ""))
+def test_filters_that_travel(oracle, case):
+    """Two sets of splitters with four patch slots beside a ring of filter stages, and the forms that find their pixel late."""
+    c, k, h, w, f, n, onto = case
+    pads = same_pads(h, w, f, f, 1)
+    rng = np.random.default_rng(c + k + f)
+    x = rng.uniform(-1, 1, (n, c, h, w)).astype(np.float32) * (8.0 ** (np.arange(n) % 5 - 2)).astype(np.float32)[:, None, None, None]
+    x, wt = P.pack_activation(x), P.pack_conv_filter(rng.normal(0, np.sqrt(2.0 / (c * f * f)), (k, c, f, f)).astype(np.float32))
+    seed = rng.uniform(-1, 1, (n, k * h * w)).astype(np.float32) if onto else None
+    I, F, O = fbuf(x), fbuf(wt), fbuf(seed) if onto else S.FloatBuffer(n * k * h * w)
+    Fp = S.FloatBuffer(2 * F.size())
+    S.prepare_filter_3xTF32(f, f, k, c, F, Fp)
+    S.Conv2D_3xTF32(f, f, 1, *pads, k, c, h, w, I, Fp, None, O, partial=onto, batch=n)
+    got = O.numpy().reshape(n, -1)
+    assert _lib.device_status() == 0
+    some = np.unique(np.linspace(0, n - 1, 8).astype(int))
+    want = oracle_conv_batch(oracle, shape(c, k, h, w, f, f, 1, pads, CB), x[some], wt, seed=seed[some] if onto else None)
+    for i, ref in zip(some, want):
+        assert rel_max_err(got[i], ref) <= 1e-5  # as above
