@@ -526,6 +526,36 @@ bool fit(PatchArgs &a, int NT)
                 return true;
     return plan(false, 2, 2);
 }
+// Where conv_u8_ring.cu is the shorter way.  Its tiles are 128 outputs each and no junk; here small images under large windows leave
+// few outputs a tile, and a filter that does not stay is fetched for each of them again.
+//   Cycles of a step of 32 bytes: here 100 a tile while the filter stays, else what its bytes take, by bulk copies or 16 at a time, but not
+// less than 1.6 for every 16 bytes of pixels; there 800 for the first tile of an SM, which waits for its gathers, and 650 for a tile more, with
+// zero points that want further columns 1350 and 1400 (to 1700); with some room for what this leaves out.
+// us, there and here: 64 -> 64 7x7 with a stride of two at 8x17, 1024 images 55 and 113; 192 -> 192 3x3 / 2 at 20x11, 256 images 34 and 58;
+// 192 -> 192 7x7 / 2 at 23x23, 64 images 130 and 152; 256 -> 256 1x3 / 2 at 8x8, 1024 images 18.6 and 24.4; but 96 -> 48 7x7 / 2 at
+// 6x6, 1024 images 63 and 53.
+//   Launches of a few steps: the sums of the filter, which padding with a byte other than zero needs, take longer than the ring's
+// steps: 16 -> 32 1x3 / 2 at 25x19 4.2 and 5.2, 32 -> 16 2x2 / 2 at 7x9, 8 images 4.3 and 5.1; 16 -> 96 2x2 / 2 at 3x3, 16 images 5.5 and 5.0.
+// Windows that meet a pixel once or twice, few channels: 32 -> 16 2x2 / 2 at 25x25, 1024 images 14.8 and 19.9, 32 -> 32 2x2 at 18x18, 256 images
+// 9.1 and 10.7, 16 -> 64 2x2 at 11x11 (1.8 times as many tiles), 1024 images 15.2 and 17.7.
+// Of 2000 random layers some 40 were slower here than there by more than 2 %, behind this line 6, by 9 % at most.
+bool ring_is_shorter(const PatchArgs &a, int nt)
+{
+    const bool plain = a.zero_filt == -128 && (a.zero_in == 0 || a.zero_in == -128);
+    const int few = a.taps * ((a.cbs + 1) / 2); // the ring's steps
+    const bool little = a.planes == 4 && few <= 6 && a.K <= 32;
+    const int sms = num_sms(), blocks = (a.K + nt - 1) / nt, side = std::max(1, sms / blocks);
+    const long long rounds = (a.tiles + side - 1) / side, ring = ((long long)a.N * a.Ho * a.Wo + BM - 1) / BM;
+    if (rounds == 1)
+        return plain && a.zero_in != 0 && ((a.K <= 64 && few <= 4) || little);
+    if (plain && (little || (a.zero_in != 0 && few <= 4 && (a.planes == 4 || a.K <= 32))))
+        return true;
+    if (few <= 4 && a.tiles > 1.3 * ring)
+        return true;
+    const double step = a.resident ? 100. : a.in_order ? std::max(105., 2.5 * nt) : std::max(165., 4.2 * nt);
+    const double here = rounds * std::max(step, 3.2 * a.units / a.taps), tiles = (double)ring * ((a.K + 127) / 128) / sms;
+    return here > (plain ? std::max(840., 680. * tiles) : std::max(1750., 1800. * tiles));
+}
 } // namespace
 
 namespace sb
@@ -609,6 +639,8 @@ int conv2d_u8_patch(const small_b200_layer *L, const uint8_t *in, const uint8_t 
     while (!fit(a, nt))
         if ((nt /= 2) < 16)
             return -1;
+    if (ring_is_shorter(a, nt))
+        return -1;
 #define SB_PATCH(NT_) return a.taps == 9 ? launch_patch<NT_, true>(a, in, filt, bias, out, st) : launch_patch<NT_, false>(a, in, filt, bias, out, st)
     switch (nt)
     {

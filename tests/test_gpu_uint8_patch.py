@@ -51,6 +51,31 @@ def test_conv2d_u8_patch(oracle, case, zp):
     _check_conv(oracle, case, pads, _quant(rng, C * Fh * Fw, zp), rng, zp[0] != 0, None)
 
 
+RING = [
+    # what conv_u8_ring.cu does sooner (see ring_is_shorter), and windows of more taps than the patch kernel has room for
+    (16, 16, 19, 19, 1, 3, 2, "same", 1, (-128, -128)),
+    (32, 16, 7, 9, 2, 2, 2, "valid", 8, (-128, -128)),
+    (32, 64, 3, 3, 1, 3, 1, "same", 2, (-128, -128)),
+    (32, 16, 25, 25, 2, 2, 2, "valid", 300, (0, -128)),
+    (64, 64, 8, 17, 7, 7, 2, "same", 592, (0, -128)),
+    (16, 64, 11, 11, 2, 2, 1, (1, 1, 1, 1), 600, (-113, -121)),
+    (256, 256, 8, 8, 1, 3, 2, (0, 0, 1, 1), 1024, (-128, -128)),
+    (16, 16, 20, 20, 8, 8, 1, "same", 3, (0, -128)),
+    (32, 48, 20, 11, 5, 12, 2, "same", 3, (-128, -128)),
+    (16, 32, 20, 20, 10, 5, 1, "same", 2, (-113, -121)),
+]
+
+
+@pytest.mark.parametrize("case", RING, ids=lambda c: _case_id(c[:9]) + "_zi{}_zf{}".format(*c[9]))
+def test_layers_that_stay_with_the_ring(oracle, case):
+    from oracle.bindings import same_pads
+    C, K, H, W, Fh, Fw, s, pm, N, zp = case
+    pads = same_pads(H, W, Fh, Fw, s) if pm == "same" else (0, 0, 0, 0) if pm == "valid" else pm
+    rng = np.random.default_rng(C + H + W + N)
+    _check_conv(oracle, case[:9], pads, _quant(rng, C * Fh * Fw, zp), rng, zp[0] != 0, None)
+    assert _lib.last_kernel() == "conv_u8_ring_kernel"
+
+
 @pytest.mark.parametrize("shift", [0, 1], ids=lambda r: f"rshift{r}")
 def test_quantisers_outside_the_common_form(oracle, shift):
     from oracle.bindings import Quant, same_pads
