@@ -424,6 +424,13 @@ int conv2d_u8_rgb(const small_b200_layer *L, const uint8_t *in, const uint8_t *f
     if (best < 0 || best > 0x3fffffff)
         return -1;
     a.tiles = (int)best;
+    // Tiles with few outputs, of images a little too large for one: from half of one on where a tile's pixels are fetched for several parts of the
+    // channels, a third where for one.  us, the CUDA cores' form and this: 3 -> 32 at 11x11, 2048 images (0.24 of a tile, two parts)
+    // 12.1 and 18.5, 3 -> 64 at 38x9, 2048 images (0.33, four) 43.6 and 61.6, at 30x30 / 2, 1024 images (0.44, two) 18.9 and 21.4; but at
+    // 18x18, 1024 images (0.63, four) 23.6 and 19.5, 3 -> 16 at 15x15, 2048 images (0.44) 13.6 and 11.9.
+    const double filled = (double)a.N * a.Ho * a.Wo / ((double)a.tiles * BM * G);
+    if (filled < (a.K > (a.stride == 2 && a.K % (2 * CB) == 0 ? 2 * CB : CB) && a.Fh > 2 ? 0.5 : 0.35))
+        return -1;
     a.rows_in = (a.TH - 1) * a.stride + a.Fh;
     a.units = a.rows_in * a.PW;
     a.E = std::max(BM + more_r * a.PW + 1, (a.rows_in + a.stride - 1) / a.stride * a.PW);

@@ -4,6 +4,7 @@ than 3x3, the zero points whose padding is a byte."""
 import numpy as np
 import pytest
 
+from smallframework_b200 import _lib
 from tests.test_gpu_uint8 import _case_id, _check_conv, _quant
 
 pytestmark = pytest.mark.gpu
@@ -36,6 +37,17 @@ def test_conv2d_u8_rgb(oracle, case, zp):
     pads = same_pads(H, W, Fh, Fw, s) if pm == "same" else (0, 0, 0, 0) if pm == "valid" else pm
     rng = np.random.default_rng(K * 100 + H * 10 + W + zp[0] + 1000)
     _check_conv(oracle, case, pads, _quant(rng, C * Fh * Fw, zp), rng, zp[0] != 0, None)
+
+
+@pytest.mark.parametrize("case", [
+    (3, 48, 35, 38, 3, 3, 2, (1, 1, 1, 1), 640, "conv_u8_rgb_kernel"), (3, 48, 30, 31, 3, 3, 2, (1, 1, 1, 1), 840, "conv2d_u8_onestep_kernel"),
+    (3, 16, 300, 3, 3, 3, 2, (1, 1, 1, 1), 700, "conv_u8_rgb_kernel"), (3, 16, 300, 1, 3, 3, 2, (1, 1, 1, 1), 1340, "conv2d_u8_onestep_kernel"),
+    (3, 64, 18, 18, 3, 3, 1, (1, 1, 1, 1), 620, "conv_u8_rgb_kernel"), (3, 64, 38, 9, 3, 3, 1, (1, 1, 1, 1), 600, "conv2d_u8_onestep_kernel"),
+], ids=lambda c: _case_id(c[:9]))
+def test_how_full_tiles_are(oracle, case):
+    rng = np.random.default_rng(case[1] + case[2])
+    _check_conv(oracle, case[:9], case[7], _quant(rng, 27, (-113, -121)), rng, True, None)
+    assert _lib.last_kernel() == case[9]
 
 
 @pytest.mark.parametrize("shift", [0, 1], ids=lambda r: f"rshift{r}")
