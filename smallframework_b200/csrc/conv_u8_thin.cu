@@ -27,13 +27,13 @@ constexpr int THREADS = (EPI_WARPS + PRODUCERS + ISSUERS) * 32;
 constexpr uint32_t HALF = BM * CB; // 128 pixels of a plane
 // Where this kernel is the faster one.  us, before (16 channels: the CUDA cores' kernel of quint8.cu, else conv_u8_tc.cu) -> this: 16 -> 16 at
 // 48x48, 64 images (2.4 million results) 3.8 -> 4.2, 256 images 9.4 -> 7.4; 16 -> 32 at 24x24, 64 images 3.3 -> 3.9, 256 images (4.7
-// million) 5.3 -> 5.1; 16 -> 64 at 24x24, 1 image 3.9 -> 3.7, 64 images 4.3 -> 4.2; 32 -> 64 at 12x12, 128 images (18 432 pixels) 4.1 -> 4.5,
+// million) 5.3 -> 5.1; 16 -> 64 at 24x24, 1 image 3.9 -> 3.7, 64 images 4.3 -> 4.2, but up to 128 pixels (a CTA there) 3.0 to 3.3 -> 3.7; 32 -> 64 at 12x12, 128 images (18 432 pixels) 4.1 -> 4.5,
 // 256 images 5.2 -> 4.6; 64 -> 64 at 12x12, 64 images 4.2 -> 4.6, 256 images 5.6 -> 5.3.  128 channels stay where they were: 128 -> 128 at
 // 14x14, 64 images 5.6 -> 6.8, at 8x8, 2048 images 14.4 -> 17.6.
 constexpr long long MIN_RESULTS = 4 << 20, MIN_PIXELS = 30000;
 bool large_enough(int C, int K, long long pixels)
 {
-    return C > CB ? pixels >= MIN_PIXELS : K >= 64 || pixels * K >= MIN_RESULTS;
+    return C > CB ? pixels >= MIN_PIXELS : (K >= 64 && pixels > BM) || pixels * K >= MIN_RESULTS;
 }
 constexpr int MAX_STEPS = 2;             // reduction steps: up to 64 channels
 constexpr int SMEM_LIMIT = 2 * MAX_STEPS * (STAGES * (int)HALF + 80 * 16);

@@ -48,6 +48,15 @@ def test_quantisers_outside_the_common_form(oracle, shift, C):
     _check_conv(oracle, (C, 32, 32, 32, 1, 1, 1, "valid", 130), (0, 0, 0, 0), Quant(-3, -120, 2 - 2 * shift, shift, 1 << 19, 0), rng, True, None)
 
 
+@pytest.mark.parametrize("case", [(16, 64, 8, 16, 1, 1, 1, "valid", 1), (16, 64, 3, 43, 1, 1, 1, "valid", 1), (16, 96, 2, 2, 1, 1, 1, "valid", 32),
+                                  (16, 128, 5, 26, 1, 1, 1, "valid", 1)], ids=_case_id)
+def test_where_a_few_pixels_go(oracle, case):
+    """16 channels to 64 and more: from 129 pixels on this kernel."""
+    rng = np.random.default_rng(case[1] + case[2])
+    _check_conv(oracle, case, (0, 0, 0, 0), _quant(rng, 16, (-113, -121)), rng, True, None)
+    assert (_lib.last_kernel() == "conv_u8_thin_kernel") == (case[2] * case[3] * case[8] > 128)
+
+
 def test_planes_beyond_a_fifteenth_of_31_bits(oracle):
     """One image of 143 million pixels (4.6 GB): the runs of a tile that lie in other images are counted in 32 bits."""
     C, K, H, W = 32, 16, 11970, 11969
