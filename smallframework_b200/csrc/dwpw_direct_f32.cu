@@ -214,9 +214,9 @@ int dwpw_direct_f32(const small_b200_layer *D, const small_b200_layer *L, const 
     const int S = D->stride, K = L->K;
     // Where it is the shorter way, by outputs: 32 channels from 16384 on (24x24: one image 6.4 us there and 7.6 here, 128 images 12.3 and
     // 10.7); a stride of two, where a warp's reads meet in pairs of banks, for 16 -> 32 up to 131072 (48x48: 16 images 6.5 and
-    // 5.0, 2048 87 and 89; 32 -> 16 36 and 77).
+    // 5.0, 2048 87 and 89; 32 -> 16 36 and 77) and from 40 on (6x6, one image 5.4 there and 5.7 here, 33x7 6.3 and 4.1).
     const long long outputs = (long long)D->N * L->H * L->W;
-    if (S == 2 ? D->C != 16 || K != 32 || outputs > 131072 : D->C > 16 && outputs < 16384)
+    if (S == 2 ? D->C != 16 || K != 32 || outputs < 40 || outputs > 131072 : D->C > 16 && outputs < 16384)
         return -1;
     if (D->C > 32 || (K != 16 && K != 32) || (reinterpret_cast<uintptr_t>(in) & 15) != 0 || (reinterpret_cast<uintptr_t>(out) & 31) != 0)
         return -1;
@@ -249,6 +249,12 @@ int dwpw_direct_f32(const small_b200_layer *D, const small_b200_layer *L, const 
     if (int rc = make_tensor_map(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, in, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B))
         return rc;
     const int threads = (a.TW * (TH / V) + 31) & ~31;
+    // 32 channels, where the gain is small: not in tiles of one warp, which leave an SM with three of them (18x5, 256 images 7.9 us there and
+    // 9.7 here), and not where threads without outputs and pixels fetched for several tiles, or for none, are four times what is
+    // needed (5x126, 256 images 22.0 and 27.8).
+    const double slots = (double)tiles * threads * V / outputs, fetched = (double)tiles * a.PR * a.PW / outputs;
+    if (a.C > CB && (threads == 32 || (K == 32 && slots * fetched > 4)))
+        return -1;
     const size_t smem = (size_t)a.cbs * a.patch_bytes + (size_t)(a.C * 9 + a.C * K + a.C + K) * sizeof(float);
 #define SB_DIRECT(K_, S_) \
     if (K == K_ && S == S_) \

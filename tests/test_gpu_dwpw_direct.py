@@ -54,6 +54,21 @@ def test_against_the_two_layers(oracle, case):
     assert rel_max_err(got, want) <= 1e-6  # two fp32 sums of 9 and at most 32 products in the same precision
 
 
+LINES = [
+    # to either side of the lines between the two kernels
+    (32, 16, 18, 5, 1, "same", 200, "dwpw_f32_kernel"), (32, 16, 24, 24, 1, "same", 30, "dwpw_direct_f32_kernel"),
+    (32, 32, 126, 5, 1, "same", 40, "dwpw_direct_f32_kernel"), (32, 32, 5, 126, 1, "same", 40, "dwpw_f32_kernel"),
+    (16, 32, 12, 13, 2, "same", 1, "dwpw_direct_f32_kernel"), (16, 32, 12, 11, 2, "same", 1, "dwpw_f32_kernel"),
+]
+
+
+@pytest.mark.parametrize("case", LINES, ids=lambda c: "C{}_K{}_{}x{}_s{}_{}_n{}".format(*c[:7]))
+def test_which_kernel(oracle, case):
+    got, want = _run(oracle, case[:7], *_operands(case[:7]))
+    assert _lib.last_kernel() == case[7]
+    assert rel_max_err(got, want) <= (1e-6 if "direct" in case[7] else 1e-5)  # as above; pairs of tf32 words, 2^-21 of a product
+
+
 @pytest.mark.parametrize("value", [np.inf, np.nan, 1e38], ids=str)
 def test_values_without_a_finite_sum(oracle, value):
     case = CASES[0]
