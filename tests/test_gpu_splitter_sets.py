@@ -69,3 +69,37 @@ def test_filters_that_travel(oracle, case):
     want = oracle_conv_batch(oracle, shape(c, k, h, w, f, f, 1, pads, CB), x[some], wt, seed=seed[some] if onto else None)
     for i, ref in zip(some, want):
         assert rel_max_err(got[i], ref) <= 1e-5  # as above
+
+
+def test_pooled_with_wide_tiles_and_infinities(oracle):
+    """The pooled form with two sets of splitters (an input beyond L2): images with a pixel 2^30 and more above its neighbours, whose tiles are
+    summed on the FMA pipe, and with an infinity, beside ordinary ones."""
+    c, k, h, n = 16, 32, 208, 51
+    rng = np.random.default_rng(3)
+    x = rng.uniform(-1, 1, (n, c, h, h)).astype(np.float32)
+    spots = {4: (57, 91), 23: (0, 0), 50: (207, 130)}
+    for i, (r, q) in spots.items():
+        x[i] *= 1e-5
+        x[i, 3, r, q] = 3e4
+    x[30, 5, 100, 33], x[31, 0, 207, 207] = np.inf, -np.inf
+    wt = rng.normal(0, np.sqrt(2.0 / (c * 9)), (k, c, 3, 3)).astype(np.float32)
+    I, F = fbuf(P.pack_activation(x)), fbuf(P.pack_conv_filter(wt))
+    Fp, O = S.FloatBuffer(2 * F.size()), S.FloatBuffer(n * k * h * h // 4)
+    S.prepare_filter_3xTF32(3, 3, k, c, F, Fp)
+    S.Conv2D_Maxpool2D_3xTF32(3, 3, (1, 1, 1, 1), k, c, h, h, I, Fp, None, O, batch=n)
+    got = P.unpack_activation(O.numpy().reshape(n, -1), k, h // 2, h // 2)
+    assert _lib.device_status() == 0
+    some = [3, *spots, 24, 30, 31, 32]
+    want = oracle_conv_batch(oracle, shape(c, k, h, h, 3, 3, 1, (1, 1, 1, 1), CB), P.pack_activation(x[some]), P.pack_conv_filter(wt))
+    for i, ref in zip(some, want):
+        ref = P.unpack_activation(oracle.pool2d_f32(shape(k, k, h, h, 2, 2, 2, (0, 0, 0, 0), CB), ref)[None], k, h // 2, h // 2)[0]
+        mine, fin = got[i], np.isfinite(ref)
+        assert np.array_equal(np.isposinf(mine), np.isposinf(ref)) and np.array_equal(np.isfinite(mine), fin)
+        assert fin.all() == (i not in (30, 31))
+        if i in spots:
+            r, q = (v // 2 for v in spots[i])
+            near = np.zeros_like(fin)
+            near[:, max(0, r - 1):r + 2, max(0, q - 1):q + 2] = True
+            assert rel_max_err(mine[near], ref[near]) <= 1e-5
+            fin = ~near # to the size of the sums around, 10^9 below
+        assert rel_max_err(mine[fin], ref[fin]) <= 1e-5
