@@ -1587,9 +1587,9 @@ bool fit_rings(TcArgs &a, bool need_two)
             if (p[1] % issuers)
                 continue;
             // Four slots serve two sets of splitters, each with its next patch on the way while the MMAs read its last one (two
-            // slots and four, us: 256 -> 32 channels 3x3 at 94x23, 128 images 330 and 280; 64 -> 32 7x7 at 135x96, 64 images 667 and 624; 128 -> 16
-            // 1x1 at 22x184, 32 images 29.3 and 24.0).  Six filter stages beside them only where a group is a whole window: 128 -> 32 3x3
-            // at 8x13, 128 images 17.4 with six and 17.9 with three, but 256 -> 16 5x5 at 81x92, 64 images 851 and 742.
+            // slots and four, us: 256 -> 32 channels 3x3 at 23x94, 128 images 330 and 280; 64 -> 32 7x7 at 96x135, 64 images 667 and 624; 128 -> 16
+            // 1x1 at 184x22, 32 images 29.3 and 24.0).  Six filter stages beside them only where a group is a whole window: 128 -> 32 3x3
+            // at 13x8, 128 images 17.4 with six and 17.9 with three, but 256 -> 16 5x5 at 92x81, 64 images 851 and 742.
             if (p[0] == 4 && (a.split_sets != 2 || any || (p[1] == 6 && a.group != a.taps)))
                 continue;
             const int xs = p[0] < a.cbs || persistent ? p[0] : a.cbs;
@@ -2072,8 +2072,8 @@ int run_tc(const small_b200_layer *L, const small_b200_layer *pool, const float 
     a.tile_base = (int)base; a.total_tiles = (int)std::min(tiles, base + room);
     const unsigned grid = (unsigned)(a.persistent ? std::min(blocks, tiles - base) : blocks);
     // Tiles of many patches: LATE, since what the other form keeps in registers over the sums costs more in every group than the
-    // epilogue then gains.  us, the other form and this: onto what is there 256 -> 16 channels 3x3 at 162x43, 64 images 428 and 414, 128 -> 16
-    // at 30x52, one image 20.4 and 19.1; but 16 -> 16 at 112x112, 256 images 178 and 207, 64 -> 64 1x1 at 32x32, 1024 images 133 and 159.
+    // epilogue then gains.  us, the other form and this: onto what is there 256 -> 16 channels 3x3 at 43x162, 64 images 428 and 414, 128 -> 16
+    // at 52x30, one image 20.4 and 19.1; but 16 -> 16 at 112x112, 256 images 178 and 207, 64 -> 64 1x1 at 32x32, 1024 images 133 and 159.
     const bool two = a.split_sets == 2, late = a.cg == 1 && a.cbs > 4;
 #define SB_LAUNCH_PIXM(M, P, SETS, LATE) \
     conv_f16x3_kernel<true, false, true, M, P, SETS, LATE><<<grid, num_threads(SETS), a.smem_bytes, as_stream(stream)>>>(\
