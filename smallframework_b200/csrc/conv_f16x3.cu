@@ -1525,13 +1525,14 @@ conv_f16x3_kernel(const __grid_constant__ CUtensorMap map_x, const float *__rest
 // 154.7 -> 147.1, 32 -> 16 1x1 onto what is there at 112x112, 16 images 17.2 -> 16.8) and whose kernel leaves the accumulation
 // warps more registers, where those also read what is there (16 -> 16 at 32x32, 1024 images onto the shortcut: 80 and
 // 85), and before a pool, which makes them the slower ones while the input comes from L2 (16 -> 32 at 208x208, 16 images
-// 43.2 and 44.6; 64 images, 177 MB from memory, 152.2 and 146.6).
+// 43.2 and 44.6; 64 images, 177 MB from memory, 152.2 and 146.6) or a tile is two patches and two groups (32 -> 32 3x3 at 58x340, 256
+// images 508.6 and 548.5, at 240x200, 64 images 297.7 and 304.8).
 bool want_two_sets(const TcArgs &a)
 {
     constexpr long long L2_BYTES = 126ll << 20;
     const long long tiles = (long long)a.N * a.px_tiles * a.k_tiles, blocks = std::min<long long>(tiles, num_sms());
     return a.merged && !a.accumulate && (a.cbs > 1 || tiles > 3 * blocks) &&
-           (!a.pool || (long long)a.N * a.C * a.H * a.W * (long long)sizeof(float) > L2_BYTES);
+           (!a.pool || ((long long)a.N * a.C * a.H * a.W * (long long)sizeof(float) > L2_BYTES && (a.cbs != 2 || a.group != a.taps)));
 }
 
 // Picks ring depths for the patch / filter sizes already in `a`.  Narrow layers run persistent (one
