@@ -1,7 +1,7 @@
 // conv_u8_ring.cu -- small::Conv2D<QUInt8Buffer> (include/small/interface_abstract.hpp:229-404, loop nest
 // include/small/q_abstract_layer.hpp:894-1571) for every window, stride and padding as an implicit GEMM on
 // tcgen05.mma.kind::i8.  Layers of blocks of channels with windows of more than one tap go to conv_u8_patch.cu where a tap outside
-// the image has a byte; here run the first layers, 1x1 windows and the other zero points.
+// the image has a byte; here run the first layers, 1x1 windows, the other zero points, and what takes longer there.
 //
 // A tile is 128 consecutive output pixels of the batch (pixel index = image * Ho*Wo + oh * Wo + ow) times
 // NT output channels; the reduction runs over (kernel row, kernel column, pair of input channel blocks)

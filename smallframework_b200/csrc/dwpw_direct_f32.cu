@@ -9,8 +9,8 @@
 // A CTA is one tile: rows of the full width where that is at most 64, one TMA box per 16 channels (zeros outside the image) in the
 // 64-byte swizzle, in which the reads of eight neighbouring pixels' same four channels fall into different banks.  Three CTAs an SM
 // hide each other's fetches (160 threads of 128 registers; two of 192 take 5 to 10 % longer).
-// What bounds it: shared memory (16 -> 16 at 48x48: 51 % of its passes, 46 % of the issue slots) and the latency of a dozen
-// warps; the memory of that block alone is 92 us at 2048 images.
+// What bounds it: shared memory (16 -> 16 at 48x48, 1024 images: 52 % of its passes, 54 % of the issue slots, 52 % of the FMA pipe) and
+// the latency of a dozen warps; the memory of that block alone is 92 us at 2048 images.
 // us, dwpw_f32.cu -> this: 16 -> 16 at 48x48, 2048 images 336 -> 125, 128 images 22.7 -> 11.4, one 5.7 -> 5.2; 32 -> 32 at 24x24, 2048 images
 // 118 -> 104; against fp64 4.5e-7 -> 0.9e-7 (2-norm).
 #include "tc_common.cuh"

@@ -388,7 +388,6 @@ net_u8_tc_kernel(const __grid_constant__ NetArgs a, const uint8_t *__restrict__ 
                     if (three && to_right)
                         *reinterpret_cast<uint4 *>(p1 + copy_bytes - CB) = o; // copy kw = 2, entry q + W - 1
                 };
-                // its channels' sums: a depthwise layer's first half, second half or (a group of four warps) both in turn
                 // its channels' sums: a depthwise layer's first half, second half or (a group of four warps) both in turn.  (One wait on
                 // a barrier chosen beforehand: 4096 images 139.5 us.)
                 const bool late = PARTS > 1 && cb0 * 2 >= KB;
