@@ -540,8 +540,10 @@ bool fit(PatchArgs &a, int NT)
 // Windows that meet a pixel once or twice, few channels: 32 -> 16 2x2 / 2 at 25x25, 1024 images 14.8 and 19.9, 32 -> 32 2x2 at 18x18, 256 images
 // 9.1 and 10.7, 16 -> 64 2x2 at 11x11 (1.8 times as many tiles), 1024 images 15.2 and 17.7.
 // Of 2000 random layers some 40 were slower here than there by more than 2 %, behind this line 6, by 9 % at most.
-bool ring_is_shorter(const PatchArgs &a, int nt)
+bool ring_is_shorter(const PatchArgs &a, int nt, const int32_t *bias)
 {
+    if ((reinterpret_cast<uintptr_t>(bias) & 15) != 0)
+        return false; // which the ring does not take
     const bool plain = a.zero_filt == -128 && (a.zero_in == 0 || a.zero_in == -128);
     const int few = a.taps * ((a.cbs + 1) / 2); // the ring's steps
     const bool little = a.planes == 4 && few <= 6 && a.K <= 32;
@@ -640,7 +642,7 @@ int conv2d_u8_patch(const small_b200_layer *L, const uint8_t *in, const uint8_t 
     while (!fit(a, nt))
         if ((nt /= 2) < 16)
             return -1;
-    if (ring_is_shorter(a, nt))
+    if (ring_is_shorter(a, nt, bias))
         return -1;
 #define SB_PATCH(NT_) return a.taps == 9 ? launch_patch<NT_, true>(a, in, filt, bias, out, st) : launch_patch<NT_, false>(a, in, filt, bias, out, st)
     switch (nt)

@@ -76,6 +76,27 @@ def test_layers_that_stay_with_the_ring(oracle, case):
     assert _lib.last_kernel() == "conv_u8_ring_kernel"
 
 
+def test_biases_that_the_ring_does_not_take(oracle):
+    """Four bytes past a 16-byte boundary: a layer that the ring does sooner stays on the tensor cores all the same."""
+    rng = np.random.default_rng(8)
+    C, K, H, W, N = 16, 32, 25, 19, 2
+    x, w = rng.integers(0, 256, N * C * H * W).astype(np.uint8), rng.integers(0, 256, K * C * 3).astype(np.uint8)
+    b = rng.integers(-1024, 1025, K + 1).astype(np.int32)
+    q = _quant(rng, C * 3, (-128, -128))
+    L = _lib.Layer(N, C, K, H, W, 1, 3, 2, 0, 0, 1, 1, 0, 0, 0.0, q.zero_in, q.zero_filt, q.lshift, q.rshift, q.multiplier, q.k_zero)
+    ho, wo = L.out_hw()
+    xd, wd, bd = (torch.from_numpy(v).cuda() for v in (x, w, b))
+    out = torch.empty(N, K * ho * wo, dtype=torch.uint8, device="cuda")
+    for skip, kernel in ((0, "conv_u8_ring_kernel"), (1, "conv_u8_patch_kernel")):
+        _lib.check(_lib.lib().small_b200_conv2d_u8(ctypes.byref(L), xd.data_ptr(), wd.data_ptr(), bd.data_ptr() + 4 * skip, out.data_ptr(),
+                                                   torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        assert _lib.last_kernel() == kernel
+        sh = shape(C, K, H, W, 1, 3, 2, (0, 0, 1, 1), 16)
+        want = np.stack([oracle.conv2d_u8(sh, q, v, w, bias=b[skip:skip + K]) for v in x.reshape(N, -1)])
+        assert np.array_equal(out.cpu().numpy(), want) and want.min() < want.max()
+
+
 @pytest.mark.parametrize("shift", [0, 1], ids=lambda r: f"rshift{r}")
 def test_quantisers_outside_the_common_form(oracle, shift):
     from oracle.bindings import Quant, same_pads
